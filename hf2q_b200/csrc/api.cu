@@ -1478,7 +1478,7 @@ HF2Q_API int32_t hf2q_cuda_router_logits(hf2q_ctx* ctx, void* stream, const void
     if (x_dtype != HF2Q_DT_F32 && x_dtype != HF2Q_DT_BF16) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "router_logits: x_dtype %u (want F32 or BF16)", x_dtype);
     if (n_tokens == 0) return HF2Q_OK;
     DeviceGuard dg(ctx->device);
-    const cudaError_t e = launch_router_logits(x, x_dtype == HF2Q_DT_BF16, router, logits, n_tokens, n_experts, hidden, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_router_logits(x, x_dtype == HF2Q_DT_BF16, router, logits, n_tokens, n_experts, hidden, ctx_sm_count(ctx), static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "router_logits launch");
     ctx->launches += 1;
     return HF2Q_OK;

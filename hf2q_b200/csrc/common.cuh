@@ -157,6 +157,15 @@ __device__ __forceinline__ float byte_to_float(uint32_t w, int k) {
     return __uint_as_float(bits) - (8388608.0f + static_cast<float>(BIAS));
 }
 
+// two f32 values in a 64-bit register; one instruction works on both (IEEE arithmetic on each half)
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 f2_both(float a) { f2 d; asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a)); return d; }
+__device__ __forceinline__ float2 f2_parts(f2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a)); return r; }
+__device__ __forceinline__ float f2_sum(f2 a) { float x, y; asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); return x + y; }
+
 // ---- mbarrier / bulk-copy PTX (sm_90+; used here for sm_100a only) ----------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -4,11 +4,15 @@
 // dense_swiglu_cpu_ref (src/inference/models/qwen35/ffn.rs:91-112) and moe_ffn_cpu_ref
 // (ffn.rs:179-336); the reference's GPU builders dispatch dispatch_silu_mul /
 // dispatch_moe_weighted_reduce for the same steps (gpu_ffn.rs:1086-1351, 2313-2802).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.h"
+#include "seq_common.cuh"
 
 namespace hf2q {
 namespace {
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }     // ffn.rs:24-26
 
@@ -64,54 +68,200 @@ __global__ void __launch_bounds__(256) rowdot_kernel(const float* __restrict__ x
 
 // Router logits of an MoE layer: out[t, e] = sum_h x[t, h] * w[e, h], all f32 (the router is a small
 // dense f32 matrix in the reference as well: phase 1 of the six-phase graph at gpu_ffn.rs:2347-2359).
-// Classic shared-memory tiling: a CTA computes 64 tokens x 64 experts, 4 x 4 outputs per thread.
-constexpr int RT = 64, RKT = 16;
-__global__ void __launch_bounds__(256) router_logits_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
-                                                            float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
-    __shared__ float xs[RKT][RT + 4], ws[RKT][RT + 4];
+//
+// Up to RV_TOKENS tokens: bound by the latency of one pass over the router (2 MB for 256 experts of 2048), so every
+// expert has a CTA of its own whose threads request sixteen values of its row at a time (256 experts, one token: 2.6 us;
+// tiles of 64 tokens, four CTAs in all, took 180 us).
+constexpr int RV_TOKENS = 8, RV_THREADS = 128, RV_AHEAD = 4;
+
+__device__ __forceinline__ float4 load4(const void* p, uint32_t bf16, size_t i) {
+    if (!bf16) return *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i);
+    const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p) + i);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float load1(const void* p, uint32_t bf16, size_t i) {
+    return bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]) : static_cast<const float*>(p)[i];
+}
+
+// VEC: h is a multiple of 4, and x and w allow loads of four elements.
+template <bool VEC>
+__global__ void __launch_bounds__(RV_THREADS) router_vector_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
+                                                                   float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
+    __shared__ float part[RV_TOKENS][RV_THREADS / 32];
+    const uint32_t e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* row = w + static_cast<size_t>(e) * h;
+    float acc[RV_TOKENS] = {};
+    seq::pdl_trigger();
+    seq::pdl_wait();
+    if constexpr (VEC) {
+        for (uint32_t i0 = 4 * threadIdx.x; i0 < h; i0 += RV_AHEAD * 4 * RV_THREADS) {
+            float4 wv[RV_AHEAD];
+#pragma unroll
+            for (int a = 0; a < RV_AHEAD; ++a) {
+                const uint32_t i = i0 + a * 4 * RV_THREADS;
+                wv[a] = i < h ? __ldg(reinterpret_cast<const float4*>(row + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int t = 0; t < RV_TOKENS; ++t) {
+                if (t >= n_tokens) break;
+#pragma unroll
+                for (int a = 0; a < RV_AHEAD; ++a) {
+                    const uint32_t i = i0 + a * 4 * RV_THREADS;
+                    if (i >= h) break;
+                    const float4 v = load4(x, x_bf16, static_cast<size_t>(t) * h + i);
+                    acc[t] += wv[a].x * v.x + wv[a].y * v.y + wv[a].z * v.z + wv[a].w * v.w;
+                }
+            }
+        }
+    }
+    if constexpr (!VEC) {
+        for (uint32_t i = threadIdx.x; i < h; i += RV_THREADS) {
+            const float wv = __ldg(row + i);
+#pragma unroll
+            for (int t = 0; t < RV_TOKENS; ++t)
+                if (t < n_tokens) acc[t] += wv * load1(x, x_bf16, static_cast<size_t>(t) * h + i);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < RV_TOKENS; ++t) {
+        for (int o = 16; o > 0; o >>= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+        if (lane == 0) part[t][warp] = acc[t];
+    }
+    __syncthreads();
+    if (threadIdx.x < n_tokens) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < RV_THREADS / 32; ++i) s += part[threadIdx.x][i];
+        out[static_cast<size_t>(threadIdx.x) * n_experts + e] = s;
+    }
+}
+
+// More tokens: 64 tokens x 64 experts per tile, 4 x 4 outputs per thread in packed f32 arithmetic, the next 32 columns on
+// their way to registers while the present ones are used.  Bound by the f32 pipes (2048 tokens x 256 experts of 2048: 1.07 G
+// multiply-adds).  The CTAs of a cluster share a tile's columns where the tiles alone would leave the chip idle, and add
+// their sums through distributed shared memory in rank order (2048 tokens, 256 experts of 2048: 263 -> 86 us; the line at
+// RV_TOKENS lies where a CTA per expert would read more activations than weights).  Columns are stored with the group of four tokens (or
+// experts) XORed by the column's own group of four, which keeps both the transposing stores and the reads free of conflicts.
+constexpr int RT = 64, RKT = 32, RT_MAX_PARTS = 8;
+
+template <bool VEC>
+__global__ void __launch_bounds__(256) router_tile_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
+                                                          float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
+    __shared__ __align__(16) float xs[RKT][RT], ws[RKT][RT];
+    const cg::cluster_group cl = cg::this_cluster();
+    seq::pdl_trigger();
+    seq::pdl_wait();
+    const uint32_t parts = gridDim.z, part = blockIdx.z;             // the cluster is the whole z extent
     const uint32_t t0 = blockIdx.y * RT, e0 = blockIdx.x * RT;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;          // outputs: tokens 4ty..4ty+3, experts 4tx..4tx+3
-    float acc[4][4] = {};
-    for (uint32_t k0 = 0; k0 < h; k0 += RKT) {
-        for (int i = threadIdx.x; i < RT * RKT; i += 256) {
-            const int r = i / RKT, c = i % RKT;
-            const uint32_t t = t0 + r, e = e0 + r, kk = k0 + c;
-            float xv = 0.f;
-            if (t < n_tokens && kk < h)
-                xv = x_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(x)[static_cast<size_t>(t) * h + kk])
-                            : static_cast<const float*>(x)[static_cast<size_t>(t) * h + kk];
-            xs[c][r] = xv;
-            ws[c][r] = (e < n_experts && kk < h) ? w[static_cast<size_t>(e) * h + kk] : 0.f;
+    const uint32_t chunks = (h + RKT - 1) / RKT, per = (chunks + parts - 1) / parts;
+    const uint32_t c0 = min(part * per, chunks), c1 = min(c0 + per, chunks);
+    // a thread brings columns 4 kg .. 4 kg + 3 of rows r and r + 32 of both tiles
+    const uint32_t kg = threadIdx.x & 7, r = threadIdx.x >> 3;
+    float4 xr[2], wr[2];
+    auto fetch = [&](uint32_t c) {
+        const uint32_t k = c * RKT + 4 * kg;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t t = t0 + r + 32 * i, e = e0 + r + 32 * i;
+            const size_t xo = static_cast<size_t>(t) * h + k, wo = static_cast<size_t>(e) * h + k;
+            xr[i] = wr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (VEC) {
+                if (t < n_tokens && k < h) xr[i] = load4(x, x_bf16, xo);
+                if (e < n_experts && k < h) wr[i] = __ldg(reinterpret_cast<const float4*>(w + wo));
+            } else {
+                float* xp = &xr[i].x;
+                float* wp = &wr[i].x;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (t < n_tokens && k + j < h) xp[j] = load1(x, x_bf16, xo + j);
+                    if (e < n_experts && k + j < h) wp[j] = __ldg(w + wo + j);
+                }
+            }
+        }
+    };
+    f2 acc[4][2] = {};
+    if (c0 < c1) fetch(c0);
+    for (uint32_t c = c0; c < c1; ++c) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t row = r + 32 * i, at = 4 * ((row >> 2) ^ kg) + (row & 3);
+            const float xv[4] = {xr[i].x, xr[i].y, xr[i].z, xr[i].w}, wv[4] = {wr[i].x, wr[i].y, wr[i].z, wr[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                xs[4 * kg + j][at] = xv[j];
+                ws[4 * kg + j][at] = wv[j];
+            }
         }
         __syncthreads();
+        if (c + 1 < c1) fetch(c + 1);
 #pragma unroll
-        for (int c = 0; c < RKT; ++c) {
-            const float4 a = *reinterpret_cast<const float4*>(&xs[c][4 * ty]);
-            const float4 b = *reinterpret_cast<const float4*>(&ws[c][4 * tx]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        for (int k = 0; k < RKT; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[k][4 * (ty ^ (k >> 2))]);
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&ws[k][4 * (tx ^ (k >> 2))]);
+            const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * bv[j];
+            for (int i = 0; i < 4; ++i) {
+                const f2 aa = f2_both(av[i]);
+                acc[i][0] = f2_fma(aa, b.x, acc[i][0]);
+                acc[i][1] = f2_fma(aa, b.y, acc[i][1]);
+            }
         }
         __syncthreads();
     }
+    auto store = [&](uint32_t t, uint32_t e, const float4& v) {      // experts e .. e + 3 of token t
+        if (t >= n_tokens) return;
+        const float o[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j)
+            if (e + j < n_experts) out[static_cast<size_t>(t) * n_experts + e + j] = o[j];
+    };
+    if (parts == 1) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t t = t0 + 4 * ty + i, e = e0 + 4 * tx + j;
-            if (t < n_tokens && e < n_experts) out[static_cast<size_t>(t) * n_experts + e] = acc[i][j];
+        for (int i = 0; i < 4; ++i) {
+            const float2 lo = f2_parts(acc[i][0]), hi = f2_parts(acc[i][1]);
+            store(t0 + 4 * ty + i, e0 + 4 * tx, make_float4(lo.x, lo.y, hi.x, hi.y));
         }
+        return;
+    }
+    // the tile's 64 x 64 sums: rows 0..31 in the tokens' buffer, 32..63 in the experts'
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f2* d = reinterpret_cast<f2*>((4 * ty + i < RKT ? xs[4 * ty + i] : ws[4 * ty + i - RKT]) + 4 * tx);
+        d[0] = acc[i][0];
+        d[1] = acc[i][1];
+    }
+    cl.sync();
+    // this CTA's share of the tile's rows
+    const uint32_t rows = RT / parts;
+    for (uint32_t i = threadIdx.x; i < rows * (RT / 4); i += 256) {
+        const uint32_t row = part * rows + i / (RT / 4), q = 4 * (i % (RT / 4));
+        float* mine = row < RKT ? xs[row] : ws[row - RKT];
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (uint32_t p = 0; p < parts; ++p) {
+            const float4 v = *reinterpret_cast<const float4*>(cl.map_shared_rank(mine + q, p));
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        store(t0 + row, e0 + q, s);
+    }
+    cl.sync();                                                       // peers read this CTA's sums until here
 }
 
 }  // namespace
 
 cudaError_t launch_router_logits(const void* x, uint32_t x_bf16, const float* w, float* out, uint32_t n_tokens, uint32_t n_experts,
-                                 uint32_t h, cudaStream_t st) {
-    const dim3 grid((n_experts + RT - 1) / RT, (n_tokens + RT - 1) / RT);
-    router_logits_kernel<<<grid, 256, 0, st>>>(x, x_bf16, w, out, n_tokens, n_experts, h);
-    return cudaGetLastError();
+                                 uint32_t h, int sm_count, cudaStream_t st) {
+    const bool vec = h % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % (x_bf16 ? 8 : 16) == 0;
+    if (n_tokens <= RV_TOKENS)
+        return seq::launch_pdl(vec ? router_vector_kernel<true> : router_vector_kernel<false>, dim3(n_experts), dim3(RV_THREADS), 0, st, x, x_bf16, w, out,
+                               n_tokens, n_experts, h);
+    const dim3 tiles((n_experts + RT - 1) / RT, (n_tokens + RT - 1) / RT);
+    // as many parts as keep two CTAs on every SM busy
+    uint32_t parts = 1;
+    while (parts < RT_MAX_PARTS && 2ull * parts * tiles.x * tiles.y <= 2ull * sm_count && h >= 2 * parts * RKT) parts *= 2;
+    return seq::launch_pdl_cluster(vec ? router_tile_kernel<true> : router_tile_kernel<false>, dim3(tiles.x, tiles.y, parts), dim3(256), dim3(1, 1, parts), 0, st,
+                                   x, x_bf16, w, out, n_tokens, n_experts, h);
 }
 
 cudaError_t launch_silu_mul(const float* gate, const float* up, float* out, uint64_t n, int sm_count, cudaStream_t st) {

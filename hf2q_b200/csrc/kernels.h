@@ -203,7 +203,7 @@ cudaError_t launch_silu_mul(const float* gate, const float* up, float* out, uint
 cudaError_t launch_moe_combine(const float* y, const float* w, const float* shared, const float* gate_logit, const float* residual,
                                float* out, uint32_t n_tokens, uint32_t top_k, uint32_t h, cudaStream_t st);
 cudaError_t launch_router_logits(const void* x, uint32_t x_bf16, const float* w, float* out, uint32_t n_tokens, uint32_t n_experts,
-                                 uint32_t h, cudaStream_t st);
+                                 uint32_t h, int sm_count, cudaStream_t st);
 cudaError_t launch_rowdot(const float* x, const float* v, float* out, uint32_t n_tokens, uint32_t h, cudaStream_t st);
 
 }  // namespace hf2q

@@ -52,14 +52,6 @@ __device__ __forceinline__ void stage_rows(float* dst, uint32_t dst_ld, const fl
     }
 }
 
-// two f32 values in a 64-bit register; one instruction works on both (IEEE arithmetic on each half)
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 f2_both(float a) { f2 d; asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a)); return d; }
-__device__ __forceinline__ float f2_sum(f2 a) { float x, y; asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); return x + y; }
-
 template <int RQ> struct Vec {                       // a lane's RQ pairs of key channels
     f2 v[RQ];
     __device__ __forceinline__ void load(const float* p) {
