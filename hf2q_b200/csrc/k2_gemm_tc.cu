@@ -25,9 +25,13 @@
 //                       tcgen05.commit releases the activation stages and the A buffers.
 //   warps 0-7 again     epilogue: tcgen05.ld the fp32 accumulators, coalesced stores of y.
 //
+// Where the tiles leave SMs idle (few activation rows), the CTAs of a cluster share a tile's K-blocks (gemm_tc_parts
+// of them) and add their accumulators through distributed shared memory in rank order.
+//
 // TMEM: 512 columns = D (<= 256) + 2 x 128 (two A buffers of one K-block each).
 // Every mbarrier wait is bounded; a wait that gives up sets the status word and all roles drain to
-// the final barrier, where TMEM is freed.  No cluster launch, no multicast.
+// the final barrier, where TMEM is freed.  No multicast.
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <cstdlib>
@@ -44,6 +48,7 @@ namespace hf2q {
 using namespace tc;
 
 namespace {
+namespace cg = cooperative_groups;
 
 constexpr int TILE_N = 128;      // weight rows per CTA (MMA M)
 constexpr int KB = 256;          // K elements per block step
@@ -133,7 +138,8 @@ __device__ __forceinline__ void dequant_dispatch(uint32_t grp, const uint8_t* ro
 // The epilogue pairs lane l with lane l + 16 by one shuffle per value and stores silu(gate) * up: the
 // SwiGLU of build_dense_ffn_layer_gpu_q / build_moe_ffn_layer_gpu_q (gpu_ffn.rs:896-935, 2606-2760) without
 // the two f32 round trips and the dispatch_silu_mul in between.
-template <uint32_t TYPE, int NT, bool GROUPED, bool DUAL>
+// SHARED: gridDim.z CTAs, a cluster, share the tile's K-blocks.
+template <uint32_t TYPE, int NT, bool GROUPED, bool DUAL, bool SHARED>
 __global__ void __launch_bounds__(GEMM_THREADS, (two_ctas_of(NT, GROUPED) ? 2 : 1))
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
                const __grid_constant__ CUtensorMap tmap_x, const GParams p) {
@@ -170,7 +176,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         const GroupTile gt = p.tiles[blockIdx.y];
         tok0 = gt.start; tok_end = gt.start + gt.count; expert = gt.expert;
     }
-    const uint32_t nkb = p.k / KB;
+    // this CTA's K-blocks: all of them, or its share of the cluster's
+    const uint32_t parts = SHARED ? gridDim.z : 1u, part = SHARED ? blockIdx.z : 0u;
+    const uint32_t kb0 = SHARED ? p.k / KB * part / parts : 0u, nkb = SHARED ? p.k / KB * (part + 1) / parts - kb0 : p.k / KB;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < RAW_STAGES; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], DEQ_WARPS); }
@@ -200,7 +208,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                     if (gk >= RAW_STAGES) ok = mbar_wait_bounded(&raw_empty[rs], ((gk / RAW_STAGES) - 1) & 1, p.status);
                     if (!ok) break;
                     mbar_arrive_expect_tx(&raw_full[rs], raw_stage);
-                    const uint32_t byte0 = (kb * p.blk_bytes) & ~15u;       // 16-byte aligned start of the box
+                    const uint32_t byte0 = ((kb0 + kb) * p.blk_bytes) & ~15u;       // 16-byte aligned start of the box
                     if constexpr (GROUPED)
                         tma_3d(raw + rs * raw_stage, &tmap_w, static_cast<int>(byte0 >> 1), static_cast<int>(row0), static_cast<int>(expert), &raw_full[rs]);
                     else
@@ -218,7 +226,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             bool ok = true;
             const uint32_t nx = ntile * nkb * (KB / XK);
             for (uint32_t xi = 0; xi < nx && ok; ++xi) {
-                const uint32_t st = xi % X_STAGES, kx = xi % (nkb * (KB / XK));      // K position inside the current tile
+                const uint32_t st = xi % X_STAGES, kx = kb0 * (KB / XK) + xi % (nkb * (KB / XK));      // K position inside the current tile
                 if (xi >= X_STAGES) ok = mbar_wait_bounded(&x_empty[st], ((xi / X_STAGES) - 1) & 1, p.status);
                 if (!ok) break;
                 mbar_arrive_expect_tx(&x_full[st], X_STAGE);
@@ -281,7 +289,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t off = (kb * p.blk_bytes) & 15u;
+                const uint32_t off = ((kb0 + kb) * p.blk_bytes) & 15u;
                 dequant_dispatch<TYPE>(grp, raw + rs * raw_stage + src_row * p.boxw, off, tmem_a + ab * 128 + lane_addr);
                 tmem_wait_st();
                 tc_fence_before();
@@ -293,7 +301,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            if constexpr (DUAL) {
+            if constexpr (SHARED) {
+                // the cluster's sum needs them first: [token column][row] over the activation stages, which are idle now
+                float* sums = reinterpret_cast<float*>(smem);
+#pragma unroll 1
+                for (int c0 = 32 * static_cast<int>(grp); c0 < n_cols; c0 += 32 * DEQ_GROUPS) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem_d + lane_addr + c0, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sums[(c0 + j) * TILE_N + r] = __uint_as_float(v[j]);
+                }
+            } else if constexpr (DUAL) {
                 // lanes 0..15 of this warp hold gate rows, lanes 16..31 the up rows of the same 16 outputs.  Of each
                 // pair of tokens the lower lane finishes the even one and the upper lane the odd one: one exchange
                 // per pair, every lane busy.
@@ -373,6 +392,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     tc_fence_before();
     __syncthreads();
     if (warp == DEQ_WARPS + 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+    if constexpr (SHARED) {
+        const cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        // token columns part, part + parts, ... of the tile are this CTA's: all CTAs' sums in rank order, then the epilogue
+        float* sums = reinterpret_cast<float*>(smem);
+        const uint32_t row0 = tile0 * TILE_ROWS, cols = min(static_cast<uint32_t>(NT), tok_end - tok0);
+        const uint32_t out_row = threadIdx.x % TILE_ROWS, row = row0 + out_row;
+        constexpr uint32_t PER = GEMM_THREADS / TILE_ROWS;           // columns at a time
+        if (threadIdx.x < PER * TILE_ROWS && row < p.n) {
+            const uint32_t lane_of = DUAL ? (out_row / 16) * 32 + out_row % 16 : out_row;
+            for (uint32_t c = part + parts * (threadIdx.x / TILE_ROWS); c < cols; c += parts * PER) {
+                float v = 0.f, up = 0.f;
+                for (uint32_t q = 0; q < parts; ++q) {
+                    const float* s = cl.map_shared_rank(sums, q) + c * TILE_N + lane_of;
+                    v += s[0];
+                    if constexpr (DUAL) up += s[16];
+                }
+                const size_t o = static_cast<size_t>(tok0 + c) * p.ldy + row;
+                if constexpr (DUAL) p.y[o] = v / (1.0f + expf(-v)) * up;
+                else p.y[o] = p.residual ? v + __ldcg(p.residual + o) : v;
+            }
+        }
+        cl.sync();                                                   // the others read this CTA's sums until here
+    }
 }
 
 // ---------------------------------------------------------------- activations -> f16 panel
@@ -443,40 +486,75 @@ EncodeTiledFn encode_fn() {
 
 uint32_t boxw_of(uint32_t type) { return tc_boxw(type); }
 
-template <uint32_t TYPE, int NT, bool GROUPED, bool DUAL = false>
-cudaError_t launch_gemm_t(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx, const GParams& p, uint32_t grid_y, cudaStream_t st) {
-    auto kern = gemm_tc_kernel<TYPE, NT, GROUPED, DUAL>;
+template <uint32_t TYPE, int NT, bool GROUPED, bool DUAL, bool SHARED>
+cudaError_t launch_gemm_form(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx, const GParams& p, uint32_t grid_y, cudaStream_t st,
+                             uint32_t parts) {
+    auto kern = gemm_tc_kernel<TYPE, NT, GROUPED, DUAL, SHARED>;
     const size_t raw_stages = raw_stages_of(TYPE, NT, GROUPED);
     const size_t smem = 1024 + static_cast<size_t>(x_stages_of(TYPE, NT, GROUPED)) * NT * 128 + raw_stages * TILE_N * p.boxw + 512;
     static PerDeviceFlag attr;
     if (const cudaError_t e = ensure_max_dynamic_smem(kern, 227 * 1024, attr); e != cudaSuccess) return e;
     const uint32_t tile_rows = DUAL ? 64 : TILE_N;
     const uint32_t row_tiles = (p.n + tile_rows - 1) / tile_rows;
-    const dim3 grid((row_tiles + p.tiles_per_cta - 1) / p.tiles_per_cta, grid_y);
+    const dim3 grid((row_tiles + p.tiles_per_cta - 1) / p.tiles_per_cta, grid_y, parts);
+    if constexpr (SHARED) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(GEMM_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute cluster[1];
+        cluster[0].id = cudaLaunchAttributeClusterDimension;
+        cluster[0].val.clusterDim.x = cluster[0].val.clusterDim.y = 1;
+        cluster[0].val.clusterDim.z = parts;
+        cfg.attrs = cluster;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kern, tw, tw2, tx, p);
+    }
     kern<<<grid, GEMM_THREADS, smem, st>>>(tw, tw2, tx, p);
     return cudaGetLastError();
 }
 
+// parts > 1: the CTAs of a cluster share the K-blocks (dense tiles of up to 128 tokens)
+template <uint32_t TYPE, int NT, bool GROUPED, bool DUAL = false>
+cudaError_t launch_gemm_t(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx, const GParams& p, uint32_t grid_y, cudaStream_t st,
+                          uint32_t parts = 1) {
+    if constexpr (!GROUPED && NT <= 128)
+        if (parts > 1) return launch_gemm_form<TYPE, NT, GROUPED, DUAL, true>(tw, tw2, tx, p, grid_y, st, parts);
+    return launch_gemm_form<TYPE, NT, GROUPED, DUAL, false>(tw, tw2, tx, p, grid_y, st, 1);
+}
+
+// CTAs that share the K-blocks of a tile, for m rows against an n x k matrix: as many (1, 2, 4, 8) as run next to one another,
+// with two K-blocks or more for each (2560 x 9728 in Q8_0 at 37 rows, 20 tiles: 53 -> 22 us with four).  The count of tiles is the same whatever form the product takes (so that its fused and its
+// separate forms add in the same order), and such that the SwiGLU pair with its 64-row tiles still runs in one wave: up to 64
+// rows two CTAs share an SM, beyond that one.  (A pair of 2048 x 2560 at 453 rows that took a second wave ran 52 -> 65 us.)
+uint32_t gemm_tc_parts(uint32_t m, uint32_t n, uint32_t k, int sms) {
+    const uint64_t tiles = static_cast<uint64_t>((n + TILE_N - 1) / TILE_N) * (m <= 64 ? 1 : 2 * ((m + 127) / 128));
+    uint32_t parts = 1;
+    while (parts < 8 && 2 * parts * tiles <= static_cast<uint64_t>(sms) && k / KB >= 4 * parts) parts *= 2;
+    return parts;
+}
+
 template <uint32_t TYPE>
-cudaError_t launch_gemm_nt(const CUtensorMap& tw, const CUtensorMap& tx, const GParams& p, uint32_t nt, cudaStream_t st) {
+cudaError_t launch_gemm_nt(const CUtensorMap& tw, const CUtensorMap& tx, const GParams& p, uint32_t nt, cudaStream_t st, uint32_t parts) {
     const uint32_t gy = (p.m + nt - 1) / nt;
     switch (nt) {
-        case 32: return launch_gemm_t<TYPE, 32, false>(tw, tw, tx, p, gy, st);
-        case 64: return launch_gemm_t<TYPE, 64, false>(tw, tw, tx, p, gy, st);
-        case 128: return launch_gemm_t<TYPE, 128, false>(tw, tw, tx, p, gy, st);
-        default: return launch_gemm_t<TYPE, 256, false>(tw, tw, tx, p, gy, st);
+        case 32: return launch_gemm_t<TYPE, 32, false>(tw, tw, tx, p, gy, st, parts);
+        case 64: return launch_gemm_t<TYPE, 64, false>(tw, tw, tx, p, gy, st, parts);
+        case 128: return launch_gemm_t<TYPE, 128, false>(tw, tw, tx, p, gy, st, parts);
+        default: return launch_gemm_t<TYPE, 256, false>(tw, tw, tx, p, gy, st, parts);
     }
 }
 
 // the SwiGLU pair
 template <uint32_t TYPE, bool GROUPED>
 cudaError_t launch_gemm_dual_nt(const CUtensorMap& tg, const CUtensorMap& tu, const CUtensorMap& tx, const GParams& p, uint32_t nt, uint32_t gy,
-                                cudaStream_t st) {
+                                cudaStream_t st, uint32_t parts = 1) {
     switch (nt) {
-        case 32: return launch_gemm_t<TYPE, 32, GROUPED, true>(tg, tu, tx, p, gy, st);
-        case 64: return launch_gemm_t<TYPE, 64, GROUPED, true>(tg, tu, tx, p, gy, st);
-        case 128: return launch_gemm_t<TYPE, 128, GROUPED, true>(tg, tu, tx, p, gy, st);
-        default: return launch_gemm_t<TYPE, 256, GROUPED, true>(tg, tu, tx, p, gy, st);
+        case 32: return launch_gemm_t<TYPE, 32, GROUPED, true>(tg, tu, tx, p, gy, st, parts);
+        case 64: return launch_gemm_t<TYPE, 64, GROUPED, true>(tg, tu, tx, p, gy, st, parts);
+        case 128: return launch_gemm_t<TYPE, 128, GROUPED, true>(tg, tu, tx, p, gy, st, parts);
+        default: return launch_gemm_t<TYPE, 256, GROUPED, true>(tg, tu, tx, p, gy, st, parts);
     }
 }
 
@@ -548,7 +626,8 @@ cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const 
     p.blk_bytes = KB / g.elems * g.bytes;
     p.status = status;
     const uint32_t tile_rows = dual ? 64 : TILE_N;
-    const uint32_t nt = gemm_tc_token_tile(m, (n + tile_rows - 1) / tile_rows, sm_count);
+    const uint32_t parts = gemm_tc_parts(m, n, k, sm_count), best_nt = gemm_tc_token_tile(m, (n + tile_rows - 1) / tile_rows, sm_count);
+    const uint32_t nt = parts > 1 && best_nt > 128 ? 128 : best_nt;
     alignas(64) CUtensorMap tw, tw2, tx;
     for (int which = 0; which < (dual ? 2 : 1); ++which) {
         // weights: [n rows][row_bytes] viewed as u16, box = boxw bytes x 128 (pair: 64) rows, no swizzle
@@ -575,25 +654,25 @@ cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const 
     if (dual) {
         const uint32_t gy = (m + nt - 1) / nt;
         switch (type) {
-            case HF2Q_TYPE_Q4_0: return launch_gemm_dual_nt<HF2Q_TYPE_Q4_0, false>(tw, tw2, tx, p, nt, gy, st);
-            case HF2Q_TYPE_Q8_0: return launch_gemm_dual_nt<HF2Q_TYPE_Q8_0, false>(tw, tw2, tx, p, nt, gy, st);
-            case HF2Q_TYPE_Q4_K: return launch_gemm_dual_nt<HF2Q_TYPE_Q4_K, false>(tw, tw2, tx, p, nt, gy, st);
-            case HF2Q_TYPE_Q5_K: return launch_gemm_dual_nt<HF2Q_TYPE_Q5_K, false>(tw, tw2, tx, p, nt, gy, st);
-            case HF2Q_TYPE_Q6_K: return launch_gemm_dual_nt<HF2Q_TYPE_Q6_K, false>(tw, tw2, tx, p, nt, gy, st);
+            case HF2Q_TYPE_Q4_0: return launch_gemm_dual_nt<HF2Q_TYPE_Q4_0, false>(tw, tw2, tx, p, nt, gy, st, parts);
+            case HF2Q_TYPE_Q8_0: return launch_gemm_dual_nt<HF2Q_TYPE_Q8_0, false>(tw, tw2, tx, p, nt, gy, st, parts);
+            case HF2Q_TYPE_Q4_K: return launch_gemm_dual_nt<HF2Q_TYPE_Q4_K, false>(tw, tw2, tx, p, nt, gy, st, parts);
+            case HF2Q_TYPE_Q5_K: return launch_gemm_dual_nt<HF2Q_TYPE_Q5_K, false>(tw, tw2, tx, p, nt, gy, st, parts);
+            case HF2Q_TYPE_Q6_K: return launch_gemm_dual_nt<HF2Q_TYPE_Q6_K, false>(tw, tw2, tx, p, nt, gy, st, parts);
             default: return cudaErrorNotSupported;
         }
     }
     switch (type) {
-        case HF2Q_TYPE_Q4_0: return launch_gemm_nt<HF2Q_TYPE_Q4_0>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q8_0: return launch_gemm_nt<HF2Q_TYPE_Q8_0>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q4_K: return launch_gemm_nt<HF2Q_TYPE_Q4_K>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q5_K: return launch_gemm_nt<HF2Q_TYPE_Q5_K>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q6_K: return launch_gemm_nt<HF2Q_TYPE_Q6_K>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q4_1: return launch_gemm_nt<HF2Q_TYPE_Q4_1>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q5_0: return launch_gemm_nt<HF2Q_TYPE_Q5_0>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_Q5_1: return launch_gemm_nt<HF2Q_TYPE_Q5_1>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_IQ4_NL: return launch_gemm_nt<HF2Q_TYPE_IQ4_NL>(tw, tx, p, nt, st);
-        case HF2Q_TYPE_MLX_AFFINE4_GS32: return launch_gemm_nt<HF2Q_TYPE_MLX_AFFINE4_GS32>(tw, tx, p, nt, st);
+        case HF2Q_TYPE_Q4_0: return launch_gemm_nt<HF2Q_TYPE_Q4_0>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q8_0: return launch_gemm_nt<HF2Q_TYPE_Q8_0>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q4_K: return launch_gemm_nt<HF2Q_TYPE_Q4_K>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q5_K: return launch_gemm_nt<HF2Q_TYPE_Q5_K>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q6_K: return launch_gemm_nt<HF2Q_TYPE_Q6_K>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q4_1: return launch_gemm_nt<HF2Q_TYPE_Q4_1>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q5_0: return launch_gemm_nt<HF2Q_TYPE_Q5_0>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_Q5_1: return launch_gemm_nt<HF2Q_TYPE_Q5_1>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_IQ4_NL: return launch_gemm_nt<HF2Q_TYPE_IQ4_NL>(tw, tx, p, nt, st, parts);
+        case HF2Q_TYPE_MLX_AFFINE4_GS32: return launch_gemm_nt<HF2Q_TYPE_MLX_AFFINE4_GS32>(tw, tx, p, nt, st, parts);
         default: return cudaErrorInvalidValue;
     }
 }
