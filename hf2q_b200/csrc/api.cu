@@ -1622,7 +1622,7 @@ HF2Q_API int32_t hf2q_cuda_attn_prefill(hf2q_ctx* ctx, void* stream, const float
     DeviceGuard dg(ctx->device);
     const uint32_t stride = (n_q_heads + 2 * kv->n_kv_heads) * kv->head_dim;
     const cudaError_t e = launch_attn_prefill(qkv, stride, m, n_q_heads, kv->n_kv_heads, kv->head_dim, view_of(kv), pos0, out, out_dtype,
-                                              n_q_heads * kv->head_dim, static_cast<cudaStream_t>(stream));
+                                              n_q_heads * kv->head_dim, ctx->status, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "attn_prefill launch");
     ctx->launches += 1;
     return HF2Q_OK;

@@ -565,149 +565,6 @@ __global__ void __launch_bounds__(ATT_HD) attn_combine_kernel(const float* __res
     else out[static_cast<size_t>(head) * ATT_HD + d] = __float2bfloat16_rn(v);
 }
 
-// ------------------------------------------------------------------ prefill attention (causal, tensor cores)
-// grid (ceil(m / tokens per CTA), n_kv_heads), 4 warps per CTA.  A warp owns 16 rows = 16 / G query tokens x the
-// G heads of its KV head (row r: token r / G, head r % G) and walks the cached positions [0, pos0 + token] in
-// steps of 16 with the decode kernel's two products (mma.sync m16n8k16: K codes as the exact f16 integers
-// 1024 + (code + 128), V codes as f16 subnormals gathered byte-wise from pairs of rows, P * vscale straight
-// from the score accumulators), here with all 16 rows of the A operand in use.  The K / V rows of a KV head are
-// shared by the warps and CTAs of that head through L2 (1 MB per head at 8192 positions).  Heavy tiles (late
-// tokens) are scheduled first.  q is read rotated and scaled (rope_kv_append_kernel ran before).
-constexpr int PF_WARPS = 4;
-
-template <int G, typename OUT>
-__global__ void __launch_bounds__(PF_WARPS * 32) attn_prefill_kernel(const float* __restrict__ qkv, uint32_t row_stride, uint32_t m,
-                                                                     const int8_t* __restrict__ k_codes, const float* __restrict__ k_scale,
-                                                                     const int8_t* __restrict__ v_codes, const float* __restrict__ v_scale,
-                                                                     uint32_t max_seq, uint32_t pos0, OUT* __restrict__ out,
-                                                                     uint32_t out_stride) {
-    constexpr uint32_t TPW = 16 / G;                        // tokens per warp
-    const uint32_t kvh = blockIdx.y, tile = gridDim.x - 1 - blockIdx.x;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, t = lane & 3;
-    const uint32_t wtok0 = (tile * PF_WARPS + warp) * TPW;
-    if (wtok0 >= m) return;
-    const int8_t* kc = k_codes + static_cast<size_t>(kvh) * max_seq * ATT_HD;
-    const int8_t* vc = v_codes + static_cast<size_t>(kvh) * max_seq * ATT_HD;
-    const float* ksc = k_scale + static_cast<size_t>(kvh) * max_seq;
-    const float* vsc = v_scale + static_cast<size_t>(kvh) * max_seq;
-    const uint32_t wlast = pos0 + min(wtok0 + TPW, m) - 1;  // last position any row of this warp sees
-    // this lane's two rows: gid and gid + 8
-    uint32_t rtok[2], rlast[2];
-    uint32_t qa[4][8];                                      // A fragments of the 8 k-steps: [a0 a1 a2 a3][j]
-    float qfix[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t r = gid + 8 * h;
-        rtok[h] = wtok0 + r / G;
-        const bool live = rtok[h] < m;
-        rlast[h] = live ? pos0 + rtok[h] : wlast;           // (rows past the end compute on zeros and are not stored)
-        const float* q = qkv + static_cast<size_t>(live ? rtok[h] : 0) * row_stride + (static_cast<size_t>(kvh) * G + r % G) * ATT_HD + 32 * t;
-        float qsum = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float4 q4 = live ? __ldg(reinterpret_cast<const float4*>(q) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const __half2 lo2 = __floats2half2_rn(q4.x, q4.y), hi2 = __floats2half2_rn(q4.z, q4.w);
-            qa[h][j] = *reinterpret_cast<const uint32_t*>(&lo2);
-            qa[2 + h][j] = *reinterpret_cast<const uint32_t*>(&hi2);
-            qsum += (__low2float(lo2) + __high2float(lo2)) + (__low2float(hi2) + __high2float(hi2));
-        }
-        qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
-        qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
-        qfix[h] = 1152.0f * qsum;
-    }
-    float mx[2] = {-CUDART_INF_F, -CUDART_INF_F}, l[2] = {0.f, 0.f}, lfix[2] = {0.f, 0.f};
-    float o[16][4];                                         // [tile j]: rows gid (0,1) and gid + 8 (2,3), dims 32t + j and 32t + 16 + j
-#pragma unroll
-    for (int j = 0; j < 16; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    for (uint32_t p0 = 0; p0 <= wlast; p0 += 16) {
-        uint4 kq[2][2], vq[4];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            const uint4* kr = reinterpret_cast<const uint4*>(kc + static_cast<size_t>(min(p0 + 8 * nt + gid, wlast)) * ATT_HD + 32 * t);
-            kq[nt][0] = kr[0];
-            kq[nt][1] = kr[1];
-        }
-        const uint32_t pc[4] = {p0 + 2 * t, p0 + 2 * t + 1, p0 + 2 * t + 8, p0 + 2 * t + 9};
-        float kscl[4], vscl[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            vq[i] = *reinterpret_cast<const uint4*>(vc + static_cast<size_t>(min(pc[i], wlast)) * ATT_HD + 16 * gid);
-            kscl[i] = ksc[min(pc[i], wlast)];
-            vscl[i] = vsc[min(pc[i], wlast)];
-        }
-        float sc[2][4];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
-            const uint32_t kw[8] = {kq[nt][0].x, kq[nt][0].y, kq[nt][0].z, kq[nt][0].w, kq[nt][1].x, kq[nt][1].y, kq[nt][1].z, kq[nt][1].w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t x = kw[j] ^ 0x80808080u;
-                mma_m16n8k16_f16(c, qa[0][j], qa[1][j], qa[2][j], qa[3][j], __byte_perm(x, 0x64646464u, 0x4140u), __byte_perm(x, 0x64646464u, 0x4342u));
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-                    sc[h][2 * nt + i] = pc[2 * nt + i] <= rlast[h] ? (c[2 * h + i] - qfix[h]) * kscl[2 * nt + i] : -CUDART_INF_F;
-        }
-        uint32_t pa[4];                                     // a0 (row gid, tile 0), a1 (row gid + 8, tile 0), a2, a3 (tile 1)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float bm = fmaxf(fmaxf(sc[h][0], sc[h][1]), fmaxf(sc[h][2], sc[h][3]));
-            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
-            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
-            const float nm = fmaxf(mx[h], bm);              // finite from the first step on: position 0 is visible to every row
-            const float corr = __expf(mx[h] - nm);
-            float pr[4], wsum = 0.f, psum = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) pr[i] = __expf(sc[h][i] - nm);
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                const __half2 w2 = __floats2half2_rn(pr[2 * nt] * vscl[2 * nt] * 256.0f, pr[2 * nt + 1] * vscl[2 * nt + 1] * 256.0f);
-                pa[2 * nt + h] = *reinterpret_cast<const uint32_t*>(&w2);
-                wsum += __low2float(w2) + __high2float(w2);
-                psum += pr[2 * nt] + pr[2 * nt + 1];
-            }
-            psum += __shfl_xor_sync(0xffffffffu, psum, 1);
-            wsum += __shfl_xor_sync(0xffffffffu, wsum, 1);
-            psum += __shfl_xor_sync(0xffffffffu, psum, 2);
-            wsum += __shfl_xor_sync(0xffffffffu, wsum, 2);
-            l[h] = l[h] * corr + psum;
-            lfix[h] = lfix[h] * corr + wsum;
-            mx[h] = nm;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) { o[j][2 * h] *= corr; o[j][2 * h + 1] *= corr; }
-        }
-        const uint32_t va[4] = {vq[0].x ^ 0x80808080u, vq[0].y ^ 0x80808080u, vq[0].z ^ 0x80808080u, vq[0].w ^ 0x80808080u};
-        const uint32_t vb[4] = {vq[1].x ^ 0x80808080u, vq[1].y ^ 0x80808080u, vq[1].z ^ 0x80808080u, vq[1].w ^ 0x80808080u};
-        const uint32_t vc8[4] = {vq[2].x ^ 0x80808080u, vq[2].y ^ 0x80808080u, vq[2].z ^ 0x80808080u, vq[2].w ^ 0x80808080u};
-        const uint32_t vd[4] = {vq[3].x ^ 0x80808080u, vq[3].y ^ 0x80808080u, vq[3].z ^ 0x80808080u, vq[3].w ^ 0x80808080u};
-#pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
-            const uint32_t lo01 = __byte_perm(va[c4], vb[c4], 0x5410u), hi01 = __byte_perm(va[c4], vb[c4], 0x7632u);
-            const uint32_t lo89 = __byte_perm(vc8[c4], vd[c4], 0x5410u), hi89 = __byte_perm(vc8[c4], vd[c4], 0x7632u);
-            const uint32_t b0[4] = {lo01 & 0x00FF00FFu, __byte_perm(lo01, 0u, 0x4341u), hi01 & 0x00FF00FFu, __byte_perm(hi01, 0u, 0x4341u)};
-            const uint32_t b1[4] = {lo89 & 0x00FF00FFu, __byte_perm(lo89, 0u, 0x4341u), hi89 & 0x00FF00FFu, __byte_perm(hi89, 0u, 0x4341u)};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) mma_m16n8k16_f16(o[4 * c4 + i], pa[0], pa[1], pa[2], pa[3], b0[i], b1[i]);
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        if (rtok[h] >= m) continue;
-        const uint32_t r = gid + 8 * h;
-        const float inv = l[h] > 0.f ? 1.0f / l[h] : 0.f, off = 128.0f * lfix[h] * (1.0f / 256.0f);
-        OUT* dst = out + static_cast<size_t>(rtok[h]) * out_stride + (static_cast<size_t>(kvh) * G + r % G) * ATT_HD + 32 * t;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float v0 = (o[j][2 * h] * 65536.0f - off) * inv, v1 = (o[j][2 * h + 1] * 65536.0f - off) * inv;
-            if constexpr (sizeof(OUT) == 4) { dst[j] = v0; dst[16 + j] = v1; }
-            else { dst[j] = __float2bfloat16_rn(v0); dst[16 + j] = __float2bfloat16_rn(v1); }
-        }
-    }
-}
-
 // ------------------------------------------------------------------ greedy arg-max (+ position advance)
 // The index of the largest logit (the lowest index on ties, NaN never wins) goes to *out_id; if
 // pos != nullptr the position counter is advanced by one -- the decode loop's hand-over to the next
@@ -854,31 +711,6 @@ cudaError_t launch_attn_decode_fused(const float* qkv, uint32_t n_q, uint32_t n_
 #define HF2Q_CASE(GG) case GG: \
         if (f32) return cudaLaunchKernelEx(&cfg, attn_decode_fused_kernel<GG, float>, qkv, n_q, n_kv, theta, qs, kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, pos, part, counters, static_cast<float*>(out), status); \
         return cudaLaunchKernelEx(&cfg, attn_decode_fused_kernel<GG, __nv_bfloat16>, qkv, n_q, n_kv, theta, qs, kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, pos, part, counters, static_cast<__nv_bfloat16*>(out), status);
-        HF2Q_CASE(1) HF2Q_CASE(2) HF2Q_CASE(4) HF2Q_CASE(8)
-#undef HF2Q_CASE
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-template <int G, typename OUT>
-static cudaError_t launch_prefill_g(const float* qkv, uint32_t row_stride, uint32_t m, const KvCacheView& kv, uint32_t n_kv, uint32_t pos0,
-                                    OUT* out, uint32_t out_stride, cudaStream_t st) {
-    constexpr uint32_t TOK = PF_WARPS * (16 / G);           // query tokens per CTA
-    const dim3 grid((m + TOK - 1) / TOK, n_kv);
-    attn_prefill_kernel<G, OUT><<<grid, PF_WARPS * 32, 0, st>>>(qkv, row_stride, m, kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, pos0,
-                                                                out, out_stride);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_attn_prefill(const float* qkv, uint32_t row_stride, uint32_t m, uint32_t n_q, uint32_t n_kv, uint32_t hd,
-                                const KvCacheView& kv, uint32_t pos0, void* out, uint32_t out_dtype, uint32_t out_stride, cudaStream_t st) {
-    if (hd != ATT_HD || n_kv == 0 || n_q % n_kv) return cudaErrorInvalidValue;
-    const uint32_t G = n_q / n_kv;
-    const bool f32 = out_dtype == HF2Q_DT_F32;
-    if (!f32 && out_dtype != HF2Q_DT_BF16) return cudaErrorInvalidValue;
-    switch (G) {
-#define HF2Q_CASE(GG) case GG: return f32 ? launch_prefill_g<GG, float>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<float*>(out), out_stride, st) \
-                                          : launch_prefill_g<GG, __nv_bfloat16>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<__nv_bfloat16*>(out), out_stride, st);
         HF2Q_CASE(1) HF2Q_CASE(2) HF2Q_CASE(4) HF2Q_CASE(8)
 #undef HF2Q_CASE
         default: return cudaErrorInvalidValue;

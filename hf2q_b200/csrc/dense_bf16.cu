@@ -278,13 +278,6 @@ constexpr int TC_M = 128, TC_K = 64, TC_THREADS = 192;
 __host__ __device__ constexpr int tc_stages(int nt) { return nt == 256 ? 4 : nt == 128 ? 6 : 8; }
 __host__ __device__ constexpr uint32_t tc_stage_bytes(int nt) { return (TC_M + nt) * TC_K * 2; }
 
-__device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void st_global_v8(float* p, const float* v) {
     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
                  "f"(v[6]), "f"(v[7])
@@ -371,7 +364,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_gemm_tc_kernel(const __gr
                     tc::tc_fence_after();
                     const uint64_t da = tc::smem_desc_sw128(smem_u32(smem + s * SB)), db = tc::smem_desc_sw128(smem_u32(smem + s * SB + TC_M * TC_K * 2));
 #pragma unroll
-                    for (uint32_t kk = 0; kk < TC_K / 16; ++kk) umma_ss(tmem + b * NT, da + 2 * kk, db + 2 * kk, IDESC, (kb | kk) ? 1u : 0u);
+                    for (uint32_t kk = 0; kk < TC_K / 16; ++kk) tc::umma_ss(tmem + b * NT, da + 2 * kk, db + 2 * kk, IDESC, (kb | kk) ? 1u : 0u);
                     tc::tc_commit(&empty[s]);
                 }
                 if (ok) tc::tc_commit(&d_full[b]);

@@ -188,7 +188,7 @@ size_t attn_decode_scratch_bytes(uint32_t n_kv, uint32_t group, uint32_t n_split
 cudaError_t launch_attn_decode(const float* q, uint32_t n_q, uint32_t n_kv, uint32_t hd, const KvCacheView& kv, const uint32_t* pos,
                                void* out, uint32_t out_dtype, float* scratch, uint32_t n_splits, cudaStream_t st);
 cudaError_t launch_attn_prefill(const float* qkv, uint32_t row_stride, uint32_t m, uint32_t n_q, uint32_t n_kv, uint32_t hd,
-                                const KvCacheView& kv, uint32_t pos0, void* out, uint32_t out_dtype, uint32_t out_stride, cudaStream_t st);
+                                const KvCacheView& kv, uint32_t pos0, void* out, uint32_t out_dtype, uint32_t out_stride, uint32_t* status, cudaStream_t st);
 // scratch: 1 + 2 * 64 + 1 zero-initialised words owned by the caller (the context), one arg-max at a time
 cudaError_t launch_argmax(const float* logits, uint32_t n, uint32_t* out_id, uint32_t* pos, uint32_t* scratch, cudaStream_t st);
 // rotary embedding of the query, append of the new position, split attention and merge in one launch;

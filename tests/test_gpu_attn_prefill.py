@@ -1,0 +1,53 @@
+"""Prompt attention over the 8-bit cache: the tensor-core kernel against softmax attention in 64 bits on the same codes."""
+import ctypes as C
+
+import pytest
+import torch
+
+from hf2q_b200 import _lib, decoder, ops
+
+pytestmark = pytest.mark.gpu
+HD = 128
+
+
+def case(group, n_kv, pos0, m, k_scale, v_scale, growing, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    T, S = pos0 + m, pos0 + m + 3
+    codes = [torch.randint(-127, 128, (n_kv, S, HD), generator=g, device="cuda", dtype=torch.int8) for _ in range(2)]
+    scales = [s * (0.5 + torch.rand((n_kv, S), generator=g, device="cuda")) / 127 for s in (k_scale, v_scale)]
+    if growing:                                          # scores grow with the position: the running maximum rises in every block
+        scales[0] = scales[0] * torch.linspace(0.05, 4.0, S, device="cuda")
+    scales[0][:, T:], scales[1][:, T:] = float("nan"), float("nan")          # what no row sees is not touched
+    qkv = torch.randn((m, (group + 2) * n_kv * HD), generator=g, device="cuda") * HD ** -0.5
+    return qkv, codes, scales, T, S
+
+
+@pytest.mark.parametrize("group,n_kv,pos0,m,k_scale,v_scale,growing,dtype", [
+    (4, 8, 0, 1, 1.0, 1.0, False, torch.float32),
+    (4, 2, 0, 63, 1.0, 1.0, False, torch.float32),
+    (4, 2, 0, 65, 2.0, 1.0, True, torch.float32),
+    (8, 1, 5, 300, 2.0, 1.0, True, torch.bfloat16),
+    (1, 3, 130, 257, 2.0, 1.0, True, torch.float32),
+    (2, 2, 1000, 129, 1.0, 5e3, True, torch.float32),    # V scales at which the exponentials may not pass 1
+    (4, 2, 4001, 97, 3.0, 1.0, False, torch.bfloat16),
+    (1, 1, 64, 64, 1.0, 1e-4, False, torch.float32),
+])
+def test_prompt_attention_matches_softmax(gpu_ctx, group, n_kv, pos0, m, k_scale, v_scale, growing, dtype):
+    qkv, codes, scales, T, S = case(group, n_kv, pos0, m, k_scale, v_scale, growing, seed=m)
+    nq = group * n_kv
+    kv = decoder._KvCache(codes[0].data_ptr(), scales[0].data_ptr(), codes[1].data_ptr(), scales[1].data_ptr(), n_kv, HD, S)
+    out = torch.full((m, nq * HD), float("nan"), device="cuda", dtype=dtype)
+    lib = _lib.load()
+    gpu_ctx._check(lib.hf2q_cuda_attn_prefill(gpu_ctx._h, torch.cuda.current_stream().cuda_stream, qkv.data_ptr(), m, nq, C.byref(kv), pos0,
+                                              out.data_ptr(), ops.DT_F32 if dtype == torch.float32 else ops.DT_BF16))
+    gpu_ctx.check_status()
+    k, v = ((c[:, :T].double() * s[:, :T, None].double()) for c, s in zip(codes, scales))
+    q = qkv[:, :nq * HD].double().view(m, n_kv, group, HD)
+    s = torch.einsum("tgrd,gpd->gtrp", q, k)
+    hidden = torch.arange(T, device="cuda")[None] > pos0 + torch.arange(m, device="cuda")[:, None]
+    want = torch.einsum("gtrp,gpd->tgrd", torch.softmax(s.masked_fill(hidden[None, :, None], -float("inf")), dim=-1), v).reshape(m, nq * HD)
+    # probability * v_scale and q are f16: 2^-11 of the value each, the second times the spread of a score; bf16 results 2^-9 more
+    spread = s.masked_fill(hidden[None, :, None], 0).std().item()
+    bound = 2 ** -11 * (1 + spread) + (2 ** -9 if dtype == torch.bfloat16 else 0)
+    err = (out.double() - want).norm() / want.norm()
+    assert err < bound, (err.item(), bound)
