@@ -157,6 +157,13 @@ class GreedyDecoder:
         return out
 
 
+def to_device(t: torch.Tensor, device) -> torch.Tensor:
+    """A copy that the host does not wait for: host tensors go through pinned memory."""
+    if t.device.type == "cpu" and torch.device(device).type == "cuda" and t.numel():
+        return t.pin_memory().to(device, non_blocking=True)
+    return t.to(device)
+
+
 class SlotDecoder(GreedyDecoder):
     """A decoder whose sequences live in the slots of a ``StatePool``; steps run one sequence at a time.
 
@@ -214,7 +221,9 @@ class SlotDecoder(GreedyDecoder):
         if n == 0 or start + n > self.max_seq:
             raise ops.Hf2qError(_lib.ERR_INVALID_ARGUMENT, f"{n} tokens after {start}: the model was loaded for sequences of 1..{self.max_seq}")
         self.bind(slot)
-        ids = ids.to(self.dev, torch.int32).contiguous()
+        ids = ids.to(torch.int32).contiguous()
+        if n > 1:
+            ids = to_device(ids, self.dev)
         want = list(want)
         out = torch.empty((len(want), self.cfg.vocab), dtype=torch.float32, device=self.dev)
         for c0 in range(0, n, self.chunk):
@@ -223,19 +232,23 @@ class SlotDecoder(GreedyDecoder):
             last = c0 + m == n
             self.pos.fill_(start + c0)
             if m == 1 and self.on_layer is None:
-                self.tok.copy_(ids[c0:c0 + 1])
+                # nothing here waits for the device, so that the host prepares the next step while this one runs
+                if ids.device.type == "cpu":
+                    self.tok.fill_(int(ids[0]))
+                else:
+                    self.tok.copy_(ids[c0:c0 + 1])
                 self.ensure_graph()
                 self._graph.replay()
-                if here:
-                    out[[j for j, _ in here]] = self.logits
+                for j, _ in here:
+                    out[j:j + 1].copy_(self.logits)
                 continue
             self._start = start + c0
-            x = self._portion(ids[c0:c0 + m], m)
+            x = self._portion(ids[c0:c0 + m].to(self.dev), m)
             self._start = None
             rows = [p for _, p in here]
             logits = self._head_rows(x, rows + [m - 1]) if last or rows else None
             if rows:
-                out[torch.tensor([j for j, _ in here], device=self.dev)] = logits[:len(rows)]
+                out[to_device(torch.tensor([j for j, _ in here]), self.dev)] = logits[:len(rows)]
             if last:
                 self.logits.copy_(logits[-1:])
                 self.sop.argmax(self.logits, self.tok)

@@ -10,6 +10,8 @@ from dataclasses import dataclass
 
 import torch
 
+from .decoder import to_device
+
 
 @dataclass
 class Entry:
@@ -33,13 +35,15 @@ class Engine:
             slot = self._slots[e.id]
             order = sorted(range(len(e.want)), key=lambda j: e.want[j])
             got = self.model.extend(slot, torch.tensor(e.tokens, dtype=torch.int32), [e.want[j] for j in order])
-            back = torch.empty(len(order), dtype=torch.long)
-            back[order] = torch.arange(len(order))
-            if len(order):
-                rows.append(got[back.to(got.device)])
+            if len(order) and order == list(range(len(order))):
+                rows.append(got)
+            elif len(order):
+                back = torch.empty(len(order), dtype=torch.long)
+                back[order] = torch.arange(len(order))
+                rows.append(got[to_device(back, got.device)])
         for i in end:
             self.model.close_slot(self._slots.pop(i))
-        return torch.cat(rows) if rows else None
+        return (rows[0] if len(rows) == 1 else torch.cat(rows)) if rows else None
 
     def generate(self, prompts, n_new: int) -> list[list[int]]:
         """Greedy continuations of the prompts (lists of token ids), n_new tokens each."""
