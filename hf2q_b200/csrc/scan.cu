@@ -5,10 +5,17 @@
 //   ssd     scalar decay per head and token (Mamba-2)
 //
 // All keep S[key channel][value column] and treat a value column independently, so the state lives in registers:
-// sixteen lanes share a column (each holds key channels 32 c + 2 l and + 1), a warp carries two columns, a CTA of eight
-// warps sixteen columns of one head: the token chain is latency-bound, so many short warps beat few long ones.  A token costs no block barrier; sums over the key channels are four shuffles.
-// Tokens are staged in shared memory in batches by asynchronous copies, two batches in flight.  The state in memory
-// is [head][column][key channel, padded to 32] (f32), which makes a lane's channels consecutive.
+// sixteen lanes share a column (each holds key channels 32 c + 2 l and + 1), and sums over the key channels are shuffles.
+// The state in memory is [head][column][key channel, padded to 32] (f32), which makes a lane's channels consecutive.
+//
+// Prompt portions (the scans): a group of sixteen lanes carries C columns.  What a token costs a warp is the k, q (and g)
+// words that each lane reads from shared memory -- the register file takes one 32-lane word per clock and SM, whether or
+// not lanes read the same one -- so several columns share them; a column alone (two a warp, eight warps an SM) spent 260
+// to 300 of its 490 to 570 clocks a token there.  One warp of the CTA only fetches: it stages the next batch of tokens by
+// asynchronous copies (and makes the gate factors) while the others work through this one, with one barrier per batch.
+// Portions of 2048 tokens: mlstm (8 heads of 128 x 128) 509 -> 217 us with two columns a group (one: 256 us), delta (16 of
+// 128 x 128) 594 -> 314 us with two (346 us one token at a time), ssd (64 of 128 x 64) 547 -> 268 us with two in eight warps
+// (280 us with four in four).  What bounds them now is the issue of a token's multiply-adds, two clocks for each pair.
 #include <math_constants.h>
 
 #include "seq_common.cuh"
@@ -17,7 +24,8 @@ namespace hf2q {
 namespace {
 using namespace seq;
 
-constexpr int SC_WARPS = 8, SC_COLS = 16, SC_TB = 16, SC_THREADS = SC_WARPS * 32;
+constexpr int SC_WARPS = 8, SC_COLS = 16, SC_THREADS = SC_WARPS * 32;       // one-token kernels: a group to a column
+constexpr int SC_TB = 32;                                                   // scans: tokens of a batch
 
 __device__ __forceinline__ float group_sum(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -26,10 +34,11 @@ __device__ __forceinline__ float group_sum(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 8);
     return v;
 }
-// Sums of sixteen values over the sixteen lanes of a group, transposed: lane l ends with the sum of v[l] (15 shuffles).
-__device__ __forceinline__ float group_transpose_sum(float (&v)[16], uint32_t l) {
+// Sums of K values over the sixteen lanes of a group, transposed: lane l ends with the sum of v[l % K].
+template <int K>
+__device__ __forceinline__ float group_transpose_sum(float (&v)[K], uint32_t l) {
 #pragma unroll
-    for (int w = 8; w > 0; w >>= 1) {
+    for (int w = K / 2; w > 0; w >>= 1) {
         const bool up = l & w;
 #pragma unroll
         for (int i = 0; i < w; ++i) {
@@ -37,18 +46,39 @@ __device__ __forceinline__ float group_transpose_sum(float (&v)[16], uint32_t l)
             v[i] = (up ? v[i + w] : v[i]) + other;
         }
     }
+#pragma unroll
+    for (int w = K; w < 16; w *= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], w);
     return v[0];
 }
-// rows of `count` floats -> shared memory, asynchronously, 16 bytes at a time where both sides allow it; a warp takes
-// whole rows
+// rows of `count` floats -> shared memory, asynchronously, by one warp; 16 bytes at a time where both sides allow it
 __device__ __forceinline__ void stage_rows(float* dst, uint32_t dst_ld, const float* src, size_t src_ld, uint32_t rows, uint32_t count) {
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31;
     if (count % 4 == 0 && src_ld % 4 == 0 && dst_ld % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-        for (uint32_t r = warp; r < rows; r += SC_WARPS)
-            for (uint32_t c = 4 * lane; c < count; c += 128) cp_async16(dst + r * dst_ld + c, src + r * src_ld + c);
+        if (count <= 64) {                                   // several short rows at once
+            const uint32_t per = count <= 8 ? 2 : count <= 16 ? 4 : count <= 32 ? 8 : 16, c = 4 * (lane % per);
+            if (c < count)
+                for (uint32_t r = lane / per; r < rows; r += 32 / per) cp_async16(dst + r * dst_ld + c, src + r * src_ld + c);
+        } else {
+            for (uint32_t c = 4 * lane; c < count; c += 128)
+#pragma unroll 4
+                for (uint32_t r = 0; r < rows; ++r) cp_async16(dst + r * dst_ld + c, src + r * src_ld + c);
+        }
     } else {
-        for (uint32_t r = warp; r < rows; r += SC_WARPS)
-            for (uint32_t c = lane; c < count; c += 32) cp_async4(dst + r * dst_ld + c, src + r * src_ld + c);
+        for (uint32_t c = lane; c < count; c += 32)
+#pragma unroll 4
+            for (uint32_t r = 0; r < rows; ++r) cp_async4(dst + r * dst_ld + c, src + r * src_ld + c);
+    }
+}
+template <int C>
+__device__ __forceinline__ void load_values(float (&v)[C], const float* p) {
+    if constexpr (C == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else if constexpr (C == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        v[0] = x.x; v[1] = x.y;
+    } else {
+        v[0] = *p;
     }
 }
 
@@ -73,6 +103,12 @@ template <int RQ> struct Vec {                       // a lane's RQ pairs of key
         for (int c = 1; c < RQ; ++c) s[c & 1] = f2_fma(v[c], k.v[c], s[c & 1]);
         return f2_sum(RQ > 1 ? f2_add(s[0], s[1]) : s[0]);
     }
+    __device__ __forceinline__ Vec operator*(const Vec& k) const {
+        Vec r;
+#pragma unroll
+        for (int c = 0; c < RQ; ++c) r.v[c] = f2_mul(v[c], k.v[c]);
+        return r;
+    }
     __device__ __forceinline__ void scale(const Vec& k) {
 #pragma unroll
         for (int c = 0; c < RQ; ++c) v[c] = f2_mul(v[c], k.v[c]);
@@ -89,119 +125,188 @@ template <int RQ> struct Vec {                       // a lane's RQ pairs of key
     }
 };
 
+// Where a thread of a scan stands: W working warps of two groups with C columns each, then the fetching warp.
+template <int RQ, int C, int W>
+struct ScanPlace {
+    static constexpr uint32_t DP = 32 * RQ, COLS = 2 * C * W, GROUP = 16 / C;        // GROUP: tokens whose sums fill a group's lanes
+    uint32_t warp, lane, lg, group, col0, col, n_cols;
+    bool fetches;
+    __device__ __forceinline__ ScanPlace(uint32_t slice, uint32_t vdim) {
+        warp = threadIdx.x >> 5;
+        lane = threadIdx.x & 31;
+        lg = lane & 15;
+        group = warp * 2 + (lane >> 4);
+        col0 = slice * COLS;
+        col = col0 + group * C;                              // the group's first column
+        n_cols = min(COLS, vdim - col0);
+        fetches = warp == W;
+    }
+};
+// Batches of SC_TB tokens in two buffers: stage(t0, buffer) by the fetching warp, batch(t0, buffer, tokens) by the others.
+template <typename Stage, typename Batch>
+__device__ __forceinline__ void scan_batches(bool fetches, uint32_t m, Stage stage, Batch batch) {
+    if (fetches) { stage(0u, 0u); cp_async_wait<0>(); }
+    __syncthreads();
+    for (uint32_t t0 = 0, b = 0; t0 < m; t0 += SC_TB, b ^= 1) {
+        if (fetches) {
+            if (t0 + SC_TB < m) { stage(t0 + SC_TB, b ^ 1); cp_async_wait<0>(); }
+        } else {
+            batch(t0, b, min(static_cast<uint32_t>(SC_TB), m - t0));
+        }
+        __syncthreads();
+    }
+}
+// The whole groups of a batch's n tokens: form(j0, sums) makes a lane's partial sums, done(j0, sums) adds them up and stores.
+// A group's sums are finished beside the next group's tokens, whose arithmetic hides the shuffles.  Returns the tokens taken.
+template <typename Sums, uint32_t GROUP, typename Form, typename Done>
+__device__ __forceinline__ uint32_t scan_groups(uint32_t n, Form form, Done done) {
+    if (n < GROUP) return 0;
+    Sums last;
+    form(0u, last);
+    uint32_t j0 = GROUP;
+    for (; j0 + GROUP <= n; j0 += GROUP) {
+        Sums now;
+        form(j0, now);
+        done(j0 - GROUP, last);
+        last = now;
+    }
+    done(j0 - GROUP, last);
+    return j0;
+}
+// channels past `dim` stay zero in shared memory, so the padded part of the state stays zero too
+__device__ __forceinline__ void clear_padding(float* sm, uint32_t n, bool padded) {
+    if (!padded) return;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sm[i] = 0.f;
+    __syncthreads();
+}
+// Shared memory of a scan's launch.  It asks for so much that no SM takes more CTAs than an even spread puts there: the CTAs
+// start while the preceding kernel's last ones still run, and would otherwise pile up on the SMs that are free first.
+constexpr size_t SCAN_STATIC = 9 * 1024, SCAN_MAX = 227 * 1024 - SCAN_STATIC;       // static arrays: at most
+inline size_t scan_smem(size_t need, dim3 grid, int sms) {
+    const size_t ctas = static_cast<size_t>(grid.x) * grid.y, per_sm = (ctas + sms - 1) / sms;
+    const size_t even = 228 * 1024 / per_sm, claim = even > SCAN_STATIC + 1024 ? even - SCAN_STATIC - 1024 : 0;
+    return claim > need ? claim : need;
+}
+
 // ---------------------------------------------------------------- mLSTM
-template <int RQ>
-__global__ void __launch_bounds__(SC_THREADS) mlstm_kernel(const __grid_constant__ hf2q_mlstm a, uint32_t m, float* __restrict__ out) {
-    constexpr uint32_t DP = 32 * RQ;
+// A CTA carries the 16 columns that share a normaliser and a maximum.
+template <int RQ, int C>
+__global__ void __launch_bounds__((8 / C + 1) * 32, 1) mlstm_kernel(const __grid_constant__ hf2q_mlstm a, uint32_t m, float* __restrict__ out) {
+    constexpr uint32_t W = 8 / C;
+    using Place = ScanPlace<RQ, C, W>;
+    constexpr uint32_t DP = Place::DP;
     extern __shared__ __align__(16) float dsm[];                    // k, q: [2][SC_TB][DP] each
     float* ks = dsm;
     float* qs = dsm + 2 * SC_TB * DP;
     __shared__ __align__(16) float vs[2][SC_TB][SC_COLS];
-    __shared__ float gk[2][SC_TB], gw[2][SC_TB], ge[2][SC_TB];     // keep, write, exp(-maximum)
+    __shared__ __align__(8) float2 gs[2][SC_TB];                    // keep, write
+    __shared__ float ge[2][SC_TB];                                  // exp(-maximum)
     pdl_trigger();
     pdl_wait();
     const uint32_t h = blockIdx.x, slice = blockIdx.y, n_slices = gridDim.y;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = lane & 15;
-    const uint32_t col_s = warp * 2 + (lane >> 4), col0 = slice * SC_COLS, col = col0 + col_s;
-    const uint32_t n_cols = min(static_cast<uint32_t>(SC_COLS), a.vdim - col0);
-    const bool live = col < a.vdim;
+    const Place at(slice, a.vdim);
     const float q_scale = 1.0f / sqrtf(static_cast<float>(a.dim));
     float* mp = a.mx + static_cast<size_t>(h) * n_slices + slice;
-    float mx = *mp;                                          // carried by the last warp
-    // channels past dim stay zero in shared memory, so the padded part of the state stays zero too
-    for (uint32_t i = threadIdx.x; i < 4 * SC_TB * DP; i += SC_THREADS) dsm[i] = 0.f;
-    for (uint32_t i = threadIdx.x; i < 2 * SC_TB * SC_COLS; i += SC_THREADS) (&vs[0][0][0])[i] = 0.f;
-    __syncthreads();
+    float mx = *mp;                                          // carried by the fetching warp
+    clear_padding(dsm, 4 * SC_TB * DP, a.dim < DP);
     auto stage = [&](uint32_t t0, uint32_t b) {
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
+        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0), lane = at.lane;
         const float* row = a.proj + static_cast<size_t>(t0) * a.ld;
         stage_rows(ks + b * SC_TB * DP, DP, row + a.k_off + h * a.dim, a.ld, n, a.dim);
         stage_rows(qs + b * SC_TB * DP, DP, row + a.q_off + h * a.dim, a.ld, n, a.dim);
-        stage_rows(vs[b][0], SC_COLS, row + a.v_off + h * a.vdim + col0, a.ld, n, n_cols);
-        // gate factors of the batch, by the last warp (lane = token): the running maximum is a max-plus scan over the
-        // pairs (f, i), m_t = max(m + f_1 + .. + f_t, max_s (i_s + f_(s+1) + .. + f_t))
-        if (warp == SC_WARPS - 1) {
-            float f = 0.f, x = -CUDART_INF_F;
-            if (lane < n) {
-                const float* g = row + static_cast<size_t>(lane) * a.ld + h;
-                x = a.gate_cap * tanhf((g[a.i_off] + a.i_bias[h]) / a.gate_cap);
-                f = -softplusf(-a.gate_cap * tanhf((g[a.f_off] + a.f_bias[h]) / a.gate_cap));
-            }
-            const float f_own = f, x_own = x;
-#pragma unroll
-            for (int d = 1; d < SC_TB; d *= 2) {
-                const float fo = __shfl_up_sync(0xffffffffu, f, d), xo = __shfl_up_sync(0xffffffffu, x, d);
-                if (lane >= d) { x = fmaxf(xo + f, x); f += fo; }
-            }
-            const float m_t = fmaxf(mx + f, x);
-            float before = __shfl_up_sync(0xffffffffu, m_t, 1);
-            if (lane == 0) before = mx;
-            if (lane < n) {
-                gk[b][lane] = expf(f_own + before - m_t);
-                gw[b][lane] = expf(x_own - m_t);
-                ge[b][lane] = expf(-m_t);
-            }
-            mx = __shfl_sync(0xffffffffu, m_t, n - 1);
-        }
+        stage_rows(vs[b][0], SC_COLS, row + a.v_off + h * a.vdim + at.col0, a.ld, n, at.n_cols);
         cp_async_commit();
+        // gate factors of the batch (lane = token): the running maximum is a max-plus scan over the pairs (f, i),
+        // m_t = max(m + f_1 + .. + f_t, max_s (i_s + f_(s+1) + .. + f_t))
+        float f = 0.f, x = -CUDART_INF_F;
+        if (lane < n) {
+            const float* g = row + static_cast<size_t>(lane) * a.ld + h;
+            x = a.gate_cap * tanhf((g[a.i_off] + a.i_bias[h]) / a.gate_cap);
+            f = -softplusf(-a.gate_cap * tanhf((g[a.f_off] + a.f_bias[h]) / a.gate_cap));
+        }
+        const float f_own = f, x_own = x;
+#pragma unroll
+        for (int d = 1; d < SC_TB; d *= 2) {
+            const float fo = __shfl_up_sync(0xffffffffu, f, d), xo = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) { x = fmaxf(xo + f, x); f += fo; }
+        }
+        const float m_t = fmaxf(mx + f, x);
+        float before = __shfl_up_sync(0xffffffffu, m_t, 1);
+        if (lane == 0) before = mx;
+        if (lane < n) {
+            gs[b][lane] = make_float2(expf(f_own + before - m_t), expf(x_own - m_t));
+            ge[b][lane] = expf(-m_t);
+        }
+        mx = __shfl_sync(0xffffffffu, m_t, n - 1);
     };
-    Vec<RQ> S, N;
-    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + (live ? col : 0)) * DP + 2 * lg;
-    float* np = a.n + (static_cast<size_t>(h) * n_slices + slice) * DP + 2 * lg;
-    if (live) S.load(sp); else S.zero();
-    N.load(np);
-    stage(0, 0);
-    for (uint32_t t0 = 0, b = 0; t0 < m; t0 += SC_TB, b ^= 1) {
-        if (t0 + SC_TB < m) { stage(t0 + SC_TB, b ^ 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        __syncthreads();
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
+    Vec<RQ> S[C], N;
+    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + at.col) * DP + 2 * at.lg;
+    float* np = a.n + (static_cast<size_t>(h) * n_slices + slice) * DP + 2 * at.lg;
+    if (!at.fetches) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (at.col + c < a.vdim) S[c].load(sp + c * DP); else S[c].zero();
+        N.load(np);
+    }
+    scan_batches(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
         // a token's operands are read one token ahead of their use
-        struct Operands { Vec<RQ> k, q; float keep, write, v; };
+        struct Operands { Vec<RQ> k, q; float2 g; float v[C]; };
         auto fetch = [&](uint32_t j) {
             Operands t;
-            t.k.load(ks + (b * SC_TB + j) * DP + 2 * lg);
-            t.q.load(qs + (b * SC_TB + j) * DP + 2 * lg);
-            t.keep = gk[b][j];
-            t.write = gw[b][j];
-            t.v = vs[b][j][col_s];
+            t.k.load(ks + (b * SC_TB + j) * DP + 2 * at.lg);
+            t.q.load(qs + (b * SC_TB + j) * DP + 2 * at.lg);
+            t.g = gs[b][j];
+            load_values(t.v, &vs[b][j][at.group * C]);
             return t;
         };
-        auto token = [&](const Operands& t, float& num, float& den) {      // this lane's part of both sums
-            S.decay_axpy(t.keep, t.k, t.write * t.v);
-            N.decay_axpy(t.keep, t.k, t.write);
-            num = S.dot(t.q);
+        auto token = [&](const Operands& t, float* num, float& den) {      // this lane's part of the sums
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                S[c].decay_axpy(t.g.x, t.k, t.g.y * t.v[c]);
+                num[c] = S[c].dot(t.q);
+            }
+            N.decay_axpy(t.g.x, t.k, t.g.y);
             den = N.dot(t.q);
         };
-        auto finish = [&](uint32_t j, float num, float den) {
-            if (live)
+        auto finish = [&](uint32_t j, uint32_t col, float num, float den) {
+            if (col < a.vdim)
                 out[static_cast<size_t>(t0 + j) * a.heads * a.vdim + static_cast<size_t>(h) * a.vdim + col] = num * q_scale / (fmaxf(fabsf(den * q_scale), ge[b][j]) + 1e-6f);
         };
-        uint32_t j0 = 0;
-        for (; j0 + 16 <= n; j0 += 16) {                     // sixteen tokens without a branch; lane i of a group finishes token i
-            float num[16], den[16];
-            Operands t = fetch(j0);
+        struct Sums { float num[16], den[Place::GROUP]; };
+        uint32_t j0 = scan_groups<Sums, Place::GROUP>(
+            n,
+            [&](uint32_t j, Sums& r) {
+                Operands t = fetch(j);
 #pragma unroll
-            for (uint32_t u = 0; u < 16; ++u) {
-                const Operands next = fetch(j0 + (u < 15 ? u + 1 : 15));
-                token(t, num[u], den[u]);
-                t = next;
-            }
-            const float x = group_transpose_sum(num, lg), y = group_transpose_sum(den, lg);
-            finish(j0 + lg, x, y);
-        }
+                for (uint32_t u = 0; u < Place::GROUP; ++u) {
+                    const Operands next = fetch(j + (u + 1 < Place::GROUP ? u + 1 : u));
+                    token(t, r.num + u * C, r.den[u]);
+                    t = next;
+                }
+            },
+            [&](uint32_t j, Sums& r) {                           // lane i of a group finishes token i / C, column i % C
+                const float x = group_transpose_sum(r.num, at.lg), y = group_transpose_sum(r.den, at.lg);
+                finish(j + at.lg / C, at.col + at.lg % C, x, C == 1 ? y : __shfl_sync(0xffffffffu, y, (at.lane & 16) + at.lg / C));
+            });
         for (; j0 < n; ++j0) {
-            float x, y;
-            token(fetch(j0), x, y);
-            x = group_sum(x);
-            y = group_sum(y);
-            if (lg == 0) finish(j0, x, y);
+            float num[C], den;
+            token(fetch(j0), num, den);
+            den = group_sum(den);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float x = group_sum(num[c]);
+                if (at.lg == c) finish(j0, at.col + c, x, den);
+            }
         }
-        __syncthreads();
+    });
+    if (!at.fetches) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (at.col + c < a.vdim) S[c].store(sp + c * DP);
+        if (at.warp == 0 && at.lane < 16) N.store(np);
+    } else if (at.lane == 0) {
+        *mp = mx;
     }
-    if (live) S.store(sp);
-    if (warp == 0 && lane < 16) N.store(np);
-    if (warp == SC_WARPS - 1 && lane == 0) *mp = mx;
 }
 
 // ---------------------------------------------------------------- gated delta rule
@@ -219,78 +324,122 @@ __device__ __forceinline__ float delta_token(Vec<RQ>& S, const DeltaOperands<RQ>
     return S.dot(t.q);
 }
 
-template <int RQ>
-__global__ void __launch_bounds__(SC_THREADS) delta_scan_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, const float* __restrict__ qkv,
-                                                                const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ out) {
-    constexpr uint32_t DP = 32 * RQ;
+template <int RQ, int C, int W, int PER_SM>
+__global__ void __launch_bounds__((W + 1) * 32, PER_SM) delta_scan_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, const float* __restrict__ qkv,
+                                                                  const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ out) {
+    using Place = ScanPlace<RQ, C, W>;
+    constexpr uint32_t DP = Place::DP;
     extern __shared__ __align__(16) float dsm[];                    // k, q, g: [2][SC_TB][DP] each
     float* ks = dsm;
     float* qs = dsm + 2 * SC_TB * DP;
     float* gs = dsm + 4 * SC_TB * DP;
-    __shared__ __align__(16) float vs[2][SC_TB][SC_COLS];
+    __shared__ __align__(16) float vs[2][SC_TB][Place::COLS];
     __shared__ float bs[2][SC_TB];
     pdl_trigger();
     pdl_wait();
-    const uint32_t h = blockIdx.x, slice = blockIdx.y, kvh = h / (a.heads / a.kv_heads);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = lane & 15;
-    const uint32_t col_s = warp * 2 + (lane >> 4), col0 = slice * SC_COLS, col = col0 + col_s;
-    const uint32_t n_cols = min(static_cast<uint32_t>(SC_COLS), a.vdim - col0);
-    const bool live = col < a.vdim;
+    const uint32_t h = blockIdx.x, kvh = h / (a.heads / a.kv_heads);
+    const Place at(blockIdx.y, a.vdim);
     const uint32_t qk = a.kv_heads * a.dim, ld = 2 * qk + a.heads * a.vdim;
-    for (uint32_t i = threadIdx.x; i < 6 * SC_TB * DP; i += SC_THREADS) dsm[i] = 0.f;
-    for (uint32_t i = threadIdx.x; i < 2 * SC_TB * SC_COLS; i += SC_THREADS) (&vs[0][0][0])[i] = 0.f;
-    __syncthreads();
+    clear_padding(dsm, 6 * SC_TB * DP, a.dim < DP);
     auto stage = [&](uint32_t t0, uint32_t b) {
         const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
         const float* row = qkv + static_cast<size_t>(t0) * ld;
         stage_rows(qs + b * SC_TB * DP, DP, row + kvh * a.dim, ld, n, a.dim);
         stage_rows(ks + b * SC_TB * DP, DP, row + qk + kvh * a.dim, ld, n, a.dim);
-        stage_rows(vs[b][0], SC_COLS, row + 2 * qk + h * a.vdim + col0, ld, n, n_cols);
+        stage_rows(vs[b][0], Place::COLS, row + 2 * qk + h * a.vdim + at.col0, ld, n, at.n_cols);
         stage_rows(gs + b * SC_TB * DP, DP, g + (static_cast<size_t>(t0) * a.heads + h) * a.dim, static_cast<size_t>(a.heads) * a.dim, n, a.dim);
-        if (threadIdx.x < n) bs[b][threadIdx.x] = beta[static_cast<size_t>(t0 + threadIdx.x) * a.heads + h];
+        if (at.lane < n) cp_async4(&bs[b][at.lane], beta + static_cast<size_t>(t0 + at.lane) * a.heads + h);
         cp_async_commit();
     };
-    Vec<RQ> S;
-    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + (live ? col : 0)) * DP + 2 * lg;
-    if (live) S.load(sp); else S.zero();
-    stage(0, 0);
-    for (uint32_t t0 = 0, b = 0; t0 < m; t0 += SC_TB, b ^= 1) {
-        if (t0 + SC_TB < m) { stage(t0 + SC_TB, b ^ 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        __syncthreads();
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
-        auto fetch = [&](uint32_t j) {                       // read one token ahead of their use
-            const uint32_t o = (b * SC_TB + j) * DP + 2 * lg;
-            DeltaOperands<RQ> t;
+    Vec<RQ> S[C];
+    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + at.col) * DP + 2 * at.lg;
+    if (!at.fetches) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (at.col + c < a.vdim) S[c].load(sp + c * DP); else S[c].zero();
+    }
+    scan_batches(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
+        struct Operands { Vec<RQ> g, k, q; float v[C], beta; };
+        auto fetch = [&](uint32_t j) {                       // read one step ahead of their use
+            const uint32_t o = (b * SC_TB + j) * DP + 2 * at.lg;
+            Operands t;
             t.g.load(gs + o);
             t.k.load(ks + o);
             t.q.load(qs + o);
-            t.v = vs[b][j][col_s];
+            load_values(t.v, &vs[b][j][at.group * C]);
             t.beta = bs[b][j];
             return t;
         };
-        float* dst = out + static_cast<size_t>(t0) * a.heads * a.vdim + static_cast<size_t>(h) * a.vdim + col;
-        const size_t row_o = static_cast<size_t>(a.heads) * a.vdim;
-        uint32_t j0 = 0;
-        for (; j0 + 16 <= n; j0 += 16) {                     // sixteen tokens without a branch; lane i of a group stores token i
-            float r[16];
-            DeltaOperands<RQ> t = fetch(j0);
+        auto token = [&](const Operands& t, float* r) {      // this lane's part of o
 #pragma unroll
-            for (uint32_t u = 0; u < 16; ++u) {
-                const DeltaOperands<RQ> next = fetch(j0 + (u < 15 ? u + 1 : 15));
-                r[u] = delta_token<RQ>(S, t);
-                t = next;
+            for (int c = 0; c < C; ++c) {
+                S[c].scale(t.g);
+                S[c].axpy(t.k, t.beta * (t.v[c] - group_sum(S[c].dot(t.k))));
+                r[c] = S[c].dot(t.q);
             }
-            const float x = group_transpose_sum(r, lg);
-            if (live) dst[(j0 + lg) * row_o] = x;
-        }
+        };
+        // Two tokens at a time: what the second one reads off the state is taken from the state before the first,
+        //   S1^T (g2 k2) = S0^T (g1 g2 k2) + (k1 . g2 k2) u1,
+        // so that one chain of shuffles serves both.
+        auto pair = [&](const Operands& t1, const Operands& t2, float* r) {
+            const Vec<RQ> gk = t1.g * t1.k, g2k = t2.g * t2.k, ggk = t1.g * g2k, gq = t1.g * t1.q, gg = t1.g * t2.g, kg = t1.k * t2.g;
+            float d[2 * C + 1];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                d[2 * c] = S[c].dot(gk);
+                d[2 * c + 1] = S[c].dot(ggk);
+            }
+            d[2 * C] = t1.k.dot(g2k);
+            const float kq = t1.k.dot(t1.q);
+#pragma unroll
+            for (int w = 1; w < 16; w *= 2)
+#pragma unroll
+                for (int i = 0; i < 2 * C + 1; ++i) d[i] += __shfl_xor_sync(0xffffffffu, d[i], w);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float u1 = t1.beta * (t1.v[c] - d[2 * c]), u2 = t2.beta * (t2.v[c] - fmaf(d[2 * C], u1, d[2 * c + 1]));
+                r[c] = fmaf(kq, u1, S[c].dot(gq));
+                S[c].scale(gg);
+                S[c].axpy(kg, u1);
+                S[c].axpy(t2.k, u2);
+                r[C + c] = S[c].dot(t2.q);
+            }
+        };
+        float* dst = out + static_cast<size_t>(t0) * a.heads * a.vdim + static_cast<size_t>(h) * a.vdim;
+        const size_t row_o = static_cast<size_t>(a.heads) * a.vdim;
+        struct Sums { float r[16]; };
+        uint32_t j0 = scan_groups<Sums, Place::GROUP>(
+            n,
+            [&](uint32_t j, Sums& s) {
+                Operands t1 = fetch(j), t2 = fetch(j + 1);
+#pragma unroll
+                for (uint32_t u = 0; u < Place::GROUP; u += 2) {
+                    const Operands n1 = fetch(j + (u + 2 < Place::GROUP ? u + 2 : u)), n2 = fetch(j + (u + 3 < Place::GROUP ? u + 3 : u));
+                    pair(t1, t2, s.r + u * C);
+                    t1 = n1;
+                    t2 = n2;
+                }
+            },
+            [&](uint32_t j, Sums& s) {                           // lane i of a group stores token i / C, column i % C
+                const float x = group_transpose_sum(s.r, at.lg);
+                const uint32_t col = at.col + at.lg % C;
+                if (col < a.vdim) dst[(j + at.lg / C) * row_o + col] = x;
+            });
         for (; j0 < n; ++j0) {
-            const float r = group_sum(delta_token<RQ>(S, fetch(j0)));
-            if (lg == 0 && live) dst[j0 * row_o] = r;
+            float r[C];
+            token(fetch(j0), r);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float x = group_sum(r[c]);
+                if (at.lg == c && at.col + c < a.vdim) dst[j0 * row_o + at.col + c] = x;
+            }
         }
-        __syncthreads();
+    });
+    if (!at.fetches) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (at.col + c < a.vdim) S[c].store(sp + c * DP);
     }
-    if (live) S.store(sp);
 }
 
 // convolution + SiLU of channel `ch` (0 .. 2 qk + heads vdim) for one token; before(j): the input j tokens back
@@ -444,90 +593,96 @@ __global__ void __launch_bounds__(256) delta_decay_kernel(const float* __restric
 __device__ __forceinline__ uint32_t ssd_channels(const hf2q_ssd& a) { return a.heads * a.vdim + 2 * a.groups * a.state; }
 
 // S <- keep S + dt B x^T;  y = S^T C + d x
-template <int RQ>
-__global__ void __launch_bounds__(SC_THREADS) ssd_scan_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, const float* __restrict__ xbc,
-                                                              const float* __restrict__ dt, const float* __restrict__ la, float* __restrict__ y) {
-    constexpr uint32_t DP = 32 * RQ;
+template <int RQ, int C, int W>
+__global__ void __launch_bounds__((W + 1) * 32, 1) ssd_scan_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, const float* __restrict__ xbc,
+                                                                const float* __restrict__ dt, const float* __restrict__ la, float* __restrict__ y) {
+    using Place = ScanPlace<RQ, C, W>;
+    constexpr uint32_t DP = Place::DP;
     extern __shared__ __align__(16) float dsm[];                    // B, C: [2][SC_TB][DP] each
     float* ks = dsm;
     float* qs = dsm + 2 * SC_TB * DP;
-    __shared__ __align__(16) float vs[2][SC_TB][SC_COLS];
-    __shared__ float gk[2][SC_TB], gw[2][SC_TB];                    // decay, step size
+    __shared__ __align__(16) float vs[2][SC_TB][Place::COLS];
+    __shared__ __align__(8) float2 gs[2][SC_TB];                    // decay, step size
     pdl_trigger();
     pdl_wait();
-    const uint32_t h = blockIdx.x, slice = blockIdx.y, grp = h / (a.heads / a.groups);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = lane & 15;
-    const uint32_t col_s = warp * 2 + (lane >> 4), col0 = slice * SC_COLS, col = col0 + col_s;
-    const uint32_t n_cols = min(static_cast<uint32_t>(SC_COLS), a.vdim - col0);
-    const bool live = col < a.vdim;
+    const uint32_t h = blockIdx.x, grp = h / (a.heads / a.groups);
+    const Place at(blockIdx.y, a.vdim);
     const uint32_t channels = ssd_channels(a), inner = a.heads * a.vdim;
     // the convolution's reader has finished: the last inputs go to the state
-    for (uint32_t i = (blockIdx.y * gridDim.x + blockIdx.x) * SC_THREADS + threadIdx.x; i < channels; i += gridDim.x * gridDim.y * SC_THREADS) {
+    for (uint32_t i = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < channels; i += gridDim.x * gridDim.y * blockDim.x) {
         const uint32_t pos = *a.pos, keep = min(a.taps - 1, m);
         for (uint32_t j = 0; j < keep; ++j)
             a.conv_state[static_cast<size_t>(i) * a.taps + (pos + m - 1 - j) % a.taps] = a.proj[static_cast<size_t>(m - 1 - j) * a.ld + a.off + i];
     }
-    for (uint32_t i = threadIdx.x; i < 4 * SC_TB * DP; i += SC_THREADS) dsm[i] = 0.f;
-    for (uint32_t i = threadIdx.x; i < 2 * SC_TB * SC_COLS; i += SC_THREADS) (&vs[0][0][0])[i] = 0.f;
-    __syncthreads();
+    clear_padding(dsm, 4 * SC_TB * DP, a.state < DP);
     auto stage = [&](uint32_t t0, uint32_t b) {
         const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
         const float* row = xbc + static_cast<size_t>(t0) * channels;
         stage_rows(ks + b * SC_TB * DP, DP, row + inner + grp * a.state, channels, n, a.state);
         stage_rows(qs + b * SC_TB * DP, DP, row + inner + (a.groups + grp) * a.state, channels, n, a.state);
-        stage_rows(vs[b][0], SC_COLS, row + h * a.vdim + col0, channels, n, n_cols);
-        if (threadIdx.x < n) {
-            const size_t o = static_cast<size_t>(t0 + threadIdx.x) * a.heads + h;
-            gk[b][threadIdx.x] = expf(la[o]);
-            gw[b][threadIdx.x] = dt[o];
-        }
+        stage_rows(vs[b][0], Place::COLS, row + h * a.vdim + at.col0, channels, n, at.n_cols);
         cp_async_commit();
+        if (at.lane < n) {
+            const size_t o = static_cast<size_t>(t0 + at.lane) * a.heads + h;
+            gs[b][at.lane] = make_float2(expf(la[o]), dt[o]);
+        }
     };
-    Vec<RQ> S;
-    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + (live ? col : 0)) * DP + 2 * lg;
+    Vec<RQ> S[C];
+    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + at.col) * DP + 2 * at.lg;
     const float skip = a.d[h];
-    if (live) S.load(sp); else S.zero();
-    stage(0, 0);
-    for (uint32_t t0 = 0, b = 0; t0 < m; t0 += SC_TB, b ^= 1) {
-        if (t0 + SC_TB < m) { stage(t0 + SC_TB, b ^ 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        __syncthreads();
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
-        struct Operands { Vec<RQ> k, q; float keep, write, v; };
-        auto fetch = [&](uint32_t j) {
+    if (!at.fetches) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (at.col + c < a.vdim) S[c].load(sp + c * DP); else S[c].zero();
+    }
+    scan_batches(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
+        struct Operands { Vec<RQ> k, q; float2 g; float v[C]; };
+        auto fetch = [&](uint32_t j) {                       // read one token ahead of their use
             Operands t;
-            t.k.load(ks + (b * SC_TB + j) * DP + 2 * lg);
-            t.q.load(qs + (b * SC_TB + j) * DP + 2 * lg);
-            t.keep = gk[b][j];
-            t.write = gw[b][j];
-            t.v = vs[b][j][col_s];
+            t.k.load(ks + (b * SC_TB + j) * DP + 2 * at.lg);
+            t.q.load(qs + (b * SC_TB + j) * DP + 2 * at.lg);
+            t.g = gs[b][j];
+            load_values(t.v, &vs[b][j][at.group * C]);
             return t;
         };
-        auto finish = [&](uint32_t j, float s) {
-            if (live) y[static_cast<size_t>(t0 + j) * inner + static_cast<size_t>(h) * a.vdim + col] = s + skip * vs[b][j][col_s];
-        };
-        uint32_t j0 = 0;
-        for (; j0 + 16 <= n; j0 += 16) {                     // sixteen tokens without a branch; lane i of a group finishes token i
-            float r[16];
-            Operands t = fetch(j0);
+        auto token = [&](const Operands& t, float* r) {
 #pragma unroll
-            for (uint32_t u = 0; u < 16; ++u) {
-                const Operands next = fetch(j0 + (u < 15 ? u + 1 : 15));
-                S.decay_axpy(t.keep, t.k, t.write * t.v);
-                r[u] = S.dot(t.q);
-                t = next;
+            for (int c = 0; c < C; ++c) {
+                S[c].decay_axpy(t.g.x, t.k, t.g.y * t.v[c]);
+                r[c] = S[c].dot(t.q);
             }
-            finish(j0 + lg, group_transpose_sum(r, lg));
-        }
+        };
+        auto finish = [&](uint32_t j, uint32_t c, float s) {     // column c of the group
+            if (at.col + c < a.vdim) y[static_cast<size_t>(t0 + j) * inner + static_cast<size_t>(h) * a.vdim + at.col + c] = s + skip * vs[b][j][at.group * C + c];
+        };
+        struct Sums { float r[16]; };
+        uint32_t j0 = scan_groups<Sums, Place::GROUP>(
+            n,
+            [&](uint32_t j, Sums& s) {
+                Operands t = fetch(j);
+#pragma unroll
+                for (uint32_t u = 0; u < Place::GROUP; ++u) {
+                    const Operands next = fetch(j + (u + 1 < Place::GROUP ? u + 1 : u));
+                    token(t, s.r + u * C);
+                    t = next;
+                }
+            },
+            [&](uint32_t j, Sums& s) { finish(j + at.lg / C, at.lg % C, group_transpose_sum(s.r, at.lg)); });    // lane i: token i / C, column i % C
         for (; j0 < n; ++j0) {
-            const Operands t = fetch(j0);
-            S.decay_axpy(t.keep, t.k, t.write * t.v);
-            const float r = group_sum(S.dot(t.q));
-            if (lg == 0) finish(j0, r);
+            float r[C];
+            token(fetch(j0), r);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float x = group_sum(r[c]);
+                if (at.lg == c) finish(j0, c, x);
+            }
         }
-        __syncthreads();
+    });
+    if (!at.fetches) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (at.col + c < a.vdim) S[c].store(sp + c * DP);
     }
-    if (live) S.store(sp);
 }
 
 __device__ __forceinline__ void ssd_gates(const hf2q_ssd& a, uint32_t h, float raw, float& dt, float& la) {
@@ -608,12 +763,14 @@ bool ssd_ok(const hf2q_ssd* a) {
     return a && a->proj && a->conv && a->conv_bias && a->dt_bias && a->a_log && a->d && a->conv_state && a->s && a->pos && a->heads && a->groups &&
            a->heads % a->groups == 0 && a->state && a->state <= 256 && a->vdim && a->taps;
 }
-template <int RQ>
-cudaError_t launch_ssd_scan(const hf2q_ssd& a, uint32_t m, const float* xbc, const float* dt, const float* la, float* y, cudaStream_t st) {
+template <int RQ, int C, int W>
+cudaError_t launch_ssd_scan(const hf2q_ssd& a, uint32_t m, const float* xbc, const float* dt, const float* la, float* y, int sms, cudaStream_t st) {
     static PerDeviceFlag flag;
-    const size_t smem = 4ull * SC_TB * 32 * RQ * sizeof(float);
-    if (const cudaError_t e = ensure_max_dynamic_smem(ssd_scan_kernel<RQ>, static_cast<int>(smem), flag); e != cudaSuccess) return e;
-    return launch_pdl(ssd_scan_kernel<RQ>, dim3(a.heads, (a.vdim + SC_COLS - 1) / SC_COLS), dim3(SC_THREADS), smem, st, a, m, xbc, dt, la, y);
+    constexpr size_t need = 4ull * SC_TB * 32 * RQ * sizeof(float);
+    constexpr uint32_t cols = ScanPlace<RQ, C, W>::COLS;
+    const dim3 grid(a.heads, (a.vdim + cols - 1) / cols);
+    if (const cudaError_t e = ensure_max_dynamic_smem(ssd_scan_kernel<RQ, C, W>, SCAN_MAX, flag); e != cudaSuccess) return e;
+    return launch_pdl(ssd_scan_kernel<RQ, C, W>, grid, dim3((W + 1) * 32), scan_smem(need, grid, sms), st, a, m, xbc, dt, la, y);
 }
 
 bool delta_ok(const hf2q_delta* a) {
@@ -621,20 +778,34 @@ bool delta_ok(const hf2q_delta* a) {
            a->heads && a->kv_heads && a->heads % a->kv_heads == 0 && a->dim && a->dim <= 256 && a->vdim && a->taps && a->a_rank_ld % 8 == 0 &&
            a->g_rank_ld % 8 == 0 && a->a_rank_ld && a->g_rank_ld;
 }
-template <int RQ>
-cudaError_t launch_scan(const hf2q_delta& a, uint32_t m, const float* qkv, const float* beta, const float* g, float* out, cudaStream_t st) {
+template <int RQ, int C, int W, int PER_SM>
+cudaError_t launch_scan_as(const hf2q_delta& a, uint32_t m, const float* qkv, const float* beta, const float* g, float* out, dim3 grid, int sms, cudaStream_t st) {
     static PerDeviceFlag flag;
-    const size_t smem = 6ull * SC_TB * 32 * RQ * sizeof(float);
-    if (const cudaError_t e = ensure_max_dynamic_smem(delta_scan_kernel<RQ>, static_cast<int>(smem), flag); e != cudaSuccess) return e;
-    return launch_pdl(delta_scan_kernel<RQ>, dim3(a.heads, (a.vdim + SC_COLS - 1) / SC_COLS), dim3(SC_THREADS), smem, st, a, m, qkv, beta, g, out);
+    constexpr size_t need = 6ull * SC_TB * 32 * RQ * sizeof(float);
+    if (const cudaError_t e = ensure_max_dynamic_smem(delta_scan_kernel<RQ, C, W, PER_SM>, SCAN_MAX, flag); e != cudaSuccess) return e;
+    return launch_pdl(delta_scan_kernel<RQ, C, W, PER_SM>, grid, dim3((W + 1) * 32), scan_smem(need, grid, sms), st, a, m, qkv, beta, g, out);
+}
+// More CTAs than SMs: two to an SM where the batches of both fit (dim up to 128), which costs a CTA alone 6 % (200 registers)
+template <int RQ>
+cudaError_t launch_scan(const hf2q_delta& a, uint32_t m, const float* qkv, const float* beta, const float* g, float* out, int sms, cudaStream_t st) {
+    constexpr uint32_t cols = ScanPlace<RQ, 2, 4>::COLS;
+    const dim3 grid(a.heads, (a.vdim + cols - 1) / cols);
+    if (RQ <= 4 && static_cast<uint64_t>(grid.x) * grid.y > static_cast<uint64_t>(sms)) return launch_scan_as<RQ, 2, 4, RQ <= 4 ? 2 : 1>(a, m, qkv, beta, g, out, grid, sms, st);
+    return launch_scan_as<RQ, 2, 4, 1>(a, m, qkv, beta, g, out, grid, sms, st);
 }
 
-template <int RQ>
-cudaError_t launch_mlstm(const hf2q_mlstm& a, uint32_t m, float* out, cudaStream_t st) {
+template <int RQ, int C>
+cudaError_t launch_mlstm_as(const hf2q_mlstm& a, uint32_t m, float* out, int sms, cudaStream_t st) {
     static PerDeviceFlag flag;
-    const size_t smem = 4ull * SC_TB * 32 * RQ * sizeof(float);
-    if (const cudaError_t e = ensure_max_dynamic_smem(mlstm_kernel<RQ>, static_cast<int>(smem), flag); e != cudaSuccess) return e;
-    return launch_pdl(mlstm_kernel<RQ>, dim3(a.heads, (a.vdim + SC_COLS - 1) / SC_COLS), dim3(SC_THREADS), smem, st, a, m, out);
+    constexpr size_t need = 4ull * SC_TB * 32 * RQ * sizeof(float);
+    const dim3 grid(a.heads, (a.vdim + SC_COLS - 1) / SC_COLS);
+    if (const cudaError_t e = ensure_max_dynamic_smem(mlstm_kernel<RQ, C>, SCAN_MAX, flag); e != cudaSuccess) return e;
+    return launch_pdl(mlstm_kernel<RQ, C>, grid, dim3((8 / C + 1) * 32), m == 1 ? need : scan_smem(need, grid, sms), st, a, m, out);
+}
+// one token: every warp reads as little of the state as it can
+template <int RQ>
+cudaError_t launch_mlstm(const hf2q_mlstm& a, uint32_t m, float* out, int sms, cudaStream_t st) {
+    return m == 1 ? launch_mlstm_as<RQ, 1>(a, m, out, sms, st) : launch_mlstm_as<RQ, 2>(a, m, out, sms, st);
 }
 
 #define HF2Q_RQ_CASES(F) F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8)
@@ -656,7 +827,7 @@ HF2Q_API int32_t hf2q_cuda_mlstm(hf2q_ctx* ctx, void* stream, const hf2q_mlstm* 
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaErrorInvalidValue;
     switch ((a->dim + 31) / 32) {
-#define F(RQ) case RQ: e = launch_mlstm<RQ>(*a, m, out, st); break;
+#define F(RQ) case RQ: e = launch_mlstm<RQ>(*a, m, out, ctx_sm_count(ctx), st); break;
         HF2Q_RQ_CASES(F)
 #undef F
         default: break;
@@ -712,7 +883,7 @@ HF2Q_API int32_t hf2q_cuda_delta_scan(hf2q_ctx* ctx, void* stream, const hf2q_de
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaErrorInvalidValue;
     switch ((a->dim + 31) / 32) {
-#define F(RQ) case RQ: e = launch_scan<RQ>(*a, m, qkv, beta, g, out, st); break;
+#define F(RQ) case RQ: e = launch_scan<RQ>(*a, m, qkv, beta, g, out, ctx_sm_count(ctx), st); break;
         HF2Q_RQ_CASES(F)
 #undef F
         default: break;
@@ -747,7 +918,7 @@ HF2Q_API int32_t hf2q_cuda_ssd_scan(hf2q_ctx* ctx, void* stream, const hf2q_ssd*
     if (m == 0) return HF2Q_OK;
     cudaError_t e = cudaErrorInvalidValue;
     switch ((a->state + 31) / 32) {
-#define F(RQ) case RQ: e = launch_ssd_scan<RQ>(*a, m, xbc, dt, la, y, static_cast<cudaStream_t>(stream)); break;
+#define F(RQ) case RQ: e = launch_ssd_scan<RQ, 2, 8>(*a, m, xbc, dt, la, y, ctx_sm_count(ctx), static_cast<cudaStream_t>(stream)); break;
         HF2Q_RQ_CASES(F)
 #undef F
         default: break;
