@@ -3,13 +3,14 @@
 // plain rows of keys and values, with a part of every key shared by the heads (expanded latents).
 //
 //   append    prefill: normalised queries to a buffer, normalised keys and values to the cache
-//   prefill   bf16 cache: tiles of 64 queries x 64 keys on the tensor cores (f32 scores, softmax and accumulators, bf16
-//             product operands); f32 cache: one warp per query in f32
+//   prefill   bf16 cache: tiles on the tensor cores (f32 scores, softmax and accumulators, bf16 product operands), of 128
+//             queries on tcgen05 where a key has 65..192 and a value up to 128 elements; f32 cache: one warp per query in f32
 //   decode    one launch: norm, append, window split over CTAs, merge by the CTA that arrives last
 #include <math_constants.h>
 
 #include "mma_sync.cuh"
 #include "seq_common.cuh"
+#include "tc_common.cuh"
 
 namespace hf2q {
 namespace {
@@ -345,7 +346,289 @@ __global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_co
         for (uint32_t i = a.heads * a.vdim + lane; i < ldo; i += 32) out[static_cast<size_t>(t) * ldo + i] = from_f32<OUT>(0.f);
 }
 
-// ---------------------------------------------------------------- prefill, bf16 cache, tensor cores
+// ---------------------------------------------------------------- prefill, bf16 cache, tcgen05
+// One CTA owns 128 queries of one head and walks the keys from the first one that its first query sees, 64 at a time:
+//
+//   warps 4-7   copy keys and values (16 bytes a time, asynchronously) to shared memory with the 128-byte swizzle, two blocks
+//               deep; K is the K-major B operand of the scores, V, in the same layout, the MN-major one of the output.
+//   warp 8      one lane issues the products: the scores of the next block before the output of this one.
+//   warps 0-3   softmax, a thread to a query: scores from tensor memory are scaled, biased, masked and put back, then read
+//               again for the exponentials (64 of them would not fit the registers beside the rest); P takes their place.
+//               The output rows of a warp are rescaled wherever one's running maximum grew: with the true maximum the largest
+//               weight is 1, which bf16 holds exactly (an older one within 2^8 was no faster and doubled the error of peaked rows).
+//
+// 256 tensor-memory columns (S 2 x 64, O 128).  Two CTAs per SM with keys of up to 128 elements, one with 192.  It is bound by
+// the latency of a block's chain (scores, maximum, exponentials, output).  2048 queries x 16 heads of 128 with 2048 keys each
+// take 171 us (the warp-level kernel below took 397), with keys of 192 elements 233 us (519).
+constexpr uint32_t WT_Q = 128, WT_K = 64, WT_V = 128, WT_THREADS = 288, WT_COLS = 256, WT_O = 128, WT_PANEL = WT_K * 128;
+constexpr uint32_t wt_smem(uint32_t dk) { return WT_Q * dk * 2 + 2 * WT_K * dk * 2 + 2 * WT_K * WT_V * 2 + 1024; }
+
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float lg2(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// 16-byte chunk c of a row, in panels of `rows` rows x 64 elements
+__device__ __forceinline__ uint32_t wt_chunk(uint32_t rows, uint32_t row, uint32_t c) { return (c >> 3) * rows * 128 + row * 128 + (((c & 7) ^ (row & 7)) << 4); }
+
+template <int DK, typename OUT, bool PLAIN>
+__global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_tc_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m,
+                                                                                          const __nv_bfloat16* __restrict__ q, const float* __restrict__ gate,
+                                                                                          uint32_t ldg, OUT* __restrict__ out, uint32_t ldo, uint32_t* status) {
+    extern __shared__ __align__(16) uint8_t wt_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    constexpr uint32_t Q_BYTES = WT_Q * DK * 2, K_BYTES = WT_K * DK * 2, V_BYTES = WT_K * WT_V * 2;
+    uint8_t *qs = smem, *ks = smem + Q_BYTES, *vs = ks + 2 * K_BYTES;
+    __shared__ uint64_t k_full[2], v_full[2], s_full[2], p_full[2], o_done[2];
+    __shared__ uint32_t tmem_slot;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t h = blockIdx.y, t0 = (gridDim.x - 1 - blockIdx.x) * WT_Q;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&k_full[i], 4);
+            mbar_init(&v_full[i], 4);
+            mbar_init(&s_full[i], 1);
+            mbar_init(&p_full[i], 4);
+            mbar_init(&o_done[i], 1);
+        }
+        mbar_fence_init();
+    }
+    if (warp == 8) { tc::tmem_alloc(&tmem_slot, WT_COLS); tc::tmem_relinquish(); }
+    __syncthreads();
+    pdl_trigger();                                             // (dependents may claim tensor memory too: not before this CTA has its own)
+    pdl_wait();
+    const uint32_t pos0 = *a.pos;
+    const KeyRows<__nv_bfloat16, PLAIN> rows(a, h / (a.heads / a.kv_heads), pos0);
+    const uint32_t dq = rows.dp + rows.sp, dvp = pad8(a.vdim), nk = (dq + 15) / 16;
+    const uint32_t q_lo = pos0 + t0, q_hi = pos0 + min(t0 + WT_Q, m) - 1;
+    const uint32_t j0 = q_lo + 1 > a.window ? q_lo + 1 - a.window : 0u, nb = (q_hi - j0) / WT_K + 1;
+    if (dq < DK || dvp < WT_V) {                               // elements past dim / vdim must be finite zeros
+        for (uint32_t i = threadIdx.x; i < (2 * K_BYTES + 2 * V_BYTES) / 16; i += WT_THREADS) reinterpret_cast<uint4*>(ks)[i] = make_uint4(0, 0, 0, 0);
+    }
+    const bool wide_q = reinterpret_cast<uintptr_t>(q) % 16 == 0;          // rows are whole 16-byte groups
+    for (uint32_t i = threadIdx.x; i < WT_Q * (DK / 8); i += WT_THREADS) {
+        const uint32_t r = i / (DK / 8), c = i % (DK / 8);
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (t0 + r < m && 8 * c < dq) {
+            const __nv_bfloat16* src = q + (static_cast<size_t>(t0 + r) * a.heads + h) * dq + 8 * c;
+            if (wide_q) {
+                v = *reinterpret_cast<const uint4*>(src);
+            } else {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
+                v = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+        *reinterpret_cast<uint4*>(qs + wt_chunk(WT_Q, r, c)) = v;
+    }
+    proxy_fence();
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp >= 4 && warp < 8) {
+        const uint32_t tid = threadIdx.x - 128, c0 = tid & 7, row0 = tid >> 3, ck = dq / 8, cv = dvp / 8, cd = rows.dp / 8;
+        bool ok = true;
+        // iteration j starts the copies of block j and hands over those of block j - 1
+        for (uint32_t j = 0; j <= nb; ++j) {
+            const uint32_t b = j & 1, par = ((j >> 1) - 1) & 1;
+            if (j < nb) {
+                if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&s_full[b], par, status));        // S(j-2) is there: its K block is free
+                if (!ok) break;
+#pragma unroll
+                for (uint32_t i = 0; i < WT_K / 16; ++i) {
+                    const uint32_t r = row0 + 16 * i, key = min(j0 + j * WT_K + r, q_hi);             // keys past the last visible one repeat it
+                    const __nv_bfloat16* src = rows.key(key);
+                    for (uint32_t c = c0; c < ck; c += 8) {
+                        const __nv_bfloat16* from = !PLAIN || c < cd ? src + 8 * c : rows.shared_key(key) + 8 * (c - cd);
+                        cp_async16(ks + b * K_BYTES + wt_chunk(WT_K, r, c), from);
+                    }
+                }
+            }
+            cp_async_commit();
+            if (j > 0) {
+                cp_async_wait<2>();                            // all but the copies of V(j-1) and K(j)
+                proxy_fence();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&k_full[b ^ 1]);
+                cp_async_wait<1>();
+                proxy_fence();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&v_full[b ^ 1]);
+            }
+            if (j < nb) {
+                if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&o_done[b], par, status));        // the output of j-2 is in: its V block is free
+                if (!ok) break;
+#pragma unroll
+                for (uint32_t i = 0; i < WT_K / 16; ++i) {
+                    const uint32_t r = row0 + 16 * i;
+                    const __nv_bfloat16* src = rows.value(min(j0 + j * WT_K + r, q_hi));
+                    for (uint32_t c = c0; c < cv; c += 8) cp_async16(vs + b * V_BYTES + wt_chunk(WT_K, r, c), src + 8 * c);
+                }
+            }
+            cp_async_commit();
+        }
+        cp_async_wait<0>();
+    } else if (warp == 8) {
+        if (lane == 0) {
+            // D f32, A and B bf16, M = 128; S: both K-major, N = 64; O: B MN-major, N = 128
+            constexpr uint32_t ID = (1u << 4) | (1u << 7) | (1u << 10) | ((WT_Q >> 4) << 24), ID_S = ID | ((WT_K >> 3) << 17), ID_O = ID | (1u << 16) | ((WT_V >> 3) << 17);
+            bool ok = true;
+            auto scores = [&](uint32_t j) {
+                const uint32_t b = j & 1;
+                ok = mbar_wait_bounded(&k_full[b], (j >> 1) & 1, status);
+                if (ok && j >= 2) ok = mbar_wait_bounded(&o_done[b], ((j >> 1) - 1) & 1, status);   // P(j-2) is read: S(j) takes its place
+                if (!ok) return;
+                tc::tc_fence_after();
+#pragma unroll
+                for (uint32_t kk = 0; kk < DK / 16; ++kk)
+                    if (kk < nk)
+                        tc::umma_ss(tmem + b * WT_K, tc::smem_desc_sw128(smem_u32(qs + (kk >> 2) * (WT_Q * 128))) + 2 * (kk & 3),
+                                    tc::smem_desc_sw128(smem_u32(ks + b * K_BYTES + (kk >> 2) * WT_PANEL)) + 2 * (kk & 3), ID_S, kk ? 1u : 0u);
+                tc::tc_commit(&s_full[b]);
+            };
+            scores(0);
+            for (uint32_t j = 0; j < nb && ok; ++j) {
+                const uint32_t b = j & 1;
+                if (j + 1 < nb) scores(j + 1);
+                if (ok) ok = mbar_wait_bounded(&v_full[b], (j >> 1) & 1, status);
+                if (ok) ok = mbar_wait_bounded(&p_full[b], (j >> 1) & 1, status);
+                if (!ok) break;
+                tc::tc_fence_after();
+#pragma unroll
+                for (uint32_t kk = 0; kk < WT_K / 16; ++kk)
+                    tc::umma_ts(tmem + WT_O, tmem + b * WT_K + 8 * kk, tc::smem_desc_mn_sw128(smem_u32(vs + b * V_BYTES), WT_PANEL) + kk * (16 * 128 >> 4), ID_O, (j | kk) ? 1u : 0u);
+                tc::tc_commit(&o_done[b]);
+            }
+        }
+    } else {
+        const uint32_t t = t0 + threadIdx.x, at = tmem + ((warp * 32u) << 16), qp = pos0 + t;
+        const bool live = t < m, bias = a.r1 != nullptr;       // (rows past the end compute on zeros and are not stored)
+        const float r1 = bias ? a.r1[h] : 0.f, r2 = bias ? a.r2[h] : 0.f, scale = a.scale * 1.4426950408889634f;      // scores in units of log2
+        float mx = -CUDART_INF_F, sum[2] = {0.f, 0.f};
+        bool ok = true;
+        for (uint32_t j = 0; j < nb; ++j) {
+            const uint32_t b = j & 1, key0 = j0 + j * WT_K;
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&s_full[b], (j >> 1) & 1, status));
+            if (!ok) break;
+            tc::tc_fence_after();
+            // some query of the tile does not see all of the block
+            const bool edge = key0 + WT_K - 1 > q_lo || key0 + a.window <= pos0 + t0 + WT_Q - 1;
+            float top[2] = {-CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+            for (uint32_t half = 0; half < 2; ++half) {
+                uint32_t r[32];
+                tc::tmem_ld32(at + b * WT_K + 32 * half, r);
+                tc::tmem_wait_ld();
+                const uint32_t d0 = qp - key0 - 32 * half;     // distance to the first key; wraps for keys after the query
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    float v = __uint_as_float(r[i]) * scale;
+                    if (bias) v -= r1 * lg2(fmaf(r2, static_cast<float>(d0 - i), 1.0f));
+                    r[i] = __float_as_uint(v);
+                }
+                if (edge) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) r[i] = d0 - i < a.window ? r[i] : __float_as_uint(-CUDART_INF_F);
+                }
+#pragma unroll
+                for (int i = 0; i < 32; ++i) top[i & 1] = fmaxf(top[i & 1], __uint_as_float(r[i]));
+                tc::tmem_st32(at + b * WT_K + 32 * half, r);
+            }
+            tc::tmem_wait_st();
+            const float bm = fmaxf(top[0], top[1]);
+            const bool grew = bm > mx;
+            if (j == 0) {
+                mx = bm;
+            } else if (__any_sync(0xffffffffu, grew)) {
+                const float to = grew ? bm : mx, corr = grew ? ex2(mx - to) : 1.0f;
+                mx = to;
+                sum[0] *= corr;
+                sum[1] *= corr;
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(&o_done[b ^ 1], ((j - 1) >> 1) & 1, status));
+                if (!ok) break;
+                tc::tc_fence_after();
+#pragma unroll 1
+                for (uint32_t c = 0; c < WT_V; c += 32) {
+                    uint32_t o[32];
+                    tc::tmem_ld32(at + WT_O + c, o);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                    tc::tmem_st32(at + WT_O + c, o);
+                }
+            }
+            const float nm = mx == -CUDART_INF_F ? 0.f : mx;   // nothing visible yet: every weight is 2^-inf = 0
+#pragma unroll
+            for (uint32_t c = 0; c < WT_K / 16; ++c) {
+                uint32_t r[16], p[8];
+                tc::tmem_ld16(at + b * WT_K + 16 * c, r);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float x = ex2(__uint_as_float(r[2 * i]) - nm), y = ex2(__uint_as_float(r[2 * i + 1]) - nm);
+                    sum[0] += x;
+                    sum[1] += y;
+                    p[i] = pack_bf16(x, y);
+                }
+                tc::tmem_st8(at + b * WT_K + 8 * c, p);        // over scores that have been read
+            }
+            tc::tmem_wait_st();
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[b]);
+        }
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&o_done[(nb - 1) & 1], ((nb - 1) >> 1) & 1, status));
+        if (ok) {
+            tc::tc_fence_after();
+            const float inv = 1.0f / (sum[0] + sum[1]);
+            OUT* dst = out + static_cast<size_t>(live ? t : 0) * ldo + h * a.vdim;
+            const float* gr = gate ? gate + static_cast<size_t>(live ? t : 0) * ldg + h * a.vdim : nullptr;
+            const bool wide = (reinterpret_cast<uintptr_t>(out) | ldo * sizeof(OUT) | a.vdim * sizeof(OUT)) % 16 == 0 &&
+                              (!gate || (reinterpret_cast<uintptr_t>(gate) | ldg * sizeof(float) | a.vdim * sizeof(float)) % 16 == 0);
+#pragma unroll 1
+            for (uint32_t c = 0; c < a.vdim; c += 16) {
+                uint32_t o[16];
+                tc::tmem_ld16(at + WT_O + c, o);
+                tc::tmem_wait_ld();
+                if (!live) continue;
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(o[i]) * inv;
+                if (wide && c + 16 <= a.vdim) {
+                    if (gr) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 g = *reinterpret_cast<const float4*>(gr + c + 4 * i);
+                            v[4 * i] *= sigmoidf(g.x);
+                            v[4 * i + 1] *= sigmoidf(g.y);
+                            v[4 * i + 2] *= sigmoidf(g.z);
+                            v[4 * i + 3] *= sigmoidf(g.w);
+                        }
+                    }
+                    if constexpr (sizeof(OUT) == 4) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + c + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            *reinterpret_cast<uint4*>(dst + c + 8 * i) = make_uint4(pack_bf16(v[8 * i], v[8 * i + 1]), pack_bf16(v[8 * i + 2], v[8 * i + 3]),
+                                                                                    pack_bf16(v[8 * i + 4], v[8 * i + 5]), pack_bf16(v[8 * i + 6], v[8 * i + 7]));
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (c + i < a.vdim) dst[c + i] = from_f32<OUT>(gr ? v[i] * sigmoidf(gr[c + i]) : v[i]);
+                }
+            }
+            if (live && h == a.heads - 1)
+                for (uint32_t i = a.heads * a.vdim; i < ldo; ++i) out[static_cast<size_t>(t) * ldo + i] = from_f32<OUT>(0.f);
+        }
+        tc::tc_fence_before();
+    }
+    __syncthreads();
+    if (warp == 8) { tc::tc_fence_after(); tc::tmem_dealloc(tmem, WT_COLS); }
+}
+
+// ---------------------------------------------------------------- prefill, bf16 cache, other sizes: warp-level products
 constexpr int WP_WARPS = 4, WP_Q = 16 * WP_WARPS, WP_K = 64;
 
 // grid (query tiles, heads); DK >= dim + shared_dim, DV >= vdim.  Keys are walked from the first one the tile's first
@@ -570,17 +853,27 @@ cudaError_t launch_prefill_dm(const hf2q_window_attn& a, uint32_t m, const void*
     return launch_pdl(window_prefill_mma_kernel<DK, DV, OUT, PLAIN>, dim3((m + WP_Q - 1) / WP_Q, a.heads), dim3(WP_WARPS * 32), smem, st, a, m,
                       static_cast<const __nv_bfloat16*>(q), gate, ldg, static_cast<OUT*>(out), ldo);
 }
+template <int DK, typename OUT, bool PLAIN>
+cudaError_t launch_prefill_tc(const hf2q_window_attn& a, uint32_t m, const void* q, const float* gate, uint32_t ldg, void* out, uint32_t ldo, uint32_t* status,
+                              cudaStream_t st) {
+    static PerDeviceFlag flag;
+    constexpr uint32_t smem = wt_smem(DK);
+    if (const cudaError_t e = ensure_max_dynamic_smem(window_prefill_tc_kernel<DK, OUT, PLAIN>, static_cast<int>(smem), flag); e != cudaSuccess) return e;
+    return launch_pdl(window_prefill_tc_kernel<DK, OUT, PLAIN>, dim3((m + WT_Q - 1) / WT_Q, a.heads), dim3(WT_THREADS), smem, st, a, m,
+                      static_cast<const __nv_bfloat16*>(q), gate, ldg, static_cast<OUT*>(out), ldo, status);
+}
 template <typename OUT>
-cudaError_t launch_prefill_mma(const hf2q_window_attn& a, uint32_t m, const void* q, const float* gate, uint32_t ldg, void* out, uint32_t ldo, cudaStream_t st) {
+cudaError_t launch_prefill_mma(const hf2q_window_attn& a, uint32_t m, const void* q, const float* gate, uint32_t ldg, void* out, uint32_t ldo, uint32_t* status,
+                               cudaStream_t st) {
     const uint32_t k = pad8(a.dim) + pad8(a.shared_dim), v = a.vdim;
     if (a.linear) {
         if (k <= 64 && v <= 64) return launch_prefill_dm<64, 64, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
-        if (k <= 128 && v <= 128) return launch_prefill_dm<128, 128, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
-        if (k <= 192 && v <= 128) return launch_prefill_dm<192, 128, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
+        if (k <= 128 && v <= 128) return launch_prefill_tc<128, OUT, true>(a, m, q, gate, ldg, out, ldo, status, st);
+        if (k <= 192 && v <= 128) return launch_prefill_tc<192, OUT, true>(a, m, q, gate, ldg, out, ldo, status, st);
         return launch_prefill_dm<QK_MAX, 256, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
     }
     if (k <= 64 && v <= 64) return launch_prefill_dm<64, 64, OUT, false>(a, m, q, gate, ldg, out, ldo, st);
-    if (k <= 128 && v <= 128) return launch_prefill_dm<128, 128, OUT, false>(a, m, q, gate, ldg, out, ldo, st);
+    if (k <= 128 && v <= 128) return launch_prefill_tc<128, OUT, false>(a, m, q, gate, ldg, out, ldo, status, st);
     return launch_prefill_dm<256, 256, OUT, false>(a, m, q, gate, ldg, out, ldo, st);
 }
 
@@ -638,9 +931,9 @@ HF2Q_API int32_t hf2q_cuda_window_attn_prefill(hf2q_ctx* ctx, void* stream, cons
         if (out_dtype == HF2Q_DT_F32)
             e = a->linear ? launch_prefill_f32<float, float, true>(*a, m, q, gate, ldg, out, ldo, st) : launch_prefill_f32<float, float, false>(*a, m, q, gate, ldg, out, ldo, st);
     } else if (out_dtype == HF2Q_DT_BF16) {
-        e = launch_prefill_mma<__nv_bfloat16>(*a, m, q, gate, ldg, out, ldo, st);
+        e = launch_prefill_mma<__nv_bfloat16>(*a, m, q, gate, ldg, out, ldo, ctx_status_word(ctx), st);
     } else if (out_dtype == HF2Q_DT_F32) {
-        e = launch_prefill_mma<float>(*a, m, q, gate, ldg, out, ldo, st);
+        e = launch_prefill_mma<float>(*a, m, q, gate, ldg, out, ldo, ctx_status_word(ctx), st);
     }
     return ctx_cuda_result(ctx, e, "window_attn_prefill", 1);
 }
