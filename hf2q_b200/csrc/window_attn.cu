@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_co
 //
 // 256 tensor-memory columns (S 2 x 64, O 128).  Two CTAs per SM with keys of up to 128 elements, one with 192.  It is bound by
 // the latency of a block's chain (scores, maximum, exponentials, output).  2048 queries x 16 heads of 128 with 2048 keys each
-// take 171 us (the warp-level kernel below took 397), with keys of 192 elements 233 us (519).
+// take 168 us (the warp-level kernel below took 397), with keys of 192 elements 229 us (519).
 constexpr uint32_t WT_Q = 128, WT_K = 64, WT_V = 128, WT_THREADS = 288, WT_COLS = 256, WT_O = 128, WT_PANEL = WT_K * 128;
 constexpr uint32_t wt_smem(uint32_t dk) { return WT_Q * dk * 2 + 2 * WT_K * dk * 2 + 2 * WT_K * WT_V * 2 + 1024; }
 
@@ -520,10 +520,11 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
                 tc::tmem_wait_ld();
                 const uint32_t d0 = qp - key0 - 32 * half;     // distance to the first key; wraps for keys after the query
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    float v = __uint_as_float(r[i]) * scale;
-                    if (bias) v -= r1 * lg2(fmaf(r2, static_cast<float>(d0 - i), 1.0f));
-                    r[i] = __float_as_uint(v);
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
+                if (bias) {
+                    const float d0f = static_cast<float>(static_cast<int>(d0));        // (whole numbers; what is hidden may become NaN here)
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) - r1 * lg2(fmaf(r2, d0f - i, 1.0f)));
                 }
                 if (edge) {
 #pragma unroll
