@@ -40,7 +40,10 @@ constexpr uint32_t HD = 128, ROWS = 128, BP = 64;                  // head dim, 
 constexpr uint32_t Q_BYTES = ROWS * HD * 2, KV_BYTES = BP * HD * 2, PANEL = BP * 128;
 constexpr uint32_t AP_SMEM = Q_BYTES + 4 * KV_BYTES + 1024;        // Q, two K and two V blocks, alignment
 constexpr uint32_t AP_THREADS = 288, COLS = 256, COL_O = 128;
-constexpr uint32_t SLOTS = 4;                                      // scales of a block: written up to three blocks ahead of their use
+// Scales of a block have a barrier per slot.  They are written up to two blocks ahead of the softmax, and no phase of sc_full
+// passes its waiter: slot j % 4 is written next for block j + 4, after s_full of j + 2, which follows o_done of j, which follows
+// the P(j) of every softmax warp.  (k_full, two deep, can run a phase ahead of the softmax: K(j + 2) waits for S(j) alone.)
+constexpr uint32_t SLOTS = 4;
 constexpr float LAZY_LOG2 = 3.0f, LAZY_VMAX = 16.0f;
 
 __device__ __forceinline__ float exp2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
     uint8_t *qs = smem, *ks = smem + Q_BYTES, *vs = ks + 2 * KV_BYTES;
     __shared__ __align__(16) float s_ks[SLOTS][BP], s_vs[SLOTS][BP];
     __shared__ float s_vmax[SLOTS][2];
-    __shared__ uint64_t k_full[2], v_full[2], s_full[2], p_full[2], o_done[2];
+    __shared__ uint64_t k_full[2], v_full[2], s_full[2], p_full[2], o_done[2], sc_full[SLOTS];
     __shared__ uint32_t tmem_slot;
     constexpr uint32_t TOK = ROWS / G;
     const uint32_t kvh = blockIdx.x % n_kv, tok0 = ((gridDim.x - 1 - blockIdx.x) / n_kv) * TOK;
@@ -97,6 +100,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
             mbar_init(&p_full[i], 4);
             mbar_init(&o_done[i], 1);
         }
+        for (uint32_t i = 0; i < SLOTS; ++i) mbar_init(&sc_full[i], 4);
         mbar_fence_init();
     }
     if (warp == 8) { tmem_alloc(&tmem_slot, COLS); tmem_relinquish(); }
@@ -146,7 +150,10 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
             }
             proxy_fence();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&k_full[b]);
+            if (lane == 0) {
+                mbar_arrive(&sc_full[slot]);
+                mbar_arrive(&k_full[b]);
+            }
             if (j + 1 < nb) {
                 load(kc, j + 1, kq);
                 sc = __ldg(scale + min((j + 1) * BP + (tid & 63), last));
@@ -200,9 +207,8 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
         bool ok = true;
         for (uint32_t j = 0; j < nb; ++j) {
             const uint32_t b = j & 1, slot = j % SLOTS;
-            // the scales come with the K block: s_full follows it
             ok = mbar_wait_bounded(&s_full[b], (j >> 1) & 1, status);
-            if (ok) ok = mbar_wait_bounded(&k_full[b], (j >> 1) & 1, status);
+            if (ok) ok = mbar_wait_bounded(&sc_full[slot], (j / SLOTS) & 1, status);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();

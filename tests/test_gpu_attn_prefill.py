@@ -51,3 +51,22 @@ def test_prompt_attention_matches_softmax(gpu_ctx, group, n_kv, pos0, m, k_scale
     bound = 2 ** -11 * (1 + spread) + (2 ** -9 if dtype == torch.bfloat16 else 0)
     err = (out.double() - want).norm() / want.norm()
     assert err < bound, (err.item(), bound)
+
+
+def attend(ctx, qkv, codes, scales, S, m, nq, n_kv, pos0, out):
+    kv = decoder._KvCache(codes[0].data_ptr(), scales[0].data_ptr(), codes[1].data_ptr(), scales[1].data_ptr(), n_kv, HD, S)
+    ctx._check(_lib.load().hf2q_cuda_attn_prefill(ctx._h, torch.cuda.current_stream().cuda_stream, qkv.data_ptr(), m, nq, C.byref(kv), pos0, out.data_ptr(),
+                                                  ops.DT_F32 if out.dtype == torch.float32 else ops.DT_BF16))
+
+
+@pytest.mark.parametrize("pos0,m", [(0, 1500), (64, 700), (640, 2048)])
+def test_waves_of_ctas_agree(gpu_ctx, pos0, m):
+    """CTAs of all lengths (1 block to dozens) side by side and in several waves, many times: every wait ends, every run has the same bits."""
+    qkv, codes, scales, T, S = case(4, 8, pos0, m, 2.0, 1.0, True, seed=m)
+    first, again = (torch.full((m, 32 * HD), float("nan"), device="cuda") for _ in range(2))
+    attend(gpu_ctx, qkv, codes, scales, S, m, 32, 8, pos0, first)
+    for _ in range(40):
+        attend(gpu_ctx, qkv, codes, scales, S, m, 32, 8, pos0, again)
+        assert torch.equal(first, again)
+    gpu_ctx.check_status()
+    assert first.isfinite().all()
