@@ -295,28 +295,30 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
                 uint32_t o[32];
                 tmem_ld32(at + COL_O + c, o);
                 tmem_wait_ld();
-                if (!live) continue;
-                float v[32];
+                if (live) {
+                    float v[32];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * inv;
-                if constexpr (std::is_same_v<OUT, float>) {
-                    if (wide) {
+                    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * inv;
+                    if constexpr (std::is_same_v<OUT, float>) {
+                        if (wide) {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) reinterpret_cast<float4*>(dst + c)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                            for (int i = 0; i < 8; ++i) reinterpret_cast<float4*>(dst + c)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                        } else {
+                            for (int i = 0; i < 32; ++i) dst[c + i] = v[i];
+                        }
                     } else {
-                        for (int i = 0; i < 32; ++i) dst[c + i] = v[i];
-                    }
-                } else {
-                    __nv_bfloat162 h[16];
+                        __nv_bfloat162 h[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                    if (wide) {
+                        for (int i = 0; i < 16; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                        if (wide) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(dst + c)[i] = reinterpret_cast<const uint4*>(h)[i];
-                    } else {
-                        for (int i = 0; i < 16; ++i) { dst[c + 2 * i] = h[i].x; dst[c + 2 * i + 1] = h[i].y; }
+                            for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(dst + c)[i] = reinterpret_cast<const uint4*>(h)[i];
+                        } else {
+                            for (int i = 0; i < 16; ++i) { dst[c + 2 * i] = h[i].x; dst[c + 2 * i + 1] = h[i].y; }
+                        }
                     }
                 }
+                __syncwarp();                                  // the next load from tensor memory is the whole warp's
             }
         }
         tc_fence_before();

@@ -590,35 +590,37 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
                 uint32_t o[16];
                 tc::tmem_ld16(at + WT_O + c, o);
                 tc::tmem_wait_ld();
-                if (!live) continue;
-                float v[16];
+                if (live) {
+                    float v[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(o[i]) * inv;
-                if (wide && c + 16 <= a.vdim) {
-                    if (gr) {
+                    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(o[i]) * inv;
+                    if (wide && c + 16 <= a.vdim) {
+                        if (gr) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float4 g = *reinterpret_cast<const float4*>(gr + c + 4 * i);
-                            v[4 * i] *= sigmoidf(g.x);
-                            v[4 * i + 1] *= sigmoidf(g.y);
-                            v[4 * i + 2] *= sigmoidf(g.z);
-                            v[4 * i + 3] *= sigmoidf(g.w);
+                            for (int i = 0; i < 4; ++i) {
+                                const float4 g = *reinterpret_cast<const float4*>(gr + c + 4 * i);
+                                v[4 * i] *= sigmoidf(g.x);
+                                v[4 * i + 1] *= sigmoidf(g.y);
+                                v[4 * i + 2] *= sigmoidf(g.z);
+                                v[4 * i + 3] *= sigmoidf(g.w);
+                            }
                         }
-                    }
-                    if constexpr (sizeof(OUT) == 4) {
+                        if constexpr (sizeof(OUT) == 4) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + c + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + c + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i)
+                                *reinterpret_cast<uint4*>(dst + c + 8 * i) = make_uint4(pack_bf16(v[8 * i], v[8 * i + 1]), pack_bf16(v[8 * i + 2], v[8 * i + 3]),
+                                                                                        pack_bf16(v[8 * i + 4], v[8 * i + 5]), pack_bf16(v[8 * i + 6], v[8 * i + 7]));
+                        }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            *reinterpret_cast<uint4*>(dst + c + 8 * i) = make_uint4(pack_bf16(v[8 * i], v[8 * i + 1]), pack_bf16(v[8 * i + 2], v[8 * i + 3]),
-                                                                                    pack_bf16(v[8 * i + 4], v[8 * i + 5]), pack_bf16(v[8 * i + 6], v[8 * i + 7]));
+                        for (int i = 0; i < 16; ++i)
+                            if (c + i < a.vdim) dst[c + i] = from_f32<OUT>(gr ? v[i] * sigmoidf(gr[c + i]) : v[i]);
                     }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (c + i < a.vdim) dst[c + i] = from_f32<OUT>(gr ? v[i] * sigmoidf(gr[c + i]) : v[i]);
                 }
+                __syncwarp();                                  // the next load from tensor memory is the whole warp's
             }
             if (live && h == a.heads - 1)
                 for (uint32_t i = a.heads * a.vdim; i < ldo; ++i) out[static_cast<size_t>(t) * ldo + i] = from_f32<OUT>(0.f);

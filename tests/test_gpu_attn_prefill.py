@@ -70,3 +70,29 @@ def test_waves_of_ctas_agree(gpu_ctx, pos0, m):
         assert torch.equal(first, again)
     gpu_ctx.check_status()
     assert first.isfinite().all()
+
+
+@pytest.mark.parametrize("group,m", [(1, 1), (1, 127), (1, 129), (1, 161), (2, 65), (4, 7), (4, 33), (8, 1), (8, 17)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_tiles_that_end_inside_a_warp(gpu_ctx, group, m, dtype, shift):
+    """Rows past the last token share a warp with live ones: live rows come whole, aligned or not, and nothing else is written."""
+    qkv, codes, scales, T, S = case(group, 2, 70, m, 2.0, 1.0, True, seed=m)
+    nq = 2 * group
+    flat = torch.full((shift + (m + 3) * nq * HD,), -7.0, device="cuda", dtype=dtype)
+    out = flat[shift:shift + m * nq * HD].view(m, nq * HD)
+    whole = torch.empty((m + 128, nq * HD), device="cuda", dtype=dtype)[:m]
+    attend(gpu_ctx, qkv, codes, scales, S, m, nq, 2, 70, whole)
+    attend(gpu_ctx, qkv, codes, scales, S, m, nq, 2, 70, out)
+    gpu_ctx.check_status()
+    k, v = ((c[:, :T].double() * s[:, :T, None].double()) for c, s in zip(codes, scales))
+    q = qkv[:, :nq * HD].double().view(m, 2, group, HD)
+    s = torch.einsum("tgrd,gpd->gtrp", q, k)
+    hidden = torch.arange(T, device="cuda")[None] > 70 + torch.arange(m, device="cuda")[:, None]
+    want = torch.einsum("gtrp,gpd->tgrd", torch.softmax(s.masked_fill(hidden[None, :, None], -float("inf")), dim=-1), v).reshape(m, nq * HD)
+    spread = s.masked_fill(hidden[None, :, None], 0).std().item()
+    bound = 2 ** -11 * (1 + spread) + (2 ** -9 if dtype == torch.bfloat16 else 0)        # as above
+    row_err = (out.double() - want).norm(dim=1) / want.norm(dim=1)
+    assert row_err.max() < 4 * bound                     # a row alone: no averaging over rows
+    assert torch.equal(out, whole)
+    assert (flat[:shift] == -7).all() and (flat[shift + m * nq * HD:] == -7).all()
