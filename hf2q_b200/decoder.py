@@ -158,9 +158,10 @@ class GreedyDecoder:
 
 
 def to_device(t: torch.Tensor, device) -> torch.Tensor:
-    """A copy that the host does not wait for: host tensors go through pinned memory."""
+    """A copy that the host does not wait for: host tensors go through pinned memory of the copy's own, so that the caller
+    may change its tensor at once."""
     if t.device.type == "cpu" and torch.device(device).type == "cuda" and t.numel():
-        return t.pin_memory().to(device, non_blocking=True)
+        return torch.empty(t.shape, dtype=t.dtype, pin_memory=True).copy_(t).to(device, non_blocking=True)
     return t.to(device)
 
 
