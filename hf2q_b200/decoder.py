@@ -157,12 +157,27 @@ class GreedyDecoder:
         return out
 
 
-def to_device(t: torch.Tensor, device) -> torch.Tensor:
-    """A copy that the host does not wait for: host tensors go through pinned memory of the copy's own, so that the caller
-    may change its tensor at once."""
-    if t.device.type == "cpu" and torch.device(device).type == "cuda" and t.numel():
-        return torch.empty(t.shape, dtype=t.dtype, pin_memory=True).copy_(t).to(device, non_blocking=True)
-    return t.to(device)
+class Staging:
+    """Small host tensors reach the device through a pinned buffer of their own, and the host does not wait for them: the
+    caller may change its tensor at once, and no call allocates pinned memory (a capture gives torch's cached blocks back,
+    so allocations around the first single-token step went to the driver)."""
+
+    def __init__(self, nbytes: int, device):
+        self.device = device
+        self._buf, self._at, self._copied = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True), 0, torch.cuda.Event()
+
+    def to_device(self, t: torch.Tensor) -> torch.Tensor:
+        n = t.numel() * t.element_size()
+        if t.device.type != "cpu" or n == 0 or n > self._buf.numel() or torch.cuda.is_current_stream_capturing():
+            return t.to(self.device)
+        if self._at + n > self._buf.numel():
+            self._copied.synchronize()                # (copies run in the order of the calls, so the last one is enough)
+            self._at = 0
+        part = self._buf[self._at:self._at + n].view(t.dtype).view(t.shape)
+        out = part.copy_(t).to(self.device, non_blocking=True)
+        self._copied.record(torch.cuda.current_stream(self.device))
+        self._at += (n + 15) // 16 * 16
+        return out
 
 
 class SlotDecoder(GreedyDecoder):
@@ -180,6 +195,7 @@ class SlotDecoder(GreedyDecoder):
         self.chunk = min(prefill_chunk, max_seq)
         self.pool = StatePool(n_slots, self.dev)
         self.ws = Workspace(self.dev)
+        self.staging = Staging(8 * max_seq + (1 << 16), self.dev)      # the ids and row numbers of a call
         self.logits = torch.zeros((1, cfg.vocab), dtype=torch.float32, device=self.dev)
         self._graphs: dict[int, object] = {}
         self._slot = None
@@ -224,7 +240,7 @@ class SlotDecoder(GreedyDecoder):
         self.bind(slot)
         ids = ids.to(torch.int32).contiguous()
         if n > 1:
-            ids = to_device(ids, self.dev)
+            ids = self.staging.to_device(ids)
         want = list(want)
         out = torch.empty((len(want), self.cfg.vocab), dtype=torch.float32, device=self.dev)
         for c0 in range(0, n, self.chunk):
@@ -249,7 +265,7 @@ class SlotDecoder(GreedyDecoder):
             rows = [p for _, p in here]
             logits = self._head_rows(x, rows + [m - 1]) if last or rows else None
             if rows:
-                out[to_device(torch.tensor([j for j, _ in here]), self.dev)] = logits[:len(rows)]
+                out[self.staging.to_device(torch.tensor([j for j, _ in here]))] = logits[:len(rows)]
             if last:
                 self.logits.copy_(logits[-1:])
                 self.sop.argmax(self.logits, self.tok)

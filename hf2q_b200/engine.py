@@ -10,8 +10,6 @@ from dataclasses import dataclass
 
 import torch
 
-from .decoder import to_device
-
 
 @dataclass
 class Entry:
@@ -40,7 +38,7 @@ class Engine:
             elif len(order):
                 back = torch.empty(len(order), dtype=torch.long)
                 back[order] = torch.arange(len(order))
-                rows.append(got[to_device(back, got.device)])
+                rows.append(got[back.to(got.device)])
         for i in end:
             self.model.close_slot(self._slots.pop(i))
         return (rows[0] if len(rows) == 1 else torch.cat(rows)) if rows else None

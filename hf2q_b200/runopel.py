@@ -17,7 +17,7 @@ from pathlib import Path
 import torch
 
 from . import _lib, ops
-from .decoder import SlotDecoder, to_device
+from .decoder import SlotDecoder
 from .feedforward import FEED_FORWARDS
 from .mixers import MIXERS
 from .safetensors import SafetensorsFile
@@ -218,7 +218,7 @@ class RunopelDecoder(SlotDecoder):
         """Final norm and output head of the given tokens."""
         c, n, m = self.cfg, len(rows), portion.x.shape[0]
         if n != m or rows != list(range(m)):
-            at = to_device(torch.tensor(rows), self.dev)
+            at = self.staging.to_device(torch.tensor(rows))
             pending = portion.pending
             if pending is not None:
                 y, parts, hc = pending

@@ -21,3 +21,28 @@ def test_pinned_ids_may_be_overwritten_after_the_call(gpu_ctx):
     got = m.extend(slot, pinned, range(40))
     pinned.fill_(0)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("design", ["fomatar", "runopel"])
+def test_no_call_allocates_pinned_memory(gpu_ctx, design):
+    from tests import test_gpu_runopel as R
+    m, cfg, _ = load(gpu_ctx, "a", torch.float32) if design == "fomatar" else R.load(gpu_ctx, "a", torch.float32)
+    ids = torch.randint(0, cfg["vocab"], (70,), dtype=torch.int32)
+    torch.cuda.synchronize()
+    before = torch.cuda.host_memory_stats()["num_host_alloc"]
+    slot = m.open_slot()
+    for a, b, want in [(0, 40, [39]), (40, 41, [0]), (41, 60, [3, 7, 18]), (60, 61, []), (61, 70, [])]:
+        m.extend(slot, ids[a:b], want)
+    assert torch.cuda.host_memory_stats()["num_host_alloc"] == before
+
+
+def test_staging_wraps_behind_its_copies(gpu_ctx):
+    from hf2q_b200.decoder import Staging
+    st, sent, got = Staging(256, torch.device("cuda", 0)), [], []
+    torch.cuda.synchronize()
+    torch.cuda._sleep(LONG // 8)
+    for i in range(1, 90):                               # sizes on both sides of the buffer's
+        sent.append(torch.arange(i, dtype=torch.int64) * 1000 + i)
+        got.append(st.to_device(sent[-1]))
+    for a, b in zip(sent, got):
+        assert torch.equal(a, b.cpu())
