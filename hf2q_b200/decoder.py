@@ -18,6 +18,7 @@ graph and replayed once per generated token.
 from __future__ import annotations
 
 import ctypes as C
+from contextlib import contextmanager
 from dataclasses import dataclass
 
 import numpy as np
@@ -200,6 +201,7 @@ class SlotDecoder(GreedyDecoder):
         self._graphs: dict[int, object] = {}
         self._slot = None
         self._start = None              # position of the running portion's first token, None in decode steps
+        self._done = torch.cuda.Event()                               # the end of the latest call's work
         self.on_layer = None            # callable(run index, residual [m, width]) after every layer run: a probe for tests
 
     def _portion(self, ids, m: int):
@@ -208,9 +210,24 @@ class SlotDecoder(GreedyDecoder):
     def _head_rows(self, portion, rows) -> torch.Tensor:
         raise NotImplementedError
 
+    @contextmanager
+    def _ordered(self):
+        """Calls return before the device has finished, and all of them work on the same state and scratch buffers: each
+        starts on its stream when the last one's work is done, on whatever stream that was."""
+        if torch.cuda.is_current_stream_capturing():
+            yield
+            return
+        stream = torch.cuda.current_stream(self.dev)
+        stream.wait_event(self._done)
+        try:
+            yield
+        finally:
+            self._done.record(stream)
+
     # ---- slots ----------------------------------------------------------------------------------
     def open_slot(self) -> int:
-        return self.pool.open()
+        with self._ordered():
+            return self.pool.open()
 
     def close_slot(self, slot: int) -> None:
         self.pool.close(slot)
@@ -238,10 +255,15 @@ class SlotDecoder(GreedyDecoder):
         if n == 0 or start + n > self.max_seq:
             raise ops.Hf2qError(_lib.ERR_INVALID_ARGUMENT, f"{n} tokens after {start}: the model was loaded for sequences of 1..{self.max_seq}")
         self.bind(slot)
+        with self._ordered():
+            out = self._extend(ids, n, start, list(want))
+        self.pool.length[slot] = start + n
+        return out
+
+    def _extend(self, ids, n: int, start: int, want: list) -> torch.Tensor:
         ids = ids.to(torch.int32).contiguous()
         if n > 1:
             ids = self.staging.to_device(ids)
-        want = list(want)
         out = torch.empty((len(want), self.cfg.vocab), dtype=torch.float32, device=self.dev)
         for c0 in range(0, n, self.chunk):
             m = min(self.chunk, n - c0)
@@ -270,13 +292,13 @@ class SlotDecoder(GreedyDecoder):
                 self.logits.copy_(logits[-1:])
                 self.sop.argmax(self.logits, self.tok)
                 self.pos.fill_(start + n)
-        self.pool.length[slot] = start + n
         return out
 
     def generate(self, n: int, use_graph: bool = True, collect: bool = True):
         if self.pool.length[self._slot] + n > self.max_seq:
             raise ops.Hf2qError(_lib.ERR_INVALID_ARGUMENT, f"{n} more tokens do not fit the {self.max_seq} the model was loaded for")
-        out = super().generate(n, use_graph, collect)
+        with self._ordered():
+            out = super().generate(n, use_graph, collect)
         self.pool.length[self._slot] += n
         return out
 

@@ -25,7 +25,9 @@ class Engine:
 
     def step(self, entries, end=()) -> torch.Tensor | None:
         """Runs every entry's tokens from the state its earlier steps left; returns the wanted logits, rows in the order
-        of the entries and of ``want`` (None if nothing is wanted).  ``end``: requests that give back their slot."""
+        of the entries and of ``want`` (None if nothing is wanted).  ``end``: requests that give back their slot.
+        It returns before the device has finished: the rows are ready in the order of the current stream.  A later step may
+        come on another stream (the decoder orders them)."""
         rows = []
         for e in entries:
             if e.id not in self._slots:

@@ -88,6 +88,8 @@ class Workspace:
         need = rows * cols
         b = self._bufs.get(key)
         if b is None or b.numel() < need:
+            if b is not None and b.is_cuda:
+                b.record_stream(torch.cuda.current_stream(b.device))       # work on it may still run, on another stream than it came from
             b = torch.zeros(need, dtype=dtype, device=self.device)
             self._bufs[key] = b
         return b[:need].view(rows, cols)

@@ -46,3 +46,26 @@ def test_staging_wraps_behind_its_copies(gpu_ctx):
         got.append(st.to_device(sent[-1]))
     for a, b in zip(sent, got):
         assert torch.equal(a, b.cpu())
+
+
+def test_calls_on_alternating_streams(gpu_ctx):
+    """Each call works on what the last one left, although that may still be waiting on another stream."""
+    from hf2q_b200.engine import Engine, Entry
+    cuts, ids = [40, 1, 1, 90, 2, 1, 1], None
+
+    def rows(streams):
+        nonlocal ids
+        m, cfg, _ = load(gpu_ctx, "a", torch.float32, prefill_chunk=64)          # (the larger portion grows the scratch buffers)
+        ids = U.tokens(cfg, sum(cuts)) if ids is None else ids
+        e, out, at = Engine(m), [], 0
+        torch.cuda.synchronize()
+        for i, n in enumerate(cuts):
+            with torch.cuda.stream(streams[i % len(streams)]):
+                torch.cuda._sleep(LONG // 4)
+                out.append(e.step([Entry("r", list(ids[at:at + n]), [n - 1])]))
+            at += n
+        torch.cuda.synchronize()
+        return torch.cat(out)
+
+    one = rows([torch.cuda.Stream()])
+    assert torch.equal(rows([torch.cuda.Stream(), torch.cuda.Stream()]), one)
