@@ -274,7 +274,7 @@ class FomatarDecoder(SlotDecoder):
     def _head_rows(self, x, rows) -> torch.Tensor:
         """Final norm and output head of the given residual rows."""
         c, n = self.cfg, len(rows)
-        xs = x if n == x.shape[0] else x.index_select(0, self.staging.to_device(torch.tensor(rows)))
+        xs = x if rows == list(range(x.shape[0])) else x.index_select(0, self.staging.to_device(torch.tensor(rows)))
         xn = self.ws.get("head.xn", n, pad8(c.width), self.act)
         self.sop.pre_norm(self._pre(xs, None, self.final_norm), n, xn)
         out = torch.empty((n, c.vocab), dtype=torch.float32, device=self.dev)

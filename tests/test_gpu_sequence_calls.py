@@ -69,3 +69,15 @@ def test_calls_on_alternating_streams(gpu_ctx):
 
     one = rows([torch.cuda.Stream()])
     assert torch.equal(rows([torch.cuda.Stream(), torch.cuda.Stream()]), one)
+
+
+@pytest.mark.parametrize("design", ["fomatar", "runopel"])
+@pytest.mark.parametrize("n,want", [(2, [1]), (3, [0, 2]), (4, [1, 1, 2]), (3, [2, 2]), (1, [0])])
+def test_as_many_rows_as_tokens(gpu_ctx, design, n, want):
+    """The rows asked for and the last one can be as many as the portion's tokens without being those tokens."""
+    from tests import test_gpu_runopel as R
+    m, cfg, _ = load(gpu_ctx, "a", torch.float32, n_slots=2) if design == "fomatar" else R.load(gpu_ctx, "a", torch.float32, n_slots=2)
+    ids = torch.tensor(U.tokens(cfg, n), dtype=torch.int32)
+    every = m.extend(m.open_slot(), ids, range(n))
+    some = m.extend(m.open_slot(), ids, want)
+    assert (some - every[want]).norm() <= 1e-5 * every[want].norm()          # (other row counts take other products of the head)
