@@ -69,9 +69,10 @@ __device__ __forceinline__ void store_codes(uint8_t* block, uint32_t row, uint32
     *reinterpret_cast<uint4*>(at + (((c + 1 - flip) ^ (row & 7)) << 4)) = flip ? lo : hi;
 }
 
-// two scores of positions p and p + 1 for a row whose last position is `seen`
-__device__ __forceinline__ float2 hide(float2 x, uint32_t p, uint32_t seen) {
-    return make_float2(p <= seen ? x.x : -CUDART_INF_F, p + 1 <= seen ? x.y : -CUDART_INF_F);
+// two values of positions p and p + 1 for a row whose last position is `seen`: scores, or weights (what is hidden has none,
+// also where its V scale is infinite or NaN)
+__device__ __forceinline__ float2 hide(float2 x, uint32_t p, uint32_t seen, float hidden) {
+    return make_float2(p <= seen ? x.x : hidden, p + 1 <= seen ? x.y : hidden);
 }
 
 template <int G, typename OUT>
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
                     for (int i = 0; i < 16; ++i) {
                         const ulonglong2 k = k2[8 * half + i / 2];
                         float2 x = f2_parts(f2_mul(f2_pack(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x));
-                        if constexpr (decltype(masked)::value) x = hide(x, j * BP + 32 * half + 2 * i, seen);
+                        if constexpr (decltype(masked)::value) x = hide(x, j * BP + 32 * half + 2 * i, seen, -CUDART_INF_F);
                         top[2 * (i & 1)] = fmaxf(top[2 * (i & 1)], x.x);
                         top[2 * (i & 1) + 1] = fmaxf(top[2 * (i & 1) + 1], x.y);
                     }
@@ -268,10 +269,11 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
                     for (int i = 0; i < 8; ++i) {
                         const ulonglong2 k = k2[4 * c + i / 2], v = v2[4 * c + i / 2];
                         float2 d = f2_parts(f2_fma(f2_pack(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x, nm));
-                        if constexpr (decltype(masked)::value) d = hide(d, j * BP + 16 * c + 2 * i, seen);
+                        if constexpr (decltype(masked)::value) d = hide(d, j * BP + 16 * c + 2 * i, seen, -CUDART_INF_F);
                         const f2 e = f2_pack(exp2_fast(d.x), exp2_fast(d.y));
                         part = f2_add(part, e);
-                        const float2 w = f2_parts(f2_mul(e, i & 1 ? v.y : v.x));
+                        float2 w = f2_parts(f2_mul(e, i & 1 ? v.y : v.x));
+                        if constexpr (decltype(masked)::value) w = hide(w, j * BP + 16 * c + 2 * i, seen, 0.f);
                         p[i] = pack_h2(w.x, w.y);
                     }
                     tmem_st8(at + b * BP + 8 * c, p);          // over scores that have been read

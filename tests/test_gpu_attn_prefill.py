@@ -96,3 +96,25 @@ def test_tiles_that_end_inside_a_warp(gpu_ctx, group, m, dtype, shift):
     assert row_err.max() < 4 * bound                     # a row alone: no averaging over rows
     assert torch.equal(out, whole)
     assert (flat[:shift] == -7).all() and (flat[shift + m * nq * HD:] == -7).all()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("which", [0, 1])
+@pytest.mark.parametrize("pos0,m,at", [(0, 200, 77), (30, 129, 30 + 128), (64, 100, 64 + 1)])
+def test_hidden_scales_do_not_reach_a_row(gpu_ctx, bad, which, pos0, m, at):
+    """A K or V scale that is not finite shows in the rows that see its position and in no other of the tile."""
+    qkv, codes, scales, T, S = case(2, 2, pos0, m, 2.0, 1.0, True, seed=m)
+    clean = [s.clone() for s in scales]
+    scales[which][:, at] = bad
+    out = torch.empty((m, 4 * HD), device="cuda")
+    attend(gpu_ctx, qkv, codes, scales, S, m, 4, 2, pos0, out)
+    gpu_ctx.check_status()
+    k, v = ((c[:, :T].double() * s[:, :T, None].double()) for c, s in zip(codes, clean))
+    s = torch.einsum("tgrd,gpd->gtrp", qkv[:, :4 * HD].double().view(m, 2, 2, HD), k)
+    hidden = torch.arange(T, device="cuda")[None] > pos0 + torch.arange(m, device="cuda")[:, None]
+    want = torch.einsum("gtrp,gpd->tgrd", torch.softmax(s.masked_fill(hidden[None, :, None], -float("inf")), dim=-1), v).reshape(m, 4 * HD)
+    n = at - pos0                                        # the first row that sees the position
+    bound = 2 ** -11 * (1 + s.masked_fill(hidden[None, :, None], 0).std().item())
+    assert (out[:n].double() - want[:n]).norm() < bound * want[:n].norm()
+    if which == 1:
+        assert not out[n].isfinite().any()
