@@ -313,24 +313,20 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_decode_kernel(const __gr
 constexpr uint32_t QK_MAX = 320;                        // dim and shared_dim together, padded
 
 // ---------------------------------------------------------------- prefill, f32: one warp per (query, head)
+// query t of head h by one warp; qs [QK_MAX] and ps [32] of this warp in shared memory
 template <typename T, typename OUT, int NC, bool PLAIN>
-__global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m, const T* __restrict__ q,
-                                                                 const float* __restrict__ gate, uint32_t ldg, OUT* __restrict__ out, uint32_t ldo) {
-    __shared__ __align__(16) float qs[8][QK_MAX];
-    __shared__ float ps[8][32];
-    pdl_trigger();
-    pdl_wait();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, t = blockIdx.x * 8 + warp;
-    if (t >= m) return;
-    const KeyRows<T, PLAIN> kv(a, h / (a.heads / a.kv_heads), *a.pos);
+__device__ __forceinline__ void f32_query(const hf2q_window_attn& a, uint32_t pos0, uint32_t t, uint32_t h, const T* __restrict__ q, const float* __restrict__ gate,
+                                          uint32_t ldg, OUT* __restrict__ out, uint32_t ldo, float* qs, float* ps) {
+    const uint32_t lane = threadIdx.x & 31;
+    const KeyRows<T, PLAIN> kv(a, h / (a.heads / a.kv_heads), pos0);
     const uint32_t dq = kv.dp + kv.sp;
-    for (uint32_t i = lane; i < dq; i += 32) qs[warp][i] = to_f32(q[(static_cast<size_t>(t) * a.heads + h) * dq + i]);
+    for (uint32_t i = lane; i < dq; i += 32) qs[i] = to_f32(q[(static_cast<size_t>(t) * a.heads + h) * dq + i]);
     __syncwarp();
-    const uint32_t pos = *a.pos + t, n = min(pos + 1, a.window), hi = pos + 1;
+    const uint32_t pos = pos0 + t, n = min(pos + 1, a.window), hi = pos + 1;
     const float r1[1] = {a.r1 ? a.r1[h] : 0.f}, r2[1] = {a.r1 ? a.r2[h] : 0.f};
     WarpAttn<T, 1, NC, PLAIN> w;
     w.init();
-    for (uint32_t p0 = hi - n; p0 < hi; p0 += 32) w.keys(a, kv.k, kv.v, &kv, qs[warp], ps[warp], r1, r2, pos, p0, hi);
+    for (uint32_t p0 = hi - n; p0 < hi; p0 += 32) w.keys(a, kv.k, kv.v, &kv, qs, ps, r1, r2, pos, p0, hi);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -345,6 +341,17 @@ __global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_co
     if (h == a.heads - 1)
         for (uint32_t i = a.heads * a.vdim + lane; i < ldo; i += 32) out[static_cast<size_t>(t) * ldo + i] = from_f32<OUT>(0.f);
 }
+template <typename T, typename OUT, int NC, bool PLAIN>
+__global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m, const T* __restrict__ q,
+                                                                 const float* __restrict__ gate, uint32_t ldg, OUT* __restrict__ out, uint32_t ldo) {
+    __shared__ __align__(16) float qs[8][QK_MAX];
+    __shared__ float ps[8][32];
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t warp = threadIdx.x >> 5, t = blockIdx.x * 8 + warp;
+    if (t >= m) return;
+    f32_query<T, OUT, NC, PLAIN>(a, *a.pos, t, blockIdx.y, q, gate, ldg, out, ldo, qs[warp], ps[warp]);
+}
 
 // ---------------------------------------------------------------- prefill, bf16 cache, tcgen05
 // One CTA owns 128 queries of one head and walks the keys from the first one that its first query sees, 64 at a time:
@@ -356,6 +363,9 @@ __global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_co
 //               again for the exponentials (64 of them would not fit the registers beside the rest); P takes their place.
 //               The output rows of a warp are rescaled wherever one's running maximum grew: with the true maximum the largest
 //               weight is 1, which bf16 holds exactly (an older one within 2^8 was no faster and doubled the error of peaked rows).
+//
+// The weight of a key that a query does not see is zero, but zero times a value that is not finite is NaN.  So warps 4-7 look
+// for such values in the blocks that some query does not see whole; a tile that has one is done again in f32, a warp to a query.
 //
 // 256 tensor-memory columns (S 2 x 64, O 128).  Two CTAs per SM with keys of up to 128 elements, one with 192.  It is bound by
 // the latency of a block's chain (scores, maximum, exponentials, output).  2048 queries x 16 heads of 128 with 2048 keys each
@@ -369,6 +379,15 @@ __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.
 // 16-byte chunk c of a row, in panels of `rows` rows x 64 elements
 __device__ __forceinline__ uint32_t wt_chunk(uint32_t rows, uint32_t row, uint32_t c) { return (c >> 3) * rows * 128 + row * 128 + (((c & 7) ^ (row & 7)) << 4); }
 
+// the queries t0 .. t0 + n of head h again, in f32; work: WT_THREADS / 32 x (QK_MAX + 32) floats of shared memory
+template <typename OUT, bool PLAIN>
+__device__ __noinline__ void wt_again(const hf2q_window_attn& a, uint32_t pos0, uint32_t t0, uint32_t n, uint32_t h, const __nv_bfloat16* q, const float* gate,
+                                      uint32_t ldg, OUT* out, uint32_t ldo, float* work) {
+    float* qs = work + (threadIdx.x >> 5) * (QK_MAX + 32);
+    for (uint32_t t = threadIdx.x >> 5; t < n; t += WT_THREADS / 32)
+        f32_query<__nv_bfloat16, OUT, WT_V / 64, PLAIN>(a, pos0, t0 + t, h, q, gate, ldg, out, ldo, qs, qs + QK_MAX);
+}
+
 template <int DK, typename OUT, bool PLAIN>
 __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_tc_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m,
                                                                                           const __nv_bfloat16* __restrict__ q, const float* __restrict__ gate,
@@ -378,10 +397,11 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
     constexpr uint32_t Q_BYTES = WT_Q * DK * 2, K_BYTES = WT_K * DK * 2, V_BYTES = WT_K * WT_V * 2;
     uint8_t *qs = smem, *ks = smem + Q_BYTES, *vs = ks + 2 * K_BYTES;
     __shared__ uint64_t k_full[2], v_full[2], s_full[2], p_full[2], o_done[2];
-    __shared__ uint32_t tmem_slot;
+    __shared__ uint32_t tmem_slot, again;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t h = blockIdx.y, t0 = (gridDim.x - 1 - blockIdx.x) * WT_Q;
     if (threadIdx.x == 0) {
+        again = 0;
         for (int i = 0; i < 2; ++i) {
             mbar_init(&k_full[i], 4);
             mbar_init(&v_full[i], 4);
@@ -400,6 +420,8 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
     const uint32_t dq = rows.dp + rows.sp, dvp = pad8(a.vdim), nk = (dq + 15) / 16;
     const uint32_t q_lo = pos0 + t0, q_hi = pos0 + min(t0 + WT_Q, m) - 1;
     const uint32_t j0 = q_lo + 1 > a.window ? q_lo + 1 - a.window : 0u, nb = (q_hi - j0) / WT_K + 1;
+    // some query of the tile (those past the end included) does not see all of block j
+    auto edge = [&](uint32_t j) { return j0 + j * WT_K + WT_K - 1 > q_lo || q_lo + WT_Q - 1 - (j0 + j * WT_K) >= a.window; };
     if (dq < DK || dvp < WT_V) {                               // elements past dim / vdim must be finite zeros
         for (uint32_t i = threadIdx.x; i < (2 * K_BYTES + 2 * V_BYTES) / 16; i += WT_THREADS) reinterpret_cast<uint4*>(ks)[i] = make_uint4(0, 0, 0, 0);
     }
@@ -465,6 +487,17 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
                 }
             }
             cp_async_commit();
+            if (j > 0 && edge(j - 1)) {                        // this thread's copies of V(j-1): a value whose exponent is all ones?
+                uint32_t top = 0;
+                auto full = [](uint32_t w) { return (w & 0x7F807F80u) + 0x00800080u; };       // bit 15 of a half: its exponent was
+#pragma unroll
+                for (uint32_t i = 0; i < WT_K / 16; ++i)
+                    for (uint32_t c = c0; c < cv; c += 8) {
+                        const uint4 w = *reinterpret_cast<const uint4*>(vs + (b ^ 1) * V_BYTES + wt_chunk(WT_K, row0 + 16 * i, c));
+                        top |= full(w.x) | full(w.y) | full(w.z) | full(w.w);
+                    }
+                if (top & 0x80008000u) again = 1;
+            }
         }
         cp_async_wait<0>();
     } else if (warp == 8) {
@@ -510,8 +543,6 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
             ok = __all_sync(0xffffffffu, mbar_wait_bounded(&s_full[b], (j >> 1) & 1, status));
             if (!ok) break;
             tc::tc_fence_after();
-            // some query of the tile does not see all of the block
-            const bool edge = key0 + WT_K - 1 > q_lo || key0 + a.window <= pos0 + t0 + WT_Q - 1;
             float top[2] = {-CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
             for (uint32_t half = 0; half < 2; ++half) {
@@ -526,7 +557,7 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) - r1 * lg2(fmaf(r2, d0f - i, 1.0f)));
                 }
-                if (edge) {
+                if (edge(j)) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = d0 - i < a.window ? r[i] : __float_as_uint(-CUDART_INF_F);
                 }
@@ -629,6 +660,7 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
     }
     __syncthreads();
     if (warp == 8) { tc::tc_fence_after(); tc::tmem_dealloc(tmem, WT_COLS); }
+    if (again) wt_again<OUT, PLAIN>(a, pos0, t0, min(WT_Q, m - t0), h, q, gate, ldg, out, ldo, reinterpret_cast<float*>(smem));
 }
 
 // ---------------------------------------------------------------- prefill, bf16 cache, other sizes: warp-level products
