@@ -538,7 +538,30 @@ __global__ void __launch_bounds__(SC_THREADS) delta_step_kernel(const __grid_con
     }
 }
 
-constexpr uint32_t PREP_TOKENS = 16;
+// Tokens of a CTA of the four-tap kernels (`columns` CTAs to a run of tokens): 16, so that inputs and weights are read once and
+// not four times through L2 (8 with wide heads, a lane of which has eight channels), or as few as put PREP_CTAS on every SM, for
+// a CTA is a chain of its tokens.  delta, 8 + 8 + 16 heads of 128: 64 tokens 17.1 us a token a CTA, 20.6 at 16, 3.5 as here; 2048
+// tokens 56.9, 41.0 and 41.0.  2 CTAs an SM: 4.6 at 64 tokens; 8: the same to 15 % slower at 128.  ssd, 64 heads of 128 x 64:
+// 2048 tokens 57.8 us a token a CTA, 28.0 as here.
+constexpr uint32_t PREP_CTAS = 4;
+inline uint32_t prep_tokens(uint32_t m, uint32_t columns, int sms, bool wide = false) {
+    uint32_t per = wide ? 8 : 16;
+    while (per > 1 && static_cast<uint64_t>((m + per - 1) / per) * columns < static_cast<uint64_t>(PREP_CTAS) * sms) per /= 2;
+    return per;
+}
+// f(t, x[t * ld]) for t = 0 .. n, the inputs of U tokens on their way together (a load behind each store would be a chain)
+template <uint32_t U, typename F>
+__device__ __forceinline__ void for_inputs(const float* x, size_t ld, uint32_t n, F f) {
+    for (uint32_t t0 = 0; t0 < n; t0 += U) {
+        float now[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u)
+            if (t0 + u < n) now[u] = x[(t0 + u) * ld];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u)
+            if (t0 + u < n) f(t0 + u, now[u]);
+    }
+}
 // A channel's running window over the four taps of its convolution: the last three inputs and the weights in registers.
 struct FourTaps {
     float w0, w1, w2, w3, x1, x2, x3;
@@ -554,15 +577,14 @@ struct FourTaps {
         return siluf(s);
     }
 };
-// Four taps: 16 tokens a CTA, so that inputs and weights are read once and not four times through L2.  Columns of CTAs: heads
-// of q and k (a warp each, NJ channels a lane), channels of v (a thread each), then the gates and low-rank rows.
-// 2048 tokens of 8 + 8 + 16 heads of 128: 60 -> 45 us.
+// Four taps, `per` tokens a CTA.  Columns of CTAs: heads of q and k (a warp each, NJ channels a lane), channels of v (a thread
+// each), then the gates and low-rank rows.
 template <int NJ, typename LR>
-__global__ void __launch_bounds__(256) delta_prep4_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, uint32_t qk_columns, float* __restrict__ qkv,
+__global__ void __launch_bounds__(256) delta_prep4_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, uint32_t per, uint32_t qk_columns, float* __restrict__ qkv,
                                                           float* __restrict__ beta, LR* __restrict__ a1, LR* __restrict__ g1) {
     pdl_trigger();
     pdl_wait();
-    const uint32_t t0 = blockIdx.x * PREP_TOKENS, n = min(PREP_TOKENS, m - t0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t t0 = blockIdx.x * per, n = min(per, m - t0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t pos = *a.pos, qk = a.kv_heads * a.dim;
     const size_t ld = a.ld, ld_o = 2 * qk + a.heads * a.vdim;
     const float* rows = a.proj + t0 * ld;
@@ -580,24 +602,30 @@ __global__ void __launch_bounds__(256) delta_prep4_kernel(const __grid_constant_
             if (i < a.dim) tap[j].start(w + static_cast<size_t>(c0 + i) * 4, x + i, ld, a.conv_state + static_cast<size_t>((is_k ? qk : 0u) + c0 + i) * 4, pos, t0);
         }
         float* to = dst + (is_k ? qk : 0u) + c0;
-#pragma unroll 4
-        for (uint32_t t = 0; t < n; ++t) {
-            float v[NJ], s = 0.f;
+        constexpr uint32_t U = NJ == 4 ? 4 : 2;                      // tokens whose inputs are on their way together
+        for (uint32_t t1 = 0; t1 < n; t1 += U) {
+            float now[U][NJ];
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                const uint32_t i = lane + 32 * j;
-                v[j] = 0.f;
-                if (i < a.dim) {
-                    const float now = x[t * ld + i];
-                    v[j] = tap[j].next(now, now * tap[j].w3);
+            for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+                    if (t1 + u < n && lane + 32 * j < a.dim) now[u][j] = x[(t1 + u) * ld + lane + 32 * j];
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t t = t1 + u;
+                if (t >= n) break;
+                float v[NJ], s = 0.f;
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    v[j] = lane + 32 * j < a.dim ? tap[j].next(now[u][j], now[u][j] * tap[j].w3) : 0.f;
+                    s += v[j] * v[j];
                 }
-                s += v[j] * v[j];
-            }
-            float inv = 1.0f / sqrtf(warp_sum(s) + 1e-6f);
-            if (!is_k) inv /= sqrtf(static_cast<float>(a.dim));
+                float inv = 1.0f / sqrtf(warp_sum(s) + 1e-6f);
+                if (!is_k) inv /= sqrtf(static_cast<float>(a.dim));
 #pragma unroll
-            for (int j = 0; j < NJ; ++j)
-                if (lane + 32 * j < a.dim) to[t * ld_o + lane + 32 * j] = v[j] * inv;
+                for (int j = 0; j < NJ; ++j)
+                    if (lane + 32 * j < a.dim) to[t * ld_o + lane + 32 * j] = v[j] * inv;
+            }
         }
     } else if (blockIdx.y + 1 < gridDim.y) {
         const uint32_t c = (blockIdx.y - qk_columns) * 256 + threadIdx.x;
@@ -605,11 +633,7 @@ __global__ void __launch_bounds__(256) delta_prep4_kernel(const __grid_constant_
         const float* x = rows + a.v_off + c;
         FourTaps tap;
         tap.start(a.v_conv + static_cast<size_t>(c) * 4, x, ld, a.conv_state + static_cast<size_t>(2 * qk + c) * 4, pos, t0);
-#pragma unroll 8
-        for (uint32_t t = 0; t < n; ++t) {
-            const float now = x[t * ld];
-            dst[t * ld_o + 2 * qk + c] = tap.next(now, now * tap.w3);
-        }
+        for_inputs<8>(x, ld, n, [&](uint32_t t, float now) { dst[t * ld_o + 2 * qk + c] = tap.next(now, now * tap.w3); });
     } else {
         for (uint32_t t = 0; t < n; ++t) {
             const float* row = rows + t * ld;
@@ -778,13 +802,12 @@ __device__ __forceinline__ float conv_bias_silu(const float* w, float bias, uint
     return siluf(s);
 }
 
-// Four taps: a thread takes one channel over 16 tokens, with its taps and the last three inputs in registers (a token a CTA read
-// every input and weight four times through L2).  Bound by memory; the last CTA column makes the gates.  2048 tokens of 5120
-// channels: 60 -> 26 us.
-__global__ void __launch_bounds__(256) ssd_prep4_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, float* __restrict__ xbc, float* __restrict__ dt, float* __restrict__ la) {
+// Four taps: a thread takes one channel over `per` tokens, with its taps and the last three inputs in registers (a token a CTA read
+// every input and weight four times through L2).  Bound by memory; the last CTA column makes the gates.
+__global__ void __launch_bounds__(256) ssd_prep4_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, uint32_t per, float* __restrict__ xbc, float* __restrict__ dt, float* __restrict__ la) {
     pdl_trigger();
     pdl_wait();
-    const uint32_t t0 = blockIdx.x * PREP_TOKENS, n = min(PREP_TOKENS, m - t0), pos = *a.pos, channels = ssd_channels(a);
+    const uint32_t t0 = blockIdx.x * per, n = min(per, m - t0), pos = *a.pos, channels = ssd_channels(a);
     const float* row = a.proj + static_cast<size_t>(t0) * a.ld + a.off;
     if (blockIdx.y + 1 == gridDim.y) {
         for (uint32_t i = threadIdx.x; i < n * a.heads; i += 256) {
@@ -801,11 +824,7 @@ __global__ void __launch_bounds__(256) ssd_prep4_kernel(const __grid_constant__ 
     tap.start(a.conv + static_cast<size_t>(c) * 4, x, a.ld, a.conv_state + static_cast<size_t>(c) * 4, pos, t0);
     const float bias = a.conv_bias[c];
     float* dst = xbc + static_cast<size_t>(t0) * channels + c;
-#pragma unroll 8
-    for (uint32_t t = 0; t < n; ++t) {
-        const float now = x[static_cast<size_t>(t) * a.ld];
-        dst[static_cast<size_t>(t) * channels] = tap.next(now, fmaf(now, tap.w3, bias));
-    }
+    for_inputs<8>(x, a.ld, n, [&](uint32_t t, float now) { dst[static_cast<size_t>(t) * channels] = tap.next(now, fmaf(now, tap.w3, bias)); });
 }
 
 // One CTA per token.
@@ -908,12 +927,13 @@ cudaError_t launch_scan(const hf2q_delta& a, uint32_t m, const float* qkv, const
 
 // four taps, as such layers are built; other counts a CTA a token
 template <typename LR>
-cudaError_t launch_delta_prep(const hf2q_delta& a, uint32_t m, float* qkv, float* beta, LR* a1, LR* g1, cudaStream_t st) {
+cudaError_t launch_delta_prep(const hf2q_delta& a, uint32_t m, float* qkv, float* beta, LR* a1, LR* g1, int sms, cudaStream_t st) {
     const uint32_t qk_columns = (2 * a.kv_heads + 7) / 8, columns = qk_columns + (a.heads * a.vdim + 255) / 256 + 1;
     if (a.taps != 4 || columns > 65535) return launch_pdl(delta_prep_kernel<LR>, dim3(m), dim3(256), 0, st, a, qkv, beta, a1, g1);
-    const dim3 grid((m + PREP_TOKENS - 1) / PREP_TOKENS, columns);
-    if (a.dim <= 128) return launch_pdl(delta_prep4_kernel<4, LR>, grid, dim3(256), 0, st, a, m, qk_columns, qkv, beta, a1, g1);
-    return launch_pdl(delta_prep4_kernel<8, LR>, grid, dim3(256), 0, st, a, m, qk_columns, qkv, beta, a1, g1);
+    const uint32_t per = prep_tokens(m, columns, sms, a.dim > 128);
+    const dim3 grid((m + per - 1) / per, columns);
+    if (a.dim <= 128) return launch_pdl(delta_prep4_kernel<4, LR>, grid, dim3(256), 0, st, a, m, per, qk_columns, qkv, beta, a1, g1);
+    return launch_pdl(delta_prep4_kernel<8, LR>, grid, dim3(256), 0, st, a, m, per, qk_columns, qkv, beta, a1, g1);
 }
 
 template <int RQ, int C>
@@ -980,8 +1000,8 @@ HF2Q_API int32_t hf2q_cuda_delta_prep(hf2q_ctx* ctx, void* stream, const hf2q_de
     if (m == 0) return HF2Q_OK;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaErrorInvalidValue;
-    if (lr_dtype == HF2Q_DT_F32) e = launch_delta_prep(*a, m, qkv, beta, static_cast<float*>(a1), static_cast<float*>(g1), st);
-    else if (lr_dtype == HF2Q_DT_BF16) e = launch_delta_prep(*a, m, qkv, beta, static_cast<__nv_bfloat16*>(a1), static_cast<__nv_bfloat16*>(g1), st);
+    if (lr_dtype == HF2Q_DT_F32) e = launch_delta_prep(*a, m, qkv, beta, static_cast<float*>(a1), static_cast<float*>(g1), ctx_sm_count(ctx), st);
+    else if (lr_dtype == HF2Q_DT_BF16) e = launch_delta_prep(*a, m, qkv, beta, static_cast<__nv_bfloat16*>(a1), static_cast<__nv_bfloat16*>(g1), ctx_sm_count(ctx), st);
     return ctx_cuda_result(ctx, e, "delta_prep", 1);
 }
 
@@ -1031,7 +1051,8 @@ HF2Q_API int32_t hf2q_cuda_ssd_prep(hf2q_ctx* ctx, void* stream, const hf2q_ssd*
     if (m == 0) return HF2Q_OK;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t columns = (a->heads * a->vdim + 2 * a->groups * a->state + 255) / 256 + 1;
-    const cudaError_t e = a->taps == 4 && columns <= 65535 ? launch_pdl(ssd_prep4_kernel, dim3((m + PREP_TOKENS - 1) / PREP_TOKENS, columns), dim3(256), 0, st, *a, m, xbc, dt, la)
+    const uint32_t per = prep_tokens(m, columns, ctx_sm_count(ctx));
+    const cudaError_t e = a->taps == 4 && columns <= 65535 ? launch_pdl(ssd_prep4_kernel, dim3((m + per - 1) / per, columns), dim3(256), 0, st, *a, m, per, xbc, dt, la)
                                                            : launch_pdl(ssd_prep_kernel, dim3(m), dim3(256), 0, st, *a, xbc, dt, la);
     return ctx_cuda_result(ctx, e, "ssd_prep", 1);
 }

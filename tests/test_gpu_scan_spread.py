@@ -32,3 +32,50 @@ def test_many_heads(gpu_ctx, heads, state, vdim, m):
     bound = 2 ** -24 * (state + m)
     assert (y.view_as(want).double() - want).norm() < bound * want.norm()
     assert (s[..., :state].double() - S0).norm() < bound * S0.norm()
+
+
+# tokens of a CTA: 1 .. 16, by the size of the portion; the last CTA's share is shorter
+@pytest.mark.parametrize("m,at", [(1, 5), (2, 0), (7, 3), (17, 1), (130, 2), (700, 0), (2100, 6)])
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 40, 24), (16, 128, 128), (6, 200, 300)])
+def test_convolution_inputs(gpu_ctx, m, at, heads, dim, vdim):
+    """delta_prep and ssd_prep behind `at` earlier tokens of a sequence (four taps)."""
+    sop, g, kvh = S.SeqOps(gpu_ctx), torch.Generator(device=DEV).manual_seed(m + dim), heads // 2
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)
+    pos = torch.tensor([at], dtype=torch.int32, device=DEV)
+
+    def ring(x):                                          # the last three inputs before `at`, column t % 4 of a channel
+        st = torch.zeros(x.shape[1], 4, device=DEV)
+        for t in range(max(0, at - 3), at):
+            st[:, t % 4] = x[t]
+        return st
+
+    def conv(x, w, bias=0.0):
+        ext = torch.cat([torch.zeros(3, x.shape[1], dtype=torch.float64, device=DEV), x.double()])
+        y = sum(ext[j:j + len(x)] * w.double()[:, j] for j in range(4)) + bias
+        return (y * torch.sigmoid(y))[at:]
+
+    close = lambda got, want: (got.double() - want).norm() <= 1e-6 * want.norm()          # four products and a few functions in f32
+    C1 = 2 * kvh * dim + heads * vdim
+    x, low = rand(at + m, C1 + heads), rand(at + m, 16)
+    proj, w = torch.cat([x, low], 1).contiguous(), rand(C1, 4)
+    qkv, beta, a1, g1, one = rand(m, C1), rand(m, heads), rand(m, 8), rand(m, 8), rand(heads * dim)
+    a = S.struct(S.Delta, proj=proj[at:], ld=proj.shape[1], q_off=0, k_off=kvh * dim, v_off=2 * kvh * dim, b_off=C1, a1_off=C1 + heads, g1_off=C1 + heads + 8,
+                 q_conv=w, k_conv=w[kvh * dim:], v_conv=w[2 * kvh * dim:], a_log=one, dt_bias=one, a2=one, g2=one, conv_state=(st := ring(x[:, :C1])), s=one, pos=pos,
+                 heads=heads, kv_heads=kvh, dim=dim, vdim=vdim, taps=4, a_rank_ld=8, g_rank_ld=8)
+    sop.delta_prep(a, m, qkv, beta, a1, g1)
+    y = conv(x[:, :C1], w)
+    q, k = (y[:, i * kvh * dim:(i + 1) * kvh * dim].view(m, kvh, dim) for i in (0, 1))
+    unit = lambda v: v / (v.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    assert close(qkv, torch.cat([(unit(q) * dim ** -0.5).reshape(m, -1), unit(k).reshape(m, -1), y[:, 2 * kvh * dim:]], 1))
+    assert close(beta, torch.sigmoid(x[at:, C1:].double()))
+    assert torch.equal(a1, low[at:, :8]) and torch.equal(g1, low[at:, 8:])
+    C2 = heads * vdim + 2 * dim
+    x, w, bias, dt_bias, a_log = rand(at + m, C2 + heads), rand(C2, 4), rand(C2), rand(heads), rand(heads)
+    xbc, dt, la = rand(m, C2), rand(m, heads), rand(m, heads)
+    b = S.struct(S.Ssd, proj=x[at:], ld=C2 + heads, off=0, conv=w, conv_bias=bias, dt_bias=dt_bias, a_log=a_log, d=one, conv_state=(st2 := ring(x[:, :C2])), s=one,
+                 heads=heads, groups=1, state=dim, vdim=vdim, taps=4, pos=pos)
+    sop.ssd_prep(b, m, xbc, dt, la)
+    gpu_ctx.check_status()
+    assert close(xbc, conv(x[:, :C2], w, bias.double()))
+    steps = torch.nn.functional.softplus(x[at:, C2:].double() + dt_bias.double())
+    assert close(dt, steps) and close(la, -torch.exp(a_log.double()) * steps)
