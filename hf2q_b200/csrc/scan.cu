@@ -25,7 +25,7 @@ namespace {
 using namespace seq;
 
 constexpr int SC_WARPS = 8, SC_COLS = 16, SC_THREADS = SC_WARPS * 32;       // one-token kernels: a group to a column
-constexpr int SC_TB = 32;                                                   // scans: tokens of a batch
+constexpr int SC_TB = 32, SC_FEW = 8;                                       // scans: tokens of a batch, and of one of a short portion
 
 __device__ __forceinline__ float group_sum(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -142,25 +142,25 @@ struct ScanPlace {
         fetches = warp == W;
     }
 };
-// Batches of SC_TB tokens in two buffers: stage(t0, buffer) by the fetching warp, batch(t0, buffer, tokens) by the others.
-template <typename Stage, typename Batch>
+// Batches of TB tokens in two buffers: stage(t0, buffer) by the fetching warp, batch(t0, buffer, tokens) by the others.
+template <uint32_t TB, typename Stage, typename Batch>
 __device__ __forceinline__ void scan_batches(bool fetches, uint32_t m, Stage stage, Batch batch) {
     if (fetches) { stage(0u, 0u); cp_async_wait<0>(); }
     __syncthreads();
-    for (uint32_t t0 = 0, b = 0; t0 < m; t0 += SC_TB, b ^= 1) {
+    for (uint32_t t0 = 0, b = 0; t0 < m; t0 += TB, b ^= 1) {
         if (fetches) {
-            if (t0 + SC_TB < m) { stage(t0 + SC_TB, b ^ 1); cp_async_wait<0>(); }
+            if (t0 + TB < m) { stage(t0 + TB, b ^ 1); cp_async_wait<0>(); }
         } else {
-            batch(t0, b, min(static_cast<uint32_t>(SC_TB), m - t0));
+            batch(t0, b, min(TB, m - t0));
         }
         __syncthreads();
     }
 }
 // The whole groups of a batch's n tokens: form(j0, sums) makes a lane's partial sums, done(j0, sums) adds them up and stores.
 // A group's sums are finished beside the next group's tokens, whose arithmetic hides the shuffles.  Returns the tokens taken.
-template <typename Sums, uint32_t GROUP, typename Form, typename Done>
+template <typename Sums, uint32_t GROUP, uint32_t TB, typename Form, typename Done>
 __device__ __forceinline__ uint32_t scan_groups(uint32_t n, Form form, Done done) {
-    if (n < GROUP) return 0;
+    if (TB < GROUP || n < GROUP) return 0;
     Sums last;
     form(0u, last);
     uint32_t j0 = GROUP;
@@ -190,17 +190,17 @@ inline size_t scan_smem(size_t need, dim3 grid, int sms) {
 
 // ---------------------------------------------------------------- mLSTM
 // A CTA carries the 16 columns that share a normaliser and a maximum.
-template <int RQ, int C>
-__global__ void __launch_bounds__((8 / C + 1) * 32, 1) mlstm_kernel(const __grid_constant__ hf2q_mlstm a, uint32_t m, float* __restrict__ out) {
+template <int RQ, int C, uint32_t TB>
+__global__ void __launch_bounds__((8 / C + 1) * 32, TB == SC_TB ? 1 : 2) mlstm_kernel(const __grid_constant__ hf2q_mlstm a, uint32_t m, float* __restrict__ out) {
     constexpr uint32_t W = 8 / C;
     using Place = ScanPlace<RQ, C, W>;
     constexpr uint32_t DP = Place::DP;
-    extern __shared__ __align__(16) float dsm[];                    // k, q: [2][SC_TB][DP] each
+    extern __shared__ __align__(16) float dsm[];                    // k, q: [2][TB][DP] each
     float* ks = dsm;
-    float* qs = dsm + 2 * SC_TB * DP;
-    __shared__ __align__(16) float vs[2][SC_TB][SC_COLS];
-    __shared__ __align__(8) float2 gs[2][SC_TB];                    // keep, write
-    __shared__ float ge[2][SC_TB];                                  // exp(-maximum)
+    float* qs = dsm + 2 * TB * DP;
+    __shared__ __align__(16) float vs[2][TB][SC_COLS];
+    __shared__ __align__(8) float2 gs[2][TB];                    // keep, write
+    __shared__ float ge[2][TB];                                  // exp(-maximum)
     pdl_trigger();
     pdl_wait();
     const uint32_t h = blockIdx.x, slice = blockIdx.y, n_slices = gridDim.y;
@@ -208,12 +208,12 @@ __global__ void __launch_bounds__((8 / C + 1) * 32, 1) mlstm_kernel(const __grid
     const float q_scale = 1.0f / sqrtf(static_cast<float>(a.dim));
     float* mp = a.mx + static_cast<size_t>(h) * n_slices + slice;
     float mx = *mp;                                          // carried by the fetching warp
-    clear_padding(dsm, 4 * SC_TB * DP, a.dim < DP);
+    clear_padding(dsm, 4 * TB * DP, a.dim < DP);
     auto stage = [&](uint32_t t0, uint32_t b) {
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0), lane = at.lane;
+        const uint32_t n = min(TB, m - t0), lane = at.lane;
         const float* row = a.proj + static_cast<size_t>(t0) * a.ld;
-        stage_rows(ks + b * SC_TB * DP, DP, row + a.k_off + h * a.dim, a.ld, n, a.dim);
-        stage_rows(qs + b * SC_TB * DP, DP, row + a.q_off + h * a.dim, a.ld, n, a.dim);
+        stage_rows(ks + b * TB * DP, DP, row + a.k_off + h * a.dim, a.ld, n, a.dim);
+        stage_rows(qs + b * TB * DP, DP, row + a.q_off + h * a.dim, a.ld, n, a.dim);
         stage_rows(vs[b][0], SC_COLS, row + a.v_off + h * a.vdim + at.col0, a.ld, n, at.n_cols);
         cp_async_commit();
         // gate factors of the batch (lane = token): the running maximum is a max-plus scan over the pairs (f, i),
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__((8 / C + 1) * 32, 1) mlstm_kernel(const __grid
         }
         const float f_own = f, x_own = x;
 #pragma unroll
-        for (int d = 1; d < SC_TB; d *= 2) {
+        for (int d = 1; d < TB; d *= 2) {
             const float fo = __shfl_up_sync(0xffffffffu, f, d), xo = __shfl_up_sync(0xffffffffu, x, d);
             if (lane >= d) { x = fmaxf(xo + f, x); f += fo; }
         }
@@ -248,13 +248,13 @@ __global__ void __launch_bounds__((8 / C + 1) * 32, 1) mlstm_kernel(const __grid
             if (at.col + c < a.vdim) S[c].load(sp + c * DP); else S[c].zero();
         N.load(np);
     }
-    scan_batches(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
+    scan_batches<TB>(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
         // a token's operands are read one token ahead of their use
         struct Operands { Vec<RQ> k, q; float2 g; float v[C]; };
         auto fetch = [&](uint32_t j) {
             Operands t;
-            t.k.load(ks + (b * SC_TB + j) * DP + 2 * at.lg);
-            t.q.load(qs + (b * SC_TB + j) * DP + 2 * at.lg);
+            t.k.load(ks + (b * TB + j) * DP + 2 * at.lg);
+            t.q.load(qs + (b * TB + j) * DP + 2 * at.lg);
             t.g = gs[b][j];
             load_values(t.v, &vs[b][j][at.group * C]);
             return t;
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__((8 / C + 1) * 32, 1) mlstm_kernel(const __grid
                 out[static_cast<size_t>(t0 + j) * a.heads * a.vdim + static_cast<size_t>(h) * a.vdim + col] = num * q_scale / (fmaxf(fabsf(den * q_scale), ge[b][j]) + 1e-6f);
         };
         struct Sums { float num[16], den[Place::GROUP]; };
-        uint32_t j0 = scan_groups<Sums, Place::GROUP>(
+        uint32_t j0 = scan_groups<Sums, Place::GROUP, TB>(
             n,
             [&](uint32_t j, Sums& r) {
                 Operands t = fetch(j);
@@ -324,30 +324,30 @@ __device__ __forceinline__ float delta_token(Vec<RQ>& S, const DeltaOperands<RQ>
     return S.dot(t.q);
 }
 
-template <int RQ, int C, int W, int PER_SM>
+template <int RQ, int C, int W, uint32_t TB, int PER_SM>
 __global__ void __launch_bounds__((W + 1) * 32, PER_SM) delta_scan_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, const float* __restrict__ qkv,
                                                                   const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ out) {
     using Place = ScanPlace<RQ, C, W>;
     constexpr uint32_t DP = Place::DP;
-    extern __shared__ __align__(16) float dsm[];                    // k, q, g: [2][SC_TB][DP] each
+    extern __shared__ __align__(16) float dsm[];                    // k, q, g: [2][TB][DP] each
     float* ks = dsm;
-    float* qs = dsm + 2 * SC_TB * DP;
-    float* gs = dsm + 4 * SC_TB * DP;
-    __shared__ __align__(16) float vs[2][SC_TB][Place::COLS];
-    __shared__ float bs[2][SC_TB];
+    float* qs = dsm + 2 * TB * DP;
+    float* gs = dsm + 4 * TB * DP;
+    __shared__ __align__(16) float vs[2][TB][Place::COLS];
+    __shared__ float bs[2][TB];
     pdl_trigger();
     pdl_wait();
     const uint32_t h = blockIdx.x, kvh = h / (a.heads / a.kv_heads);
     const Place at(blockIdx.y, a.vdim);
     const uint32_t qk = a.kv_heads * a.dim, ld = 2 * qk + a.heads * a.vdim;
-    clear_padding(dsm, 6 * SC_TB * DP, a.dim < DP);
+    clear_padding(dsm, 6 * TB * DP, a.dim < DP);
     auto stage = [&](uint32_t t0, uint32_t b) {
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
+        const uint32_t n = min(TB, m - t0);
         const float* row = qkv + static_cast<size_t>(t0) * ld;
-        stage_rows(qs + b * SC_TB * DP, DP, row + kvh * a.dim, ld, n, a.dim);
-        stage_rows(ks + b * SC_TB * DP, DP, row + qk + kvh * a.dim, ld, n, a.dim);
+        stage_rows(qs + b * TB * DP, DP, row + kvh * a.dim, ld, n, a.dim);
+        stage_rows(ks + b * TB * DP, DP, row + qk + kvh * a.dim, ld, n, a.dim);
         stage_rows(vs[b][0], Place::COLS, row + 2 * qk + h * a.vdim + at.col0, ld, n, at.n_cols);
-        stage_rows(gs + b * SC_TB * DP, DP, g + (static_cast<size_t>(t0) * a.heads + h) * a.dim, static_cast<size_t>(a.heads) * a.dim, n, a.dim);
+        stage_rows(gs + b * TB * DP, DP, g + (static_cast<size_t>(t0) * a.heads + h) * a.dim, static_cast<size_t>(a.heads) * a.dim, n, a.dim);
         if (at.lane < n) cp_async4(&bs[b][at.lane], beta + static_cast<size_t>(t0 + at.lane) * a.heads + h);
         cp_async_commit();
     };
@@ -358,10 +358,10 @@ __global__ void __launch_bounds__((W + 1) * 32, PER_SM) delta_scan_kernel(const 
         for (int c = 0; c < C; ++c)
             if (at.col + c < a.vdim) S[c].load(sp + c * DP); else S[c].zero();
     }
-    scan_batches(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
+    scan_batches<TB>(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
         struct Operands { Vec<RQ> g, k, q; float v[C], beta; };
         auto fetch = [&](uint32_t j) {                       // read one step ahead of their use
-            const uint32_t o = (b * SC_TB + j) * DP + 2 * at.lg;
+            const uint32_t o = (b * TB + j) * DP + 2 * at.lg;
             Operands t;
             t.g.load(gs + o);
             t.k.load(ks + o);
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__((W + 1) * 32, PER_SM) delta_scan_kernel(const 
         float* dst = out + static_cast<size_t>(t0) * a.heads * a.vdim + static_cast<size_t>(h) * a.vdim;
         const size_t row_o = static_cast<size_t>(a.heads) * a.vdim;
         struct Sums { float r[16]; };
-        uint32_t j0 = scan_groups<Sums, Place::GROUP>(
+        uint32_t j0 = scan_groups<Sums, Place::GROUP, TB>(
             n,
             [&](uint32_t j, Sums& s) {
                 Operands t1 = fetch(j), t2 = fetch(j + 1);
@@ -699,16 +699,16 @@ __global__ void __launch_bounds__(256) delta_decay_kernel(const float* __restric
 __device__ __forceinline__ uint32_t ssd_channels(const hf2q_ssd& a) { return a.heads * a.vdim + 2 * a.groups * a.state; }
 
 // S <- keep S + dt B x^T;  y = S^T C + d x
-template <int RQ, int C, int W>
-__global__ void __launch_bounds__((W + 1) * 32, 1) ssd_scan_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, const float* __restrict__ xbc,
+template <int RQ, int C, int W, uint32_t TB>
+__global__ void __launch_bounds__((W + 1) * 32, TB == SC_TB ? 1 : RQ <= 4 ? 4 : 2) ssd_scan_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, const float* __restrict__ xbc,
                                                                 const float* __restrict__ dt, const float* __restrict__ la, float* __restrict__ y) {
     using Place = ScanPlace<RQ, C, W>;
     constexpr uint32_t DP = Place::DP;
-    extern __shared__ __align__(16) float dsm[];                    // B, C: [2][SC_TB][DP] each
+    extern __shared__ __align__(16) float dsm[];                    // B, C: [2][TB][DP] each
     float* ks = dsm;
-    float* qs = dsm + 2 * SC_TB * DP;
-    __shared__ __align__(16) float vs[2][SC_TB][Place::COLS];
-    __shared__ __align__(8) float2 gs[2][SC_TB];                    // decay, step size
+    float* qs = dsm + 2 * TB * DP;
+    __shared__ __align__(16) float vs[2][TB][Place::COLS];
+    __shared__ __align__(8) float2 gs[2][TB];                    // decay, step size
     pdl_trigger();
     pdl_wait();
     const uint32_t h = blockIdx.x, grp = h / (a.heads / a.groups);
@@ -720,12 +720,12 @@ __global__ void __launch_bounds__((W + 1) * 32, 1) ssd_scan_kernel(const __grid_
         for (uint32_t j = 0; j < keep; ++j)
             a.conv_state[static_cast<size_t>(i) * a.taps + (pos + m - 1 - j) % a.taps] = a.proj[static_cast<size_t>(m - 1 - j) * a.ld + a.off + i];
     }
-    clear_padding(dsm, 4 * SC_TB * DP, a.state < DP);
+    clear_padding(dsm, 4 * TB * DP, a.state < DP);
     auto stage = [&](uint32_t t0, uint32_t b) {
-        const uint32_t n = min(static_cast<uint32_t>(SC_TB), m - t0);
+        const uint32_t n = min(TB, m - t0);
         const float* row = xbc + static_cast<size_t>(t0) * channels;
-        stage_rows(ks + b * SC_TB * DP, DP, row + inner + grp * a.state, channels, n, a.state);
-        stage_rows(qs + b * SC_TB * DP, DP, row + inner + (a.groups + grp) * a.state, channels, n, a.state);
+        stage_rows(ks + b * TB * DP, DP, row + inner + grp * a.state, channels, n, a.state);
+        stage_rows(qs + b * TB * DP, DP, row + inner + (a.groups + grp) * a.state, channels, n, a.state);
         stage_rows(vs[b][0], Place::COLS, row + h * a.vdim + at.col0, channels, n, at.n_cols);
         cp_async_commit();
         if (at.lane < n) {
@@ -741,12 +741,12 @@ __global__ void __launch_bounds__((W + 1) * 32, 1) ssd_scan_kernel(const __grid_
         for (int c = 0; c < C; ++c)
             if (at.col + c < a.vdim) S[c].load(sp + c * DP); else S[c].zero();
     }
-    scan_batches(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
+    scan_batches<TB>(at.fetches, m, stage, [&](uint32_t t0, uint32_t b, uint32_t n) {
         struct Operands { Vec<RQ> k, q; float2 g; float v[C]; };
         auto fetch = [&](uint32_t j) {                       // read one token ahead of their use
             Operands t;
-            t.k.load(ks + (b * SC_TB + j) * DP + 2 * at.lg);
-            t.q.load(qs + (b * SC_TB + j) * DP + 2 * at.lg);
+            t.k.load(ks + (b * TB + j) * DP + 2 * at.lg);
+            t.q.load(qs + (b * TB + j) * DP + 2 * at.lg);
             t.g = gs[b][j];
             load_values(t.v, &vs[b][j][at.group * C]);
             return t;
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__((W + 1) * 32, 1) ssd_scan_kernel(const __grid_
             if (at.col + c < a.vdim) y[static_cast<size_t>(t0 + j) * inner + static_cast<size_t>(h) * a.vdim + at.col + c] = s + skip * vs[b][j][at.group * C + c];
         };
         struct Sums { float r[16]; };
-        uint32_t j0 = scan_groups<Sums, Place::GROUP>(
+        uint32_t j0 = scan_groups<Sums, Place::GROUP, TB>(
             n,
             [&](uint32_t j, Sums& s) {
                 Operands t = fetch(j);
@@ -894,14 +894,23 @@ bool ssd_ok(const hf2q_ssd* a) {
     return a && a->proj && a->conv && a->conv_bias && a->dt_bias && a->a_log && a->d && a->conv_state && a->s && a->pos && a->heads && a->groups &&
            a->heads % a->groups == 0 && a->state && a->state <= 256 && a->vdim && a->taps;
 }
-template <int RQ, int C, int W>
-cudaError_t launch_ssd_scan(const hf2q_ssd& a, uint32_t m, const float* xbc, const float* dt, const float* la, float* y, int sms, cudaStream_t st) {
+template <int RQ, int C, int W, uint32_t TB>
+cudaError_t launch_ssd_scan_as(const hf2q_ssd& a, uint32_t m, const float* xbc, const float* dt, const float* la, float* y, int sms, cudaStream_t st) {
     static PerDeviceFlag flag;
-    constexpr size_t need = 4ull * SC_TB * 32 * RQ * sizeof(float);
+    constexpr size_t need = 4ull * TB * 32 * RQ * sizeof(float);
     constexpr uint32_t cols = ScanPlace<RQ, C, W>::COLS;
     const dim3 grid(a.heads, (a.vdim + cols - 1) / cols);
-    if (const cudaError_t e = ensure_max_dynamic_smem(ssd_scan_kernel<RQ, C, W>, SCAN_MAX, flag); e != cudaSuccess) return e;
-    return launch_pdl(ssd_scan_kernel<RQ, C, W>, grid, dim3((W + 1) * 32), scan_smem(need, grid, sms), st, a, m, xbc, dt, la, y);
+    if (const cudaError_t e = ensure_max_dynamic_smem(ssd_scan_kernel<RQ, C, W, TB>, SCAN_MAX, flag); e != cudaSuccess) return e;
+    return launch_pdl(ssd_scan_kernel<RQ, C, W, TB>, grid, dim3((W + 1) * 32), TB == SC_TB ? scan_smem(need, grid, sms) : need, st, a, m, xbc, dt, la, y);
+}
+// Few tokens and more CTAs than SMs: one column a group in batches of 8, four CTAs to an SM (128 heads of 128 x 64, 5 tokens:
+// 5.8 us, with two columns 6.6; 64 heads: 5.2 and 4.4).
+template <int RQ>
+cudaError_t launch_ssd_scan(const hf2q_ssd& a, uint32_t m, const float* xbc, const float* dt, const float* la, float* y, int sms, cudaStream_t st) {
+    constexpr uint32_t cols = ScanPlace<RQ, 2, 8>::COLS;
+    if (m < 8 && static_cast<uint64_t>(a.heads) * ((a.vdim + cols - 1) / cols) > static_cast<uint64_t>(sms))
+        return launch_ssd_scan_as<RQ, 1, 8, SC_FEW>(a, m, xbc, dt, la, y, sms, st);
+    return launch_ssd_scan_as<RQ, 2, 8, SC_TB>(a, m, xbc, dt, la, y, sms, st);
 }
 
 bool delta_ok(const hf2q_delta* a) {
@@ -909,20 +918,25 @@ bool delta_ok(const hf2q_delta* a) {
            a->heads && a->kv_heads && a->heads % a->kv_heads == 0 && a->dim && a->dim <= 256 && a->vdim && a->taps && a->a_rank_ld % 8 == 0 &&
            a->g_rank_ld % 8 == 0 && a->a_rank_ld && a->g_rank_ld;
 }
-template <int RQ, int C, int W, int PER_SM>
-cudaError_t launch_scan_as(const hf2q_delta& a, uint32_t m, const float* qkv, const float* beta, const float* g, float* out, dim3 grid, int sms, cudaStream_t st) {
+template <int RQ, int C, int W, uint32_t TB, int PER_SM>
+cudaError_t launch_scan_as(const hf2q_delta& a, uint32_t m, const float* qkv, const float* beta, const float* g, float* out, int sms, cudaStream_t st) {
     static PerDeviceFlag flag;
-    constexpr size_t need = 6ull * SC_TB * 32 * RQ * sizeof(float);
-    if (const cudaError_t e = ensure_max_dynamic_smem(delta_scan_kernel<RQ, C, W, PER_SM>, SCAN_MAX, flag); e != cudaSuccess) return e;
-    return launch_pdl(delta_scan_kernel<RQ, C, W, PER_SM>, grid, dim3((W + 1) * 32), scan_smem(need, grid, sms), st, a, m, qkv, beta, g, out);
+    constexpr size_t need = 6ull * TB * 32 * RQ * sizeof(float);
+    constexpr uint32_t cols = ScanPlace<RQ, C, W>::COLS;
+    const dim3 grid(a.heads, (a.vdim + cols - 1) / cols);
+    if (const cudaError_t e = ensure_max_dynamic_smem(delta_scan_kernel<RQ, C, W, TB, PER_SM>, SCAN_MAX, flag); e != cudaSuccess) return e;
+    return launch_pdl(delta_scan_kernel<RQ, C, W, TB, PER_SM>, grid, dim3((W + 1) * 32), TB == SC_TB ? scan_smem(need, grid, sms) : need, st, a, m, qkv, beta, g, out);
 }
-// More CTAs than SMs: two to an SM where the batches of both fit (dim up to 128), which costs a CTA alone 6 % (200 registers)
+// Few tokens: one column a group and batches of 8, as below (16 heads of 256 x 256: 33 tokens 27.3 us with two columns a group;
+// of 128 x 128: 8 tokens 5.6 with one, 3.9 with two).  More CTAs than SMs: two to an SM where the batches of both fit (dim up to
+// 128), which costs a CTA alone 6 % (200 registers).
 template <int RQ>
 cudaError_t launch_scan(const hf2q_delta& a, uint32_t m, const float* qkv, const float* beta, const float* g, float* out, int sms, cudaStream_t st) {
+    if (m < (RQ > 4 ? 64u : 8u)) return launch_scan_as<RQ, 1, 8, SC_FEW, 2>(a, m, qkv, beta, g, out, sms, st);
     constexpr uint32_t cols = ScanPlace<RQ, 2, 4>::COLS;
-    const dim3 grid(a.heads, (a.vdim + cols - 1) / cols);
-    if (RQ <= 4 && static_cast<uint64_t>(grid.x) * grid.y > static_cast<uint64_t>(sms)) return launch_scan_as<RQ, 2, 4, RQ <= 4 ? 2 : 1>(a, m, qkv, beta, g, out, grid, sms, st);
-    return launch_scan_as<RQ, 2, 4, 1>(a, m, qkv, beta, g, out, grid, sms, st);
+    if (RQ <= 4 && static_cast<uint64_t>(a.heads) * ((a.vdim + cols - 1) / cols) > static_cast<uint64_t>(sms))
+        return launch_scan_as<RQ, 2, 4, SC_TB, RQ <= 4 ? 2 : 1>(a, m, qkv, beta, g, out, sms, st);
+    return launch_scan_as<RQ, 2, 4, SC_TB, 1>(a, m, qkv, beta, g, out, sms, st);
 }
 
 // four taps, as such layers are built; other counts a CTA a token
@@ -936,18 +950,22 @@ cudaError_t launch_delta_prep(const hf2q_delta& a, uint32_t m, float* qkv, float
     return launch_pdl(delta_prep4_kernel<8, LR>, grid, dim3(256), 0, st, a, m, per, qk_columns, qkv, beta, a1, g1);
 }
 
-template <int RQ, int C>
+template <int RQ, int C, uint32_t TB>
 cudaError_t launch_mlstm_as(const hf2q_mlstm& a, uint32_t m, float* out, int sms, cudaStream_t st) {
     static PerDeviceFlag flag;
-    constexpr size_t need = 4ull * SC_TB * 32 * RQ * sizeof(float);
+    constexpr size_t need = 4ull * TB * 32 * RQ * sizeof(float);
     const dim3 grid(a.heads, (a.vdim + SC_COLS - 1) / SC_COLS);
-    if (const cudaError_t e = ensure_max_dynamic_smem(mlstm_kernel<RQ, C>, SCAN_MAX, flag); e != cudaSuccess) return e;
-    return launch_pdl(mlstm_kernel<RQ, C>, grid, dim3((8 / C + 1) * 32), m == 1 ? need : scan_smem(need, grid, sms), st, a, m, out);
+    if (const cudaError_t e = ensure_max_dynamic_smem(mlstm_kernel<RQ, C, TB>, SCAN_MAX, flag); e != cudaSuccess) return e;
+    return launch_pdl(mlstm_kernel<RQ, C, TB>, grid, dim3((8 / C + 1) * 32), TB == SC_TB ? scan_smem(need, grid, sms) : need, st, a, m, out);
 }
-// one token: every warp reads as little of the state as it can
+// Few tokens (a decode step among them): what counts is how soon a token's chain starts and that the CTAs share the SMs, so one
+// column a group, eight warps, and a batch of 8 tokens, whose buffers let several CTAs on an SM.  The line lies where two columns
+// a group take whole groups of tokens: 16 heads of 128 x 128, 8 tokens 6.0 us with one column, 3.7 with two; 5 tokens 4.8 and
+// 4.8.  32 such heads, one token: 3.4 us, a CTA an SM took 5.3.
 template <int RQ>
 cudaError_t launch_mlstm(const hf2q_mlstm& a, uint32_t m, float* out, int sms, cudaStream_t st) {
-    return m == 1 ? launch_mlstm_as<RQ, 1>(a, m, out, sms, st) : launch_mlstm_as<RQ, 2>(a, m, out, sms, st);
+    if (m < (RQ > 4 ? 16u : 8u)) return launch_mlstm_as<RQ, 1, SC_FEW>(a, m, out, sms, st);
+    return launch_mlstm_as<RQ, 2, SC_TB>(a, m, out, sms, st);
 }
 
 #define HF2Q_RQ_CASES(F) F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8)
@@ -1063,7 +1081,7 @@ HF2Q_API int32_t hf2q_cuda_ssd_scan(hf2q_ctx* ctx, void* stream, const hf2q_ssd*
     if (m == 0) return HF2Q_OK;
     cudaError_t e = cudaErrorInvalidValue;
     switch ((a->state + 31) / 32) {
-#define F(RQ) case RQ: e = launch_ssd_scan<RQ, 2, 8>(*a, m, xbc, dt, la, y, ctx_sm_count(ctx), static_cast<cudaStream_t>(stream)); break;
+#define F(RQ) case RQ: e = launch_ssd_scan<RQ>(*a, m, xbc, dt, la, y, ctx_sm_count(ctx), static_cast<cudaStream_t>(stream)); break;
         HF2Q_RQ_CASES(F)
 #undef F
         default: break;

@@ -34,6 +34,70 @@ def test_many_heads(gpu_ctx, heads, state, vdim, m):
     assert (s[..., :state].double() - S0).norm() < bound * S0.norm()
 
 
+# portions of one batch of tokens or several, of up to 8 tokens (one column a lane group) or more (two), on fewer or more CTAs than SMs
+PORTIONS = [(6, 128, 128, 1), (32, 128, 128, 8), (32, 128, 128, 9), (150, 40, 9, 33), (19, 64, 130, 70), (3, 256, 33, 40), (16, 256, 256, 16), (20, 100, 128, 3)]
+
+
+@pytest.mark.parametrize("heads,dim,vdim,m", PORTIONS)
+def test_delta_portions(gpu_ctx, heads, dim, vdim, m):
+    sop, g, kvh = S.SeqOps(gpu_ctx), torch.Generator(device=DEV).manual_seed(heads + m), heads if heads % 2 else heads // 2
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k, v = unit(rand(m, kvh, dim)) * dim ** -0.5, unit(rand(m, kvh, dim)), rand(m, heads, vdim)
+    qkv = torch.cat([x.reshape(m, -1) for x in (q, k, v)], 1).contiguous()
+    beta, decay = torch.rand((m, heads), generator=g, device=DEV), torch.exp(-0.1 * torch.rand((m, heads, dim), generator=g, device=DEV))
+    s = rand(heads, vdim, S.pad32(dim))
+    s[..., dim:] = 0
+    S0, out, one, pos = s[..., :dim].double(), torch.empty(m, heads * vdim, device=DEV), rand(heads * 8), torch.zeros(1, dtype=torch.int32, device=DEV)
+    a = S.struct(S.Delta, proj=one, ld=8, q_conv=one, k_conv=one, v_conv=one, a_log=one, dt_bias=one, a2=one, g2=one, conv_state=one, s=s, pos=pos,
+                 heads=heads, kv_heads=kvh, dim=dim, vdim=vdim, taps=4, a_rank_ld=8, g_rank_ld=8)
+    sop.delta_scan(a, m, qkv, beta, decay, out)
+    gpu_ctx.check_status()
+    Q, K = (x.double().repeat_interleave(heads // kvh, 1) for x in (q, k))
+    want = torch.empty(m, heads, vdim, dtype=torch.float64, device=DEV)
+    for t in range(m):
+        S0 = S0 * decay[t].double()[:, None]
+        u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hvk,hk->hv", S0, K[t]))
+        S0 = S0 + u[..., None] * K[t][:, None]
+        want[t] = torch.einsum("hvk,hk->hv", S0, Q[t])
+    bound = 2 ** -24 * (dim + m)                          # as above
+    assert (out.view_as(want).double() - want).norm() < bound * want.norm()
+    assert (s[..., :dim].double() - S0).norm() < bound * S0.norm()
+    assert (s[..., dim:] == 0).all()
+
+
+@pytest.mark.parametrize("heads,dim,vdim,m", PORTIONS)
+def test_mlstm_portions(gpu_ctx, heads, dim, vdim, m):
+    sop, g, cap = S.SeqOps(gpu_ctx), torch.Generator(device=DEV).manual_seed(heads + m), 15.0
+    o, slices = heads * (2 * dim + vdim), -(-vdim // 16)
+    proj = torch.randn((m, o + 2 * heads), generator=g, device=DEV)
+    proj[:, heads * dim:2 * heads * dim] += 0.5           # (normalisers away from zero, where a quotient keeps no digits)
+    proj[:, :heads * dim] += 0.5
+    ib, fb = torch.randn(heads, generator=g, device=DEV), 3 + torch.randn(heads, generator=g, device=DEV)
+    s, n, mx = torch.zeros(heads, vdim, S.pad32(dim), device=DEV), torch.zeros(heads, slices, S.pad32(dim), device=DEV), torch.zeros(heads, slices, device=DEV)
+    out = torch.empty(m, heads * vdim, device=DEV)
+    a = S.struct(S.MLstm, proj=proj, ld=proj.shape[1], q_off=0, k_off=heads * dim, v_off=2 * heads * dim, i_off=o, f_off=o + heads, i_bias=ib, f_bias=fb, s=s,
+                 n=n, mx=mx, heads=heads, dim=dim, vdim=vdim, gate_cap=cap)
+    sop.mlstm(a, m, out)
+    gpu_ctx.check_status()
+    P = proj.double()
+    q, k, v = (P[:, i:j].view(m, heads, -1) for i, j in ((0, heads * dim), (heads * dim, 2 * heads * dim), (2 * heads * dim, o)))
+    ig, fg = (cap * torch.tanh((P[:, i:i + heads] + b.double()) / cap) for i, b in ((o, ib), (o + heads, fb)))
+    fg = -torch.nn.functional.softplus(-fg)
+    S0, N, M = torch.zeros(heads, vdim, dim, dtype=torch.float64, device=DEV), torch.zeros(heads, dim, dtype=torch.float64, device=DEV), torch.zeros(heads, dtype=torch.float64, device=DEV)
+    want = torch.empty(m, heads, vdim, dtype=torch.float64, device=DEV)
+    for t in range(m):
+        new = torch.maximum(fg[t] + M, ig[t])
+        keep, write, M = torch.exp(fg[t] + M - new), torch.exp(ig[t] - new), new
+        S0, N = keep[:, None, None] * S0 + (write[:, None] * v[t])[..., None] * k[t][:, None], keep[:, None] * N + write[:, None] * k[t]
+        num, den = (torch.einsum(e, x, q[t]) * dim ** -0.5 for e, x in (("hvk,hk->hv", S0), ("hk,hk->h", N)))
+        want[t] = num / (torch.maximum(den.abs(), torch.exp(-M)) + 1e-6)[:, None]
+    bound = 2 ** -24 * (dim + 16 * m)                     # gate logarithms of up to 15 are carried in f32, over m tokens
+    assert (s[..., :dim].double() - S0).norm() < bound * S0.norm()
+    assert (out.view_as(want).double() - want).norm() < 4 * bound * want.norm()
+    assert (n[..., :dim].double() - N[:, None]).norm() < bound * N.norm() * slices ** 0.5
+
+
 # tokens of a CTA: 1 .. 16, by the size of the portion; the last CTA's share is shorter
 @pytest.mark.parametrize("m,at", [(1, 5), (2, 0), (7, 3), (17, 1), (130, 2), (700, 0), (2100, 6)])
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 40, 24), (16, 128, 128), (6, 200, 300)])
