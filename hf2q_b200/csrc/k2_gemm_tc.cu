@@ -63,8 +63,14 @@ constexpr int raw_stages_of(uint32_t type, int nt, bool grouped) {
 constexpr int a_bufs_of(int nt, bool grouped) { return two_ctas_of(nt, grouped) ? 1 : 2; }
 constexpr uint32_t tmem_cols_of(int nt, bool grouped) { return two_ctas_of(nt, grouped) ? 256u : 512u; }
 // activation stages: one stage is NT rows x 64 elements; keep ~128 KB of them in flight so that the
-// copies for the next K-blocks are issued long before the MMA warp needs them
-constexpr int x_stages_of(uint32_t type, int nt, bool grouped) {
+// copies for the next K-blocks are issued long before the MMA warp needs them.  A SwiGLU pair of 64 tokens whose K-blocks are shared
+// keeps as many as let two CTAs fit an SM, which the rule for their number counts on (with eight, Q6_K and Q8_0 took a second
+// wave: 6144 x 4096 at 64 rows in Q6_K 42.0 us, now 30.5; the plain product never has more CTAs than SMs)
+constexpr int x_stages_of(uint32_t type, int nt, bool grouped, bool shared_pair) {
+    if (shared_pair && nt == 64) {
+        const int fit = static_cast<int>((113 * 1024 - 1536 - 2 * TILE_N * tc_boxw(type)) / (64 * 128));
+        return fit < 8 ? fit : 8;
+    }
     return nt >= 256 ? (type == HF2Q_TYPE_Q8_0 ? 4 : 5) : (grouped && nt == 128) ? 3 : 8;
 }
 constexpr int DEQ_GROUPS = 2;                        // groups of 4 dequantiser warps; group g takes quarters g*2, g*2+1
@@ -146,7 +152,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     constexpr uint32_t X_STAGE = NT * 128;                       // NT rows x 64 f16, 128B-swizzled
-    constexpr int X_STAGES = x_stages_of(TYPE, NT, GROUPED);
+    constexpr int X_STAGES = x_stages_of(TYPE, NT, GROUPED, SHARED && DUAL);
+    static_assert(!SHARED || X_STAGES >= 4, "the sums of a shared tile lie over the activation stages");
     uint8_t* xs = smem;                                          // X_STAGES x X_STAGE (1024-aligned)
     constexpr int RAW_STAGES = raw_stages_of(TYPE, NT, GROUPED);
     constexpr uint32_t TILE_ROWS = DUAL ? 64 : TILE_N;           // output rows of one tile
@@ -516,7 +523,7 @@ cudaError_t launch_gemm_form(const CUtensorMap& tw, const CUtensorMap& tw2, cons
                              uint32_t parts) {
     auto kern = gemm_tc_kernel<TYPE, NT, GROUPED, DUAL, SHARED>;
     const size_t raw_stages = raw_stages_of(TYPE, NT, GROUPED);
-    const size_t smem = 1024 + static_cast<size_t>(x_stages_of(TYPE, NT, GROUPED)) * NT * 128 + raw_stages * TILE_N * p.boxw + 512;
+    const size_t smem = 1024 + static_cast<size_t>(x_stages_of(TYPE, NT, GROUPED, SHARED && DUAL)) * NT * 128 + raw_stages * TILE_N * p.boxw + 512;
     static PerDeviceFlag attr;
     if (const cudaError_t e = ensure_max_dynamic_smem(kern, 227 * 1024, attr); e != cudaSuccess) return e;
     const uint32_t tile_rows = DUAL ? 64 : TILE_N;
@@ -650,7 +657,9 @@ cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const 
     p.blk_bytes = KB / g.elems * g.bytes;
     p.status = status;
     const uint32_t tile_rows = dual ? 64 : TILE_N;
-    const uint32_t parts = gemm_tc_parts(m, n, k, sm_count), best_nt = gemm_tc_token_tile(m, (n + tile_rows - 1) / tile_rows, sm_count);
+    // the CTAs of all parts fill the chip: counted without them, 128 rows took tiles of 64 tokens and decoded every weight twice
+    // (pair of 4096 x 4096 in Q6_K: 44.3 us, now 25.0)
+    const uint32_t parts = gemm_tc_parts(m, n, k, sm_count), best_nt = gemm_tc_token_tile(m, (n + tile_rows - 1) / tile_rows * parts, sm_count);
     const uint32_t nt = parts > 1 && best_nt > 128 ? 128 : best_nt;
     alignas(64) CUtensorMap tw, tw2, tx;
     for (int which = 0; which < (dual ? 2 : 1); ++which) {

@@ -58,3 +58,23 @@ def test_shared_k_blocks(ctx, ggml_type, m, n, k):
     silu = torch.empty_like(y)
     ctx._check(ctx._lib.hf2q_cuda_silu_mul(ctx._h, ctx._stream(), y.data_ptr(), act.data_ptr(), silu.data_ptr(), y.numel()))
     assert torch.equal(both, silu)
+
+
+# products whose shares come as one or two CTAs an SM, in tiles of 64 or 128 tokens
+@pytest.mark.parametrize("ggml_type", [8, 13, 14])
+@pytest.mark.parametrize("m,n,k", [(33, 6144, 2048), (64, 6144, 2048), (100, 4096, 2048), (128, 4000, 2048), (300, 1024, 2048), (1000, 512, 2048)])
+def test_shares_of_wide_products(ctx, ggml_type, m, n, k):
+    test_shared_k_blocks(ctx, ggml_type, m, n, k)
+
+
+@pytest.mark.parametrize("m", [9, 130, 2500])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_activations_off_a_vector_boundary(ctx, m, dtype):
+    n, k = 64, 512
+    w = hq.load_quant_weight(ctx, make_quant_weight(12, n, k, seed=1), 12, n, k)
+    flat = torch.randn(m * k + 1, generator=torch.Generator().manual_seed(m)).to(dtype).cuda()
+    y, z = torch.empty((m, n), device="cuda"), torch.empty((m, n), device="cuda")
+    hq.quantized_matmul_ggml(ctx, flat[1:].view(m, k), w, y, w.matmul_params(m))
+    hq.quantized_matmul_ggml(ctx, flat[1:].clone().view(m, k), w, z, w.matmul_params(m))
+    ctx.check_status()
+    assert torch.equal(y, z) and y.isfinite().all()
