@@ -3,8 +3,8 @@
 // plain rows of keys and values, with a part of every key shared by the heads (expanded latents).
 //
 //   append    prefill: normalised queries to a buffer, normalised keys and values to the cache
-//   prefill   bf16 cache: tiles on the tensor cores (f32 scores, softmax and accumulators, bf16 product operands), of 128
-//             queries on tcgen05 where a key has 65..192 and a value up to 128 elements; f32 cache: one warp per query in f32
+//   prefill   bf16 cache: tiles on the tensor cores (f32 scores, softmax and accumulators, bf16 product operands): of 128
+//             queries on tcgen05 or of 64 on warps, by size (prefill_on_tcgen05); f32 cache: one warp per query in f32
 //   decode    one launch: norm, append, window split over CTAs, merge by the CTA that arrives last
 #include <math_constants.h>
 
@@ -663,7 +663,9 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
     if (again) wt_again<OUT, PLAIN>(a, pos0, t0, min(WT_Q, m - t0), h, q, gate, ldg, out, ldo, reinterpret_cast<float*>(smem));
 }
 
-// ---------------------------------------------------------------- prefill, bf16 cache, other sizes: warp-level products
+// ---------------------------------------------------------------- prefill, bf16 cache: warp-level products
+// 2048 queries x 16 heads with 2048 keys each take 147 us with 64 elements a key and value (on tcgen05, whose tiles hold 128 each,
+// 146), 952 with ring keys of 192 (no tcgen05 form of those is built; rows: 229) and 1328 with 256.
 constexpr int WP_WARPS = 4, WP_Q = 16 * WP_WARPS, WP_K = 64;
 
 // grid (query tiles, heads); DK >= dim + shared_dim, DV >= vdim.  Keys are walked from the first one the tile's first
@@ -897,18 +899,42 @@ cudaError_t launch_prefill_tc(const hf2q_window_attn& a, uint32_t m, const void*
     return launch_pdl(window_prefill_tc_kernel<DK, OUT, PLAIN>, dim3((m + WT_Q - 1) / WT_Q, a.heads), dim3(WT_THREADS), smem, st, a, m,
                       static_cast<const __nv_bfloat16*>(q), gate, ldg, static_cast<OUT*>(out), ldo, status);
 }
+// Keys of 65..128 (or values of 65..128 beside shorter keys), in tiles of 64 queries on warps or of 128 on tcgen05?  While the
+// tiles leave SMs idle both are bound by the latency of a block of 64 keys, 3.5 us on tcgen05 and, by the size of a key and a
+// value, 3.6 to 4.6 on warps, and tcgen05 pays 2 us more at the start and walks the longer tile; once two of the smaller tiles
+// stand on every SM it is the amount of work.  us, warps / tcgen05, with keys before the portion:
+//   128 + 128 elements, 16 heads, 256 queries: window 256 26.6 / 29.9, window 512 44.7 / 43.8, window 2048 153 / 128
+//                                2048 queries: window 64 30.5 / 24.7, window 2048 358 / 157
+//   96 + 64 elements, 16 heads, 256 queries: window 512 36.8 / 43.8, window 2048 125 / 130
+//                               1024 queries: window 256 30.4 / 33.7, window 512 50.9 / 49.9;  2048: window 256 50.2 / 37.1
+// Rows with a shared key part cost the warps more (64 + 32 and 64 elements, window 2048: 127 / 99 with 64 queries).
+bool prefill_on_tcgen05(const hf2q_window_attn& a, uint32_t m, int sms) {
+    const uint64_t tiles = static_cast<uint64_t>((m + WP_Q - 1) / WP_Q) * a.heads;
+    const uint32_t k = pad8(a.dim) + pad8(a.shared_dim);
+    if (a.linear && a.shared_dim) return a.window > 256 || tiles > 2ull * sms;
+    if (k + pad8(a.vdim) >= 224) return a.window > 256 || (a.window >= 64 && tiles > 2ull * sms);
+    return (a.window >= 512 && tiles > static_cast<uint64_t>(sms)) || (a.window >= 256 && tiles > 2ull * sms);
+}
 template <typename OUT>
-cudaError_t launch_prefill_mma(const hf2q_window_attn& a, uint32_t m, const void* q, const float* gate, uint32_t ldg, void* out, uint32_t ldo, uint32_t* status,
-                               cudaStream_t st) {
+cudaError_t launch_prefill_bf16(const hf2q_window_attn& a, uint32_t m, const void* q, const float* gate, uint32_t ldg, void* out, uint32_t ldo, uint32_t* status,
+                                int sms, cudaStream_t st) {
     const uint32_t k = pad8(a.dim) + pad8(a.shared_dim), v = a.vdim;
+    const bool tc = prefill_on_tcgen05(a, m, sms);
     if (a.linear) {
         if (k <= 64 && v <= 64) return launch_prefill_dm<64, 64, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
-        if (k <= 128 && v <= 128) return launch_prefill_tc<128, OUT, true>(a, m, q, gate, ldg, out, ldo, status, st);
+        if (k <= 128 && v <= 128) {
+            if (tc) return launch_prefill_tc<128, OUT, true>(a, m, q, gate, ldg, out, ldo, status, st);
+            return launch_prefill_dm<128, 128, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
+        }
+        // 192: on warps a block of 64 keys takes 7 us, so tcgen05 from the second block on (one block: 8.2 / 7.7)
         if (k <= 192 && v <= 128) return launch_prefill_tc<192, OUT, true>(a, m, q, gate, ldg, out, ldo, status, st);
         return launch_prefill_dm<QK_MAX, 256, OUT, true>(a, m, q, gate, ldg, out, ldo, st);
     }
     if (k <= 64 && v <= 64) return launch_prefill_dm<64, 64, OUT, false>(a, m, q, gate, ldg, out, ldo, st);
-    if (k <= 128 && v <= 128) return launch_prefill_tc<128, OUT, false>(a, m, q, gate, ldg, out, ldo, status, st);
+    if (k <= 128 && v <= 128) {
+        if (tc) return launch_prefill_tc<128, OUT, false>(a, m, q, gate, ldg, out, ldo, status, st);
+        return launch_prefill_dm<128, 128, OUT, false>(a, m, q, gate, ldg, out, ldo, st);
+    }
     return launch_prefill_dm<256, 256, OUT, false>(a, m, q, gate, ldg, out, ldo, st);
 }
 
@@ -966,9 +992,9 @@ HF2Q_API int32_t hf2q_cuda_window_attn_prefill(hf2q_ctx* ctx, void* stream, cons
         if (out_dtype == HF2Q_DT_F32)
             e = a->linear ? launch_prefill_f32<float, float, true>(*a, m, q, gate, ldg, out, ldo, st) : launch_prefill_f32<float, float, false>(*a, m, q, gate, ldg, out, ldo, st);
     } else if (out_dtype == HF2Q_DT_BF16) {
-        e = launch_prefill_mma<__nv_bfloat16>(*a, m, q, gate, ldg, out, ldo, ctx_status_word(ctx), st);
+        e = launch_prefill_bf16<__nv_bfloat16>(*a, m, q, gate, ldg, out, ldo, ctx_status_word(ctx), ctx_sm_count(ctx), st);
     } else if (out_dtype == HF2Q_DT_F32) {
-        e = launch_prefill_mma<float>(*a, m, q, gate, ldg, out, ldo, ctx_status_word(ctx), st);
+        e = launch_prefill_bf16<float>(*a, m, q, gate, ldg, out, ldo, ctx_status_word(ctx), ctx_sm_count(ctx), st);
     }
     return ctx_cuda_result(ctx, e, "window_attn_prefill", 1);
 }

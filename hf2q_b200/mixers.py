@@ -92,6 +92,7 @@ class ParallelWindowMLstm:
     def prefill(self, run: LayerRun, ws: Workspace, proj, x, m: int):
         left, right, sop = self.left, self.right, self.sop
         attn = self._attn(run, proj)
+        attn.window = min(self.window, run.start + m)          # no more tokens are there: what the kernel is chosen by
         q = ws.get("q", m, left["heads"] * pad8(left["dim"]), self.cache_dtype)
         att = ws.get("att", m, self.lo.k, self.act)
         mem = ws.get("mem", m, right["heads"] * right["vdim"])
@@ -294,7 +295,7 @@ class LatentAttention:
             if hi > lo:
                 sop.matmul(cache[slot:slot + hi - lo], self.ukv, kv[lo:hi], hi - lo)
         att, out = ws.get("att", m, self.o.k, self.act), ws.get("y", m, self.width)
-        w = struct(WindowAttn, qkv=proj, k_cache=kv, v_cache=_off(kv, H * self.dp), heads=H, kv_heads=H, dim=c["dim"], vdim=c["vdim"], window=self.window,
+        w = struct(WindowAttn, qkv=proj, k_cache=kv, v_cache=_off(kv, H * self.dp), heads=H, kv_heads=H, dim=c["dim"], vdim=c["vdim"], window=min(self.window, run.start + m),
                    capacity=self.capacity, cache_dtype=a.cache_dtype, scale=c["scale"], eps=self.eps, pos=run.pos, linear=1, row_stride=self.ukv.n,
                    k_head_stride=self.dp, v_head_stride=self.vp, k_shared=_off(cache, self.rp), shared_dim=c["rot_dim"], shared_stride=self.row,
                    shared_capacity=self.capacity)
