@@ -329,9 +329,83 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
     if (warp == 8) { tc_fence_after(); tmem_dealloc(tmem, COLS); }
 }
 
+// Few positions in all: the tcgen05 kernel's start (barriers, tensor memory, one block's chain of four steps) takes 7 us however
+// few there are.  Here the codes of one KV head go to shared memory and a warp takes a row in f32: lane = position for the
+// scores, lane = four dims for the output.  Bound by the latency of its loads.
+constexpr uint32_t FEW = 48, FEW_WARPS = 8;
+
+template <int G, typename OUT>
+__global__ void __launch_bounds__(FEW_WARPS * 32) attn_prefill_few_kernel(const float* __restrict__ qkv, uint32_t row_stride, uint32_t m,
+                                                                          const int8_t* __restrict__ k_codes, const float* __restrict__ k_scale,
+                                                                          const int8_t* __restrict__ v_codes, const float* __restrict__ v_scale,
+                                                                          uint32_t max_seq, uint32_t pos0, OUT* __restrict__ out, uint32_t out_stride) {
+    __shared__ uint32_t ks[FEW][HD / 4 + 1], vs[FEW][HD / 4 + 1];  // code + 128 in every byte
+    __shared__ float k_s[FEW], v_s[FEW];
+    __shared__ __align__(16) float qs[FEW_WARPS][HD];
+    const uint32_t kvh = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.x * FEW_WARPS + warp, tok = row / G;
+    const uint32_t n = pos0 + min((blockIdx.x * FEW_WARPS + FEW_WARPS - 1) / G, m - 1) + 1;        // positions that a row of this CTA sees
+    const size_t first = static_cast<size_t>(kvh) * max_seq;
+    for (uint32_t i = threadIdx.x; i < n * 8; i += FEW_WARPS * 32) {
+        const uint32_t p = i >> 3, c = i & 7;
+        const uint4 k = __ldg(reinterpret_cast<const uint4*>(k_codes + (first + p) * HD) + c), v = __ldg(reinterpret_cast<const uint4*>(v_codes + (first + p) * HD) + c);
+        const uint32_t kw[4] = {k.x, k.y, k.z, k.w}, vw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            ks[p][4 * c + j] = kw[j] ^ 0x80808080u;
+            vs[p][4 * c + j] = vw[j] ^ 0x80808080u;
+        }
+    }
+    if (threadIdx.x < n) {
+        k_s[threadIdx.x] = __ldg(k_scale + first + threadIdx.x);
+        v_s[threadIdx.x] = __ldg(v_scale + first + threadIdx.x);
+    }
+    if (tok < m)
+        reinterpret_cast<float4*>(qs[warp])[lane] = __ldg(reinterpret_cast<const float4*>(qkv + static_cast<size_t>(tok) * row_stride + (static_cast<size_t>(kvh) * G + row % G) * HD) + lane);
+    __syncthreads();
+    if (tok >= m) return;
+    const uint32_t seen = pos0 + tok, p0 = min(lane, n - 1), p1 = min(lane + 32, n - 1);
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
+    for (uint32_t w = 0; w < HD / 4; ++w) {
+        const float4 q = reinterpret_cast<const float4*>(qs[warp])[w];
+        const float qv[4] = {q.x, q.y, q.z, q.w};
+        const uint32_t k0 = ks[p0][w], k1 = ks[p1][w];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            s0 = fmaf(qv[j], byte_to_float<128>(k0, j), s0);
+            s1 = fmaf(qv[j], byte_to_float<128>(k1, j), s1);
+        }
+    }
+    s0 = lane <= seen ? s0 * k_s[p0] : -CUDART_INF_F;
+    s1 = lane + 32 <= seen ? s1 * k_s[p1] : -CUDART_INF_F;
+    float mx = fmaxf(s0, s1);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float e0 = expf(s0 - mx), e1 = expf(s1 - mx);
+    float l = e0 + e1, o[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
+    for (uint32_t p = 0; p <= seen; ++p) {
+        const float w = __shfl_sync(0xffffffffu, p < 32 ? e0 : e1, p & 31) * v_s[p];
+        const uint32_t v = vs[p][lane];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = fmaf(w, byte_to_float<128>(v, j), o[j]);
+    }
+    const float inv = l > 0.f ? 1.0f / l : 0.f;
+    OUT* dst = out + static_cast<size_t>(tok) * out_stride + (static_cast<size_t>(kvh) * G + row % G) * HD + 4 * lane;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if constexpr (std::is_same_v<OUT, float>) dst[j] = o[j] * inv;
+        else dst[j] = __float2bfloat16_rn(o[j] * inv);
+    }
+}
+
 template <int G, typename OUT>
 cudaError_t launch_prefill_g(const float* qkv, uint32_t row_stride, uint32_t m, const KvCacheView& kv, uint32_t n_kv, uint32_t pos0, OUT* out,
                              uint32_t out_stride, uint32_t* status, cudaStream_t st) {
+    if (static_cast<uint64_t>(pos0) + m <= FEW) {
+        attn_prefill_few_kernel<G, OUT><<<dim3((m * G + FEW_WARPS - 1) / FEW_WARPS, n_kv), FEW_WARPS * 32, 0, st>>>(
+            qkv, row_stride, m, kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, pos0, out, out_stride);
+        return cudaGetLastError();
+    }
     static PerDeviceFlag flag;
     if (const cudaError_t e = ensure_max_dynamic_smem(attn_prefill_kernel<G, OUT>, AP_SMEM, flag); e != cudaSuccess) return e;
     constexpr uint32_t TOK = ROWS / G;

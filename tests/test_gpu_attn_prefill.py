@@ -118,3 +118,23 @@ def test_hidden_scales_do_not_reach_a_row(gpu_ctx, bad, which, pos0, m, at):
     assert (out[:n].double() - want[:n]).norm() < bound * want[:n].norm()
     if which == 1:
         assert not out[n].isfinite().any()
+
+
+@pytest.mark.parametrize("group,n_kv,pos0,m", [(1, 3, 0, 1), (2, 2, 7, 1), (4, 8, 0, 33), (8, 1, 40, 8), (4, 2, 0, 48), (8, 2, 1, 47), (1, 2, 0, 49), (2, 1, 47, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_few_positions(gpu_ctx, group, n_kv, pos0, m, dtype):
+    """Up to 48 positions in all a kernel in f32, above that the tensor cores; infinite scales of later tokens reach no row."""
+    qkv, codes, scales, T, S = case(group, n_kv, pos0, m, 3.0, 1.0, True, seed=m)
+    clean, nq = [s.clone() for s in scales], group * n_kv
+    if m > 1:
+        scales[0][:, T - 1], scales[1][:, T - 1] = float("nan"), float("inf")
+    out = torch.full((m, nq * HD), float("nan"), device="cuda", dtype=dtype)
+    attend(gpu_ctx, qkv, codes, scales, S, m, nq, n_kv, pos0, out)
+    gpu_ctx.check_status()
+    k, v = ((c[:, :T].double() * s[:, :T, None].double()) for c, s in zip(codes, clean))
+    s = torch.einsum("tgrd,gpd->gtrp", qkv[:, :nq * HD].double().view(m, n_kv, group, HD), k)
+    hidden = torch.arange(T, device="cuda")[None] > pos0 + torch.arange(m, device="cuda")[:, None]
+    want = torch.einsum("gtrp,gpd->tgrd", torch.softmax(s.masked_fill(hidden[None, :, None], -float("inf")), dim=-1), v).reshape(m, nq * HD)
+    spread, n = s.masked_fill(hidden[None, :, None], 0).abs().max().item(), max(m - 1, 1)
+    bound = (2 ** -23 * (12 + spread) if T <= 48 else 2 ** -11 * (1 + spread)) + (2 ** -9 if dtype == torch.bfloat16 else 0)     # sums of 128 terms; a score's error is its size's
+    assert (out[:n].double() - want[:n]).norm() < bound * want[:n].norm()
