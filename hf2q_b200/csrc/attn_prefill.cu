@@ -22,8 +22,10 @@
 //
 // What bounds it: shared-memory traffic and the exponentials, about level (a block of 64 positions moves 98 KB: Q and K
 // of the scores 48, V 16, the converted operands 32; and takes 8192 exponentials, 512 cycles).  Measured: a prompt of 8192
-// tokens in portions of 2048, 32 heads over 8, takes 269 us a portion and layer (256 TFLOP/s); warp-level products with
-// every warp converting its own codes took 1031 us.
+// tokens in portions of 2048, 32 heads over 8, takes 269 us a portion and layer (137 GFLOP, 511 TFLOP/s); warp-level products
+// with every warp converting its own codes took 1031 us.
+//
+// Up to 48 positions in all a kernel without tensor cores (attn_prefill_few_kernel).
 #include <math_constants.h>
 
 #include <type_traits>
@@ -46,9 +48,7 @@ constexpr uint32_t AP_THREADS = 288, COLS = 256, COL_O = 128;
 constexpr uint32_t SLOTS = 4;
 constexpr float LAZY_LOG2 = 3.0f, LAZY_VMAX = 16.0f;
 
-__device__ __forceinline__ float exp2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ f2 f2_pack(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
-__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // sixteen signed bytes -> sixteen f16 whole numbers, as the two 16-byte chunks of a swizzled row; odd panels store their
 // chunks in the other order (the lanes of a quarter-warp then meet all banks)
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
             if (j == 0) {
                 mx = bm;                                           // finite: position 0 is visible to every row
             } else if (__any_sync(0xffffffffu, grew)) {
-                const float to = grew ? bm : mx, corr = grew ? exp2_fast(mx - to) : 1.0f;
+                const float to = grew ? bm : mx, corr = grew ? ex2(mx - to) : 1.0f;
                 mx = to;
                 const f2 c2 = f2_both(corr);
                 sum = f2_mul(sum, c2);
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
                         const ulonglong2 k = k2[4 * c + i / 2], v = v2[4 * c + i / 2];
                         float2 d = f2_parts(f2_fma(f2_pack(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x, nm));
                         if constexpr (decltype(masked)::value) d = hide(d, j * BP + 16 * c + 2 * i, seen, -CUDART_INF_F);
-                        const f2 e = f2_pack(exp2_fast(d.x), exp2_fast(d.y));
+                        const f2 e = f2_pack(ex2(d.x), ex2(d.y));
                         part = f2_add(part, e);
                         float2 w = f2_parts(f2_mul(e, i & 1 ? v.y : v.x));
                         if constexpr (decltype(masked)::value) w = hide(w, j * BP + 16 * c + 2 * i, seen, 0.f);
@@ -331,7 +331,9 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
 
 // Few positions in all: the tcgen05 kernel's start (barriers, tensor memory, one block's chain of four steps) takes 7 us however
 // few there are.  Here the codes of one KV head go to shared memory and a warp takes a row in f32: lane = position for the
-// scores, lane = four dims for the output.  Bound by the latency of its loads.
+// scores, lane = four dims for the output.  Bound by the latency of its loads.  32 heads over 8, first portion of a sequence:
+// 1 token 3.5 us (tcgen05 7.0), 17 tokens 5.1 (9.2), 33 tokens 5.7 (10.9); a lane has room for 64 positions, and at 48 a block
+// of the other kernel is three quarters full.
 constexpr uint32_t FEW = 48, FEW_WARPS = 8;
 
 template <int G, typename OUT>

@@ -373,9 +373,7 @@ __global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_co
 constexpr uint32_t WT_Q = 128, WT_K = 64, WT_V = 128, WT_THREADS = 288, WT_COLS = 256, WT_O = 128, WT_PANEL = WT_K * 128;
 constexpr uint32_t wt_smem(uint32_t dk) { return WT_Q * dk * 2 + 2 * WT_K * dk * 2 + 2 * WT_K * WT_V * 2 + 1024; }
 
-__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float lg2(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // 16-byte chunk c of a row, in panels of `rows` rows x 64 elements
 __device__ __forceinline__ uint32_t wt_chunk(uint32_t rows, uint32_t row, uint32_t c) { return (c >> 3) * rows * 128 + row * 128 + (((c & 7) ^ (row & 7)) << 4); }
 
@@ -440,7 +438,7 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
         }
         *reinterpret_cast<uint4*>(qs + wt_chunk(WT_Q, r, c)) = v;
     }
-    proxy_fence();
+    tc::proxy_fence();
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
@@ -468,11 +466,11 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
             cp_async_commit();
             if (j > 0) {
                 cp_async_wait<2>();                            // all but the copies of V(j-1) and K(j)
-                proxy_fence();
+                tc::proxy_fence();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&k_full[b ^ 1]);
                 cp_async_wait<1>();
-                proxy_fence();
+                tc::proxy_fence();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&v_full[b ^ 1]);
             }
@@ -571,7 +569,7 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
             if (j == 0) {
                 mx = bm;
             } else if (__any_sync(0xffffffffu, grew)) {
-                const float to = grew ? bm : mx, corr = grew ? ex2(mx - to) : 1.0f;
+                const float to = grew ? bm : mx, corr = grew ? tc::ex2(mx - to) : 1.0f;
                 mx = to;
                 sum[0] *= corr;
                 sum[1] *= corr;
@@ -596,7 +594,7 @@ __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_
                 tc::tmem_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const float x = ex2(__uint_as_float(r[2 * i]) - nm), y = ex2(__uint_as_float(r[2 * i + 1]) - nm);
+                    const float x = tc::ex2(__uint_as_float(r[2 * i]) - nm), y = tc::ex2(__uint_as_float(r[2 * i + 1]) - nm);
                     sum[0] += x;
                     sum[1] += y;
                     p[i] = pack_bf16(x, y);
