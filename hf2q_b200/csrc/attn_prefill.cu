@@ -332,8 +332,8 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
 // Few positions in all: the tcgen05 kernel's start (barriers, tensor memory, one block's chain of four steps) takes 7 us however
 // few there are.  Here the codes of one KV head go to shared memory and a warp takes a row in f32: lane = position for the
 // scores, lane = four dims for the output.  Bound by the latency of its loads.  32 heads over 8, first portion of a sequence:
-// 1 token 3.5 us (tcgen05 7.0), 17 tokens 5.1 (9.2), 33 tokens 5.7 (10.9); a lane has room for 64 positions, and at 48 a block
-// of the other kernel is three quarters full.
+// 1 token 3.5 us (tcgen05 7.0), 17 tokens 5.1 (9.2), 33 tokens 5.7 (10.9).  The line: 64 heads over 8 take as long
+// either way at 48 positions (10.1, 10.5); 32 over 8 would gain up to 64 of them (64: 9.0, 10.6).
 constexpr uint32_t FEW = 48, FEW_WARPS = 8;
 
 template <int G, typename OUT>
