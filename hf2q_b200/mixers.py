@@ -92,7 +92,8 @@ class ParallelWindowMLstm:
     def prefill(self, run: LayerRun, ws: Workspace, proj, x, m: int):
         left, right, sop = self.left, self.right, self.sop
         attn = self._attn(run, proj)
-        attn.window = min(self.window, run.start + m)          # no more tokens are there: what the kernel is chosen by
+        if run.start is not None:
+            attn.window = min(self.window, run.start + m)      # no more tokens are there: what the kernel is chosen by
         q = ws.get("q", m, left["heads"] * pad8(left["dim"]), self.cache_dtype)
         att = ws.get("att", m, self.lo.k, self.act)
         mem = ws.get("mem", m, right["heads"] * right["vdim"])
