@@ -140,9 +140,11 @@ __global__ void __launch_bounds__(RV_THREADS) router_vector_kernel(const void* _
 // More tokens: 64 tokens x 64 experts per tile, 4 x 4 outputs per thread in packed f32 arithmetic, the next 32 columns on
 // their way to registers while the present ones are used.  Bound by the f32 pipes (2048 tokens x 256 experts of 2048: 1.07 G
 // multiply-adds).  The CTAs of a cluster share a tile's columns where the tiles alone would leave the chip idle, and add
-// their sums through distributed shared memory in rank order (2048 tokens, 256 experts of 2048: 263 -> 86 us; the line at
-// RV_TOKENS lies where a CTA per expert would read more activations than weights).  Columns are stored with the group of four tokens (or
-// experts) XORed by the column's own group of four, which keeps both the transposing stores and the reads free of conflicts.
+// their sums through distributed shared memory in rank order (2048 tokens, 256 experts of 2048: 263 -> 86 us).  The line at
+// RV_TOKENS is the number of sums a thread of the other kernel keeps in registers; there the tiles are still behind (us a CTA per
+// expert / tiles, 8 and 16 tokens: 256 experts of 2048 7.9 / 13.9 and 12.6 / 13.9, 8 of 4096 10.7 / 20.9 and 19.7 / 21.1).
+// Columns are stored with the group of four tokens (or experts) XORed by the column's own group of four, which keeps both the
+// transposing stores and the reads free of conflicts.
 constexpr int RT = 64, RKT = 32, RT_MAX_PARTS = 8;
 
 template <bool VEC>

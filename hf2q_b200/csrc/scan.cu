@@ -180,7 +180,9 @@ __device__ __forceinline__ void clear_padding(float* sm, uint32_t n, bool padded
     __syncthreads();
 }
 // Shared memory of a scan's launch.  It asks for so much that no SM takes more CTAs than an even spread puts there: the CTAs
-// start while the preceding kernel's last ones still run, and would otherwise pile up on the SMs that are free first.
+// start while the preceding kernel's last ones still run, and would otherwise pile up on the SMs that are free first.  The price:
+// scans of two streams do not share SMs.  Two of 2048 tokens side by side: delta (16 heads) 512 us a pair, one alone 299; ssd (64
+// heads) 443 and 256; mlstm (8 heads, both fit) 213 and 213.  (The former kernels shared SMs and took 1087, 869 and 586 a pair.)
 constexpr size_t SCAN_STATIC = 9 * 1024, SCAN_MAX = 227 * 1024 - SCAN_STATIC;       // static arrays: at most
 inline size_t scan_smem(size_t need, dim3 grid, int sms) {
     const size_t ctas = static_cast<size_t>(grid.x) * grid.y, per_sm = (ctas + sms - 1) / sms;
