@@ -48,7 +48,6 @@ constexpr uint32_t AP_THREADS = 288, COLS = 256, COL_O = 128;
 constexpr uint32_t SLOTS = 4;
 constexpr float LAZY_LOG2 = 3.0f, LAZY_VMAX = 16.0f;
 
-__device__ __forceinline__ f2 f2_pack(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
 
 // sixteen signed bytes -> sixteen f16 whole numbers, as the two 16-byte chunks of a swizzled row; odd panels store their
 // chunks in the other order (the lanes of a quarter-warp then meet all banks)
@@ -226,7 +225,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const ulonglong2 k = k2[8 * half + i / 2];
-                        float2 x = f2_parts(f2_mul(f2_pack(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x));
+                        float2 x = f2_parts(f2_mul(f2_of(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x));
                         if constexpr (decltype(masked)::value) x = hide(x, j * BP + 32 * half + 2 * i, seen, -CUDART_INF_F);
                         top[2 * (i & 1)] = fmaxf(top[2 * (i & 1)], x.x);
                         top[2 * (i & 1) + 1] = fmaxf(top[2 * (i & 1) + 1], x.y);
@@ -268,9 +267,9 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const ulonglong2 k = k2[4 * c + i / 2], v = v2[4 * c + i / 2];
-                        float2 d = f2_parts(f2_fma(f2_pack(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x, nm));
+                        float2 d = f2_parts(f2_fma(f2_of(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), i & 1 ? k.y : k.x, nm));
                         if constexpr (decltype(masked)::value) d = hide(d, j * BP + 16 * c + 2 * i, seen, -CUDART_INF_F);
-                        const f2 e = f2_pack(ex2(d.x), ex2(d.y));
+                        const f2 e = f2_of(ex2(d.x), ex2(d.y));
                         part = f2_add(part, e);
                         float2 w = f2_parts(f2_mul(e, i & 1 ? v.y : v.x));
                         if constexpr (decltype(masked)::value) w = hide(w, j * BP + 16 * c + 2 * i, seen, 0.f);

@@ -311,6 +311,47 @@ __global__ void __launch_bounds__((8 / C + 1) * 32, TB == SC_TB ? 1 : 2) mlstm_k
     }
 }
 
+// One token: nothing is staged, each lane brings its own channels and every thread makes the gate factors for itself, so that the
+// loads are one latency and no barrier stands in the chain.  8 heads of 128 x 128 1.95 us (a scan of one token 2.8, the kernel
+// before the scans of several columns 2.7), 32 heads 2.7 (3.1; 3.0), 16 heads of 256 x 256 2.7 (3.8; 3.9).
+template <int RQ>
+__global__ void __launch_bounds__(SC_THREADS) mlstm_step_kernel(const __grid_constant__ hf2q_mlstm a, float* __restrict__ out) {
+    constexpr uint32_t DP = 32 * RQ;
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t h = blockIdx.x, slice = blockIdx.y, n_slices = gridDim.y, lane = threadIdx.x & 31, lg = lane & 15;
+    const uint32_t col = slice * SC_COLS + (threadIdx.x >> 4);
+    const bool live = col < a.vdim;
+    Vec<RQ> S, N, k, q;
+    float* sp = a.s + (static_cast<size_t>(h) * a.vdim + (live ? col : 0)) * DP + 2 * lg;
+    float* np = a.n + (static_cast<size_t>(h) * n_slices + slice) * DP + 2 * lg;
+    float* mp = a.mx + static_cast<size_t>(h) * n_slices + slice;
+    if (live) S.load(sp); else S.zero();
+    N.load(np);
+    const float *kr = a.proj + a.k_off + h * a.dim, *qr = a.proj + a.q_off + h * a.dim;
+#pragma unroll
+    for (int c = 0; c < RQ; ++c) {
+        const uint32_t i = 32 * c + 2 * lg;
+        const bool in0 = i < a.dim, in1 = i + 1 < a.dim;
+        k.v[c] = f2_of(in0 ? kr[i] : 0.f, in1 ? kr[i + 1] : 0.f);
+        q.v[c] = f2_of(in0 ? qr[i] : 0.f, in1 ? qr[i + 1] : 0.f);
+    }
+    const float v = live ? a.proj[a.v_off + h * a.vdim + col] : 0.f, mx = *mp;
+    const float x = a.gate_cap * tanhf((a.proj[a.i_off + h] + a.i_bias[h]) / a.gate_cap);
+    const float f = -softplusf(-a.gate_cap * tanhf((a.proj[a.f_off + h] + a.f_bias[h]) / a.gate_cap));
+    const float top = fmaxf(mx + f, x), keep = expf(f + mx - top), write = expf(x - top);
+    S.decay_axpy(keep, k, write * v);
+    N.decay_axpy(keep, k, write);
+    const float num = group_sum(S.dot(q)), den = group_sum(N.dot(q)), q_scale = 1.0f / sqrtf(static_cast<float>(a.dim));
+    if (live) {
+        S.store(sp);
+        if (lg == 0) out[h * a.vdim + col] = num * q_scale / (fmaxf(fabsf(den * q_scale), expf(-top)) + 1e-6f);
+    }
+    __syncthreads();                                         // all threads have read the normaliser and the maximum
+    if (threadIdx.x < 16) N.store(np);
+    if (threadIdx.x == 0) *mp = top;
+}
+
 // ---------------------------------------------------------------- gated delta rule
 // S <- g S;  u = beta (v - S^T k);  S <- S + k u;  o = S^T q
 template <int RQ>
@@ -960,12 +1001,12 @@ cudaError_t launch_mlstm_as(const hf2q_mlstm& a, uint32_t m, float* out, int sms
     if (const cudaError_t e = ensure_max_dynamic_smem(mlstm_kernel<RQ, C, TB>, SCAN_MAX, flag); e != cudaSuccess) return e;
     return launch_pdl(mlstm_kernel<RQ, C, TB>, grid, dim3((8 / C + 1) * 32), TB == SC_TB ? scan_smem(need, grid, sms) : need, st, a, m, out);
 }
-// Few tokens (a decode step among them): what counts is how soon a token's chain starts and that the CTAs share the SMs, so one
-// column a group, eight warps, and a batch of 8 tokens, whose buffers let several CTAs on an SM.  The line lies where two columns
-// a group take whole groups of tokens: 16 heads of 128 x 128, 8 tokens 6.0 us with one column, 3.7 with two; 5 tokens 4.8 and
-// 4.8.  32 such heads, one token: 3.4 us, a CTA an SM took 5.3.
+// Few tokens: what counts is how soon a token's chain starts and that the CTAs share the SMs, so one column a group, eight warps,
+// and a batch of 8 tokens, whose buffers let several CTAs on an SM.  The line lies where two columns a group take whole groups of
+// tokens: 16 heads of 128 x 128, 8 tokens 6.0 us with one column, 3.7 with two; 5 tokens 4.8 and 4.8.
 template <int RQ>
 cudaError_t launch_mlstm(const hf2q_mlstm& a, uint32_t m, float* out, int sms, cudaStream_t st) {
+    if (m == 1) return launch_pdl(mlstm_step_kernel<RQ>, dim3(a.heads, (a.vdim + SC_COLS - 1) / SC_COLS), dim3(SC_THREADS), 0, st, a, out);
     if (m < (RQ > 4 ? 16u : 8u)) return launch_mlstm_as<RQ, 1, SC_FEW>(a, m, out, sms, st);
     return launch_mlstm_as<RQ, 2, SC_TB>(a, m, out, sms, st);
 }
