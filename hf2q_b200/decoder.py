@@ -161,7 +161,7 @@ class GreedyDecoder:
 class Staging:
     """Small host tensors reach the device through a pinned buffer of their own, and the host does not wait for them: the
     caller may change its tensor at once, and no call allocates pinned memory (a capture gives torch's cached blocks back,
-    so allocations around the first single-token step went to the driver)."""
+    so allocations around the first single-token step went to the CUDA driver)."""
 
     def __init__(self, nbytes: int, device):
         self.device = device
