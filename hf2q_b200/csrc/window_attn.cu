@@ -5,7 +5,8 @@
 //   append    prefill: normalised queries to a buffer, normalised keys and values to the cache
 //   prefill   bf16 cache: tiles on the tensor cores (f32 scores, softmax and accumulators, bf16 product operands): of 128
 //             queries on tcgen05 or of 64 on warps, by size (prefill_on_tcgen05); f32 cache: one warp per query in f32
-//   decode    one launch: norm, append, window split over CTAs, merge by the CTA that arrives last
+//   decode    one launch: norm, append, window split over the CTAs of a cluster and merged by it
+#include <cooperative_groups.h>
 #include <math_constants.h>
 
 #include "mma_sync.cuh"
@@ -15,6 +16,7 @@
 namespace hf2q {
 namespace {
 using namespace seq;
+namespace cg = cooperative_groups;
 
 __host__ __device__ constexpr uint32_t pad8(uint32_t n) { return (n + 7) & ~7u; }
 
@@ -201,21 +203,53 @@ struct WarpAttn {
 };
 
 // ---------------------------------------------------------------- decode
-constexpr int WD_WARPS = 8;
+// One token: WD_WARPS warps of a CTA take 16 keys each, 256 a pass.  Bound by the latency of its dependent steps, so what can be
+// is asked for at once: a pair of lanes holds a key's row and a lane four columns of 16 values in registers, and the first tile
+// is on its way before the query is normed.  The splits of a short window are a cluster and merge through distributed shared
+// memory; a long one has more splits, whose last CTA merges them (cluster_splits).  Window 2048, 530 tokens there, 16 heads over 4 of
+// 128: 9.8 us in a decode step; a lane per key, rows read four at a time and a merge through memory took 22.8.
+constexpr int WD_WARPS = 16, WD_KEYS = 16;
+constexpr uint32_t WD_PASS = WD_WARPS * WD_KEYS, WD_CLUSTER = 8;
 __host__ __device__ constexpr uint32_t wd_part(uint32_t vdim) { return 4 + pad8(vdim); }
 
-// grid (kv_heads * groups of GR query heads, splits); scratch: counters [grid.x] (256-byte multiple), then
-// [grid.x][splits][GR][max, sum, 2 pad, acc]
-template <typename T, int GR, int NC>
+// eight elements of a key row, four of a value row, as they lie in memory
+template <typename T> struct Raw;
+template <> struct Raw<__nv_bfloat16> {
+    typedef uint4 Eight;
+    typedef uint2 Four;
+    static __device__ __forceinline__ void open(const uint4& v, float (&o)[8]) {
+        o[0] = bf_lo(v.x); o[1] = bf_hi(v.x); o[2] = bf_lo(v.y); o[3] = bf_hi(v.y);
+        o[4] = bf_lo(v.z); o[5] = bf_hi(v.z); o[6] = bf_lo(v.w); o[7] = bf_hi(v.w);
+    }
+    static __device__ __forceinline__ void open(const uint2& v, float (&o)[4]) { o[0] = bf_lo(v.x); o[1] = bf_hi(v.x); o[2] = bf_lo(v.y); o[3] = bf_hi(v.y); }
+};
+template <> struct Raw<float> {
+    struct Eight { float4 a, b; };
+    typedef float4 Four;
+    static __device__ __forceinline__ void open(const Eight& v, float (&o)[8]) {
+        o[0] = v.a.x; o[1] = v.a.y; o[2] = v.a.z; o[3] = v.a.w; o[4] = v.b.x; o[5] = v.b.y; o[6] = v.b.z; o[7] = v.b.w;
+    }
+    static __device__ __forceinline__ void open(const float4& v, float (&o)[4]) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+};
+
+// grid (kv_heads * groups of GR query heads, splits), NC: values of up to 128 NC elements.  CLUSTER: the splits are a cluster;
+// else scratch: counters [grid.x] (256-byte multiple), then [grid.x][splits][GR][max, sum, 2 pad, acc].
+template <typename T, int GR, int NC, bool CLUSTER>
 __global__ void __launch_bounds__(WD_WARPS * 32) window_decode_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t groups, float* __restrict__ out,
                                                                       uint32_t* __restrict__ counters, float* __restrict__ part) {
+    typedef typename Raw<T>::Eight Eight;
+    typedef typename Raw<T>::Four Four;
+    constexpr int HOLD = GR * NC >= 16 ? 32 : GR * NC >= 8 ? 64 : 128;      // bytes of a key's half and of values that a lane holds
+    constexpr int KB = HOLD / sizeof(Eight), VB = HOLD / (4 * NC * sizeof(T));       // groups of eight, value rows
+    static_assert(VB >= 1 && WD_KEYS % VB == 0, "");
     extern __shared__ __align__(16) float sm[];
-    const uint32_t dp = pad8(a.dim), dvp = pad8(a.vdim), PP = wd_part(a.vdim);
+    const uint32_t dp = pad8(a.dim), dvp = pad8(a.vdim), PP = wd_part(a.vdim), n8 = dp / 8;
     float* qs = sm;                                        // [GR][dp]
-    float* ps = qs + GR * dp;                              // [warps][GR][32]
-    float* rm = ps + WD_WARPS * GR * 32;                   // [warps][GR] max, then sums
+    float* ps = qs + GR * dp;                              // [warps][GR][16]
+    float* rm = ps + WD_WARPS * GR * WD_KEYS;              // [warps][GR] max, then sums
     float* rl = rm + WD_WARPS * GR;
     float* ra = rl + WD_WARPS * GR;                        // [warps][GR][dvp]
+    float* sum = ra + WD_WARPS * GR * dvp;                 // CLUSTER: [GR][max, sum, 2 pad, acc] of this CTA
     __shared__ uint32_t is_last;
     pdl_trigger();
     pdl_wait();
@@ -227,18 +261,45 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_decode_kernel(const __gr
     const uint32_t lo = first + min(split * chunk, n), hi = first + min(split * chunk + chunk, n);
     T* kc = static_cast<T*>(a.k_cache) + static_cast<size_t>(kvh) * a.capacity * dp;
     T* vc = static_cast<T*>(a.v_cache) + static_cast<size_t>(kvh) * a.capacity * dvp;
-    for (uint32_t g = warp; g < GR; g += WD_WARPS) {
+    const uint32_t half = lane & 1;
+    Eight kr[KB];
+    Four vr[VB][NC];
+    // groups 2 (c0 + j) + half of key p; rows v0 .. v0 + VB of the tile at p0 (columns past the row: the row's start)
+    auto load_k = [&](uint32_t p, uint32_t c0) {
+        const Eight* row = reinterpret_cast<const Eight*>(kc + static_cast<size_t>(p % a.capacity) * dp);
+#pragma unroll
+        for (int j = 0; j < KB; ++j)
+            if (2 * (c0 + j) + half < n8) kr[j] = row[2 * (c0 + j) + half];
+    };
+    auto load_v = [&](uint32_t p, int i) {
+        const T* row = vc + static_cast<size_t>(p % a.capacity) * dvp;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const uint32_t d = 4 * lane + 128 * c;
+            vr[i][c] = *reinterpret_cast<const Four*>(row + (d < dvp ? d : 0u));
+        }
+    };
+    auto load_rows = [&](uint32_t p0, uint32_t v0) {       // (past the end: the tile's first row, with weight zero)
+#pragma unroll
+        for (int i = 0; i < VB; ++i) load_v(p0 + v0 + i < hi ? p0 + v0 + i : p0, i);
+    };
+    // ahead of the query; the new position's row is not there yet
+    uint32_t p0 = lo + warp * WD_KEYS;
+    if (p0 < hi) {
+        load_k(min(p0 + lane / 2, hi - 1), 0);
+        load_rows(p0, 0);
+    }
+    if (warp < GR) {
         HeadVec v;
-        v.load(a.qkv + a.q_off + (h0 + min(g, n_g - 1)) * a.dim, a.dim, lane);
+        v.load(a.qkv + a.q_off + (h0 + min(warp, n_g - 1)) * a.dim, a.dim, lane);
         if (a.q_norm) v.norm(a.q_norm, a.eps, a.dim, lane);
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (lane + 32 * j < dp) qs[g * dp + lane + 32 * j] = to_f32(from_f32<T>(v.v[j]));      // the prefill's operand precision
-    }
-    if (pos >= lo && pos < hi && warp < 2) {               // the new position, by the CTAs whose range holds it
+            if (lane + 32 * j < dp) qs[warp * dp + lane + 32 * j] = to_f32(from_f32<T>(v.v[j]));      // the prefill's operand precision
+    } else if (pos >= lo && pos < hi && warp < GR + 2) {   // the new position, by the CTAs whose range holds it
         const uint32_t slot = pos % a.capacity;
         HeadVec v;
-        if (warp == 0) {
+        if (warp == GR) {
             v.load(a.qkv + a.k_off + kvh * a.dim, a.dim, lane);
             if (a.k_norm) v.norm(a.k_norm, a.eps, a.dim, lane);
             v.store(kc + static_cast<size_t>(slot) * dp, a.dim, lane);
@@ -254,37 +315,140 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_decode_kernel(const __gr
         r2[g] = a.r1 ? a.r2[h0 + min(static_cast<uint32_t>(g), n_g - 1)] : 0.f;
     }
     __syncthreads();
-    WarpAttn<T, GR, NC, false> w;
-    w.init();
-    for (uint32_t p0 = lo + warp * 32; p0 < hi; p0 += WD_WARPS * 32) w.keys(a, kc, vc, nullptr, qs, ps + warp * GR * 32, r1, r2, pos, p0, hi);
+    if (p0 < hi && pos >= p0 && pos < p0 + WD_KEYS) {      // this tile holds the new position (its last key): its rows as they are now
+        if (p0 + lane / 2 >= pos) load_k(pos, 0);
+#pragma unroll
+        for (int i = 0; i < VB; ++i)
+            if (p0 + i == pos) load_v(pos, i);
+    }
+    float mx[GR], l[GR], acc[GR][NC][4];
 #pragma unroll
     for (int g = 0; g < GR; ++g) {
-        if (lane == 0) { rm[warp * GR + g] = w.mx[g]; rl[warp * GR + g] = w.l[g]; }
+        mx[g] = -CUDART_INF_F;
+        l[g] = 0.f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc[g][c][0] = acc[g][c][1] = acc[g][c][2] = acc[g][c][3] = 0.f;
+    }
+    float* pw = ps + warp * GR * WD_KEYS;
+    for (bool held = true; p0 < hi; p0 += WD_PASS, held = false) {
+        const uint32_t p = min(p0 + lane / 2, hi - 1);
+        const bool live = p0 + lane / 2 < hi;
+        if (!held) { load_k(p, 0); load_rows(p0, 0); }
+        float s[GR];
+#pragma unroll
+        for (int g = 0; g < GR; ++g) s[g] = 0.f;
+        for (uint32_t c0 = 0; 2 * c0 < n8; c0 += KB) {
+            if (c0) load_k(p, c0);
+#pragma unroll
+            for (int j = 0; j < KB; ++j) {
+                const uint32_t c = 2 * (c0 + j) + half;
+                if (c < n8) {
+                    float k[8];
+                    Raw<T>::open(kr[j], k);
+#pragma unroll
+                    for (int g = 0; g < GR; ++g) {
+                        const float4 x = *reinterpret_cast<const float4*>(qs + g * dp + 8 * c), y = *reinterpret_cast<const float4*>(qs + g * dp + 8 * c + 4);
+                        s[g] += k[0] * x.x + k[1] * x.y + k[2] * x.z + k[3] * x.w + k[4] * y.x + k[5] * y.y + k[6] * y.z + k[7] * y.w;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < GR; ++g) {
+            const float dot = s[g] + __shfl_xor_sync(0xffffffffu, s[g], 1);
+            const float sc = live ? score_of(dot, a.scale, r1[g], r2[g], pos - p, a.r1 != nullptr) : -CUDART_INF_F;
+            float bm = sc;
+            for (int o = 16; o > 1; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+            const float nm = fmaxf(mx[g], bm);
+            const float corr = expf(mx[g] - nm), pr = live ? expf(sc - nm) : 0.f;
+            float total = pr;
+            for (int o = 16; o > 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+            l[g] = l[g] * corr + total;
+            mx[g] = nm;
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[g][c][u] *= corr;
+            if (half == 0) pw[g * WD_KEYS + lane / 2] = pr;
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t v0 = 0; v0 < WD_KEYS; v0 += VB) {
+            if (v0) load_rows(p0, v0);
+#pragma unroll
+            for (int i = 0; i < VB; ++i) {
+                const bool there = p0 + v0 + i < hi;       // (a row past the end may hold anything: it does not enter, finite or not)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    float v[4];
+                    Raw<T>::open(vr[i][c], v);
+                    if (there)
+#pragma unroll
+                        for (int g = 0; g < GR; ++g) {
+                            const float w = pw[g * WD_KEYS + v0 + i];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) acc[g][c][u] = fmaf(w, v[u], acc[g][c][u]);
+                        }
+                }
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int g = 0; g < GR; ++g) {
+        if (lane == 0) { rm[warp * GR + g] = mx[g]; rl[warp * GR + g] = l[g]; }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const uint32_t d = 2 * lane + 64 * c;
-            if (d < dvp) *reinterpret_cast<float2*>(ra + (warp * GR + g) * dvp + d) = make_float2(w.acc[g][c][0], w.acc[g][c][1]);
+            const uint32_t d = 4 * lane + 128 * c;
+            if (d < dvp) *reinterpret_cast<float4*>(ra + (warp * GR + g) * dvp + d) = make_float4(acc[g][c][0], acc[g][c][1], acc[g][c][2], acc[g][c][3]);
         }
     }
     __syncthreads();
-    float* mine = part + (static_cast<size_t>(blockIdx.x) * nsplit + split) * GR * PP;
+    float* mine = CLUSTER ? sum : part + (static_cast<size_t>(blockIdx.x) * nsplit + split) * GR * PP;
     for (uint32_t i = threadIdx.x; i < GR * dvp; i += WD_WARPS * 32) {
         const uint32_t g = i / dvp, d = i % dvp;
-        float m = -CUDART_INF_F, l = 0.f, s = 0.f;
+        float m = -CUDART_INF_F, t = 0.f, v = 0.f;
+#pragma unroll
         for (int k = 0; k < WD_WARPS; ++k) m = fmaxf(m, rm[k * GR + g]);
+#pragma unroll
         for (int k = 0; k < WD_WARPS; ++k) {
             const float c = rm[k * GR + g] == -CUDART_INF_F ? 0.f : expf(rm[k * GR + g] - m);
-            l += rl[k * GR + g] * c;
-            s += ra[(k * GR + g) * dvp + d] * c;
+            t += rl[k * GR + g] * c;
+            v += ra[(k * GR + g) * dvp + d] * c;
         }
         if (nsplit == 1) {
-            if (g < n_g && d < a.vdim) out[(h0 + g) * a.vdim + d] = s / l;
+            if (g < n_g && d < a.vdim) out[(h0 + g) * a.vdim + d] = v / t;
         } else {
-            if (d == 0) { mine[g * PP] = m; mine[g * PP + 1] = l; }
-            mine[g * PP + 4 + d] = s;
+            if (d == 0) { mine[g * PP] = m; mine[g * PP + 1] = t; }
+            mine[g * PP + 4 + d] = v;
         }
     }
     if (nsplit == 1) return;
+    if constexpr (CLUSTER) {
+        const cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        // the outputs are spread over the cluster; every CTA's sums in split order
+        for (uint32_t i = split * (WD_WARPS * 32) + threadIdx.x; i < n_g * a.vdim; i += nsplit * (WD_WARPS * 32)) {
+            const uint32_t g = i / a.vdim, d = i % a.vdim;
+            float mk[WD_CLUSTER], lk[WD_CLUSTER], vk[WD_CLUSTER], m = -CUDART_INF_F, t = 0.f, v = 0.f;
+#pragma unroll
+            for (uint32_t k = 0; k < WD_CLUSTER; ++k) {
+                const float* src = cl.map_shared_rank(sum, k < nsplit ? k : 0u) + g * PP;
+                mk[k] = k < nsplit ? src[0] : -CUDART_INF_F; lk[k] = src[1]; vk[k] = src[4 + d];
+                m = fmaxf(m, mk[k]);
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < WD_CLUSTER; ++k)
+                if (mk[k] != -CUDART_INF_F) {
+                    const float c = expf(mk[k] - m);
+                    t += lk[k] * c;
+                    v += vk[k] * c;
+                }
+            out[(h0 + g) * a.vdim + d] = v / t;
+        }
+        cl.sync();                                                   // the others read this CTA's sums until here
+        return;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -298,15 +462,15 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_decode_kernel(const __gr
     const float* all = part + static_cast<size_t>(blockIdx.x) * nsplit * GR * PP;
     for (uint32_t i = threadIdx.x; i < n_g * a.vdim; i += WD_WARPS * 32) {
         const uint32_t g = i / a.vdim, d = i % a.vdim;
-        float m = -CUDART_INF_F, l = 0.f, s = 0.f;
+        float m = -CUDART_INF_F, t = 0.f, v = 0.f;
         for (uint32_t k = 0; k < nsplit; ++k) m = fmaxf(m, __ldcg(all + (k * GR + g) * PP));
         for (uint32_t k = 0; k < nsplit; ++k) {
             const float* src = all + (k * GR + g) * PP;
             const float mk = __ldcg(src), c = mk == -CUDART_INF_F ? 0.f : expf(mk - m);
-            l += __ldcg(src + 1) * c;
-            s += __ldcg(src + 4 + d) * c;
+            t += __ldcg(src + 1) * c;
+            v += __ldcg(src + 4 + d) * c;
         }
-        out[(h0 + g) * a.vdim + d] = s / l;
+        out[(h0 + g) * a.vdim + d] = v / t;
     }
 }
 
@@ -847,20 +1011,32 @@ uint32_t decode_splits(const hf2q_window_attn& a, int sms) {
 }
 size_t counter_bytes(const hf2q_window_attn& a) { return (static_cast<size_t>(a.kv_heads) * decode_groups(a) * 4 + 255) & ~static_cast<size_t>(255); }
 
+// Splits of a window as one cluster, 0 for more of them than a cluster has: up to four passes of a CTA.
+uint32_t cluster_splits(const hf2q_window_attn& a) {
+    const uint32_t s = (a.window + WD_PASS - 1) / WD_PASS;
+    return s <= WD_CLUSTER ? s : s <= 4 * WD_CLUSTER ? WD_CLUSTER : 0;
+}
 template <typename T, int GR, int NC>
 cudaError_t launch_decode(const hf2q_window_attn& a, float* out, uint8_t* scratch, int sms, cudaStream_t st) {
+    const size_t smem = (static_cast<size_t>(GR) * pad8(a.dim) + WD_WARPS * GR * (2 + WD_KEYS + pad8(a.vdim)) + GR * wd_part(a.vdim)) * sizeof(float);
+    const uint32_t groups = decode_groups(a), cluster = cluster_splits(a);
+    uint32_t* counters = reinterpret_cast<uint32_t*>(scratch);
+    float* part = reinterpret_cast<float*>(scratch + counter_bytes(a));
+    if (cluster) {
+        static PerDeviceFlag flag;
+        const auto kern = window_decode_kernel<T, GR, NC, true>;
+        if (const cudaError_t e = ensure_max_dynamic_smem(kern, 200 * 1024, flag); e != cudaSuccess) return e;
+        return launch_pdl_cluster(kern, dim3(a.kv_heads * groups, cluster), dim3(WD_WARPS * 32), dim3(1, cluster, 1), smem, st, a, groups, out, counters, part);
+    }
     static PerDeviceFlag flag;
-    const size_t smem = (static_cast<size_t>(GR) * pad8(a.dim) + WD_WARPS * GR * (34 + pad8(a.vdim))) * sizeof(float);
-    if (const cudaError_t e = ensure_max_dynamic_smem(window_decode_kernel<T, GR, NC>, 100 * 1024, flag); e != cudaSuccess) return e;
-    const uint32_t groups = decode_groups(a);
-    return launch_pdl(window_decode_kernel<T, GR, NC>, dim3(a.kv_heads * groups, decode_splits(a, sms)), dim3(WD_WARPS * 32), smem, st, a, groups, out,
-                      reinterpret_cast<uint32_t*>(scratch), reinterpret_cast<float*>(scratch + counter_bytes(a)));
+    const auto kern = window_decode_kernel<T, GR, NC, false>;
+    if (const cudaError_t e = ensure_max_dynamic_smem(kern, 200 * 1024, flag); e != cudaSuccess) return e;
+    return launch_pdl(kern, dim3(a.kv_heads * groups, decode_splits(a, sms)), dim3(WD_WARPS * 32), smem, st, a, groups, out, counters, part);
 }
 template <typename T, int GR>
 cudaError_t launch_decode_nc(const hf2q_window_attn& a, float* out, uint8_t* scratch, int sms, cudaStream_t st) {
-    if (a.vdim <= 64) return launch_decode<T, GR, 1>(a, out, scratch, sms, st);
-    if (a.vdim <= 128) return launch_decode<T, GR, 2>(a, out, scratch, sms, st);
-    return launch_decode<T, GR, 4>(a, out, scratch, sms, st);
+    if (a.vdim <= 128) return launch_decode<T, GR, 1>(a, out, scratch, sms, st);
+    return launch_decode<T, GR, 2>(a, out, scratch, sms, st);
 }
 template <typename T>
 cudaError_t launch_decode_gr(const hf2q_window_attn& a, float* out, uint8_t* scratch, int sms, cudaStream_t st) {
