@@ -49,6 +49,11 @@ SIGNATURES = {
     "hf2q_cuda_qmatmul_swiglu_ws": (i32, [vp, vp, vp, u32, vp, vp, vp, u32, u32, u32, u32, vp, u64]),
     "hf2q_cuda_qmatmul_add_ws_supported": (i32, [vp, u32, u32, u32, u32, u32]),
     "hf2q_cuda_qmatmul_add_ws": (i32, [vp, vp, vp, u32, vp, vp, vp, u32, u32, u32, u32, vp, u64]),
+    "hf2q_cuda_panel_supported": (i32, [vp, u32, u32, u32, u32]),
+    "hf2q_cuda_rms_norm_panel": (i32, [vp, vp, vp, vp, vp, C.c_float, vp, u32, u32]),
+    "hf2q_cuda_attn_prefill_panel": (i32, [vp, vp, vp, u32, u32, vp, u32, vp]),
+    "hf2q_cuda_qmatmul_panel": (i32, [vp, vp, vp, vp, u32, vp, vp, u32, u32]),
+    "hf2q_cuda_qmatmul_swiglu_panel": (i32, [vp, vp, vp, u32, vp, vp, vp, u32, u32, u32, u32, vp, u64]),
     "hf2q_cuda_qmatmul_host": (i32, [vp, vp, u32, vp, vp, u32, u32, u32, u32]),
     "hf2q_cuda_qmatmul_host_async": (i32, [vp, vp, u32, vp, vp, u32, u32, u32, u32]),
     "hf2q_cuda_host_sync": (i32, [vp]),

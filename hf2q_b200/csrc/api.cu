@@ -690,6 +690,67 @@ HF2Q_API int32_t hf2q_cuda_qmatmul_add_ws(hf2q_ctx* ctx, void* stream, const voi
     return HF2Q_OK;
 }
 
+// ---- the tensor-core products on a panel: activations as the f16 [m][k] they multiply, written by the kernel in front ----
+
+HF2Q_API int32_t hf2q_cuda_panel_supported(hf2q_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, uint32_t type) {
+    return m > 8 && hf2q_cuda_qmatmul_add_ws_supported(ctx, m, n, k, type, HF2Q_DT_F32);
+}
+
+HF2Q_API int32_t hf2q_cuda_qmatmul_panel(hf2q_ctx* ctx, void* stream, const void* panel, const hf2q_row_segment* segs, uint32_t n_segs, const float* residual,
+                                         float* y, uint32_t m, uint32_t k) {
+    if (!ctx) return HF2Q_ERR_INVALID_ARGUMENT;
+    const char* who = "qmatmul_panel";
+    if (!panel || !segs || !y || n_segs == 0 || n_segs > 16 || (residual && n_segs != 1))
+        return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: null pointer, n_segs=%u not in 1..16, or a residual for several ranges", who, n_segs);
+    uint64_t n = 0;
+    for (uint32_t i = 0; i < n_segs; ++i) {
+        if (!segs[i].w) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: segment %u has no weights", who, i);
+        const int32_t rc = check_matmul_shape(ctx, segs[i].ggml_type, segs[i].rows, k, who);
+        if (rc) return rc;
+        if (!hf2q_cuda_panel_supported(ctx, m, segs[i].rows, k, segs[i].ggml_type) || !gemm_tc_supported(segs[i].ggml_type, segs[i].w, segs[i].rows, k))
+            return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: needs more than 8 rows, 16-byte aligned weight rows and k %% 256 == 0 (ask hf2q_cuda_panel_supported)", who);
+        n += segs[i].rows;
+    }
+    if (n > 0xffffffffull || reinterpret_cast<uintptr_t>(panel) % 16 || (reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) % 4)
+        return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: misaligned buffer or %llu rows", who, (unsigned long long)n);
+    DeviceGuard dg(ctx->device);
+    uint32_t col0 = 0;
+    for (uint32_t i = 0; i < n_segs; ++i) {
+        int nl = 0;
+        const cudaError_t e = launch_gemm_tc(segs[i].ggml_type, segs[i].w, nullptr, HF2Q_DT_F16, y + col0, m, segs[i].rows, k, const_cast<void*>(panel), ctx->status,
+                                             ctx->dev.sm_count, static_cast<cudaStream_t>(stream), &nl, static_cast<uint32_t>(n), true, residual);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_panel launch");
+        ctx->launches += nl;
+        col0 += segs[i].rows;
+    }
+    return HF2Q_OK;
+}
+
+HF2Q_API int32_t hf2q_cuda_qmatmul_swiglu_panel(hf2q_ctx* ctx, void* stream, const void* x, uint32_t x_dtype, const void* w_gate, const void* w_up,
+                                                void* y_panel, uint32_t m, uint32_t n, uint32_t k, uint32_t type, void* workspace, uint64_t workspace_bytes) {
+    if (!ctx) return HF2Q_ERR_INVALID_ARGUMENT;
+    const char* who = "qmatmul_swiglu_panel";
+    if (!x || !w_gate || !w_up || !y_panel || x_dtype > HF2Q_DT_BF16) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: null pointer or x_dtype %u", who, x_dtype);
+    const int32_t rc = check_matmul_shape(ctx, type, n, k, who);
+    if (rc) return rc;
+    const bool ready = x_dtype == HF2Q_DT_F16;
+    if (reinterpret_cast<uintptr_t>(x) % (ready ? 16 : dtype_size(x_dtype)) || reinterpret_cast<uintptr_t>(y_panel) % 16)
+        return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: misaligned buffer", who);
+    if (!hf2q_cuda_panel_supported(ctx, m, n, k, type) || !gemm_tc_swiglu_supported(type) || !gemm_tc_supported(type, w_gate, n, k) || !gemm_tc_supported(type, w_up, n, k))
+        return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: needs more than 8 rows, one of the five main formats, 16-byte aligned weight rows and k %% 256 == 0", who);
+    if (!ready && (!workspace || workspace_bytes < gemm_tc_workspace_bytes(m, k)))
+        return fail(ctx, HF2Q_ERR_WORKSPACE, "%s: m=%u needs a workspace of %llu bytes (got %llu)", who, m, (unsigned long long)gemm_tc_workspace_bytes(m, k),
+                    (unsigned long long)workspace_bytes);
+    if (!ready && reinterpret_cast<uintptr_t>(workspace) % 256) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "%s: workspace must be 256-byte aligned", who);
+    DeviceGuard dg(ctx->device);
+    int nl = 0;
+    const cudaError_t e = launch_gemm_tc_swiglu(type, w_gate, w_up, x, x_dtype, nullptr, m, n, k, ready ? const_cast<void*>(x) : workspace, ctx->status,
+                                                ctx->dev.sm_count, static_cast<cudaStream_t>(stream), &nl, ready, y_panel);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_swiglu_panel launch");
+    ctx->launches += nl;
+    return HF2Q_OK;
+}
+
 // ---- row-sharded mat-vec with the all-gather in its epilogue (several GPUs, one process each) ----
 
 HF2Q_API int32_t hf2q_cuda_ipc_alloc(hf2q_ctx* ctx, uint64_t bytes, void** dev, uint8_t* handle64) {
@@ -1541,8 +1602,20 @@ HF2Q_API int32_t hf2q_cuda_rms_norm(hf2q_ctx* ctx, void* stream, float* x, const
     if (out_dtype != HF2Q_DT_F32 && out_dtype != HF2Q_DT_BF16) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "rms_norm: out_dtype %u (want F32 or BF16)", out_dtype);
     if (m == 0) return HF2Q_OK;
     DeviceGuard dg(ctx->device);
-    const cudaError_t e = launch_rms_norm(x, delta, weight, eps, out, out_dtype, m, h, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_rms_norm(x, delta, weight, eps, out, out_dtype, m, h, ctx->status, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "rms_norm launch");
+    ctx->launches += 1;
+    return HF2Q_OK;
+}
+
+HF2Q_API int32_t hf2q_cuda_rms_norm_panel(hf2q_ctx* ctx, void* stream, float* x, const float* delta, const float* weight, float eps, void* panel, uint32_t m,
+                                          uint32_t h) {
+    if (!ctx) return HF2Q_ERR_INVALID_ARGUMENT;
+    if (!x || !weight || !panel || h == 0 || reinterpret_cast<uintptr_t>(panel) % 2) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "rms_norm_panel: null pointer or h == 0");
+    if (m == 0) return HF2Q_OK;
+    DeviceGuard dg(ctx->device);
+    const cudaError_t e = launch_rms_norm(x, delta, weight, eps, panel, HF2Q_DT_F16, m, h, ctx->status, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "rms_norm_panel launch");
     ctx->launches += 1;
     return HF2Q_OK;
 }
@@ -1611,8 +1684,8 @@ HF2Q_API int32_t hf2q_cuda_attn_decode_fused(hf2q_ctx* ctx, void* stream, const 
     return HF2Q_OK;
 }
 
-HF2Q_API int32_t hf2q_cuda_attn_prefill(hf2q_ctx* ctx, void* stream, const float* qkv, uint32_t m, uint32_t n_q_heads,
-                                        const hf2q_kv_cache* kv, uint32_t pos0, void* out, uint32_t out_dtype) {
+static int32_t attn_prefill_to(hf2q_ctx* ctx, void* stream, const float* qkv, uint32_t m, uint32_t n_q_heads, const hf2q_kv_cache* kv, uint32_t pos0, void* out,
+                               uint32_t out_dtype, bool panel) {
     if (!ctx) return HF2Q_ERR_INVALID_ARGUMENT;
     if (!qkv || !out) return fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "attn_prefill: null pointer");
     const int32_t rc = check_kv(ctx, kv, n_q_heads, "attn_prefill");
@@ -1621,11 +1694,22 @@ HF2Q_API int32_t hf2q_cuda_attn_prefill(hf2q_ctx* ctx, void* stream, const float
     if (m == 0) return HF2Q_OK;
     DeviceGuard dg(ctx->device);
     const uint32_t stride = (n_q_heads + 2 * kv->n_kv_heads) * kv->head_dim;
-    const cudaError_t e = launch_attn_prefill(qkv, stride, m, n_q_heads, kv->n_kv_heads, kv->head_dim, view_of(kv), pos0, out, out_dtype,
-                                              n_q_heads * kv->head_dim, ctx->status, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = (out_dtype == HF2Q_DT_F16) != panel ? cudaErrorInvalidValue
+                                                              : launch_attn_prefill(qkv, stride, m, n_q_heads, kv->n_kv_heads, kv->head_dim, view_of(kv), pos0, out, out_dtype,
+                                                                                    n_q_heads * kv->head_dim, ctx->status, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "attn_prefill launch");
     ctx->launches += 1;
     return HF2Q_OK;
+}
+
+HF2Q_API int32_t hf2q_cuda_attn_prefill(hf2q_ctx* ctx, void* stream, const float* qkv, uint32_t m, uint32_t n_q_heads,
+                                        const hf2q_kv_cache* kv, uint32_t pos0, void* out, uint32_t out_dtype) {
+    return attn_prefill_to(ctx, stream, qkv, m, n_q_heads, kv, pos0, out, out_dtype, false);
+}
+
+HF2Q_API int32_t hf2q_cuda_attn_prefill_panel(hf2q_ctx* ctx, void* stream, const float* qkv, uint32_t m, uint32_t n_q_heads,
+                                              const hf2q_kv_cache* kv, uint32_t pos0, void* panel) {
+    return attn_prefill_to(ctx, stream, qkv, m, n_q_heads, kv, pos0, panel, HF2Q_DT_F16, true);
 }
 
 HF2Q_API int32_t hf2q_cuda_argmax(hf2q_ctx* ctx, void* stream, const float* logits, uint32_t n, uint32_t* out_id, uint32_t* pos) {

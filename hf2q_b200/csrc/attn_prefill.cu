@@ -74,6 +74,13 @@ __device__ __forceinline__ float2 hide(float2 x, uint32_t p, uint32_t seen, floa
     return make_float2(p <= seen ? x.x : hidden, p + 1 <= seen ? x.y : hidden);
 }
 
+// OUT __half: the f16 activation panel of the product that follows
+template <typename OUT> __device__ __forceinline__ OUT out_value(float v, bool& clipped) {
+    if constexpr (std::is_same_v<OUT, float>) return v;
+    else if constexpr (std::is_same_v<OUT, __half>) return panel_f16(v, clipped);
+    else return __float2bfloat16_rn(v);
+}
+
 template <int G, typename OUT>
 __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float* __restrict__ qkv, uint32_t row_stride, uint32_t m,
                                                                      const int8_t* __restrict__ k_codes, const float* __restrict__ k_scale,
@@ -291,6 +298,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
             const float l = f2_sum(sum), inv = l > 0.f ? (1.0f / 256.0f) / l : 0.f;
             OUT* dst = out + static_cast<size_t>(live ? tok : 0) * out_stride + (static_cast<size_t>(kvh) * G + row % G) * HD;
             const bool wide = reinterpret_cast<uintptr_t>(out) % 16 == 0;      // rows are whole numbers of heads
+            bool clipped = false;
 #pragma unroll 1
             for (uint32_t c = 0; c < HD; c += 32) {
                 uint32_t o[32];
@@ -308,19 +316,20 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attn_prefill_kernel(const float
                             for (int i = 0; i < 32; ++i) dst[c + i] = v[i];
                         }
                     } else {
-                        __nv_bfloat162 h[16];
+                        __align__(16) OUT h[32];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                        for (int i = 0; i < 32; ++i) h[i] = out_value<OUT>(v[i], clipped);
                         if (wide) {
 #pragma unroll
                             for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(dst + c)[i] = reinterpret_cast<const uint4*>(h)[i];
                         } else {
-                            for (int i = 0; i < 16; ++i) { dst[c + 2 * i] = h[i].x; dst[c + 2 * i + 1] = h[i].y; }
+                            for (int i = 0; i < 32; ++i) dst[c + i] = h[i];
                         }
                     }
                 }
                 __syncwarp();                                  // the next load from tensor memory is the whole warp's
             }
+            if (clipped) atomicOr(status, STATUS_X_CLIPPED);
         }
         tc_fence_before();
     }
@@ -339,7 +348,8 @@ template <int G, typename OUT>
 __global__ void __launch_bounds__(FEW_WARPS * 32) attn_prefill_few_kernel(const float* __restrict__ qkv, uint32_t row_stride, uint32_t m,
                                                                           const int8_t* __restrict__ k_codes, const float* __restrict__ k_scale,
                                                                           const int8_t* __restrict__ v_codes, const float* __restrict__ v_scale,
-                                                                          uint32_t max_seq, uint32_t pos0, OUT* __restrict__ out, uint32_t out_stride) {
+                                                                          uint32_t max_seq, uint32_t pos0, OUT* __restrict__ out, uint32_t out_stride,
+                                                                          uint32_t* status) {
     __shared__ uint32_t ks[FEW][HD / 4 + 1], vs[FEW][HD / 4 + 1];  // code + 128 in every byte
     __shared__ float k_s[FEW], v_s[FEW];
     __shared__ __align__(16) float qs[FEW_WARPS][HD];
@@ -392,11 +402,10 @@ __global__ void __launch_bounds__(FEW_WARPS * 32) attn_prefill_few_kernel(const 
     }
     const float inv = l > 0.f ? 1.0f / l : 0.f;
     OUT* dst = out + static_cast<size_t>(tok) * out_stride + (static_cast<size_t>(kvh) * G + row % G) * HD + 4 * lane;
+    bool clipped = false;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if constexpr (std::is_same_v<OUT, float>) dst[j] = o[j] * inv;
-        else dst[j] = __float2bfloat16_rn(o[j] * inv);
-    }
+    for (int j = 0; j < 4; ++j) dst[j] = out_value<OUT>(o[j] * inv, clipped);
+    if (clipped) atomicOr(status, STATUS_X_CLIPPED);
 }
 
 template <int G, typename OUT>
@@ -404,7 +413,7 @@ cudaError_t launch_prefill_g(const float* qkv, uint32_t row_stride, uint32_t m, 
                              uint32_t out_stride, uint32_t* status, cudaStream_t st) {
     if (static_cast<uint64_t>(pos0) + m <= FEW) {
         attn_prefill_few_kernel<G, OUT><<<dim3((m * G + FEW_WARPS - 1) / FEW_WARPS, n_kv), FEW_WARPS * 32, 0, st>>>(
-            qkv, row_stride, m, kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, pos0, out, out_stride);
+            qkv, row_stride, m, kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, pos0, out, out_stride, status);
         return cudaGetLastError();
     }
     static PerDeviceFlag flag;
@@ -421,11 +430,12 @@ cudaError_t launch_attn_prefill(const float* qkv, uint32_t row_stride, uint32_t 
                                 const KvCacheView& kv, uint32_t pos0, void* out, uint32_t out_dtype, uint32_t out_stride, uint32_t* status,
                                 cudaStream_t st) {
     if (hd != HD || n_kv == 0 || n_q % n_kv) return cudaErrorInvalidValue;
-    const bool f32 = out_dtype == HF2Q_DT_F32;
-    if (!f32 && out_dtype != HF2Q_DT_BF16) return cudaErrorInvalidValue;
     switch (n_q / n_kv) {
-#define HF2Q_CASE(GG) case GG: return f32 ? launch_prefill_g<GG, float>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<float*>(out), out_stride, status, st) \
-                                          : launch_prefill_g<GG, __nv_bfloat16>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<__nv_bfloat16*>(out), out_stride, status, st);
+#define HF2Q_CASE(GG) case GG: \
+        if (out_dtype == HF2Q_DT_F32) return launch_prefill_g<GG, float>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<float*>(out), out_stride, status, st); \
+        if (out_dtype == HF2Q_DT_F16) return launch_prefill_g<GG, __half>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<__half*>(out), out_stride, status, st); \
+        if (out_dtype == HF2Q_DT_BF16) return launch_prefill_g<GG, __nv_bfloat16>(qkv, row_stride, m, kv, n_kv, pos0, static_cast<__nv_bfloat16*>(out), out_stride, status, st); \
+        return cudaErrorInvalidValue;
         HF2Q_CASE(1) HF2Q_CASE(2) HF2Q_CASE(4) HF2Q_CASE(8)
 #undef HF2Q_CASE
         default: return cudaErrorInvalidValue;

@@ -247,6 +247,11 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32
         ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
         : "memory");
 }
+// An element of a tensor-core product's f16 activation panel: beyond the f16 range it is clipped, and noted.
+__device__ __forceinline__ __half panel_f16(float v, bool& clipped) {
+    clipped |= fabsf(v) > 65504.0f;
+    return __float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f));
+}
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
     uint64_t pol;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));

@@ -18,6 +18,8 @@
 //   k_scale, v_scale : float [n_kv_heads][max_seq]
 #include <math_constants.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -44,11 +46,71 @@ __global__ void __launch_bounds__(256) get_rows_kernel(const uint8_t* __restrict
 
 // ------------------------------------------------------------------ RMSNorm (+ residual add)
 // x[t,:] += delta[t,:] (if delta), then out[t,:] = x[t,:] * rsqrt(mean(x^2) + eps) * weight[:]
-// (forward_cpu.rs:36-48: sum of squares in f32, sequential per row there, tree-reduced here).
+// (forward_cpu.rs:36-48: sum of squares in f32, sequential per row there, tree-reduced here).  OUT __half: the f16 activation
+// panel of a tensor-core product, so that the product needs no conversion pass.
+template <typename OUT> __device__ __forceinline__ OUT norm_out(float v, bool& clipped) {
+    if constexpr (std::is_same_v<OUT, float>) return v;
+    else if constexpr (std::is_same_v<OUT, __half>) return panel_f16(v, clipped);
+    else return __float2bfloat16_rn(v);
+}
+__device__ __forceinline__ float block_sum(float v, float* part) {       // part [32] in shared memory
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = (threadIdx.x & 31) < (blockDim.x >> 5) ? part[threadIdx.x & 31] : 0.f;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// A row per CTA, read once: each thread keeps its 16-byte groups in registers.  Bound by memory; 2048 rows of 4096 to f16 move
+// 50 MB, 7.7 us at the copy rate: 11.4 us (one element a thread and step, f32 out, and the conversion behind it: 28 + 7).  Rows of up to 4 NORM_VECS NORM_THREADS elements on 16-byte boundaries.
+constexpr int NORM_THREADS = 256, NORM_VECS = 8;
 template <typename OUT>
-__global__ void __launch_bounds__(1024) rms_norm_kernel(float* __restrict__ x, const float* __restrict__ delta,
-                                                        const float* __restrict__ weight, float eps, OUT* __restrict__ out,
-                                                        uint32_t h) {
+__global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ weight,
+                                                                float eps, OUT* __restrict__ out, uint32_t h, uint32_t* status) {
+    __shared__ float part[32];
+    const uint32_t n4 = h / 4;
+    float4* row = reinterpret_cast<float4*>(x + static_cast<size_t>(blockIdx.x) * h);
+    const float4* drow = reinterpret_cast<const float4*>(delta ? delta + static_cast<size_t>(blockIdx.x) * h : nullptr);
+    float4 v[NORM_VECS];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NORM_VECS; ++j) {
+        const uint32_t i = threadIdx.x + NORM_THREADS * j;
+        v[j] = i < n4 ? row[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (drow) {
+#pragma unroll
+        for (int j = 0; j < NORM_VECS; ++j) {
+            const uint32_t i = threadIdx.x + NORM_THREADS * j;
+            if (i < n4) {
+                const float4 d = drow[i];
+                v[j].x += d.x; v[j].y += d.y; v[j].z += d.z; v[j].w += d.w;
+                row[i] = v[j];
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NORM_VECS; ++j) ss += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
+    const float inv = 1.0f / sqrtf(block_sum(ss, part) / static_cast<float>(h) + eps);
+    bool clipped = false;
+    OUT* orow = out + static_cast<size_t>(blockIdx.x) * h;
+#pragma unroll
+    for (int j = 0; j < NORM_VECS; ++j) {
+        const uint32_t i = threadIdx.x + NORM_THREADS * j;
+        if (i < n4) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(weight) + i);
+            struct alignas(4 * sizeof(OUT)) { OUT e[4]; } o;
+            o.e[0] = norm_out<OUT>(v[j].x * inv * w.x, clipped); o.e[1] = norm_out<OUT>(v[j].y * inv * w.y, clipped);
+            o.e[2] = norm_out<OUT>(v[j].z * inv * w.z, clipped); o.e[3] = norm_out<OUT>(v[j].w * inv * w.w, clipped);
+            reinterpret_cast<decltype(o)*>(orow)[i] = o;
+        }
+    }
+    if (clipped) atomicOr(status, STATUS_X_CLIPPED);
+}
+// rows of any length and alignment
+template <typename OUT>
+__global__ void __launch_bounds__(1024) rms_norm_any_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ weight,
+                                                            float eps, OUT* __restrict__ out, uint32_t h, uint32_t* status) {
     __shared__ float part[32];
     float* row = x + static_cast<size_t>(blockIdx.x) * h;
     const float* drow = delta ? delta + static_cast<size_t>(blockIdx.x) * h : nullptr;
@@ -59,67 +121,66 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(float* __restrict__ x, c
         if (drow) { v += drow[i]; row[i] = v; }
         ss += v * v;
     }
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.f;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) part[0] = 1.0f / sqrtf(v / static_cast<float>(h) + eps);
-    }
-    __syncthreads();
-    const float inv = part[0];
-    for (uint32_t i = threadIdx.x; i < h; i += blockDim.x) {
-        const float v = row[i] * inv * weight[i];
-        if constexpr (sizeof(OUT) == 4) orow[i] = v;
-        else orow[i] = __float2bfloat16_rn(v);
-    }
+    const float inv = 1.0f / sqrtf(block_sum(ss, part) / static_cast<float>(h) + eps);
+    bool clipped = false;
+    for (uint32_t i = threadIdx.x; i < h; i += blockDim.x) orow[i] = norm_out<OUT>(row[i] * inv * weight[i], clipped);
+    if (clipped) atomicOr(status, STATUS_X_CLIPPED);
 }
 
 // ------------------------------------------------------------------ rotary embedding + KV append
-// qkv: [m][(n_q + 2 n_kv) * hd] f32 (fused QKV product).  Token t sits at position *pos + t.
-// One warp per (token, head).  q heads are rotated in place and scaled by `q_scale` (1/sqrt(hd), so
-// the attention kernels need no multiply); k heads are rotated, then k and v heads are quantized
+// qkv: [m][(n_q + 2 n_kv) * 128] f32 (fused QKV product).  Token t sits at position *pos + t.
+// One CTA per token, one warp per head at a time, four elements a lane.  The 64 angles of a token are the same for all its
+// heads: pow, sine and cosine are taken once per token, not once per head (2048 tokens, 32 + 16 heads: 43 -> 13 us).  q heads are rotated in place and scaled by `q_scale`
+// (1/sqrt(hd), so the attention kernels need no multiply); k heads are rotated, then k and v heads are quantized
 // to int8 with one scale per (head, position) and stored in the cache.  Pairs are (2i, 2i+1) with
 // angle pos * theta^(-2i/hd) -- the rotary form of the Llama architecture.
-__global__ void __launch_bounds__(256) rope_kv_append_kernel(float* __restrict__ qkv, uint32_t m, uint32_t n_q, uint32_t n_kv,
-                                                             uint32_t hd, const uint32_t* __restrict__ pos_dev, float theta,
-                                                             float q_scale, int8_t* __restrict__ k_codes, float* __restrict__ k_scale,
-                                                             int8_t* __restrict__ v_codes, float* __restrict__ v_scale,
-                                                             uint32_t max_seq, uint32_t* status) {
-    const uint32_t heads = n_q + 2 * n_kv;
-    const uint32_t wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (wid >= m * heads) return;
-    const uint32_t t = wid / heads, hidx = wid % heads;
-    const uint32_t pos = *pos_dev + t;
-    float* v = qkv + static_cast<size_t>(t) * heads * hd + static_cast<size_t>(hidx) * hd;
-    const bool is_q = hidx < n_q, is_k = !is_q && hidx < n_q + n_kv;
-    // hd <= 256: each lane owns up to 4 consecutive pairs
-    float vals[8];
-    const uint32_t per = hd / 32;                        // elements per lane (hd = 64, 128 or 256)
-    float amax = 0.f;
-    for (uint32_t j = 0; j < per; j += 2) {
-        const uint32_t e = lane * per + j;
-        float a = v[e], b = v[e + 1];
-        if (is_q || is_k) {
-            const float freq = powf(theta, -static_cast<float>(e) / static_cast<float>(hd));
-            float sn, cs;
-            sincosf(static_cast<float>(pos) * freq, &sn, &cs);
-            const float ra = a * cs - b * sn, rb = a * sn + b * cs;
-            a = ra; b = rb;
-        }
-        if (is_q) { a *= q_scale; b *= q_scale; v[e] = a; v[e + 1] = b; }
-        vals[j] = a; vals[j + 1] = b;
-        amax = fmaxf(amax, fmaxf(fabsf(a), fabsf(b)));
+constexpr uint32_t ROPE_HD = 128;
+__global__ void __launch_bounds__(256) rope_kv_append_kernel(float* __restrict__ qkv, uint32_t n_q, uint32_t n_kv, const uint32_t* __restrict__ pos_dev,
+                                                             float theta, float q_scale, int8_t* __restrict__ k_codes, float* __restrict__ k_scale,
+                                                             int8_t* __restrict__ v_codes, float* __restrict__ v_scale, uint32_t max_seq, bool wide,
+                                                             uint32_t* status) {
+    __shared__ __align__(16) float2 turn[ROPE_HD / 2];                   // cosine, sine
+    const uint32_t heads = n_q + 2 * n_kv, t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pos = *pos_dev + t;
+    if (threadIdx.x < ROPE_HD / 2) {
+        const float freq = powf(theta, -static_cast<float>(2 * threadIdx.x) / static_cast<float>(ROPE_HD));
+        float sn, cs;
+        sincosf(static_cast<float>(pos) * freq, &sn, &cs);
+        turn[threadIdx.x] = make_float2(cs, sn);
     }
-    if (is_q) return;
-    if (pos >= max_seq) { if (lane == 0) atomicOr(status, STATUS_BAD_EXPERT_ID); return; }
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = amax / 127.0f, inv = amax > 0.f ? 127.0f / amax : 0.f;
-    const uint32_t kvh = is_k ? hidx - n_q : hidx - n_q - n_kv;
-    int8_t* codes = (is_k ? k_codes : v_codes) + (static_cast<size_t>(kvh) * max_seq + pos) * hd;
-    for (uint32_t j = 0; j < per; ++j) codes[lane * per + j] = static_cast<int8_t>(__float2int_rn(vals[j] * inv));
-    if (lane == 0) (is_k ? k_scale : v_scale)[static_cast<size_t>(kvh) * max_seq + pos] = scale;
+    __syncthreads();
+    const float4 cs = *reinterpret_cast<const float4*>(&turn[2 * lane]);
+    for (uint32_t hidx = warp; hidx < heads; hidx += 8) {
+        float* v = qkv + (static_cast<size_t>(t) * heads + hidx) * ROPE_HD + 4 * lane;
+        const bool is_q = hidx < n_q, is_k = !is_q && hidx < n_q + n_kv;
+        float e[4];
+        if (wide) { const float4 f = *reinterpret_cast<const float4*>(v); e[0] = f.x; e[1] = f.y; e[2] = f.z; e[3] = f.w; }
+        else
+            for (int j = 0; j < 4; ++j) e[j] = v[j];
+        if (is_q || is_k) {
+            const float a0 = e[0] * cs.x - e[1] * cs.y, b0 = e[0] * cs.y + e[1] * cs.x, a1 = e[2] * cs.z - e[3] * cs.w, b1 = e[2] * cs.w + e[3] * cs.z;
+            e[0] = a0; e[1] = b0; e[2] = a1; e[3] = b1;
+        }
+        if (is_q) {
+            for (int j = 0; j < 4; ++j) e[j] *= q_scale;
+            if (wide) *reinterpret_cast<float4*>(v) = make_float4(e[0], e[1], e[2], e[3]);
+            else
+                for (int j = 0; j < 4; ++j) v[j] = e[j];
+            continue;
+        }
+        if (pos >= max_seq) { if (lane == 0) atomicOr(status, STATUS_BAD_EXPERT_ID); continue; }
+        float amax = fmaxf(fmaxf(fabsf(e[0]), fabsf(e[1])), fmaxf(fabsf(e[2]), fabsf(e[3])));
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        const float scale = amax / 127.0f, inv = amax > 0.f ? 127.0f / amax : 0.f;
+        const uint32_t kvh = is_k ? hidx - n_q : hidx - n_q - n_kv;
+        const size_t at = static_cast<size_t>(kvh) * max_seq + pos;
+        int8_t* codes = (is_k ? k_codes : v_codes) + at * ROPE_HD + 4 * lane;
+        int8_t c[4];
+        for (int j = 0; j < 4; ++j) c[j] = static_cast<int8_t>(__float2int_rn(e[j] * inv));
+        if (wide) *reinterpret_cast<char4*>(codes) = make_char4(c[0], c[1], c[2], c[3]);
+        else
+            for (int j = 0; j < 4; ++j) codes[j] = c[j];
+        if (lane == 0) (is_k ? k_scale : v_scale)[at] = scale;
+    }
 }
 
 // ------------------------------------------------------------------ decode attention, split over the context
@@ -645,20 +706,33 @@ cudaError_t launch_get_rows(uint32_t type, const void* w, uint64_t row_bytes, ui
     return cudaGetLastError();
 }
 
-cudaError_t launch_rms_norm(float* x, const float* delta, const float* weight, float eps, void* out, uint32_t out_dtype, uint32_t m,
-                            uint32_t h, cudaStream_t st) {
-    const unsigned threads = h >= 4096 ? 1024 : h >= 1024 ? 512 : 256;
-    if (out_dtype == HF2Q_DT_F32) rms_norm_kernel<float><<<m, threads, 0, st>>>(x, delta, weight, eps, static_cast<float*>(out), h);
-    else if (out_dtype == HF2Q_DT_BF16) rms_norm_kernel<__nv_bfloat16><<<m, threads, 0, st>>>(x, delta, weight, eps, static_cast<__nv_bfloat16*>(out), h);
-    else return cudaErrorInvalidValue;
+namespace {
+template <typename OUT>
+cudaError_t rms_norm_to(float* x, const float* delta, const float* weight, float eps, OUT* out, uint32_t m, uint32_t h, uint32_t* status, cudaStream_t st) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(out);
+    if (h % 4 == 0 && h <= 4u * NORM_VECS * NORM_THREADS && at % 16 == 0) {
+        rms_norm_kernel<OUT><<<m, NORM_THREADS, 0, st>>>(x, delta, weight, eps, out, h, status);
+    } else {
+        const unsigned threads = h >= 4096 ? 1024 : h >= 1024 ? 512 : 256;
+        rms_norm_any_kernel<OUT><<<m, threads, 0, st>>>(x, delta, weight, eps, out, h, status);
+    }
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_rms_norm(float* x, const float* delta, const float* weight, float eps, void* out, uint32_t out_dtype, uint32_t m,
+                            uint32_t h, uint32_t* status, cudaStream_t st) {
+    if (out_dtype == HF2Q_DT_F32) return rms_norm_to(x, delta, weight, eps, static_cast<float*>(out), m, h, status, st);
+    if (out_dtype == HF2Q_DT_BF16) return rms_norm_to(x, delta, weight, eps, static_cast<__nv_bfloat16*>(out), m, h, status, st);
+    return rms_norm_to(x, delta, weight, eps, static_cast<__half*>(out), m, h, status, st);
 }
 
 cudaError_t launch_rope_kv_append(float* qkv, uint32_t m, uint32_t n_q, uint32_t n_kv, uint32_t hd, const uint32_t* pos, float theta,
                                   const KvCacheView& kv, uint32_t* status, cudaStream_t st) {
-    const uint32_t warps = m * (n_q + 2 * n_kv);
-    rope_kv_append_kernel<<<(warps + 7) / 8, 256, 0, st>>>(qkv, m, n_q, n_kv, hd, pos, theta, 1.0f / sqrtf(static_cast<float>(hd)),
-                                                            kv.k_codes, kv.k_scale, kv.v_codes, kv.v_scale, kv.max_seq, status);
+    if (hd != ROPE_HD) return cudaErrorInvalidValue;
+    const bool wide = reinterpret_cast<uintptr_t>(qkv) % 16 == 0 && (reinterpret_cast<uintptr_t>(kv.k_codes) | reinterpret_cast<uintptr_t>(kv.v_codes)) % 4 == 0;
+    rope_kv_append_kernel<<<m, 256, 0, st>>>(qkv, n_q, n_kv, pos, theta, 1.0f / sqrtf(static_cast<float>(hd)), kv.k_codes, kv.k_scale, kv.v_codes,
+                                             kv.v_scale, kv.max_seq, wide, status);
     return cudaGetLastError();
 }
 

@@ -47,6 +47,14 @@ int32_t dense_ffn(hf2q_ctx* ctx, void* stream, const void* x, uint32_t x_dtype, 
     const uint64_t ws_bytes = L.total - L.ws;
     const bool fuse = !(flags & HF2Q_FFN_NO_FUSION);
     int32_t rc;
+    // more than 8 rows: the pair writes the panel that the down product multiplies
+    if (fuse && type_gate == type_up && m > 8 && x_dtype != HF2Q_DT_F16 && hf2q_cuda_qmatmul_swiglu_ws_supported(ctx, m, ffn, hidden, type_gate, x_dtype) &&
+        hf2q_cuda_panel_supported(ctx, m, hidden, ffn, type_down) && reinterpret_cast<uintptr_t>(w_down) % 16 == 0) {
+        rc = hf2q_cuda_qmatmul_swiglu_panel(ctx, stream, x, x_dtype, w_gate, w_up, act, m, ffn, hidden, type_gate, ws, ws_bytes);
+        if (rc) return rc;
+        const hf2q_row_segment down{w_down, hidden, type_down};
+        return hf2q_cuda_qmatmul_panel(ctx, stream, act, &down, 1, residual, y, m, ffn);
+    }
     if (fuse && type_gate == type_up && hf2q_cuda_qmatmul_swiglu_ws_supported(ctx, m, ffn, hidden, type_gate, x_dtype)) {
         rc = hf2q_cuda_qmatmul_swiglu_ws(ctx, stream, x, x_dtype, w_gate, w_up, act, m, ffn, hidden, type_gate, ws, ws_bytes);
         if (rc) return rc;

@@ -91,7 +91,7 @@ struct GParams {
     const uint32_t* n_tiles;
     const uint32_t* perm;
     // epilogue options: y += residual (same layout as y); DUAL kernels store silu(gate) * up, either as f32 into y
-    // or, for the expert-routed form, as f16 into act16[sorted row][n] (the down product's activation panel)
+    // or as f16 into act16[row, or sorted row][n] (the down product's activation panel)
     const float* residual;
     __half* act16;
     // expert-routed product only: instead of storing row perm[tok] of y, add route_w[perm[tok]] * value to row
@@ -339,9 +339,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                         const uint32_t tok = tok0 + c0 + j + (upper ? 1 : 0);
                         if (row < p.n && tok < tok_end) {
                             const float act = g / (1.0f + expf(-g)) * u;
-                            if (GROUPED && p.act16) {          // same clipping rule as the f32 -> f16 conversion of any activation panel
-                                clipped |= fabsf(act) > 65504.0f;
-                                p.act16[static_cast<size_t>(tok) * p.n + row] = __float2half_rn(fminf(fmaxf(act, -65504.0f), 65504.0f));
+                            if (p.act16) {
+                                p.act16[static_cast<size_t>(tok) * p.n + row] = panel_f16(act, clipped);
                             } else {
                                 p.y[static_cast<size_t>(GROUPED ? p.perm[tok] : tok) * p.ldy + row] = act;
                             }
@@ -409,6 +408,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         constexpr uint32_t PER = GEMM_THREADS / TILE_ROWS;           // columns at a time
         if (threadIdx.x < PER * TILE_ROWS && row < p.n) {
             const uint32_t lane_of = DUAL ? (out_row / 16) * 32 + out_row % 16 : out_row;
+            bool clipped = false;
             for (uint32_t c = part + parts * (threadIdx.x / TILE_ROWS); c < cols; c += parts * PER) {
                 float v = 0.f, up = 0.f;
                 for (uint32_t q = 0; q < parts; ++q) {
@@ -417,9 +417,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                     if constexpr (DUAL) up += s[16];
                 }
                 const size_t o = static_cast<size_t>(tok0 + c) * p.ldy + row;
-                if constexpr (DUAL) p.y[o] = v / (1.0f + expf(-v)) * up;
-                else p.y[o] = p.residual ? v + __ldcg(p.residual + o) : v;
+                if constexpr (DUAL) {
+                    const float act = v / (1.0f + expf(-v)) * up;
+                    if (p.act16) p.act16[static_cast<size_t>(tok0 + c) * p.n + row] = panel_f16(act, clipped);
+                    else p.y[o] = act;
+                } else p.y[o] = p.residual ? v + __ldcg(p.residual + o) : v;
             }
+            if (DUAL && clipped) atomicOr(p.status, STATUS_X_CLIPPED);
         }
         cl.sync();                                                   // the others read this CTA's sums until here
     }
@@ -443,8 +447,7 @@ __device__ __forceinline__ bool store8_f16(__half* out, const float (&v)[8]) {  
     uint32_t o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        clipped |= (fabsf(v[2 * j]) > 65504.0f) | (fabsf(v[2 * j + 1]) > 65504.0f);
-        const __half2 hh = __floats2half2_rn(fminf(fmaxf(v[2 * j], -65504.0f), 65504.0f), fminf(fmaxf(v[2 * j + 1], -65504.0f), 65504.0f));
+        const __half2 hh = __halves2half2(panel_f16(v[2 * j], clipped), panel_f16(v[2 * j + 1], clipped));
         o[j] = *reinterpret_cast<const uint32_t*>(&hh);
     }
     *reinterpret_cast<uint4*>(out) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -626,7 +629,7 @@ namespace {
 // w_up != nullptr: the SwiGLU pair (w = gate); residual != nullptr: y = product + residual
 cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const void* x, uint32_t x_dtype, float* y, uint32_t m, uint32_t n,
                           uint32_t k, void* workspace, uint32_t* status, int sm_count, cudaStream_t st, int* launches,
-                          uint32_t ldy, bool x_ready, const float* residual, uint32_t perm_head_dim = 0) {
+                          uint32_t ldy, bool x_ready, const float* residual, uint32_t perm_head_dim = 0, void* act16 = nullptr) {
     const bool dual = w_up != nullptr;
     const BlockGeom g = block_geom(type);
     const uint64_t row_bytes = static_cast<uint64_t>(k) / g.elems * g.bytes;
@@ -652,6 +655,7 @@ cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const 
     p.y = y; p.m = m; p.n = n; p.k = k;
     p.ldy = ldy ? ldy : n;
     p.residual = residual;
+    p.act16 = static_cast<__half*>(act16);
     p.tiles_per_cta = 1;
     p.boxw = boxw_of(type);
     p.blk_bytes = KB / g.elems * g.bytes;
@@ -724,8 +728,8 @@ bool gemm_tc_swiglu_supported(uint32_t type) {
 
 cudaError_t launch_gemm_tc_swiglu(uint32_t type, const void* w_gate, const void* w_up, const void* x, uint32_t x_dtype, float* y,
                                   uint32_t m, uint32_t n, uint32_t k, void* workspace, uint32_t* status, int sm_count,
-                                  cudaStream_t st, int* launches, bool x_ready) {
-    return gemm_tc_dense(type, w_gate, w_up, x, x_dtype, y, m, n, k, workspace, status, sm_count, st, launches, n, x_ready, nullptr);
+                                  cudaStream_t st, int* launches, bool x_ready, void* act16) {
+    return gemm_tc_dense(type, w_gate, w_up, x, x_dtype, y, m, n, k, workspace, status, sm_count, st, launches, n, x_ready, nullptr, 0, act16);
 }
 
 

@@ -130,7 +130,7 @@ cudaError_t launch_gemm_tc(uint32_t type, const void* w, const void* x, uint32_t
 bool gemm_tc_swiglu_supported(uint32_t type);
 cudaError_t launch_gemm_tc_swiglu(uint32_t type, const void* w_gate, const void* w_up, const void* x, uint32_t x_dtype, float* y,
                                   uint32_t m, uint32_t n, uint32_t k, void* workspace, uint32_t* status, int sm_count,
-                                  cudaStream_t st, int* launches, bool x_ready = false);
+                                  cudaStream_t st, int* launches, bool x_ready = false, void* act16 = nullptr);   // act16: f16 [m][n] in the place of y
 
 // K4: grouped expert-routed product.  moe_scratch_layout() carves the caller's scratch into header
 // (tile count, sorted-row count), tile table, permutation and the f16 activation panel;
@@ -181,7 +181,7 @@ struct KvCacheView {
 cudaError_t launch_get_rows(uint32_t type, const void* w, uint64_t row_bytes, uint32_t n_rows, uint32_t k, const uint32_t* ids,
                             uint32_t m, float* out, uint32_t* status, cudaStream_t st);
 cudaError_t launch_rms_norm(float* x, const float* delta, const float* weight, float eps, void* out, uint32_t out_dtype, uint32_t m,
-                            uint32_t h, cudaStream_t st);
+                            uint32_t h, uint32_t* status, cudaStream_t st);      // out in f16: an activation panel of the tensor-core products
 cudaError_t launch_rope_kv_append(float* qkv, uint32_t m, uint32_t n_q, uint32_t n_kv, uint32_t hd, const uint32_t* pos, float theta,
                                   const KvCacheView& kv, uint32_t* status, cudaStream_t st);
 size_t attn_decode_scratch_bytes(uint32_t n_kv, uint32_t group, uint32_t n_splits);

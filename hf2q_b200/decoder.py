@@ -342,7 +342,10 @@ class LlamaDecoder(GreedyDecoder):
         ctx._check(self.lib.hf2q_cuda_attn_decode_scratch_bytes(ctx._h, c.n_heads, c.n_kv_heads, C.byref(need)))
         self.att_scratch = torch.zeros(max(need.value, 16), dtype=torch.uint8, device=dev)
         self.prefill_chunk = prefill_chunk
-        self._pf = None                 # prefill buffers, allocated on first use
+        self._pf, self._pf_kinds = None, {}     # prefill buffers, allocated on first use: the last portion's, and of both kinds
+        # prompt portions: the kernels between the products write the f16 panels that the products multiply
+        self.panel_prefill = all(self._panel_ok(w) for lw in weights.layers for w in (lw.wqk, lw.wv, lw.wo, lw.gate, lw.up, lw.down) if w is not None) and \
+            all(lw.gate.ggml_type == lw.up.ggml_type and ops.quantized_matmul_swiglu_supported(ctx, 9, lw.gate) for lw in weights.layers)
         self._open, self._length = False, 0
         for lw in weights.layers:
             if not ops.quantized_matmul_swiglu_supported(ctx, 1, lw.gate, torch.float32):
@@ -394,6 +397,17 @@ class LlamaDecoder(GreedyDecoder):
     def _rms(self, x, delta, weight, out, m):
         self.ctx._check(self.lib.hf2q_cuda_rms_norm(self.ctx._h, self._s(), x.data_ptr(), delta.data_ptr() if delta is not None else None,
                                                     weight.data_ptr(), self.cfg.rms_eps, out.data_ptr(), ops._TORCH_DT[out.dtype], m, self.cfg.hidden))
+
+    def _panel_ok(self, w) -> bool:
+        return w.ptr % 16 == 0 and bool(self.lib.hf2q_cuda_panel_supported(self.ctx._h, 9, w.rows, w.cols, w.ggml_type))
+
+    def _rms_panel(self, x, weight, panel, m):
+        self.ctx._check(self.lib.hf2q_cuda_rms_norm_panel(self.ctx._h, self._s(), x.data_ptr(), None, weight.data_ptr(), self.cfg.rms_eps, panel.data_ptr(), m,
+                                                          self.cfg.hidden))
+
+    def _matmul_panel(self, panel, weights, out, m, residual=None):
+        self.ctx._check(self.lib.hf2q_cuda_qmatmul_panel(self.ctx._h, self._s(), panel.data_ptr(), ops.row_segments(weights), len(weights),
+                                                         residual.data_ptr() if residual is not None else None, out.data_ptr(), m, weights[0].cols))
 
     def _rope_append(self, qkv, m, layer):
         self.ctx._check(self.lib.hf2q_cuda_rope_kv_append(self.ctx._h, self._s(), qkv.data_ptr(), m, self.cfg.n_heads, self.cfg.rope_theta,
@@ -451,15 +465,20 @@ class LlamaDecoder(GreedyDecoder):
         return 1 + per_layer * self.cfg.n_layers + qkv + (2 if self.fused_norm else 3)
 
     # ---- prefill: m tokens per chunk through the GEMM path ---------------------------------------
-    def _prefill_buffers(self, m):
-        if self._pf is None or self._pf["m"] < m:
+    def _prefill_buffers(self, m, panels):
+        """Buffers of a portion of up to m tokens; with panels xn, att and g are f16 and only they, x and qkv are there."""
+        have = self._pf_kinds.get(panels)
+        if have is None or have["m"] < m:
             c = self.cfg
+            act = dict(dtype=torch.float16 if panels else torch.float32, device=self.dev)
             f32 = dict(dtype=torch.float32, device=self.dev)
-            self._pf = {"m": m, "x": torch.empty((m, c.hidden), **f32), "xn": torch.empty((m, c.hidden), **f32),
-                        "qkv": torch.empty((m, self.qkv_cols), **f32), "att": torch.empty((m, c.q_rows), **f32),
-                        "o": torch.empty((m, c.hidden), **f32), "g": torch.empty((m, c.ffn), **f32),
-                        "u": torch.empty((m, c.ffn), **f32)}
-        return self._pf
+            have = {"m": m, "x": torch.empty((m, c.hidden), **f32), "qkv": torch.empty((m, self.qkv_cols), **f32),
+                    "xn": torch.empty((m, c.hidden), **act), "att": torch.empty((m, c.q_rows), **act), "g": torch.empty((m, c.ffn), **act)}
+            if not panels:
+                have |= {"o": torch.empty((m, c.hidden), **f32), "u": torch.empty((m, c.ffn), **f32)}
+            self._pf_kinds[panels] = have
+        self._pf = have
+        return have
 
     # ---- the engine's sequence interface: one sequence at a time --------------------------------
     n_slots = 1
@@ -502,12 +521,25 @@ class LlamaDecoder(GreedyDecoder):
         ids = ids.to(self.dev, torch.int32).contiguous()
         for p0 in range(start, T, self.prefill_chunk):
             m = min(self.prefill_chunk, T - p0)
-            b = self._prefill_buffers(min(self.prefill_chunk, T - start))
-            x, xn, qkv, att, o, g, u = (b[k][:m] for k in ("x", "xn", "qkv", "att", "o", "g", "u"))
+            panels = self.panel_prefill and self.fused_prefill and m > 8
+            b = self._prefill_buffers(m if m <= 8 else min(self.prefill_chunk, T - start), panels)
+            x, xn, qkv, att, g = (b[k][:m] for k in ("x", "xn", "qkv", "att", "g"))
+            o, u = (None, None) if panels else (b["o"][:m], b["u"][:m])
             self.pos.fill_(p0)
             self._get_rows(ids[p0 - start:p0 - start + m], m, x)
             delta = None
             for i, lw in enumerate(self.w.layers):
+                if panels:
+                    self._rms_panel(x, lw.attn_norm, xn, m)
+                    self._matmul_panel(xn, self._qkv_segments(lw), qkv, m)
+                    self._rope_append(qkv, m, i)
+                    ctx._check(lib.hf2q_cuda_attn_prefill_panel(ctx._h, self._s(), qkv.data_ptr(), m, c.n_heads, C.byref(self.kv[i]), p0, att.data_ptr()))
+                    self._matmul_panel(att, [lw.wo], x, m, x)
+                    self._rms_panel(x, lw.ffn_norm, xn, m)
+                    ctx._check(lib.hf2q_cuda_qmatmul_swiglu_panel(ctx._h, self._s(), xn.data_ptr(), ops.DT_F16, lw.gate.ptr, lw.up.ptr, g.data_ptr(), m, lw.gate.rows,
+                                                                  lw.gate.cols, lw.gate.ggml_type, None, 0))
+                    self._matmul_panel(g, [lw.down], x, m, x)
+                    continue
                 self._rms(x, delta, lw.attn_norm, xn, m)                                   # x += previous layer's FFN output (unfused form)
                 ops.quantized_matmul_segments(ctx, xn, self._qkv_segments(lw), qkv, m)
                 self._rope_append(qkv, m, i)

@@ -280,6 +280,14 @@ def norm_supported(ctx: GpuContext, m: int, weight: "QuantWeight") -> bool:
     return bool(ctx._lib.hf2q_cuda_norm_supported(ctx._h, m, weight.cols, weight.ggml_type))
 
 
+def row_segments(weights):
+    """The row ranges of one matrix, as the C entries take them."""
+    segs = (_RowSegment * len(weights))()
+    for s, w in zip(segs, weights):
+        s.w, s.rows, s.ggml_type = w.ptr, w.rows, w.ggml_type
+    return segs
+
+
 def quantized_matmul_segments(ctx: GpuContext, input: torch.Tensor, weights, out: torch.Tensor, m: int,
                               workspace: torch.Tensor | None = None, norm_weight: torch.Tensor | None = None,
                               norm_eps: float = 0.0) -> None:
@@ -293,9 +301,7 @@ def quantized_matmul_segments(ctx: GpuContext, input: torch.Tensor, weights, out
         raise Hf2qError(_lib.ERR_INVALID_ARGUMENT, "all row ranges must share k")
     if out.dtype != torch.float32 or not out.is_cuda or not out.is_contiguous() or out.numel() < m * n or input.numel() < m * k:
         raise Hf2qError(_lib.ERR_INVALID_ARGUMENT, "out must be a contiguous float32 CUDA tensor of [m, n]; input [m, k]")
-    segs = (_RowSegment * len(weights))()
-    for s, w in zip(segs, weights):
-        s.w, s.rows, s.ggml_type = w.ptr, w.rows, w.ggml_type
+    segs = row_segments(weights)
     if norm_weight is not None:      # RMSNorm(input) fused into the launches (rms_norm_rows, forward_cpu.rs:36-48)
         ctx._check(ctx._lib.hf2q_cuda_norm_qmatmul_segments(ctx._h, ctx._stream(), input.data_ptr(), norm_weight.data_ptr(), norm_eps,
                                                            segs, len(weights), out.data_ptr(), m, k))

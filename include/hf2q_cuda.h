@@ -636,6 +636,25 @@ HF2Q_API int32_t hf2q_cuda_attn_decode_fused(hf2q_ctx* ctx, void* stream, const 
 HF2Q_API int32_t hf2q_cuda_attn_prefill(hf2q_ctx* ctx, void* stream, const float* qkv, uint32_t m,
                                         uint32_t n_q_heads, const hf2q_kv_cache* kv, uint32_t pos0,
                                         void* out, uint32_t out_dtype);
+
+/* ---- panels ----
+ * A panel is the f16 [m][k] that a tensor-core product multiplies: the product's own conversion of f32 or bf16 activations gives
+ * the same (beyond the f16 range clipped and noted in the status).  The entry in front of a product can write it, which saves the
+ * conversion pass and half of the store.  More than 8 rows, 16-byte boundaries. */
+HF2Q_API int32_t hf2q_cuda_panel_supported(hf2q_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, uint32_t ggml_type);
+/* hf2q_cuda_rms_norm, hf2q_cuda_attn_prefill with a panel as the output */
+HF2Q_API int32_t hf2q_cuda_rms_norm_panel(hf2q_ctx* ctx, void* stream, float* x, const float* delta, const float* weight,
+                                          float eps, void* panel, uint32_t m, uint32_t h);
+HF2Q_API int32_t hf2q_cuda_attn_prefill_panel(hf2q_ctx* ctx, void* stream, const float* qkv, uint32_t m, uint32_t n_q_heads,
+                                              const hf2q_kv_cache* kv, uint32_t pos0, void* panel);
+/* hf2q_cuda_qmatmul_segments on a panel, or with one range y = residual + product (residual may be y) */
+HF2Q_API int32_t hf2q_cuda_qmatmul_panel(hf2q_ctx* ctx, void* stream, const void* panel, const hf2q_row_segment* segs,
+                                         uint32_t n_segs, const float* residual, float* y, uint32_t m, uint32_t k);
+/* hf2q_cuda_qmatmul_swiglu_ws with a panel as the output; x f32 or bf16 (workspace as there) or a panel (F16, no workspace).  Formats:
+ * as hf2q_cuda_qmatmul_swiglu_ws_supported says. */
+HF2Q_API int32_t hf2q_cuda_qmatmul_swiglu_panel(hf2q_ctx* ctx, void* stream, const void* x, uint32_t x_dtype, const void* w_gate,
+                                                const void* w_up, void* y_panel, uint32_t m, uint32_t n, uint32_t k,
+                                                uint32_t ggml_type, void* workspace, uint64_t workspace_bytes);
 /* Greedy sampling: *out_id = index of the largest logit (lowest index on ties); if pos != NULL,
  * *pos += 1 afterwards, which hands a captured decode step over to its next replay. */
 HF2Q_API int32_t hf2q_cuda_argmax(hf2q_ctx* ctx, void* stream, const float* logits, uint32_t n,
