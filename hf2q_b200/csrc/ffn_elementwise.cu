@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(RV_THREADS) router_vector_kernel(const void* _
     const uint32_t e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* row = w + static_cast<size_t>(e) * h;
     float acc[RV_TOKENS] = {};
-    seq::pdl_trigger();
-    seq::pdl_wait();
+    pdl_trigger();
+    pdl_wait();
     if constexpr (VEC) {
         for (uint32_t i0 = 4 * threadIdx.x; i0 < h; i0 += RV_AHEAD * 4 * RV_THREADS) {
             float4 wv[RV_AHEAD];
@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(256) router_tile_kernel(const void* __restrict
                                                           float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
     __shared__ __align__(16) float xs[RKT][RT], ws[RKT][RT];
     const cg::cluster_group cl = cg::this_cluster();
-    seq::pdl_trigger();
-    seq::pdl_wait();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t parts = gridDim.z, part = blockIdx.z;             // the cluster is the whole z extent
     const uint32_t t0 = blockIdx.y * RT, e0 = blockIdx.x * RT;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;          // outputs: tokens 4ty..4ty+3, experts 4tx..4tx+3
@@ -256,13 +256,13 @@ cudaError_t launch_router_logits(const void* x, uint32_t x_bf16, const float* w,
                                  uint32_t h, int sm_count, cudaStream_t st) {
     const bool vec = h % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % (x_bf16 ? 8 : 16) == 0;
     if (n_tokens <= RV_TOKENS)
-        return seq::launch_pdl(vec ? router_vector_kernel<true> : router_vector_kernel<false>, dim3(n_experts), dim3(RV_THREADS), 0, st, x, x_bf16, w, out,
+        return launch_pdl(vec ? router_vector_kernel<true> : router_vector_kernel<false>, dim3(n_experts), dim3(RV_THREADS), 0, st, x, x_bf16, w, out,
                                n_tokens, n_experts, h);
     const dim3 tiles((n_experts + RT - 1) / RT, (n_tokens + RT - 1) / RT);
     // as many parts as keep two CTAs on every SM busy
     uint32_t parts = 1;
     while (parts < RT_MAX_PARTS && 2ull * parts * tiles.x * tiles.y <= 2ull * sm_count && h >= 2 * parts * RKT) parts *= 2;
-    return seq::launch_pdl_cluster(vec ? router_tile_kernel<true> : router_tile_kernel<false>, dim3(tiles.x, tiles.y, parts), dim3(256), dim3(1, 1, parts), 0, st,
+    return launch_pdl_cluster(vec ? router_tile_kernel<true> : router_tile_kernel<false>, dim3(tiles.x, tiles.y, parts), dim3(256), dim3(1, 1, parts), 0, st,
                                    x, x_bf16, w, out, n_tokens, n_experts, h);
 }
 

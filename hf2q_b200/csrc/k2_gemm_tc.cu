@@ -28,6 +28,9 @@
 // Where the tiles leave SMs idle (few activation rows), the CTAs of a cluster share a tile's K-blocks (gemm_tc_parts
 // of them) and add their accumulators through distributed shared memory in rank order.
 //
+// Launched early (launch_pdl): barriers, tensor memory and the first weight stages are ready when the launch in front ends
+// (gate, up and down of 2560 x 9728 in Q8_0 at 37 rows, three launches: 64 -> 57 us).
+//
 // TMEM: 512 columns = D (<= 256) + 2 x 128 (two A buffers of one K-block each).
 // Every mbarrier wait is bounded; a wait that gives up sets the status word and all roles drain to
 // the final barrier, where TMEM is freed.  No multicast.
@@ -173,6 +176,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // The next launch may start its own prologue.  What earlier launches wrote or still read -- activations, tile table,
+    // outputs -- is touched behind pdl_wait() only; weights do not change.
+    pdl_trigger();
+    if constexpr (GROUPED) pdl_wait();
     // this CTA's weight-row tiles: [tile0, tile0 + ntile)
     const uint32_t n_row_tiles = (p.n + TILE_ROWS - 1) / TILE_ROWS;
     const uint32_t tile0 = blockIdx.x * p.tiles_per_cta;
@@ -212,6 +219,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                 const uint32_t row0 = (tile0 + tl) * TILE_ROWS;
                 for (uint32_t kb = 0; kb < nkb && ok; ++kb, ++gk) {
                     const uint32_t rs = gk % RAW_STAGES;
+                    if (gk == RAW_STAGES) pdl_wait();
                     if (gk >= RAW_STAGES) ok = mbar_wait_bounded(&raw_empty[rs], ((gk / RAW_STAGES) - 1) & 1, p.status);
                     if (!ok) break;
                     mbar_arrive_expect_tx(&raw_full[rs], raw_stage);
@@ -231,6 +239,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             }
         } else if (lane == 1) {
             bool ok = true;
+            pdl_wait();
             const uint32_t nx = ntile * nkb * (KB / XK);
             for (uint32_t xi = 0; xi < nx && ok; ++xi) {
                 const uint32_t st = xi % X_STAGES, kx = kb0 * (KB / XK) + xi % (nkb * (KB / XK));      // K position inside the current tile
@@ -248,6 +257,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             const uint32_t n_mma = max(16u, (min(static_cast<uint32_t>(NT), tok_end - tok0) + 15u) & ~15u);
             const uint32_t IDESC = (1u << 4) | ((n_mma >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
             bool ok = true;
+            pdl_wait();
             for (uint32_t tl = 0, gk = 0; tl < ntile && ok; ++tl) {
                 // the previous tile's accumulators must have been read before they are overwritten
                 if (tl) ok = mbar_wait_bounded(d_empty, (tl - 1) & 1, p.status);
@@ -292,6 +302,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             for (uint32_t kb = 0; kb < nkb; ++kb, ++gk) {
                 const uint32_t rs = gk % RAW_STAGES, ab = gk % A_BUFS;
                 if (ok) ok = mbar_wait_bounded(&raw_full[rs], (gk / RAW_STAGES) & 1, p.status);
+                if (gk == A_BUFS) pdl_wait();                          // (from here on the bounded waits measure this kernel only)
                 if (ok && gk >= A_BUFS) ok = mbar_wait_bounded(&a_empty[ab * DEQ_GROUPS + grp], ((gk / A_BUFS) - 1) & 1, p.status);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
@@ -304,6 +315,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                 if (lane == 0) { mbar_arrive(&a_full[ab * DEQ_GROUPS + grp]); mbar_arrive(&raw_empty[rs]); }
             }
             // epilogue of this tile
+            pdl_wait();
             if (ok) ok = mbar_wait_bounded(d_full, tl & 1, p.status);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -400,6 +412,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     if (warp == DEQ_WARPS + 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
     if constexpr (SHARED) {
         const cg::cluster_group cl = cg::this_cluster();
+        pdl_wait();
         cl.sync();
         // token columns part, part + parts, ... of the tile are this CTA's: all CTAs' sums in rank order, then the epilogue
         float* sums = reinterpret_cast<float*>(smem);
@@ -458,6 +471,8 @@ __device__ __forceinline__ bool store8_f16(__half* out, const float (&v)[8]) {  
 // element at a time took 110.
 __global__ void __launch_bounds__(256) x_to_f16_kernel(const void* __restrict__ x, uint32_t x_bf16, __half* __restrict__ out,
                                                        uint64_t n_elems, bool wide, uint32_t* status) {
+    pdl_trigger();
+    pdl_wait();
     const uint64_t n8 = n_elems / 8, stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     bool clipped = false;
     uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -488,6 +503,8 @@ __global__ void __launch_bounds__(256) x_to_f16_kernel(const void* __restrict__ 
 // logical (t, c) is physical (h = c / head_dim, t, f = c % head_dim).  8 elements per thread.
 __global__ void __launch_bounds__(256) x_perm021_to_f16_kernel(const void* __restrict__ x, uint32_t x_bf16, __half* __restrict__ out,
                                                                uint32_t m, uint32_t k, uint32_t head_dim, uint32_t* status) {
+    pdl_trigger();
+    pdl_wait();
     const uint64_t n8 = static_cast<uint64_t>(m) * k / 8, stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     bool clipped = false;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += stride) {
@@ -532,22 +549,8 @@ cudaError_t launch_gemm_form(const CUtensorMap& tw, const CUtensorMap& tw2, cons
     const uint32_t tile_rows = DUAL ? 64 : TILE_N;
     const uint32_t row_tiles = (p.n + tile_rows - 1) / tile_rows;
     const dim3 grid((row_tiles + p.tiles_per_cta - 1) / p.tiles_per_cta, grid_y, parts);
-    if constexpr (SHARED) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(GEMM_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute cluster[1];
-        cluster[0].id = cudaLaunchAttributeClusterDimension;
-        cluster[0].val.clusterDim.x = cluster[0].val.clusterDim.y = 1;
-        cluster[0].val.clusterDim.z = parts;
-        cfg.attrs = cluster;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kern, tw, tw2, tx, p);
-    }
-    kern<<<grid, GEMM_THREADS, smem, st>>>(tw, tw2, tx, p);
-    return cudaGetLastError();
+    if constexpr (SHARED) return launch_pdl_cluster(kern, grid, dim3(GEMM_THREADS), dim3(1, 1, parts), smem, st, tw, tw2, tx, p);
+    else return launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, tw, tw2, tx, p);
 }
 
 // parts > 1: the CTAs of a cluster share the K-blocks (dense tiles of up to 128 tokens)
@@ -641,13 +644,10 @@ cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const 
     const uint64_t nx = static_cast<uint64_t>(m) * k;
     if (!x_ready) {       // (a caller that runs several products on the same activations converts them once)
         const uint64_t want = (nx / 8 + 255) / 256, cap = static_cast<uint64_t>(sm_count) * 8;
-        if (perm_head_dim) {
-            x_perm021_to_f16_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, st>>>(x, x_dtype == HF2Q_DT_BF16, xh, m, k, perm_head_dim, status);
-        } else {
-            x_to_f16_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, st>>>(x, x_dtype == HF2Q_DT_BF16, xh, nx,
-                                                                                                       reinterpret_cast<uintptr_t>(x) % 16 == 0, status);
-        }
-        cudaError_t e = cudaGetLastError();
+        const dim3 grid(static_cast<unsigned>(want < cap ? want : cap));
+        const cudaError_t e = perm_head_dim ? launch_pdl(x_perm021_to_f16_kernel, grid, dim3(256), 0, st, x, x_dtype == HF2Q_DT_BF16, xh, m, k, perm_head_dim, status)
+                                            : launch_pdl(x_to_f16_kernel, grid, dim3(256), 0, st, x, x_dtype == HF2Q_DT_BF16, xh, nx,
+                                                           reinterpret_cast<uintptr_t>(x) % 16 == 0, status);
         if (e != cudaSuccess) return e;
     }
     // 2. tensor maps
