@@ -283,9 +283,9 @@ __device__ __forceinline__ float hyper_elements(const hf2q_hyper& p, uint32_t t,
     }
     return ss;
 }
+// [S][S] mix, [S] out, [S] in; absent streams have zeros.  The whole block takes part and meets at the end.
 template <int S>
-__device__ __forceinline__ float hyper_row_s(const hf2q_hyper& p, uint32_t t, float* xs, float* coef, uint32_t lo, uint32_t hi) {
-    // [S][S] mix, [S] out, [S] in; absent streams have zeros
+__device__ __forceinline__ void hyper_coefficients(const hf2q_hyper& p, float* coef) {
     for (uint32_t i = threadIdx.x; i < S * S + 2 * S; i += blockDim.x) {
         const uint32_t a = i / S, b = i % S;
         float v = 0.f;
@@ -297,6 +297,10 @@ __device__ __forceinline__ float hyper_row_s(const hf2q_hyper& p, uint32_t t, fl
         coef[i] = v;
     }
     __syncthreads();
+}
+template <int S>
+__device__ __forceinline__ float hyper_row_s(const hf2q_hyper& p, uint32_t t, float* xs, float* coef, uint32_t lo, uint32_t hi) {
+    hyper_coefficients<S>(p, coef);
     return p.width % 4 == 0 ? hyper_elements<S, float4>(p, t, xs, coef, lo, hi) : hyper_elements<S, float>(p, t, xs, coef, lo, hi);
 }
 // Row t of the streams (hf2q_hyper): the pending update, stored for elements [lo, hi), and the row that the sublayer reads
