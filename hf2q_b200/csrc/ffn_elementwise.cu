@@ -30,22 +30,35 @@ __global__ void __launch_bounds__(256) silu_mul_tail_kernel(const float* gate, c
 }
 
 // out[t, :] = sum_s w[t*k+s] * y[t*k+s, :]  (+ sigmoid(gate_logit[t]) * shared[t, :])  (+ residual[t, :])
+// V: float, or float4 where rows are whole 16-byte groups.  Bound by memory: eight rows are asked for before they are added, in
+// slot order, as the reference sums (2048 tokens, 8 rows of 2048 each: 151 MB, 30 -> 28 us).
+__device__ __forceinline__ void add_scaled(float& a, float w, float v) { a += w * v; }
+__device__ __forceinline__ void add_scaled(float4& a, float w, const float4& v) { a.x += w * v.x; a.y += w * v.y; a.z += w * v.z; a.w += w * v.w; }
+template <typename V>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, const float* __restrict__ w,
                                                           const float* __restrict__ shared, const float* __restrict__ gate_logit,
                                                           const float* __restrict__ residual, float* __restrict__ out,
-                                                          uint32_t n_tokens, uint32_t top_k, uint32_t h) {
-    const uint32_t t = blockIdx.y;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tokens || c >= h) return;
-    float acc = 0.f;
-    for (uint32_t s = 0; s < top_k; ++s)
-        acc += w[t * top_k + s] * y[(static_cast<size_t>(t) * top_k + s) * h + c];      // slot order, as the reference sums
-    if (shared) {
-        const float gv = gate_logit ? 1.0f / (1.0f + expf(-gate_logit[t])) : 1.0f;      // ffn.rs:28-30
-        acc += gv * shared[static_cast<size_t>(t) * h + c];
+                                                          uint32_t top_k, uint32_t h) {
+    constexpr uint32_t E = sizeof(V) / 4, AHEAD = 8;
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x, n = h / E;
+    if (c >= n) return;
+    auto at = [&](const float* p, size_t row) { return reinterpret_cast<const V*>(p + row * h)[c]; };
+    V acc{};
+    for (uint32_t s0 = 0; s0 < top_k; s0 += AHEAD) {
+        V v[AHEAD];
+        float f[AHEAD];
+#pragma unroll
+        for (uint32_t s = 0; s < AHEAD; ++s)
+            if (s0 + s < top_k) { v[s] = at(y, static_cast<size_t>(t) * top_k + s0 + s); f[s] = w[static_cast<size_t>(t) * top_k + s0 + s]; }
+#pragma unroll
+        for (uint32_t s = 0; s < AHEAD; ++s)
+            if (s0 + s < top_k) add_scaled(acc, f[s], v[s]);
     }
-    if (residual) acc += residual[static_cast<size_t>(t) * h + c];
-    out[static_cast<size_t>(t) * h + c] = acc;
+    if (shared) add_scaled(acc, gate_logit ? 1.0f / (1.0f + expf(-gate_logit[t])) : 1.0f, at(shared, t));      // ffn.rs:28-30
+    if (residual) add_scaled(acc, 1.0f, at(residual, t));
+    reinterpret_cast<V*>(out + static_cast<size_t>(t) * h)[c] = acc;
 }
 
 // out[t] = sum_i v[i] * x[t, i]   (the shared expert's gate logit, a [1, h] f32 matrix)
@@ -137,35 +150,39 @@ __global__ void __launch_bounds__(RV_THREADS) router_vector_kernel(const void* _
     }
 }
 
-// More tokens: 64 tokens x 64 experts per tile, 4 x 4 outputs per thread in packed f32 arithmetic, the next 32 columns on
-// their way to registers while the present ones are used.  Bound by the f32 pipes (2048 tokens x 256 experts of 2048: 1.07 G
-// multiply-adds).  The CTAs of a cluster share a tile's columns where the tiles alone would leave the chip idle, and add
-// their sums through distributed shared memory in rank order (2048 tokens, 256 experts of 2048: 263 -> 86 us).  The line at
+// More tokens: tiles of 64 R tokens x 64 R experts, R x R blocks of 4 x 4 outputs per thread in packed f32 arithmetic, the next 32
+// columns on their way to registers while the present ones are used.  Bound by the f32 pipes (2048 tokens x 256 experts of 2048:
+// 1.07 G multiply-adds, 29 us at their peak); with R = 1 by shared memory, 32 bytes for 16 multiply-adds, R = 2 halves that (86 -> 65 us).
+// The CTAs of a cluster share a tile's columns where the tiles alone would leave the chip idle, and add
+// their sums through distributed shared memory in rank order (2048 tokens, 256 experts of 2048, R = 1: 263 -> 86 us).  The line at
 // RV_TOKENS is the number of sums a thread of the other kernel keeps in registers; there the tiles are still behind (us a CTA per
 // expert / tiles, 8 and 16 tokens: 256 experts of 2048 7.9 / 13.9 and 12.6 / 13.9, 8 of 4096 10.7 / 20.9 and 19.7 / 21.1).
 // Columns are stored with the group of four tokens (or experts) XORed by the column's own group of four, which keeps both the
 // transposing stores and the reads free of conflicts.
 constexpr int RT = 64, RKT = 32, RT_MAX_PARTS = 8;
+constexpr size_t router_smem(int R) { return 4 * (2 * RKT * RT * R > RT * R * RT * R ? 2 * RKT * RT * R : RT * R * RT * R); }
 
-template <bool VEC>
-__global__ void __launch_bounds__(256) router_tile_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
-                                                          float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
-    __shared__ __align__(16) float xs[RKT][RT], ws[RKT][RT];
+template <bool VEC, int R>
+__global__ void __launch_bounds__(256, 2) router_tile_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
+                                                             float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
+    constexpr int TILE = RT * R;
+    extern __shared__ __align__(16) float rsm[];
+    float (*xs)[TILE] = reinterpret_cast<float (*)[TILE]>(rsm), (*ws)[TILE] = xs + RKT;
     const cg::cluster_group cl = cg::this_cluster();
     pdl_trigger();
     pdl_wait();
     const uint32_t parts = gridDim.z, part = blockIdx.z;             // the cluster is the whole z extent
-    const uint32_t t0 = blockIdx.y * RT, e0 = blockIdx.x * RT;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;          // outputs: tokens 4ty..4ty+3, experts 4tx..4tx+3
+    const uint32_t t0 = blockIdx.y * TILE, e0 = blockIdx.x * TILE;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;          // outputs: tokens 64 u + 4 ty .. + 3, experts 64 v + 4 tx .. + 3
     const uint32_t chunks = (h + RKT - 1) / RKT, per = (chunks + parts - 1) / parts;
     const uint32_t c0 = min(part * per, chunks), c1 = min(c0 + per, chunks);
-    // a thread brings columns 4 kg .. 4 kg + 3 of rows r and r + 32 of both tiles
+    // a thread brings columns 4 kg .. 4 kg + 3 of every 32nd row of both tiles
     const uint32_t kg = threadIdx.x & 7, r = threadIdx.x >> 3;
-    float4 xr[2], wr[2];
+    float4 xr[2 * R], wr[2 * R];
     auto fetch = [&](uint32_t c) {
         const uint32_t k = c * RKT + 4 * kg;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 2 * R; ++i) {
             const uint32_t t = t0 + r + 32 * i, e = e0 + r + 32 * i;
             const size_t xo = static_cast<size_t>(t) * h + k, wo = static_cast<size_t>(e) * h + k;
             xr[i] = wr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -183,11 +200,11 @@ __global__ void __launch_bounds__(256) router_tile_kernel(const void* __restrict
             }
         }
     };
-    f2 acc[4][2] = {};
+    f2 acc[4 * R][2 * R] = {};
     if (c0 < c1) fetch(c0);
     for (uint32_t c = c0; c < c1; ++c) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 2 * R; ++i) {
             const uint32_t row = r + 32 * i, at = 4 * ((row >> 2) ^ kg) + (row & 3);
             const float xv[4] = {xr[i].x, xr[i].y, xr[i].z, xr[i].w}, wv[4] = {wr[i].x, wr[i].y, wr[i].z, wr[i].w};
 #pragma unroll
@@ -200,14 +217,25 @@ __global__ void __launch_bounds__(256) router_tile_kernel(const void* __restrict
         if (c + 1 < c1) fetch(c + 1);
 #pragma unroll
         for (int k = 0; k < RKT; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(&xs[k][4 * (ty ^ (k >> 2))]);
-            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&ws[k][4 * (tx ^ (k >> 2))]);
-            const float av[4] = {a.x, a.y, a.z, a.w};
+            float4 a[R];
+            ulonglong2 b[R];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const f2 aa = f2_both(av[i]);
-                acc[i][0] = f2_fma(aa, b.x, acc[i][0]);
-                acc[i][1] = f2_fma(aa, b.y, acc[i][1]);
+            for (int u = 0; u < R; ++u) {
+                a[u] = *reinterpret_cast<const float4*>(&xs[k][RT * u + 4 * (ty ^ (k >> 2))]);
+                b[u] = *reinterpret_cast<const ulonglong2*>(&ws[k][RT * u + 4 * (tx ^ (k >> 2))]);
+            }
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const float av[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const f2 aa = f2_both(av[i]);
+#pragma unroll
+                    for (int v = 0; v < R; ++v) {
+                        acc[4 * u + i][2 * v] = f2_fma(aa, b[v].x, acc[4 * u + i][2 * v]);
+                        acc[4 * u + i][2 * v + 1] = f2_fma(aa, b[v].y, acc[4 * u + i][2 * v + 1]);
+                    }
+                }
             }
         }
         __syncthreads();
@@ -219,35 +247,49 @@ __global__ void __launch_bounds__(256) router_tile_kernel(const void* __restrict
         for (int j = 0; j < 4; ++j)
             if (e + j < n_experts) out[static_cast<size_t>(t) * n_experts + e + j] = o[j];
     };
-    if (parts == 1) {
+    // the tile's sums [token][expert], over the operands
+    float* sums = rsm;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 lo = f2_parts(acc[i][0]), hi = f2_parts(acc[i][1]);
-            store(t0 + 4 * ty + i, e0 + 4 * tx, make_float4(lo.x, lo.y, hi.x, hi.y));
+    for (int i = 0; i < 4 * R; ++i)
+#pragma unroll
+        for (int v = 0; v < R; ++v) {
+            const uint32_t row = RT * (i / 4) + 4 * ty + i % 4, col = RT * v + 4 * tx;
+            if (parts == 1) {
+                const float2 lo = f2_parts(acc[i][2 * v]), hi = f2_parts(acc[i][2 * v + 1]);
+                store(t0 + row, e0 + col, make_float4(lo.x, lo.y, hi.x, hi.y));
+            } else {
+                f2* d = reinterpret_cast<f2*>(sums + row * TILE + col);
+                d[0] = acc[i][2 * v];
+                d[1] = acc[i][2 * v + 1];
+            }
         }
-        return;
-    }
-    // the tile's 64 x 64 sums: rows 0..31 in the tokens' buffer, 32..63 in the experts'
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f2* d = reinterpret_cast<f2*>((4 * ty + i < RKT ? xs[4 * ty + i] : ws[4 * ty + i - RKT]) + 4 * tx);
-        d[0] = acc[i][0];
-        d[1] = acc[i][1];
-    }
+    if (parts == 1) return;
     cl.sync();
     // this CTA's share of the tile's rows
-    const uint32_t rows = RT / parts;
-    for (uint32_t i = threadIdx.x; i < rows * (RT / 4); i += 256) {
-        const uint32_t row = part * rows + i / (RT / 4), q = 4 * (i % (RT / 4));
-        float* mine = row < RKT ? xs[row] : ws[row - RKT];
+    const uint32_t rows = TILE / parts;
+    for (uint32_t i = threadIdx.x; i < rows * (TILE / 4); i += 256) {
+        const uint32_t row = part * rows + i / (TILE / 4), q = 4 * (i % (TILE / 4));
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         for (uint32_t p = 0; p < parts; ++p) {
-            const float4 v = *reinterpret_cast<const float4*>(cl.map_shared_rank(mine + q, p));
+            const float4 v = *reinterpret_cast<const float4*>(cl.map_shared_rank(sums + row * TILE + q, p));
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
         store(t0 + row, e0 + q, s);
     }
     cl.sync();                                                       // peers read this CTA's sums until here
+}
+
+template <int R>
+cudaError_t launch_router_tiles(bool vec, const void* x, uint32_t x_bf16, const float* w, float* out, uint32_t n_tokens, uint32_t n_experts, uint32_t h, int sm_count,
+                                cudaStream_t st) {
+    const dim3 tiles((n_experts + RT * R - 1) / (RT * R), (n_tokens + RT * R - 1) / (RT * R));
+    // as many parts as keep two CTAs on every SM busy
+    uint32_t parts = 1;
+    while (parts < RT_MAX_PARTS && 2ull * parts * tiles.x * tiles.y <= 2ull * sm_count && h >= 2 * parts * RKT) parts *= 2;
+    const auto kern = vec ? router_tile_kernel<true, R> : router_tile_kernel<false, R>;
+    static PerDeviceFlag flag[2];
+    if (const cudaError_t e = ensure_max_dynamic_smem(kern, static_cast<int>(router_smem(R)), flag[vec]); e != cudaSuccess) return e;
+    return launch_pdl_cluster(kern, dim3(tiles.x, tiles.y, parts), dim3(256), dim3(1, 1, parts), router_smem(R), st, x, x_bf16, w, out, n_tokens, n_experts, h);
 }
 
 }  // namespace
@@ -258,12 +300,10 @@ cudaError_t launch_router_logits(const void* x, uint32_t x_bf16, const float* w,
     if (n_tokens <= RV_TOKENS)
         return launch_pdl(vec ? router_vector_kernel<true> : router_vector_kernel<false>, dim3(n_experts), dim3(RV_THREADS), 0, st, x, x_bf16, w, out,
                                n_tokens, n_experts, h);
-    const dim3 tiles((n_experts + RT - 1) / RT, (n_tokens + RT - 1) / RT);
-    // as many parts as keep two CTAs on every SM busy
-    uint32_t parts = 1;
-    while (parts < RT_MAX_PARTS && 2ull * parts * tiles.x * tiles.y <= 2ull * sm_count && h >= 2 * parts * RKT) parts *= 2;
-    return launch_pdl_cluster(vec ? router_tile_kernel<true> : router_tile_kernel<false>, dim3(tiles.x, tiles.y, parts), dim3(256), dim3(1, 1, parts), 0, st,
-                                   x, x_bf16, w, out, n_tokens, n_experts, h);
+    // the larger tiles where their parts still fill the chip
+    const uint64_t tiles = static_cast<uint64_t>((n_experts + 2 * RT - 1) / (2 * RT)) * ((n_tokens + 2 * RT - 1) / (2 * RT));
+    if (n_experts > RT && tiles * RT_MAX_PARTS >= static_cast<uint64_t>(sm_count)) return launch_router_tiles<2>(vec, x, x_bf16, w, out, n_tokens, n_experts, h, sm_count, st);
+    return launch_router_tiles<1>(vec, x, x_bf16, w, out, n_tokens, n_experts, h, sm_count, st);
 }
 
 cudaError_t launch_silu_mul(const float* gate, const float* up, float* out, uint64_t n, int sm_count, cudaStream_t st) {
@@ -280,9 +320,10 @@ cudaError_t launch_silu_mul(const float* gate, const float* up, float* out, uint
 
 cudaError_t launch_moe_combine(const float* y, const float* w, const float* shared, const float* gate_logit, const float* residual,
                                float* out, uint32_t n_tokens, uint32_t top_k, uint32_t h, cudaStream_t st) {
-    const dim3 grid((h + 255) / 256, n_tokens);
-    moe_combine_kernel<<<grid, 256, 0, st>>>(y, w, shared, gate_logit, residual, out, n_tokens, top_k, h);
-    return cudaGetLastError();
+    const bool vec = h % 4 == 0 && (reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+    const dim3 grid((h / (vec ? 4 : 1) + 255) / 256, n_tokens);
+    return vec ? launch_pdl(moe_combine_kernel<float4>, grid, dim3(256), 0, st, y, w, shared, gate_logit, residual, out, top_k, h)
+               : launch_pdl(moe_combine_kernel<float>, grid, dim3(256), 0, st, y, w, shared, gate_logit, residual, out, top_k, h);
 }
 
 cudaError_t launch_rowdot(const float* x, const float* v, float* out, uint32_t n_tokens, uint32_t h, cudaStream_t st) {
