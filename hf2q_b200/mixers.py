@@ -19,6 +19,11 @@ def _off(t: torch.Tensor, cols: int) -> int:
     return t.data_ptr() + cols * t.element_size()
 
 
+# Portions of this many tokens run a layer's recurrence beside its attention: a scan has fewer CTAs than the chip has SMs and each
+# token waits for the one before, so the attention's tiles take the SMs that it leaves.
+BESIDE_TOKENS = 256
+
+
 class ParallelWindowMLstm:
     """Sliding-window attention (per-head q / k norm, logarithmic distance term, sigmoid output gate) and an mLSTM matrix
     memory side by side on the same input; the result is half the sum of the two RMS-normed outputs."""
@@ -99,12 +104,23 @@ class ParallelWindowMLstm:
         mem = ws.get("mem", m, right["heads"] * right["vdim"])
         gated = ws.get("gated", m, self.ro.k, self.act)
         a, b = ws.get("a", m, self.width), ws.get("b", m, self.width)
-        sop.window_append(attn, m, q)
-        sop.window_prefill(attn, m, q, _off(proj, self.off["left.g"]), self.proj.n, att)
-        sop.mlstm(self._mlstm(run, proj), m, mem)
-        sop.gated_heads(self._right_gate(mem, proj), m, gated)
-        sop.matmul(att, self.lo, a, m)
-        sop.matmul(gated, self.ro, b, m)
+
+        def recurrence():
+            sop.mlstm(self._mlstm(run, proj), m, mem)
+            sop.gated_heads(self._right_gate(mem, proj), m, gated)
+            sop.matmul(gated, self.ro, b, m)
+
+        def attention():
+            sop.window_append(attn, m, q)
+            sop.window_prefill(attn, m, q, _off(proj, self.off["left.g"]), self.proj.n, att)
+            sop.matmul(att, self.lo, a, m)
+
+        if m < BESIDE_TOKENS:
+            attention()
+            recurrence()
+        else:
+            with ws.beside(recurrence):
+                attention()
         return a, b
 
     def delta(self, run, proj):

@@ -6,6 +6,7 @@ buffers of a slot are views into one flat f32 arena, so giving a slot to a new s
 """
 from __future__ import annotations
 
+from contextlib import contextmanager
 from dataclasses import dataclass
 
 import torch
@@ -81,7 +82,21 @@ class Workspace:
     device: object
 
     def __post_init__(self):
-        self._bufs = {}
+        self._bufs, self._side = {}, None
+
+    @contextmanager
+    def beside(self, work):
+        """``work``'s launches on a second stream, behind everything queued so far and beside those of the body; joined at its end."""
+        if self._side is None:
+            self._side = torch.cuda.Stream(self.device)
+        here, there = torch.cuda.current_stream(self.device), self._side
+        there.wait_stream(here)
+        try:
+            with torch.cuda.stream(there):
+                work()
+            yield
+        finally:
+            here.wait_stream(there)
 
     def get(self, name: str, rows: int, cols: int, dtype=torch.float32) -> torch.Tensor:
         key = (name, dtype)
