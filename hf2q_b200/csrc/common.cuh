@@ -248,7 +248,7 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32
         : "memory");
 }
 // Programmatic dependent launch.  Every kernel launched with launch_pdl() calls pdl_wait() before it touches
-// memory that an earlier kernel of the stream writes (or still reads); weights may be touched before.
+// memory that an earlier kernel of the stream writes (or still reads); weights and other parameters may be touched before.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... KArgs, typename... Args>

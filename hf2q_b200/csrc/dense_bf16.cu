@@ -76,11 +76,195 @@ struct MatvecSegs {
     uint32_t blocks0;        // CTAs of segment 0
 };
 
+// ---- row prologues with a row's 16-byte groups in registers, PRO_GROUPS per thread: constants are there before the wait for the
+// launch in front, and everything that it wrote is asked for at once.
+constexpr int PRO_GROUPS = 3;
+__device__ __forceinline__ float4 group4(const float* p, uint32_t i, bool in) { return p && in ? *reinterpret_cast<const float4*>(p + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ bool groups_fit(uint32_t width, uintptr_t pointers) { return width % 4 == 0 && width <= 4 * PRO_GROUPS * MR_THREADS && pointers % 16 == 0; }
+__device__ __forceinline__ uintptr_t bits(const void* p) { return reinterpret_cast<uintptr_t>(p); }
+
+struct NormRow {
+    const hf2q_pre_norm& q;
+    float4 norm[PRO_GROUPS], mu[PRO_GROUPS], step[PRO_GROUPS], an[PRO_GROUPS], bn[PRO_GROUPS];
+    static __device__ __forceinline__ bool fits(const hf2q_pre_norm& q) {
+        return groups_fit(q.width, bits(q.x) | bits(q.a) | bits(q.b) | bits(q.a_norm) | bits(q.b_norm) | bits(q.add0) | bits(q.step) | bits(q.norm) | bits(q.shift) |
+                                       bits(q.shift_state) | bits(q.x_out));
+    }
+    __device__ __forceinline__ explicit NormRow(const hf2q_pre_norm& p) : q(p) {
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            const bool in = 4 * i < q.width;
+            norm[g] = group4(q.norm, i, in); mu[g] = group4(q.shift, i, in); step[g] = group4(q.step, i, in);
+            an[g] = group4(q.a_norm, i, in); bn[g] = group4(q.b_norm, i, in);
+        }
+    }
+    // the row into xs; with `keep` also x_out and the shift state.  red: 96 floats
+    __device__ __forceinline__ void run(bool keep, float* xs, float* red) const {
+        float4 v[PRO_GROUPS], a[PRO_GROUPS], b[PRO_GROUPS], add[PRO_GROUPS], even[PRO_GROUPS], odd[PRO_GROUPS];
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            const bool in = 4 * i < q.width;
+            v[g] = group4(q.x, i, in); a[g] = group4(q.a, i, in); b[g] = group4(q.b, i, in); add[g] = group4(q.add0, i, in);
+            even[g] = group4(q.shift ? q.shift_state : nullptr, i, in);     // (which of the two rows is the last one's follows from the position)
+            odd[g] = group4(q.shift ? q.shift_state + q.width : nullptr, i, in);
+        }
+        const uint32_t pos = q.shift ? *q.pos : 0u;
+        const float n = static_cast<float>(q.width);
+        if (q.a) {
+            float s[2] = {0.f, 0.f};
+#pragma unroll
+            for (int g = 0; g < PRO_GROUPS; ++g) { s[0] += square_sum(a[g]); s[1] += square_sum(b[g]); }
+            block_sum(s, red);
+            const float ia = 0.5f / sqrtf(s[0] / n + q.eps), ib = 0.5f / sqrtf(s[1] / n + q.eps);
+#pragma unroll
+            for (int g = 0; g < PRO_GROUPS; ++g) {
+                v[g].x += a[g].x * ia * an[g].x + b[g].x * ib * bn[g].x; v[g].y += a[g].y * ia * an[g].y + b[g].y * ib * bn[g].y;
+                v[g].z += a[g].z * ia * an[g].z + b[g].z * ib * bn[g].z; v[g].w += a[g].w * ia * an[g].w + b[g].w * ib * bn[g].w;
+            }
+        }
+        float s[1] = {0.f};
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            if (q.add0) { v[g].x += add[g].x; v[g].y += add[g].y; v[g].z += add[g].z; v[g].w += add[g].w; }
+            if (q.step) { v[g].x += step[g].x; v[g].y += step[g].y; v[g].z += step[g].z; v[g].w += step[g].w; }
+            s[0] += square_sum(v[g]);
+        }
+        block_sum(s, red + 64);
+        const float inv = 1.0f / sqrtf(s[0] / n + q.eps);
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            if (4 * i >= q.width) continue;
+            if (keep && q.x_out) *reinterpret_cast<float4*>(q.x_out + 4 * i) = v[g];
+            float4 h = make_float4(v[g].x * inv * norm[g].x, v[g].y * inv * norm[g].y, v[g].z * inv * norm[g].z, v[g].w * inv * norm[g].w);
+            if (q.shift) {
+                if (keep) *reinterpret_cast<float4*>(q.shift_state + static_cast<size_t>(pos & 1) * q.width + 4 * i) = h;
+                const float4 was = pos & 1 ? even[g] : odd[g];              // row (pos + 1) & 1
+                h = make_float4(h.x + (was.x - h.x) * mu[g].x, h.y + (was.y - h.y) * mu[g].y, h.z + (was.z - h.z) * mu[g].z, h.w + (was.w - h.w) * mu[g].w);
+            }
+            *reinterpret_cast<float4*>(xs + 4 * i) = h;
+        }
+    }
+};
+
+struct HyperRow {
+    static constexpr int S = 4, PARTS = 4;
+    const hf2q_hyper& q;
+    float4 norm[PRO_GROUPS];
+    static __device__ __forceinline__ bool fits(const hf2q_hyper& q) {
+        return q.streams <= S && (!q.y || q.y_parts <= PARTS) && groups_fit(q.width, bits(q.x) | bits(q.x_out) | bits(q.y) | bits(q.norm) | bits(q.h_out));
+    }
+    __device__ __forceinline__ HyperRow(const hf2q_hyper& p, float* coef) : q(p) {
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) norm[g] = group4(q.norm, threadIdx.x + MR_THREADS * g, 4 * (threadIdx.x + MR_THREADS * g) < q.width);
+        hyper_coefficients<S>(q, coef);
+    }
+    // the row into xs, the new streams' elements [lo, hi) (multiples of four) and those of the row itself to memory
+    __device__ __forceinline__ void run(float* xs, const float* coef, float* red, uint32_t lo, uint32_t hi) const {
+        const float *mix = coef, *gain = coef + S * S, *in = gain + S;
+        float4 old[PRO_GROUPS][S], y[PRO_GROUPS][PARTS], u[PRO_GROUPS];
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            const bool has = 4 * i < q.width;
+#pragma unroll
+            for (int s = 0; s < S; ++s) old[g][s] = group4(q.x + (q.x_streams == 1 ? 0u : s * q.width), i, has && s < static_cast<int>(q.streams));
+#pragma unroll
+            for (int k = 0; k < PARTS; ++k) y[g][k] = group4(q.y ? q.y + k * q.width : nullptr, i, has && k < static_cast<int>(q.y_parts));
+        }
+        float s1[1] = {0.f};
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t e = 4 * (threadIdx.x + MR_THREADS * g);
+            if (4 * MR_THREADS * g >= q.width) continue;
+            float4 yv = make_float4(0.f, 0.f, 0.f, 0.f);
+            u[g] = yv;
+#pragma unroll
+            for (int k = 0; k < PARTS; ++k) axpy(yv, 1.0f, y[g][k]);
+#pragma unroll
+            for (int d = 0; d < S; ++d) {
+                if (d >= static_cast<int>(q.streams)) continue;
+                float4 v = old[g][d];
+                if (q.y) {
+                    v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int s = 0; s < S; ++s) axpy(v, mix[s * S + d], old[g][s]);
+                    axpy(v, gain[d], yv);
+                }
+                if (q.x_out && e >= lo && e < hi && e < q.width) *reinterpret_cast<float4*>(q.x_out + static_cast<size_t>(d) * q.width + e) = v;
+                axpy(u[g], in[d], v);
+            }
+            s1[0] += square_sum(u[g]);
+        }
+        block_sum(s1, red);
+        const float inv = 1.0f / sqrtf(s1[0] / static_cast<float>(q.width) + q.eps);
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t e = 4 * (threadIdx.x + MR_THREADS * g);
+            if (e >= q.width) continue;
+            const float4 h = q.norm ? make_float4(u[g].x * inv * norm[g].x, u[g].y * inv * norm[g].y, u[g].z * inv * norm[g].z, u[g].w * inv * norm[g].w) : u[g];
+            *reinterpret_cast<float4*>(xs + e) = h;
+            if (q.h_out && e >= lo && e < hi) *reinterpret_cast<float4*>(q.h_out + e) = h;
+        }
+    }
+};
+
+// Gated head outputs of heads of whole 128-element spans, a span to a warp (silu_group_norm_row and gated_heads_row take the others).
+struct GatedRow {
+    const hf2q_gated_heads& q;
+    const bool silu;
+    float4 norm[PRO_GROUPS];
+    static __device__ __forceinline__ bool fits(const hf2q_gated_heads& q) {
+        return q.head_dim % 128 == 0 && groups_fit(q.heads * q.head_dim, bits(q.o) | bits(q.gate) | bits(q.norm));
+    }
+    __device__ __forceinline__ explicit GatedRow(const hf2q_gated_heads& p) : q(p), silu(p.kind == HF2Q_GATE_SILU_FIRST) {
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            norm[g] = group4(q.norm, silu || q.norm_all ? i : i % (q.head_dim / 4), 4 * i < q.heads * q.head_dim);
+        }
+    }
+    // the row into xs.  sums: a float per span
+    __device__ __forceinline__ void run(float* xs, float* sums) const {
+        const uint32_t width = q.heads * q.head_dim, spans = q.head_dim / 128;
+        float4 v[PRO_GROUPS], x[PRO_GROUPS];
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            v[g] = group4(q.o, i, 4 * i < width); x[g] = group4(q.gate, i, 4 * i < width);
+        }
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            if (silu) v[g] = make_float4(v[g].x * siluf(x[g].x), v[g].y * siluf(x[g].y), v[g].z * siluf(x[g].z), v[g].w * siluf(x[g].w));
+            const float s = q.norm ? warp_sum(square_sum(v[g])) : 0.f;
+            if (threadIdx.x % 32 == 0) sums[(threadIdx.x + MR_THREADS * g) / 32] = s;
+        }
+        if (q.norm) __syncthreads();
+#pragma unroll
+        for (int g = 0; g < PRO_GROUPS; ++g) {
+            const uint32_t i = threadIdx.x + MR_THREADS * g;
+            if (4 * i >= width) continue;
+            float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (q.norm) {
+                float s = 0.f;
+                for (uint32_t k = 0, first = i / 32 / spans * spans; k < spans; ++k) s += sums[first + k];
+                const float inv = 1.0f / sqrtf(s / static_cast<float>(q.head_dim) + q.eps);
+                w = make_float4(norm[g].x * inv, norm[g].y * inv, norm[g].z * inv, norm[g].w * inv);
+            }
+            float4 h = make_float4(v[g].x * w.x, v[g].y * w.y, v[g].z * w.z, v[g].w * w.w);
+            if (!silu) h = make_float4(h.x * sigmoidf(x[g].x), h.y * sigmoidf(x[g].y), h.z * sigmoidf(x[g].z), h.w * sigmoidf(x[g].w));
+            *reinterpret_cast<float4*>(xs + 4 * i) = h;
+        }
+    }
+};
+
 // One-row product: the CTA's weight rows run through a MatvecStream; the layer's row prologue fills x in front of it.
 template <int PRO, bool PAIRS>
-__global__ void __launch_bounds__(MR_THREADS) dense_matvec_kernel(const __grid_constant__ MatvecSegs p, uint32_t* status) {
+__global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __grid_constant__ MatvecSegs p, uint32_t* status) {
     extern __shared__ __align__(128) uint8_t mv_smem[];                 // ring, then x [k] f32
-    __shared__ float red[64];
+    __shared__ float red[96];
     __shared__ MatvecShared sh;
     pdl_trigger();
     const bool second = blockIdx.x >= p.blocks0;
@@ -92,36 +276,58 @@ __global__ void __launch_bounds__(MR_THREADS) dense_matvec_kernel(const __grid_c
     constexpr uint32_t unit = PAIRS ? 2 : 1;
     const uint32_t units = s.n / unit;
     const uint32_t row0 = unit * static_cast<uint32_t>(static_cast<uint64_t>(units) * blk / n_blk), row1 = unit * static_cast<uint32_t>(static_cast<uint64_t>(units) * (blk + 1) / n_blk);
-    const uint32_t per_row = (s.k + MV_CHUNK - 1) / MV_CHUNK;
+    const uint32_t piece = mv_piece(s.k), per_row = (s.k + piece - 1) / piece;
     const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(s.w) + static_cast<size_t>(row0) * s.k;
-    auto chunk = [&](uint32_t c) {
-        const uint32_t k0 = (c % per_row) * MV_CHUNK;
-        return MatvecChunk{w + static_cast<size_t>(c / per_row) * s.k + k0, k0, min(static_cast<uint32_t>(MV_CHUNK), s.k - k0)};
+    auto at = [&](uint32_t row, uint32_t col) {
+        const uint32_t k0 = col * piece;
+        return MatvecChunk{w + static_cast<size_t>(row) * s.k + k0, k0, min(piece, s.k - k0)};
     };
-    MatvecStream stream(mv_smem, sh, (row1 - row0) * per_row, status);
-    stream.start(chunk);
-    pdl_wait();
+    MatvecStream stream(mv_smem, sh, row1 - row0, per_row, status);
+    stream.start(at);
+    // what the first pass of the epilogue adds to this thread's row (or pair)
+    const uint32_t mine = row0 + threadIdx.x * unit;
+    float bias0 = 0.f, bias1 = 0.f, residual = 0.f;
+    if (s.bias && mine < row1) {
+        bias0 = s.bias[mine];
+        if constexpr (PAIRS) bias1 = s.bias[mine + 1];
+    }
+    auto add_residual = [&] { if (s.epilogue == HF2Q_EPI_ADD && mine < row1) residual = s.residual[mine]; };
     if constexpr (PRO == HF2Q_PRO_NONE) {
-        for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = s.x[i];
+        pdl_wait();
+        add_residual();
+        if (s.k % 4 == 0 && bits(s.x) % 16 == 0)
+            for (uint32_t i = threadIdx.x; i < s.k / 4; i += MR_THREADS) reinterpret_cast<float4*>(xs)[i] = reinterpret_cast<const float4*>(s.x)[i];
+        else
+            for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = s.x[i];
     } else if constexpr (PRO == HF2Q_PRO_NORM) {
         const hf2q_pre_norm& q = s.pre;
-        const float inv = residual_row(q, 0, xs, red);
         const bool keep = blk == 0;
-        const uint32_t pos = q.shift ? *q.pos : 0u;
-        const float* before = q.shift_state + static_cast<size_t>((pos + 1) & 1) * q.width;
-        float* now = q.shift_state + static_cast<size_t>(pos & 1) * q.width;
-        for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) {
-            float h = 0.f;
-            if (i < q.width) {
-                const float x = xs[i];
-                if (keep && q.x_out) q.x_out[i] = x;
-                h = x * inv * q.norm[i];
-                if (q.shift) {
-                    if (keep) now[i] = h;
-                    h += (before[i] - h) * q.shift[i];
+        if (NormRow::fits(q)) {
+            const NormRow row(q);
+            pdl_wait();
+            add_residual();
+            row.run(keep, xs, red);
+            for (uint32_t i = q.width + threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = 0.f;
+        } else {
+            pdl_wait();
+            add_residual();
+            const float inv = residual_row(q, 0, xs, red);
+            const uint32_t pos = q.shift ? *q.pos : 0u;
+            const float* before = q.shift_state + static_cast<size_t>((pos + 1) & 1) * q.width;
+            float* now = q.shift_state + static_cast<size_t>(pos & 1) * q.width;
+            for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) {
+                float h = 0.f;
+                if (i < q.width) {
+                    const float x = xs[i];
+                    if (keep && q.x_out) q.x_out[i] = x;
+                    h = x * inv * q.norm[i];
+                    if (q.shift) {
+                        if (keep) now[i] = h;
+                        h += (before[i] - h) * q.shift[i];
+                    }
                 }
+                xs[i] = h;
             }
-            xs[i] = h;
         }
     } else if constexpr (PRO == HF2Q_PRO_HYPER) {
         const hf2q_hyper& q = s.hyper;
@@ -129,30 +335,48 @@ __global__ void __launch_bounds__(MR_THREADS) dense_matvec_kernel(const __grid_c
         // every CTA makes the whole row and stores its share of the new streams
         const uint32_t lo = static_cast<uint32_t>(static_cast<uint64_t>(q.width) * blk / n_blk) & ~3u;
         const uint32_t hi = blk + 1 == n_blk ? q.width : static_cast<uint32_t>(static_cast<uint64_t>(q.width) * (blk + 1) / n_blk) & ~3u;
-        const float inv = hyper_row(q, 0, xs, coef, red, lo, hi);
-        for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) {
-            const float h = i < q.width ? (q.norm ? xs[i] * inv * q.norm[i] : xs[i]) : 0.f;
-            xs[i] = h;
-            if (q.h_out && i >= lo && i < hi) q.h_out[i] = h;
+        if (HyperRow::fits(q)) {
+            const HyperRow row(q, coef);
+            pdl_wait();
+            add_residual();
+            row.run(xs, coef, red, lo, hi);
+            for (uint32_t i = q.width + threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = 0.f;
+        } else {
+            pdl_wait();
+            add_residual();
+            const float inv = hyper_row(q, 0, xs, coef, red, lo, hi);
+            for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) {
+                const float h = i < q.width ? (q.norm ? xs[i] * inv * q.norm[i] : xs[i]) : 0.f;
+                xs[i] = h;
+                if (q.h_out && i >= lo && i < hi) q.h_out[i] = h;
+            }
         }
+    } else if (GatedRow::fits(s.gated)) {
+        const GatedRow row(s.gated);
+        pdl_wait();
+        add_residual();
+        row.run(xs, red);
+        for (uint32_t i = s.gated.heads * s.gated.head_dim + threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = 0.f;
     } else {
+        pdl_wait();
+        add_residual();
         for (uint32_t i = s.gated.heads * s.gated.head_dim + threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = 0.f;
         if (s.gated.kind == HF2Q_GATE_SILU_FIRST) silu_group_norm_row<float>(s.gated, 0, xs, xs);
         else gated_heads_row<float>(s.gated, 0, xs, warp, MR_WARPS);
     }
     __syncthreads();
     if constexpr (PAIRS) {
-        stream.run<true>(chunk, xs, row1 - row0, per_row, [&](uint32_t r, float gate, float up) {
+        stream.run<true>(at, xs, [&](uint32_t r, float gate, float up) {
             const uint32_t row = row0 + r;
-            if (s.bias) { gate += s.bias[row]; up += s.bias[row + 1]; }
+            if (s.bias) { gate += row == mine ? bias0 : s.bias[row]; up += row == mine ? bias1 : s.bias[row + 1]; }
             s.y[row / 2] = glu_value(gate, up, s.epilogue, s.cap);
         });
     } else {
-        stream.run<false>(chunk, xs, row1 - row0, per_row, [&](uint32_t r, float v, float) {
+        stream.run<false>(at, xs, [&](uint32_t r, float v, float) {
             const uint32_t row = row0 + r;
-            if (s.bias) v += s.bias[row];
+            if (s.bias) v += row == mine ? bias0 : s.bias[row];
             v = epilogue_value(v, s.epilogue, s.cap);
-            if (s.epilogue == HF2Q_EPI_ADD) v += s.residual[row];
+            if (s.epilogue == HF2Q_EPI_ADD) v += row == mine ? residual : s.residual[row];
             s.y[row] = v;
         });
     }
@@ -563,7 +787,7 @@ cudaError_t dense_any(const DenseArgs& a, int sms, uint32_t* status, cudaStream_
 template <int PRO, bool PAIRS>
 cudaError_t launch_fused_as(const MatvecSegs& p, uint32_t blocks, size_t smem, uint32_t* status, cudaStream_t st) {
     static PerDeviceFlag flag;
-    if (const cudaError_t e = ensure_max_dynamic_smem(dense_matvec_kernel<PRO, PAIRS>, MR_MAX_SMEM, flag); e != cudaSuccess) return e;
+    if (const cudaError_t e = ensure_max_dynamic_smem(dense_matvec_kernel<PRO, PAIRS>, MR_RING + MR_MAX_X, flag); e != cudaSuccess) return e;
     return launch_pdl(dense_matvec_kernel<PRO, PAIRS>, dim3(blocks), dim3(MR_THREADS), smem, st, p, status);
 }
 template <int PRO>
@@ -630,7 +854,7 @@ HF2Q_API int32_t hf2q_cuda_dense_matvec(hf2q_ctx* ctx, void* stream, uint32_t pr
     uint64_t chunks[2] = {0, 0};
     for (uint32_t i = 0; i < n_segs; ++i) {
         const hf2q_matvec& s = segs[i];
-        if (!s.w || !s.y || s.n == 0 || s.k == 0 || s.k % 8 || reinterpret_cast<uintptr_t>(s.w) % 16 || MR_RING + s.k * 4ull > MR_MAX_SMEM ||
+        if (!s.w || !s.y || s.n == 0 || s.k == 0 || s.k % 8 || reinterpret_cast<uintptr_t>(s.w) % 16 || s.k * 4ull > MR_MAX_X ||
             (prologue == HF2Q_PRO_NONE && !s.x) ||
             (prologue == HF2Q_PRO_NORM && (!s.pre.x || !s.pre.norm || s.pre.width > s.k || !pre_norm_aligned(s.pre) || (s.pre.a && (!s.pre.b || !s.pre.a_norm || !s.pre.b_norm)) || (s.pre.shift && (!s.pre.shift_state || !s.pre.pos)))) ||
             (prologue == HF2Q_PRO_GATED && (!gated_ok(s.gated) || s.gated.heads * s.gated.head_dim > s.k)) ||

@@ -8,9 +8,23 @@
 namespace hf2q {
 namespace seq {
 
-constexpr int MR_WARPS = 16, MR_THREADS = MR_WARPS * 32, MV_CHUNK = 1024, MR_STAGES = 3, MR_PART = 2048;
+// One CTA an SM; its kernels say so in their launch bounds, for with all registers to give ptxas asks for a chunk's 16-byte groups and
+// a prologue's loads at once (16 warps, 25 MB: 9.4 us a product without, 7.6 with).  In a chain of up (norm prologue) and down
+// products, us a product at 2048 x 6144 / 4096 x 11264 / 3072 x 9216 / 1536 x 4096: 12 warps of 3 stages 6.6 / 16.5 / 11.9 / 5.4, of 2
+// 6.8 / 17.3 / 12.3 / 5.3, 16 of 3 7.3 / 16.9 / 12.9 / 5.6, 8 of 3 with chunks of 1536 7.5 / 17.3 / 11.3 / 5.3; two CTAs an SM 9.3 and
+// more.  Before: 9.9 / 24.7 / 17.3 / 6.7.
+constexpr int MR_WARPS = 12, MR_THREADS = MR_WARPS * 32, MR_STAGES = 3, MV_CHUNK = 1024, MR_PART = 2048;
 constexpr uint32_t MR_RING = MR_WARPS * MR_STAGES * MV_CHUNK * 2;      // bytes of dynamic shared memory
-constexpr uint32_t MR_MAX_SMEM = 208 * 1024;
+constexpr uint32_t MR_MAX_X = 112 * 1024;                              // bytes of activations
+
+// A row of k weights is cut into pieces of this many elements: a divisor of the warps to a row, so that each warp keeps to one place
+// of the rows and holds that place's activations in registers.  Longer rows: pieces of MV_CHUNK, activations from shared memory at
+// every step (16 bytes of weights meet 32 of activations there).
+__host__ __device__ constexpr uint32_t mv_piece(uint32_t k) {
+    for (uint32_t n = 1; n <= MR_WARPS; ++n)
+        if (MR_WARPS % n == 0 && k <= n * MV_CHUNK) return (k + 8 * n - 1) / (8 * n) * 8;
+    return MV_CHUNK;
+}
 
 struct MatvecShared {
     float part[2][MR_PART];
@@ -18,82 +32,126 @@ struct MatvecShared {
 };
 struct MatvecChunk {
     const __nv_bfloat16* w;      // global, 16-byte aligned
-    uint32_t x0, len;            // its activations start at xs + x0; len a multiple of 8
+    uint32_t x0, len;            // its activations start at xs + x0; len a multiple of 8, at most MV_CHUNK
 };
 
+// What a step costs beside its 32 multiply-adds a lane is what this class is about: a chunk in 950 ns and more, with the weights long
+// in shared memory, was 6 of the 10 us of a product of 25 MB.  Hence no division (places advance by a constant), no address but the
+// issuing lane's, activations in registers.
 class MatvecStream {
 public:
-    __device__ __forceinline__ MatvecStream(uint8_t* smem, MatvecShared& sh, uint32_t n_chunks, uint32_t* status)
-        : sh_(sh), n_chunks_(n_chunks), status_(status), warp_(threadIdx.x >> 5), lane_(threadIdx.x & 31),
-          ring_(reinterpret_cast<__nv_bfloat16*>(smem) + static_cast<size_t>(warp_) * MR_STAGES * MV_CHUNK) {}
-
-    // fills the ring; chunk(c) -> MatvecChunk
-    template <class F> __device__ __forceinline__ void start(F chunk) {
-        if (lane_ == 0) {
-            for (int i = 0; i < MR_STAGES; ++i) mbar_init(&sh_.bars[warp_][i], 1);
-            mbar_fence_init();
-            for (int i = 0; i < MR_STAGES; ++i) issue(i, chunk);
-        }
+    // rows of per_row pieces each
+    __device__ __forceinline__ MatvecStream(uint8_t* smem, MatvecShared& sh, uint32_t rows, uint32_t per_row, uint32_t* status)
+        : sh_(sh), rows_(rows), per_row_(per_row), status_(status), warp_(threadIdx.x >> 5), lane_(threadIdx.x & 31),
+          ring_(reinterpret_cast<__nv_bfloat16*>(smem) + static_cast<size_t>(warp_) * MR_STAGES * MV_CHUNK) {
+        down_ = MR_WARPS / per_row;
+        right_ = MR_WARPS - down_ * per_row;
+        now_.row = next_.row = warp_ / per_row;
+        now_.col = next_.col = warp_ - now_.row * per_row;
     }
-    // rows of per_row chunks each, finished one (or with PAIRS two) at a time: finish(row, sum, sum of row + 1).  Every thread
-    // of the CTA calls it, after a barrier behind the last write of xs.
-    template <bool PAIRS, class F, class G> __device__ __forceinline__ void run(F chunk, const float* xs, uint32_t rows, uint32_t per_row, G finish) {
+
+    // fills the ring; at(row, col) -> MatvecChunk
+    template <class F> __device__ __forceinline__ void start(F at) {
+        if (lane_ == 0) {
+            for (uint32_t i = 0; i < MR_STAGES; ++i) mbar_init(&sh_.bars[warp_][i], 1);
+            mbar_fence_init();
+        }
+        for (uint32_t i = 0; i < MR_STAGES; ++i) issue(i, at);
+    }
+    // The rows, finished one (or with PAIRS two) at a time: finish(row, sum, sum of row + 1).  Every thread of the CTA calls it,
+    // after a barrier behind the last write of xs.  x0 and len depend on the column only.
+    template <bool PAIRS, class F, class G> __device__ __forceinline__ void run(F at, const float* xs, G finish) {
+        if (right_ == 0) run_as<PAIRS, true>(at, xs, finish);
+        else run_as<PAIRS, false>(at, xs, finish);
+    }
+
+private:
+    struct Place { uint32_t row, col; };
+    __device__ __forceinline__ void advance(Place& p) const {              // to the warp's next chunk
+        p.row += down_;
+        p.col += right_;
+        if (p.col >= per_row_) { p.col -= per_row_; ++p.row; }
+    }
+    static constexpr int U = MV_CHUNK / 256;                               // 16-byte groups of a chunk per lane
+    template <bool PAIRS, bool HELD, class F, class G> __device__ __forceinline__ void run_as(F at, const float* xs, G finish) {
         constexpr uint32_t unit = PAIRS ? 2 : 1;
-        const uint32_t block_rows = max(unit, MR_PART / per_row / unit * unit);
-        bool ok = true;
-        uint32_t i = 0;                                                     // this warp's chunk counter
-        for (uint32_t r0 = 0, pb = 0; r0 < rows; r0 += block_rows, pb ^= 1) {
-            const uint32_t nr = min(block_rows, rows - r0), c_end = (r0 + nr) * per_row;
-            for (uint32_t c = i * MR_WARPS + warp_; c < c_end; ++i, c += MR_WARPS) {
-                const uint32_t st = i % MR_STAGES;
-                const MatvecChunk k = chunk(c);
-                if (ok) ok = mbar_wait_bounded(&sh_.bars[warp_][st], (i / MR_STAGES) & 1, status_);
-                ok = __all_sync(0xffffffffu, ok);
-                float acc = 0.f;
-                if (ok) {
-                    const uint4* wv = reinterpret_cast<const uint4*>(ring_ + st * MV_CHUNK);
-                    const float* xv = xs + k.x0;
+        const uint32_t block_rows = max(unit, MR_PART / per_row_ / unit * unit);
+        float held[HELD ? U : 1][8];
+        uint32_t len = 0;
+        if constexpr (HELD) {
+            if (now_.row < rows_) {
+                const MatvecChunk k = at(now_.row, now_.col);
+                len = k.len;
 #pragma unroll
-                    for (int u = 0; u < MV_CHUNK / 256; ++u) {
-                        const uint32_t e = lane_ + 32 * u;
-                        if (8 * e < k.len) {
-                            const uint4 v = wv[e];
-                            const float4 a = *reinterpret_cast<const float4*>(xv + 8 * e), b = *reinterpret_cast<const float4*>(xv + 8 * e + 4);
-                            acc = fmaf(bf_lo(v.x), a.x, acc); acc = fmaf(bf_hi(v.x), a.y, acc); acc = fmaf(bf_lo(v.y), a.z, acc); acc = fmaf(bf_hi(v.y), a.w, acc);
-                            acc = fmaf(bf_lo(v.z), b.x, acc); acc = fmaf(bf_hi(v.z), b.y, acc); acc = fmaf(bf_lo(v.w), b.z, acc); acc = fmaf(bf_hi(v.w), b.w, acc);
-                        }
-                    }
+                for (int u = 0; u < U; ++u) load_x(xs + k.x0, lane_ + 32 * u, len, held[u]);
+            }
+        }
+        bool ok = true;
+        uint32_t st = 0, ph = 0;                                            // ring slot and parity
+        for (uint32_t r0 = 0, pb = 0; r0 < rows_; r0 += block_rows, pb ^= 1) {
+            const uint32_t nr = min(block_rows, rows_ - r0);
+            for (; now_.row < r0 + nr; advance(now_)) {
+                const float* x = xs;
+                if constexpr (!HELD) {
+                    const MatvecChunk k = at(now_.row, now_.col);
+                    len = k.len;
+                    x += k.x0;
                 }
+                if (ok) ok = mbar_wait_bounded(&sh_.bars[warp_][st], ph, status_);
+                ok = __all_sync(0xffffffffu, ok);
+                uint4 v[U];
+                const uint4* wv = reinterpret_cast<const uint4*>(ring_ + st * MV_CHUNK);
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = ok && 8 * (lane_ + 32 * u) < len ? wv[lane_ + 32 * u] : make_uint4(0, 0, 0, 0);
                 __syncwarp();                                               // every lane has read the stage
-                if (lane_ == 0 && ok) issue(i + MR_STAGES, chunk);
-                acc = warp_sum(acc);
-                if (lane_ == 0) sh_.part[pb][c - r0 * per_row] = acc;
+                if (ok) issue(st, at);
+                if (++st == MR_STAGES) { st = 0; ph ^= 1; }
+                float acc[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    float mine[8];
+                    if constexpr (!HELD) load_x(x, lane_ + 32 * u, len, mine);
+                    const float (&f)[8] = HELD ? held[HELD ? u : 0] : mine;
+                    float a = bf_lo(v[u].x) * f[0];
+                    a = fmaf(bf_hi(v[u].x), f[1], a); a = fmaf(bf_lo(v[u].y), f[2], a); a = fmaf(bf_hi(v[u].y), f[3], a);
+                    a = fmaf(bf_lo(v[u].z), f[4], a); a = fmaf(bf_hi(v[u].z), f[5], a); a = fmaf(bf_lo(v[u].w), f[6], a); a = fmaf(bf_hi(v[u].w), f[7], a);
+                    acc[u] = a;
+                }
+                const float sum = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+                if (lane_ == 0) sh_.part[pb][(now_.row - r0) * per_row_ + now_.col] = sum;
             }
             __syncthreads();                                                // (the other half of `part` is free: its readers passed this barrier)
             for (uint32_t r = threadIdx.x * unit; r < nr; r += MR_THREADS * unit) {
                 float v = 0.f, w = 0.f;
-                for (uint32_t kc = 0; kc < per_row; ++kc) v += sh_.part[pb][r * per_row + kc];
+                for (uint32_t kc = 0; kc < per_row_; ++kc) v += sh_.part[pb][r * per_row_ + kc];
                 if constexpr (PAIRS)
-                    for (uint32_t kc = 0; kc < per_row; ++kc) w += sh_.part[pb][(r + 1) * per_row + kc];
+                    for (uint32_t kc = 0; kc < per_row_; ++kc) w += sh_.part[pb][(r + 1) * per_row_ + kc];
                 finish(r0 + r, v, w);
             }
         }
     }
-
-private:
-    template <class F> __device__ __forceinline__ void issue(uint32_t i, F& chunk) {      // this warp's chunk number i
-        const uint32_t c = i * MR_WARPS + warp_;
-        if (c >= n_chunks_) return;
-        const MatvecChunk k = chunk(c);
-        uint64_t* bar = &sh_.bars[warp_][i % MR_STAGES];
-        mbar_arrive_expect_tx(bar, k.len * 2);
-        bulk_g2s(ring_ + (i % MR_STAGES) * MV_CHUNK, k.w, k.len * 2, bar);
+    static __device__ __forceinline__ void load_x(const float* x, uint32_t e, uint32_t len, float (&out)[8]) {
+        const bool in = 8 * e < len;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a = in ? *reinterpret_cast<const float4*>(x + 8 * e) : zero, b = in ? *reinterpret_cast<const float4*>(x + 8 * e + 4) : zero;
+        out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w; out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
+    }
+    template <class F> __device__ __forceinline__ void issue(uint32_t st, F& at) {      // the next chunk of this warp into slot st
+        if (lane_ == 0 && next_.row < rows_) {
+            const MatvecChunk k = at(next_.row, next_.col);
+            uint64_t* bar = &sh_.bars[warp_][st];
+            mbar_arrive_expect_tx(bar, k.len * 2);
+            bulk_g2s(ring_ + st * MV_CHUNK, k.w, k.len * 2, bar);
+        }
+        advance(next_);
     }
     MatvecShared& sh_;
-    const uint32_t n_chunks_;
+    const uint32_t rows_, per_row_;
     uint32_t* const status_;
     const uint32_t warp_, lane_;
     __nv_bfloat16* const ring_;
+    uint32_t down_, right_;
+    Place now_, next_;
 };
 
 }  // namespace seq

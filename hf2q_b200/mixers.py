@@ -20,7 +20,9 @@ def _off(t: torch.Tensor, cols: int) -> int:
 
 
 # Portions of this many tokens run a layer's recurrence beside its attention: a scan has fewer CTAs than the chip has SMs and each
-# token waits for the one before, so the attention's tiles take the SMs that it leaves.
+# token waits for the one before, so the attention's tiles take the SMs that it leaves (four layers, two of them such ones, us in turn
+# and beside: 256 tokens 813 and 724, 2048 tokens 2441 and 2293).  Shorter ones gain as well (64: 614 and 557) where the host is ahead of
+# the device, which a portion by itself is not.
 BESIDE_TOKENS = 256
 
 

@@ -750,7 +750,8 @@ HF2Q_API int32_t hf2q_cuda_hyper_norm(hf2q_ctx* ctx, void* stream, const hf2q_hy
                                       uint32_t ldo);
 
 /* One-row products with their prologue and epilogue in the same launch (f32 arithmetic); up to two segments with
- * the same kind of prologue run side by side. */
+ * the same kind of prologue run side by side.  As in all one-token calls, parameters (weights, biases, norms, the streams'
+ * coefficients, convolution taps) may be read while the launch in front still runs. */
 enum { HF2Q_PRO_NONE = 0, HF2Q_PRO_NORM = 1, HF2Q_PRO_GATED = 2, HF2Q_PRO_HYPER = 3 };
 typedef struct hf2q_matvec {
     const void* w;
