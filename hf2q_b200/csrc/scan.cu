@@ -493,87 +493,140 @@ __device__ __forceinline__ float conv_silu(const float* w, uint32_t taps, float 
     return siluf(s);
 }
 __device__ __forceinline__ float decay_of(float a_log, float x) { return expf(-expf(a_log) * softplusf(x)); }
-__device__ __forceinline__ float low_rank_dot(const void* w, size_t row, uint32_t ld, const float* x) {
-    const __nv_bfloat16* r = static_cast<const __nv_bfloat16*>(w) + row * ld;
-    float s = 0.f;
-    for (uint32_t c = 0; c < ld; c += 8) {
-        float f[8];
-        load8(r + c, f);
+// The same for four taps from a channel's ring and its weights, both asked for before the position is known.
+__device__ __forceinline__ float ring_at(const float4& r, uint32_t i) { return (i & 2) ? ((i & 1) ? r.w : r.z) : ((i & 1) ? r.y : r.x); }
+__device__ __forceinline__ float conv4(const float4& w, const float4& ring, float now, uint32_t pos, float s0) {
+    float s = fmaf(now, w.w, s0);
+    s = fmaf(ring_at(ring, pos + 3), w.z, s);
+    s = fmaf(ring_at(ring, pos + 2), w.y, s);
+    return fmaf(ring_at(ring, pos + 1), w.x, s);
+}
+
+// Rows of a low-rank product, 16 lanes to a row: w holds the first 128 elements of N rows, fetch(c, w) brings those from c on.
+// Every lane of the group gets the sums.
+template <int N, typename F>
+__device__ __forceinline__ void low_rank_dots(uint4 (&w)[N], uint32_t ld, const float* x, F fetch, float (&s)[N]) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s = fmaf(f[i], x[c + i], s);
+    for (int r = 0; r < N; ++r) s[r] = 0.f;
+    for (uint32_t c = 0;;) {
+        const uint32_t e = c + 8 * (threadIdx.x & 15);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (e < ld) { a = *reinterpret_cast<const float4*>(x + e); b = *reinterpret_cast<const float4*>(x + e + 4); }
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            s[r] = fmaf(bf_lo(w[r].x), a.x, s[r]); s[r] = fmaf(bf_hi(w[r].x), a.y, s[r]); s[r] = fmaf(bf_lo(w[r].y), a.z, s[r]); s[r] = fmaf(bf_hi(w[r].y), a.w, s[r]);
+            s[r] = fmaf(bf_lo(w[r].z), b.x, s[r]); s[r] = fmaf(bf_hi(w[r].z), b.y, s[r]); s[r] = fmaf(bf_lo(w[r].w), b.z, s[r]); s[r] = fmaf(bf_hi(w[r].w), b.w, s[r]);
+        }
+        if ((c += 128) >= ld) break;
+        fetch(c, w);
     }
-    return s;
+#pragma unroll
+    for (int r = 0; r < N; ++r) s[r] = group_sum(s[r]);
 }
 
 // One token from the raw projection row: convolution, SiLU, unit norms, decays, gate and the state update.
+// Bound by latency: one load behind another.  The rows of the low-rank products and the taps' weights are asked for before the wait,
+// everything else right behind it; a row of a2 per thread, 16 bytes at a time, and rings read behind the position took most of a
+// launch (16 heads of 128 x 128, rank 128: 10.2 -> 4.4 us a launch of many, 64 heads of rank 64 9.3 -> 8.8).
 template <int RQ>
-__global__ void __launch_bounds__(SC_THREADS) delta_step_kernel(const __grid_constant__ hf2q_delta a, float* __restrict__ out, float* __restrict__ gate) {
-    constexpr uint32_t DP = 32 * RQ;
-    __shared__ __align__(16) float ks[DP], qs[DP], gs[DP], vs[SC_COLS];
+__global__ void __launch_bounds__(SC_THREADS, RQ <= 4 ? 2 : 1) delta_step_kernel(const __grid_constant__ hf2q_delta a, float* __restrict__ out, float* __restrict__ gate) {
+    constexpr uint32_t DP = 32 * RQ, ROWS = DP / SC_COLS, ITEMS = (2 * DP + SC_COLS + SC_THREADS - 1) / SC_THREADS;
+    __shared__ __align__(16) float xs[2 * DP + SC_COLS], gs[DP];    // q, k, v; decays
     __shared__ float red[64];
     extern __shared__ __align__(16) float lr[];                     // a1 [a_rank_ld], g1 [g_rank_ld]
     pdl_trigger();
-    const uint32_t h = blockIdx.x, slice = blockIdx.y, rep = a.heads / a.kv_heads, kvh = h / rep;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = lane & 15;
-    const uint32_t col_s = warp * 2 + (lane >> 4), col0 = slice * SC_COLS, col = col0 + col_s;
+    const uint32_t h = blockIdx.x, slice = blockIdx.y, rep = a.heads / a.kv_heads, kvh = h / rep, qk = a.kv_heads * a.dim;
+    const uint32_t lg = threadIdx.x & 15, col_s = threadIdx.x >> 4, col0 = slice * SC_COLS, col = col0 + col_s;
     const uint32_t n_cols = min(static_cast<uint32_t>(SC_COLS), a.vdim - col0);
     const bool live = col < a.vdim;
-    for (uint32_t i = threadIdx.x; i < a.dim; i += SC_THREADS)       // weights: towards L2 before the wait
-        for (uint32_t c = 0; c < a.a_rank_ld; c += 64) prefetch_l2(static_cast<const __nv_bfloat16*>(a.a2) + (static_cast<size_t>(h) * a.dim + i) * a.a_rank_ld + c);
+    // decays: rows col_s + SC_COLS r of the head; the gate: the group's own column
+    uint4 wa[ROWS], wg[1];
+    auto fetch_a = [&](uint32_t c, uint4 (&w)[ROWS]) {
+        const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.a2) + (static_cast<size_t>(h) * a.dim + col_s) * a.a_rank_ld + c + 8 * lg;
+#pragma unroll
+        for (uint32_t r = 0; r < ROWS; ++r)
+            w[r] = col_s + SC_COLS * r < a.dim && c + 8 * lg < a.a_rank_ld ? *reinterpret_cast<const uint4*>(src + static_cast<size_t>(SC_COLS) * r * a.a_rank_ld) : make_uint4(0, 0, 0, 0);
+    };
+    auto fetch_g = [&](uint32_t c, uint4 (&w)[1]) {
+        w[0] = live && c + 8 * lg < a.g_rank_ld
+                   ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.g2) + (static_cast<size_t>(h) * a.vdim + col) * a.g_rank_ld + c + 8 * lg)
+                   : make_uint4(0, 0, 0, 0);
+    };
+    fetch_a(0, wa);
+    fetch_g(0, wg);
+    // channel of an item: q, k, then the slice's v
+    struct Channel { uint32_t ring, at; const float* w; bool in, keep; };
+    auto channel = [&](uint32_t i) {
+        const uint32_t j = i < DP ? i : i < 2 * DP ? i - DP : i - 2 * DP;
+        if (i < 2 * DP) {
+            const uint32_t c = kvh * a.dim + j;
+            return Channel{i < DP ? c : qk + c, (i < DP ? a.q_off : a.k_off) + c, (i < DP ? a.q_conv : a.k_conv) + static_cast<size_t>(c) * a.taps, j < a.dim, slice == 0 && h % rep == 0};
+        }
+        const uint32_t c = h * a.vdim + col0 + j;
+        return Channel{2 * qk + c, a.v_off + c, a.v_conv + static_cast<size_t>(c) * a.taps, j < n_cols, true};
+    };
+    const bool four = a.taps == 4 && ((reinterpret_cast<uintptr_t>(a.conv_state) | reinterpret_cast<uintptr_t>(a.q_conv) | reinterpret_cast<uintptr_t>(a.k_conv) |
+                                       reinterpret_cast<uintptr_t>(a.v_conv)) & 15) == 0;
+    float4 taps[ITEMS], ring[ITEMS];
+    float now[ITEMS];
+    if (four) {
+#pragma unroll
+        for (uint32_t n = 0; n < ITEMS; ++n) {
+            const Channel c = channel(threadIdx.x + SC_THREADS * n);
+            if (c.in) taps[n] = *reinterpret_cast<const float4*>(c.w);
+        }
+    }
+    const uint32_t row = col_s + SC_COLS * lg;                      // whose decay this lane makes
+    const bool decays = lg < ROWS && row < a.dim;
+    const float bias = decays ? a.dt_bias[h * a.dim + row] : 0.f, a_log = a.a_log[h];
     pdl_wait();
     Vec<RQ> S;
     float* sp = a.s + (static_cast<size_t>(h) * a.vdim + (live ? col : 0)) * DP + 2 * lg;
     if (live) S.load(sp); else S.zero();
-    const uint32_t pos = *a.pos, qk = a.kv_heads * a.dim;
+    const uint32_t pos = *a.pos;
+    const float b = a.proj[a.b_off + h];
     for (uint32_t i = threadIdx.x; i < a.a_rank_ld; i += SC_THREADS) lr[i] = a.proj[a.a1_off + i];
     for (uint32_t i = threadIdx.x; i < a.g_rank_ld; i += SC_THREADS) lr[a.a_rank_ld + i] = a.proj[a.g1_off + i];
     // the state ring has one column more than the taps look back, so this token's column is read by nobody
-    auto channel = [&](uint32_t ch, const float* w, float now, bool keep) {
-        float* st = a.conv_state + static_cast<size_t>(ch) * a.taps;
-        const float v = conv_silu(w, a.taps, now, [&](uint32_t j) { return st[(pos + a.taps - j) % a.taps]; });
-        if (keep) st[pos % a.taps] = now;
-        return v;
-    };
+#pragma unroll
+    for (uint32_t n = 0; n < ITEMS; ++n) {
+        const Channel c = channel(threadIdx.x + SC_THREADS * n);
+        if (!c.in) continue;
+        now[n] = a.proj[c.at];
+        if (four) ring[n] = *reinterpret_cast<const float4*>(a.conv_state + static_cast<size_t>(c.ring) * 4);
+    }
     float ss[2] = {0.f, 0.f};
-    for (uint32_t i = threadIdx.x; i < DP; i += SC_THREADS) {
-        float q = 0.f, k = 0.f;
-        if (i < a.dim) {
-            const uint32_t c = kvh * a.dim + i;
-            const bool keep = slice == 0 && h % rep == 0;
-            q = channel(c, a.q_conv + static_cast<size_t>(c) * a.taps, a.proj[a.q_off + c], keep);
-            k = channel(qk + c, a.k_conv + static_cast<size_t>(c) * a.taps, a.proj[a.k_off + c], keep);
-        }
-        qs[i] = q;
-        ks[i] = k;
-        ss[0] += q * q;
-        ss[1] += k * k;
-    }
-    if (threadIdx.x < SC_COLS) {
+#pragma unroll
+    for (uint32_t n = 0; n < ITEMS; ++n) {
+        const uint32_t i = threadIdx.x + SC_THREADS * n;
+        const Channel c = channel(i);
         float v = 0.f;
-        if (threadIdx.x < n_cols) {
-            const uint32_t c = h * a.vdim + col0 + threadIdx.x;
-            v = channel(2 * qk + c, a.v_conv + static_cast<size_t>(c) * a.taps, a.proj[a.v_off + c], true);
+        if (c.in) {
+            float* st = a.conv_state + static_cast<size_t>(c.ring) * a.taps;
+            v = four ? siluf(conv4(taps[n], ring[n], now[n], pos, 0.f)) : conv_silu(c.w, a.taps, now[n], [&](uint32_t j) { return st[(pos + a.taps - j) % a.taps]; });
+            if (c.keep) st[pos % a.taps] = now[n];
         }
-        vs[threadIdx.x] = v;
+        if (i < 2 * DP + SC_COLS) xs[i] = v;
+        if (i < 2 * DP) ss[i < DP ? 0 : 1] += v * v;
     }
-    block_sum(ss, red);                                             // (its barrier also publishes lr and vs)
+    block_sum(ss, red);                                             // (its barrier also publishes lr and xs)
+    float s[ROWS], sg[1];
+    low_rank_dots(wa, a.a_rank_ld, lr, fetch_a, s);
+    low_rank_dots(wg, a.g_rank_ld, lr + a.a_rank_ld, fetch_g, sg);
+    float mine = 0.f;
+#pragma unroll
+    for (uint32_t r = 0; r < ROWS; ++r) mine = lg == r ? s[r] : mine;
+    if (lg < ROWS) gs[row] = decays ? decay_of(a_log, mine + bias) : 0.f;
+    if (live && lg == 0) gate[h * a.vdim + col] = sg[0];
     const float iq = 1.0f / sqrtf(ss[0] + 1e-6f) / sqrtf(static_cast<float>(a.dim)), ik = 1.0f / sqrtf(ss[1] + 1e-6f);
-    for (uint32_t i = threadIdx.x; i < DP; i += SC_THREADS) {
-        qs[i] *= iq;
-        ks[i] *= ik;
-        gs[i] = i < a.dim ? decay_of(a.a_log[h], low_rank_dot(a.a2, static_cast<size_t>(h) * a.dim + i, a.a_rank_ld, lr) + a.dt_bias[h * a.dim + i]) : 0.f;
-    }
-    if (threadIdx.x < n_cols) {
-        const uint32_t c = h * a.vdim + col0 + threadIdx.x;
-        gate[c] = low_rank_dot(a.g2, c, a.g_rank_ld, lr + a.a_rank_ld);
-    }
+    for (uint32_t i = threadIdx.x; i < 2 * DP; i += SC_THREADS) xs[i] *= i < DP ? iq : ik;
     __syncthreads();
     DeltaOperands<RQ> t;
     t.g.load(gs + 2 * lg);
-    t.k.load(ks + 2 * lg);
-    t.q.load(qs + 2 * lg);
-    t.v = vs[col_s];
-    t.beta = sigmoidf(a.proj[a.b_off + h]);
+    t.k.load(xs + DP + 2 * lg);
+    t.q.load(xs + 2 * lg);
+    t.v = xs[2 * DP + col_s];
+    t.beta = sigmoidf(b);
     const float r = group_sum(delta_token<RQ>(S, t));
     if (live) {
         S.store(sp);
@@ -887,49 +940,73 @@ __global__ void __launch_bounds__(256) ssd_prep_kernel(const __grid_constant__ h
     }
 }
 
-// One token from the raw projection row: convolution, SiLU, step size and the state update.
+// One token from the raw projection row: convolution, SiLU, step size and the state update.  Bound by latency: with four taps rings,
+// weights and inputs of all channels are asked for at once, the weights before the wait (64 heads of 128 x 64: 4.7 -> 2.3 us a launch of many).
 template <int RQ>
-__global__ void __launch_bounds__(SC_THREADS) ssd_step_kernel(const __grid_constant__ hf2q_ssd a, float* __restrict__ y) {
-    constexpr uint32_t DP = 32 * RQ;
-    __shared__ __align__(16) float ks[DP], qs[DP], vs[SC_COLS];
+__global__ void __launch_bounds__(SC_THREADS, 2) ssd_step_kernel(const __grid_constant__ hf2q_ssd a, float* __restrict__ y) {
+    constexpr uint32_t DP = 32 * RQ, ITEMS = (2 * DP + SC_COLS + SC_THREADS - 1) / SC_THREADS;
+    __shared__ __align__(16) float xs[2 * DP + SC_COLS];            // k, q, v
     pdl_trigger();
     const uint32_t h = blockIdx.x, slice = blockIdx.y, rep = a.heads / a.groups, grp = h / rep;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = lane & 15;
-    const uint32_t col_s = warp * 2 + (lane >> 4), col0 = slice * SC_COLS, col = col0 + col_s;
-    const uint32_t n_cols = min(static_cast<uint32_t>(SC_COLS), a.vdim - col0);
-    const bool live = col < a.vdim;
+    const uint32_t lg = threadIdx.x & 15, col_s = threadIdx.x >> 4, col0 = slice * SC_COLS, col = col0 + col_s;
+    const uint32_t n_cols = min(static_cast<uint32_t>(SC_COLS), a.vdim - col0), channels = ssd_channels(a), inner = a.heads * a.vdim;
+    const bool live = col < a.vdim, first = slice == 0 && h % rep == 0;
+    struct Channel { uint32_t c; bool in, keep; };
+    auto channel = [&](uint32_t i) {
+        const uint32_t j = i < DP ? i : i < 2 * DP ? i - DP : i - 2 * DP;
+        if (i < 2 * DP) return Channel{inner + (i < DP ? grp : a.groups + grp) * a.state + j, j < a.state, first};
+        return Channel{h * a.vdim + col0 + j, j < n_cols, true};
+    };
+    const bool four = a.taps == 4 && ((reinterpret_cast<uintptr_t>(a.conv_state) | reinterpret_cast<uintptr_t>(a.conv)) & 15) == 0;
+    float4 taps[ITEMS], ring[ITEMS];
+    float now[ITEMS], bias[ITEMS];
+#pragma unroll
+    for (uint32_t n = 0; n < ITEMS; ++n) {
+        const Channel c = channel(threadIdx.x + SC_THREADS * n);
+        if (!c.in) continue;
+        bias[n] = a.conv_bias[c.c];
+        if (four) taps[n] = *reinterpret_cast<const float4*>(a.conv + static_cast<size_t>(c.c) * 4);
+    }
+    const float skip = a.d[h];
     pdl_wait();
     Vec<RQ> S;
     float* sp = a.s + (static_cast<size_t>(h) * a.vdim + (live ? col : 0)) * DP + 2 * lg;
     if (live) S.load(sp); else S.zero();
-    const uint32_t pos = *a.pos, channels = ssd_channels(a), inner = a.heads * a.vdim;
+    const uint32_t pos = *a.pos;
     const float* row = a.proj + a.off;
-    // the state ring has one column more than the taps look back, so this token's column is read by nobody
-    auto channel = [&](uint32_t c, bool keep) {
-        float* st = a.conv_state + static_cast<size_t>(c) * a.taps;
-        const float now = row[c];
-        const float v = conv_bias_silu(a.conv + static_cast<size_t>(c) * a.taps, a.conv_bias[c], a.taps, now, [&](uint32_t j) { return st[(pos + a.taps - j) % a.taps]; });
-        if (keep) st[pos % a.taps] = now;
-        return v;
-    };
-    const bool first = slice == 0 && h % rep == 0;
-    for (uint32_t i = threadIdx.x; i < 2 * DP; i += SC_THREADS) {
-        const uint32_t j = i % DP;
-        const float v = j < a.state ? channel(inner + (i < DP ? grp : a.groups + grp) * a.state + j, first) : 0.f;
-        (i < DP ? ks : qs)[j] = v;
-    }
-    if (threadIdx.x < SC_COLS) vs[threadIdx.x] = threadIdx.x < n_cols ? channel(h * a.vdim + col0 + threadIdx.x, true) : 0.f;
     float dt, la;
     ssd_gates(a, h, row[channels + h], dt, la);
+#pragma unroll
+    for (uint32_t n = 0; n < ITEMS; ++n) {
+        const Channel c = channel(threadIdx.x + SC_THREADS * n);
+        if (!c.in) continue;
+        now[n] = row[c.c];
+        if (four) ring[n] = *reinterpret_cast<const float4*>(a.conv_state + static_cast<size_t>(c.c) * 4);
+    }
+    // the state ring has one column more than the taps look back, so this token's column is read by nobody
+#pragma unroll
+    for (uint32_t n = 0; n < ITEMS; ++n) {
+        const uint32_t i = threadIdx.x + SC_THREADS * n;
+        const Channel c = channel(i);
+        float v = 0.f;
+        if (c.in) {
+            float* st = a.conv_state + static_cast<size_t>(c.c) * a.taps;
+            v = four ? siluf(conv4(taps[n], ring[n], now[n], pos, bias[n]))
+                     : conv_bias_silu(a.conv + static_cast<size_t>(c.c) * a.taps, bias[n], a.taps, now[n], [&](uint32_t j) { return st[(pos + a.taps - j) % a.taps]; });
+            if (c.keep) st[pos % a.taps] = now[n];
+        }
+        if (i < 2 * DP + SC_COLS) xs[i] = v;
+    }
     __syncthreads();
     Vec<RQ> k, q;
-    k.load(ks + 2 * lg);
-    q.load(qs + 2 * lg);
-    S.decay_axpy(expf(la), k, dt * vs[col_s]);
+    k.load(xs + 2 * lg);
+    q.load(xs + DP + 2 * lg);
+    const float v = xs[2 * DP + col_s];
+    S.decay_axpy(expf(la), k, dt * v);
     const float r = group_sum(S.dot(q));
     if (live) {
         S.store(sp);
-        if (lg == 0) y[h * a.vdim + col] = r + a.d[h] * vs[col_s];
+        if (lg == 0) y[h * a.vdim + col] = r + skip * v;
     }
 }
 
