@@ -73,11 +73,16 @@ __device__ __forceinline__ void matvec_rows(const __nv_bfloat16* __restrict__ w,
 
 struct MatvecSegs {
     hf2q_matvec s[2];
+    MatvecPlan plan[2];
+    uint32_t share[2];       // elements of the streams that a CTA stores
     uint32_t blocks0;        // CTAs of segment 0
 };
 
 // ---- row prologues with a row's 16-byte groups in registers, PRO_GROUPS per thread: constants are there before the wait for the
 // launch in front, and everything that it wrote is asked for at once.
+// Few instructions count as much, for they come cold: a prologue over four streams of 2048 took 3.5 us with an instruction per element
+// and 2.0 with one per two, a gated row of 4096 5.2 and 3.0 with its head sums by a warp each.  Rows of 32 outputs, all of it: 7.2 -> 4.4
+// us; 2048 outputs behind a gated row 10.5 -> 7.6.
 constexpr int PRO_GROUPS = 3;
 __device__ __forceinline__ float4 group4(const float* p, uint32_t i, bool in) { return p && in ? *reinterpret_cast<const float4*>(p + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ bool groups_fit(uint32_t width, uintptr_t pointers) { return width % 4 == 0 && width <= 4 * PRO_GROUPS * MR_THREADS && pointers % 16 == 0; }
@@ -149,62 +154,72 @@ struct NormRow {
     }
 };
 
+// up to four streams; two elements an instruction
 struct HyperRow {
-    static constexpr int S = 4, PARTS = 4;
+    static constexpr int S = 4;
     const hf2q_hyper& q;
     float4 norm[PRO_GROUPS];
     static __device__ __forceinline__ bool fits(const hf2q_hyper& q) {
-        return q.streams <= S && (!q.y || q.y_parts <= PARTS) && groups_fit(q.width, bits(q.x) | bits(q.x_out) | bits(q.y) | bits(q.norm) | bits(q.h_out));
+        return q.streams <= S && groups_fit(q.width, bits(q.x) | bits(q.x_out) | bits(q.y) | bits(q.norm) | bits(q.h_out));
     }
-    __device__ __forceinline__ HyperRow(const hf2q_hyper& p, float* coef) : q(p) {
+    __device__ __forceinline__ HyperRow(const hf2q_hyper& p, f2* coef) : q(p) {
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) norm[g] = group4(q.norm, threadIdx.x + MR_THREADS * g, 4 * (threadIdx.x + MR_THREADS * g) < q.width);
         hyper_coefficients<S>(q, coef);
     }
+    static __device__ __forceinline__ ulonglong2 pairs(const float* p, uint32_t i, bool in) { return in ? *reinterpret_cast<const ulonglong2*>(p + 4 * i) : make_ulonglong2(0, 0); }
+    static __device__ __forceinline__ void axpy2(ulonglong2& d, f2 a, const ulonglong2& x) { d.x = f2_fma(a, x.x, d.x); d.y = f2_fma(a, x.y, d.y); }
     // the row into xs, the new streams' elements [lo, hi) (multiples of four) and those of the row itself to memory
-    __device__ __forceinline__ void run(float* xs, const float* coef, float* red, uint32_t lo, uint32_t hi) const {
-        const float *mix = coef, *gain = coef + S * S, *in = gain + S;
-        float4 old[PRO_GROUPS][S], y[PRO_GROUPS][PARTS], u[PRO_GROUPS];
+    __device__ __forceinline__ void run(float* xs, const f2* coef, float* red, uint32_t lo, uint32_t hi) const {
+        const f2 *mix = coef, *gain = coef + S * S, *in = gain + S;
+        const uint32_t step = q.x_streams == 1 ? 0u : q.width;
+        ulonglong2 old[PRO_GROUPS][S], y[PRO_GROUPS], u[PRO_GROUPS];
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
+            if (4 * MR_THREADS * g >= q.width) break;
             const uint32_t i = threadIdx.x + MR_THREADS * g;
             const bool has = 4 * i < q.width;
 #pragma unroll
-            for (int s = 0; s < S; ++s) old[g][s] = group4(q.x + (q.x_streams == 1 ? 0u : s * q.width), i, has && s < static_cast<int>(q.streams));
-#pragma unroll
-            for (int k = 0; k < PARTS; ++k) y[g][k] = group4(q.y ? q.y + k * q.width : nullptr, i, has && k < static_cast<int>(q.y_parts));
+            for (int s = 0; s < S; ++s) old[g][s] = pairs(q.x + s * step, i, has && s < static_cast<int>(q.streams));
+            y[g] = pairs(q.y, i, has && q.y);
         }
+        for (uint32_t k = 1; q.y && k < q.y_parts; ++k)
+#pragma unroll
+            for (int g = 0; g < PRO_GROUPS; ++g) {
+                const uint32_t i = threadIdx.x + MR_THREADS * g;
+                if (4 * i < q.width) axpy2(y[g], f2_both(1.0f), pairs(q.y + k * q.width, i, true));
+            }
         float s1[1] = {0.f};
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
+            if (4 * MR_THREADS * g >= q.width) break;
             const uint32_t e = 4 * (threadIdx.x + MR_THREADS * g);
-            if (4 * MR_THREADS * g >= q.width) continue;
-            float4 yv = make_float4(0.f, 0.f, 0.f, 0.f);
-            u[g] = yv;
-#pragma unroll
-            for (int k = 0; k < PARTS; ++k) axpy(yv, 1.0f, y[g][k]);
+            const bool own = q.x_out && e >= lo && e < hi;
+            u[g] = make_ulonglong2(0, 0);
 #pragma unroll
             for (int d = 0; d < S; ++d) {
-                if (d >= static_cast<int>(q.streams)) continue;
-                float4 v = old[g][d];
+                if (d >= static_cast<int>(q.streams)) break;
+                ulonglong2 v = old[g][d];
                 if (q.y) {
-                    v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    v = make_ulonglong2(0, 0);
 #pragma unroll
-                    for (int s = 0; s < S; ++s) axpy(v, mix[s * S + d], old[g][s]);
-                    axpy(v, gain[d], yv);
+                    for (int s = 0; s < S; ++s) axpy2(v, mix[s * S + d], old[g][s]);
+                    axpy2(v, gain[d], y[g]);
                 }
-                if (q.x_out && e >= lo && e < hi && e < q.width) *reinterpret_cast<float4*>(q.x_out + static_cast<size_t>(d) * q.width + e) = v;
-                axpy(u[g], in[d], v);
+                if (own) *reinterpret_cast<ulonglong2*>(q.x_out + static_cast<size_t>(d) * q.width + e) = v;
+                axpy2(u[g], in[d], v);
             }
-            s1[0] += square_sum(u[g]);
+            const float2 a = f2_parts(u[g].x), b = f2_parts(u[g].y);
+            s1[0] += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
         }
         block_sum(s1, red);
         const float inv = 1.0f / sqrtf(s1[0] / static_cast<float>(q.width) + q.eps);
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
             const uint32_t e = 4 * (threadIdx.x + MR_THREADS * g);
-            if (e >= q.width) continue;
-            const float4 h = q.norm ? make_float4(u[g].x * inv * norm[g].x, u[g].y * inv * norm[g].y, u[g].z * inv * norm[g].z, u[g].w * inv * norm[g].w) : u[g];
+            if (e >= q.width) break;
+            const float2 a = f2_parts(u[g].x), b = f2_parts(u[g].y);
+            const float4 h = q.norm ? make_float4(a.x * inv * norm[g].x, a.y * inv * norm[g].y, b.x * inv * norm[g].z, b.y * inv * norm[g].w) : make_float4(a.x, a.y, b.x, b.y);
             *reinterpret_cast<float4*>(xs + e) = h;
             if (q.h_out && e >= lo && e < hi) *reinterpret_cast<float4*>(q.h_out + e) = h;
         }
@@ -215,20 +230,24 @@ struct HyperRow {
 struct GatedRow {
     const hf2q_gated_heads& q;
     const bool silu;
+    const uint32_t width, spans, inv;            // of a row; of a head; x / spans = x * inv >> 16
     float4 norm[PRO_GROUPS];
     static __device__ __forceinline__ bool fits(const hf2q_gated_heads& q) {
         return q.head_dim % 128 == 0 && groups_fit(q.heads * q.head_dim, bits(q.o) | bits(q.gate) | bits(q.norm));
     }
-    __device__ __forceinline__ explicit GatedRow(const hf2q_gated_heads& p) : q(p), silu(p.kind == HF2Q_GATE_SILU_FIRST) {
+    __device__ __forceinline__ explicit GatedRow(const hf2q_gated_heads& p)
+        : q(p), silu(p.kind == HF2Q_GATE_SILU_FIRST), width(p.heads * p.head_dim), spans(p.head_dim / 128), inv((65535 + spans) / spans) {
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
             const uint32_t i = threadIdx.x + MR_THREADS * g;
-            norm[g] = group4(q.norm, silu || q.norm_all ? i : i % (q.head_dim / 4), 4 * i < q.heads * q.head_dim);
+            norm[g] = group4(q.norm, silu || q.norm_all ? i : i - first_span(g) * 32, 4 * i < width);
         }
     }
+    __device__ __forceinline__ uint32_t first_span(int g) const { return (((threadIdx.x + MR_THREADS * g) / 32 * inv) >> 16) * spans; }      // of the head
+    __device__ __forceinline__ float gate_of(float x) const { return (silu ? x : 1.0f) / (1.0f + expf(-x)); }      // siluf, sigmoidf
     // the row into xs.  sums: a float per span
     __device__ __forceinline__ void run(float* xs, float* sums) const {
-        const uint32_t width = q.heads * q.head_dim, spans = q.head_dim / 128;
+        const uint32_t lane = threadIdx.x & 31;
         float4 v[PRO_GROUPS], x[PRO_GROUPS];
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
@@ -237,24 +256,25 @@ struct GatedRow {
         }
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
-            if (silu) v[g] = make_float4(v[g].x * siluf(x[g].x), v[g].y * siluf(x[g].y), v[g].z * siluf(x[g].z), v[g].w * siluf(x[g].w));
-            const float s = q.norm ? warp_sum(square_sum(v[g])) : 0.f;
-            if (threadIdx.x % 32 == 0) sums[(threadIdx.x + MR_THREADS * g) / 32] = s;
+            if (4 * MR_THREADS * g >= width) break;
+            x[g] = make_float4(gate_of(x[g].x), gate_of(x[g].y), gate_of(x[g].z), gate_of(x[g].w));
+            if (silu) v[g] = make_float4(v[g].x * x[g].x, v[g].y * x[g].y, v[g].z * x[g].z, v[g].w * x[g].w);
+            const float s = warp_sum(square_sum(v[g]));
+            if (lane == 0) sums[(threadIdx.x + MR_THREADS * g) / 32] = s;
         }
-        if (q.norm) __syncthreads();
+        __syncthreads();
 #pragma unroll
         for (int g = 0; g < PRO_GROUPS; ++g) {
-            const uint32_t i = threadIdx.x + MR_THREADS * g;
-            if (4 * i >= width) continue;
+            const uint32_t i = threadIdx.x + MR_THREADS * g, first = first_span(g);
+            if (4 * i >= width) break;                                      // (whole warps)
             float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
             if (q.norm) {
-                float s = 0.f;
-                for (uint32_t k = 0, first = i / 32 / spans * spans; k < spans; ++k) s += sums[first + k];
-                const float inv = 1.0f / sqrtf(s / static_cast<float>(q.head_dim) + q.eps);
-                w = make_float4(norm[g].x * inv, norm[g].y * inv, norm[g].z * inv, norm[g].w * inv);
+                const float s = warp_sum((lane < spans ? sums[first + lane] : 0.f) + (lane + 32 < spans ? sums[first + lane + 32] : 0.f));
+                const float r = 1.0f / sqrtf(s / static_cast<float>(q.head_dim) + q.eps);
+                w = make_float4(norm[g].x * r, norm[g].y * r, norm[g].z * r, norm[g].w * r);
             }
             float4 h = make_float4(v[g].x * w.x, v[g].y * w.y, v[g].z * w.z, v[g].w * w.w);
-            if (!silu) h = make_float4(h.x * sigmoidf(x[g].x), h.y * sigmoidf(x[g].y), h.z * sigmoidf(x[g].z), h.w * sigmoidf(x[g].w));
+            if (!silu) h = make_float4(h.x * x[g].x, h.y * x[g].y, h.z * x[g].z, h.w * x[g].w);
             *reinterpret_cast<float4*>(xs + 4 * i) = h;
         }
     }
@@ -269,20 +289,18 @@ __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __gri
     pdl_trigger();
     const bool second = blockIdx.x >= p.blocks0;
     const hf2q_matvec& s = p.s[second];
-    const uint32_t blk = blockIdx.x - (second ? p.blocks0 : 0u), n_blk = second ? gridDim.x - p.blocks0 : p.blocks0;
+    const MatvecPlan& plan = p.plan[second];
+    const uint32_t blk = blockIdx.x - (second ? p.blocks0 : 0u);
     const uint32_t warp = threadIdx.x >> 5;
     float* xs = reinterpret_cast<float*>(mv_smem + MR_RING);
-    // rows [row0, row1) of this CTA, spread evenly
     constexpr uint32_t unit = PAIRS ? 2 : 1;
-    const uint32_t units = s.n / unit;
-    const uint32_t row0 = unit * static_cast<uint32_t>(static_cast<uint64_t>(units) * blk / n_blk), row1 = unit * static_cast<uint32_t>(static_cast<uint64_t>(units) * (blk + 1) / n_blk);
-    const uint32_t piece = mv_piece(s.k), per_row = (s.k + piece - 1) / piece;
+    const uint32_t row0 = unit * plan.first(blk), row1 = row0 + unit * plan.count(blk), piece = plan.piece;
     const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(s.w) + static_cast<size_t>(row0) * s.k;
     auto at = [&](uint32_t row, uint32_t col) {
         const uint32_t k0 = col * piece;
         return MatvecChunk{w + static_cast<size_t>(row) * s.k + k0, k0, min(piece, s.k - k0)};
     };
-    MatvecStream stream(mv_smem, sh, row1 - row0, per_row, status);
+    MatvecStream stream(mv_smem, sh, row1 - row0, plan, status);
     stream.start(at);
     // what the first pass of the epilogue adds to this thread's row (or pair)
     const uint32_t mine = row0 + threadIdx.x * unit;
@@ -331,15 +349,15 @@ __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __gri
         }
     } else if constexpr (PRO == HF2Q_PRO_HYPER) {
         const hf2q_hyper& q = s.hyper;
-        __shared__ float coef[HYPER_COEF];
+        __shared__ __align__(8) float coef[HYPER_COEF];
         // every CTA makes the whole row and stores its share of the new streams
-        const uint32_t lo = static_cast<uint32_t>(static_cast<uint64_t>(q.width) * blk / n_blk) & ~3u;
-        const uint32_t hi = blk + 1 == n_blk ? q.width : static_cast<uint32_t>(static_cast<uint64_t>(q.width) * (blk + 1) / n_blk) & ~3u;
+        const uint32_t lo = min(p.share[second] * blk, q.width), hi = min(lo + p.share[second], q.width);
         if (HyperRow::fits(q)) {
-            const HyperRow row(q, coef);
+            f2* pairs = reinterpret_cast<f2*>(coef);
+            const HyperRow row(q, pairs);
             pdl_wait();
             add_residual();
-            row.run(xs, coef, red, lo, hi);
+            row.run(xs, pairs, red, lo, hi);
             for (uint32_t i = q.width + threadIdx.x; i < s.k; i += MR_THREADS) xs[i] = 0.f;
         } else {
             pdl_wait();
@@ -870,6 +888,11 @@ HF2Q_API int32_t hf2q_cuda_dense_matvec(hf2q_ctx* ctx, void* stream, uint32_t pr
     auto ctas = [&](uint32_t i, uint64_t want) { return static_cast<uint32_t>(want < 1 ? 1 : want > segs[i].n ? segs[i].n : want); };
     uint32_t blocks = p.blocks0 = ctas(0, n_segs == 1 ? sms : (sms * chunks[0] + total / 2) / total);
     if (n_segs == 2) blocks += ctas(1, sms > p.blocks0 ? sms - p.blocks0 : 1);
+    for (uint32_t i = 0; i < n_segs; ++i) {
+        const uint32_t mine = i ? blocks - p.blocks0 : p.blocks0;
+        p.plan[i] = matvec_plan(segs[i].n, epi_pairs(segs[i].epilogue) ? 2 : 1, mine, segs[i].k);
+        p.share[i] = ((segs[i].hyper.width + 3) / 4 + mine - 1) / mine * 4;
+    }
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t smem = MR_RING + static_cast<size_t>(kmax) * 4;
     uint32_t* status = ctx_status_word(ctx);

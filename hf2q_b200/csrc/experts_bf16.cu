@@ -35,7 +35,7 @@ __device__ __forceinline__ void choose_experts(const float* logits, uint32_t exp
 
 constexpr uint32_t STEP_EXPERTS = 1024, STEP_TOP = 64;
 
-__global__ void __launch_bounds__(MR_THREADS, 1) expert_glu_kernel(const __grid_constant__ hf2q_expert_step e, uint32_t* status) {
+__global__ void __launch_bounds__(MR_THREADS, 1) expert_glu_kernel(const __grid_constant__ hf2q_expert_step e, const __grid_constant__ MatvecPlan plan, uint32_t* status) {
     extern __shared__ __align__(128) uint8_t mv_smem[];                 // ring, then h [k_in] f32
     __shared__ MatvecShared sh;
     __shared__ float z[STEP_EXPERTS], scores[STEP_TOP];
@@ -43,16 +43,14 @@ __global__ void __launch_bounds__(MR_THREADS, 1) expert_glu_kernel(const __grid_
     pdl_trigger();
     pdl_wait();
     choose_experts(e.logits, e.experts, e.top, z, ids, scores);
-    // pairs of rows of all chosen experts, spread evenly
-    const uint32_t pairs = e.top * e.ff, piece = mv_piece(e.k_in), per_row = (e.k_in + piece - 1) / piece;
-    const uint32_t row0 = 2 * static_cast<uint32_t>(static_cast<uint64_t>(pairs) * blockIdx.x / gridDim.x);
-    const uint32_t row1 = 2 * static_cast<uint32_t>(static_cast<uint64_t>(pairs) * (blockIdx.x + 1) / gridDim.x);
+    // pairs of rows of all chosen experts
+    const uint32_t row0 = 2 * plan.first(blockIdx.x), row1 = row0 + 2 * plan.count(blockIdx.x), piece = plan.piece;
     auto at = [&](uint32_t r, uint32_t col) {
         const uint32_t row = row0 + r, k0 = col * piece, slot = row / (2 * e.ff);
         const size_t w_row = static_cast<size_t>(ids[slot]) * 2 * e.ff + row % (2 * e.ff);
         return MatvecChunk{static_cast<const __nv_bfloat16*>(e.gate_up) + w_row * e.k_in + k0, k0, min(piece, e.k_in - k0)};
     };
-    MatvecStream stream(mv_smem, sh, row1 - row0, per_row, status);
+    MatvecStream stream(mv_smem, sh, row1 - row0, plan, status);
     stream.start(at);
     float* xs = reinterpret_cast<float*>(mv_smem + MR_RING);
     for (uint32_t i = threadIdx.x; i < e.k_in; i += MR_THREADS) xs[i] = e.h[i];
@@ -66,7 +64,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) expert_glu_kernel(const __grid_
     });
 }
 
-__global__ void __launch_bounds__(MR_THREADS, 1) expert_down_kernel(const __grid_constant__ hf2q_expert_step e, uint32_t* status) {
+__global__ void __launch_bounds__(MR_THREADS, 1) expert_down_kernel(const __grid_constant__ hf2q_expert_step e, const __grid_constant__ MatvecPlan plan, uint32_t* status) {
     extern __shared__ __align__(128) uint8_t mv_smem[];                 // ring, then act [top][ff] f32
     __shared__ MatvecShared sh;
     __shared__ uint32_t ids[STEP_TOP];
@@ -74,15 +72,13 @@ __global__ void __launch_bounds__(MR_THREADS, 1) expert_down_kernel(const __grid
     pdl_wait();
     for (uint32_t i = threadIdx.x; i < e.top; i += MR_THREADS) ids[i] = e.ids[i];
     __syncthreads();
-    const uint32_t piece = mv_piece(e.ff), per_slot = (e.ff + piece - 1) / piece, per_row = e.top * per_slot;
-    const uint32_t row0 = static_cast<uint32_t>(static_cast<uint64_t>(e.width) * blockIdx.x / gridDim.x);
-    const uint32_t row1 = static_cast<uint32_t>(static_cast<uint64_t>(e.width) * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t piece = plan.piece, per_slot = plan.per_row / e.top, row0 = plan.first(blockIdx.x), row1 = row0 + plan.count(blockIdx.x);
     auto at = [&](uint32_t r, uint32_t col) {                           // a row's pieces: expert after expert
         const uint32_t slot = col / per_slot, k0 = (col - slot * per_slot) * piece;
         const size_t w_row = static_cast<size_t>(ids[slot]) * e.width + row0 + r;
         return MatvecChunk{static_cast<const __nv_bfloat16*>(e.down) + w_row * e.ff + k0, slot * e.ff + k0, min(piece, e.ff - k0)};
     };
-    MatvecStream stream(mv_smem, sh, row1 - row0, per_row, status);
+    MatvecStream stream(mv_smem, sh, row1 - row0, plan, status);
     stream.start(at);
     float* xs = reinterpret_cast<float*>(mv_smem + MR_RING);
     for (uint32_t i = threadIdx.x; i < e.top * e.ff; i += MR_THREADS) xs[i] = e.act[i];
@@ -136,10 +132,10 @@ HF2Q_API int32_t hf2q_cuda_expert_glu_step(hf2q_ctx* ctx, void* stream, const hf
     if (!step_ok(e)) return ctx_fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "expert_glu_step: null or unaligned pointer, or a size outside the limits");
     static PerDeviceFlag flag;
     cudaError_t r = ensure_max_dynamic_smem(expert_glu_kernel, MR_RING + STEP_X, flag);
-    const uint32_t sms = static_cast<uint32_t>(ctx_sm_count(ctx)), pairs = e->top * e->ff;
+    const uint32_t sms = static_cast<uint32_t>(ctx_sm_count(ctx)), pairs = e->top * e->ff, ctas = pairs < sms ? pairs : sms;
     if (r == cudaSuccess)
-        r = launch_pdl(expert_glu_kernel, dim3(pairs < sms ? pairs : sms), dim3(MR_THREADS), MR_RING + static_cast<size_t>(e->k_in) * 4,
-                       static_cast<cudaStream_t>(stream), *e, ctx_status_word(ctx));
+        r = launch_pdl(expert_glu_kernel, dim3(ctas), dim3(MR_THREADS), MR_RING + static_cast<size_t>(e->k_in) * 4, static_cast<cudaStream_t>(stream), *e,
+                       matvec_plan(2 * pairs, 2, ctas, e->k_in), ctx_status_word(ctx));
     return ctx_cuda_result(ctx, r, "expert_glu_step", 1);
 }
 
@@ -148,10 +144,10 @@ HF2Q_API int32_t hf2q_cuda_expert_down_step(hf2q_ctx* ctx, void* stream, const h
     if (!step_ok(e)) return ctx_fail(ctx, HF2Q_ERR_INVALID_ARGUMENT, "expert_down_step: null or unaligned pointer, or a size outside the limits");
     static PerDeviceFlag flag;
     cudaError_t r = ensure_max_dynamic_smem(expert_down_kernel, MR_RING + STEP_X, flag);
-    const uint32_t sms = static_cast<uint32_t>(ctx_sm_count(ctx));
+    const uint32_t sms = static_cast<uint32_t>(ctx_sm_count(ctx)), ctas = e->width < sms ? e->width : sms;
     if (r == cudaSuccess)
-        r = launch_pdl(expert_down_kernel, dim3(e->width < sms ? e->width : sms), dim3(MR_THREADS), MR_RING + 4ull * e->top * e->ff,
-                       static_cast<cudaStream_t>(stream), *e, ctx_status_word(ctx));
+        r = launch_pdl(expert_down_kernel, dim3(ctas), dim3(MR_THREADS), MR_RING + 4ull * e->top * e->ff, static_cast<cudaStream_t>(stream), *e,
+                       matvec_plan(e->width, 1, ctas, e->ff, e->top), ctx_status_word(ctx));
     return ctx_cuda_result(ctx, r, "expert_down_step", 1);
 }
 

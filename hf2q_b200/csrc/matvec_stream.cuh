@@ -12,7 +12,7 @@ namespace seq {
 // a prologue's loads at once (16 warps, 25 MB: 9.4 us a product without, 7.6 with).  In a chain of up (norm prologue) and down
 // products, us a product at 2048 x 6144 / 4096 x 11264 / 3072 x 9216 / 1536 x 4096: 12 warps of 3 stages 6.6 / 16.5 / 11.9 / 5.4, of 2
 // 6.8 / 17.3 / 12.3 / 5.3, 16 of 3 7.3 / 16.9 / 12.9 / 5.6, 8 of 3 with chunks of 1536 7.5 / 17.3 / 11.3 / 5.3; two CTAs an SM 9.3 and
-// more.  Before: 9.9 / 24.7 / 17.3 / 6.7.
+// more.  Before: 9.9 / 24.7 / 17.3 / 6.7.  (With the plan below 6.4 / 16.4 / - / 5.0.)
 constexpr int MR_WARPS = 12, MR_THREADS = MR_WARPS * 32, MR_STAGES = 3, MV_CHUNK = 1024, MR_PART = 2048;
 constexpr uint32_t MR_RING = MR_WARPS * MR_STAGES * MV_CHUNK * 2;      // bytes of dynamic shared memory
 constexpr uint32_t MR_MAX_X = 112 * 1024;                              // bytes of activations
@@ -20,10 +20,24 @@ constexpr uint32_t MR_MAX_X = 112 * 1024;                              // bytes 
 // A row of k weights is cut into pieces of this many elements: a divisor of the warps to a row, so that each warp keeps to one place
 // of the rows and holds that place's activations in registers.  Longer rows: pieces of MV_CHUNK, activations from shared memory at
 // every step (16 bytes of weights meet 32 of activations there).
-__host__ __device__ constexpr uint32_t mv_piece(uint32_t k) {
+constexpr uint32_t mv_piece(uint32_t k) {
     for (uint32_t n = 1; n <= MR_WARPS; ++n)
         if (MR_WARPS % n == 0 && k <= n * MV_CHUNK) return (k + 8 * n - 1) / (8 * n) * 8;
     return MV_CHUNK;
+}
+// Who does what, worked out on the host: a kernel's first instructions come cold, and its divisions were 0.5 us of every launch.
+struct MatvecPlan {
+    uint32_t rows, extra;        // rows (or pairs) of a CTA; the first `extra` CTAs have one more
+    uint32_t piece, per_row;     // elements of a piece, pieces of a row
+    uint32_t inv;                // x / per_row = x * inv >> 16 for x <= MR_WARPS
+    uint32_t block_rows;         // rows whose sums meet at a time
+    __device__ __forceinline__ uint32_t first(uint32_t cta) const { return rows * cta + min(cta, extra); }
+    __device__ __forceinline__ uint32_t count(uint32_t cta) const { return rows + (cta < extra ? 1u : 0u); }
+};
+// rows of k weights, side of them to one sum; unit 2: in pairs
+inline MatvecPlan matvec_plan(uint32_t rows, uint32_t unit, uint32_t ctas, uint32_t k, uint32_t side = 1) {
+    const uint32_t piece = mv_piece(k), per_row = side * ((k + piece - 1) / piece), block = MR_PART / per_row / unit * unit;
+    return {rows / unit / ctas, rows / unit % ctas, piece, per_row, (65536 + per_row - 1) / per_row, block ? block : unit};
 }
 
 struct MatvecShared {
@@ -40,14 +54,13 @@ struct MatvecChunk {
 // issuing lane's, activations in registers.
 class MatvecStream {
 public:
-    // rows of per_row pieces each
-    __device__ __forceinline__ MatvecStream(uint8_t* smem, MatvecShared& sh, uint32_t rows, uint32_t per_row, uint32_t* status)
-        : sh_(sh), rows_(rows), per_row_(per_row), status_(status), warp_(threadIdx.x >> 5), lane_(threadIdx.x & 31),
+    __device__ __forceinline__ MatvecStream(uint8_t* smem, MatvecShared& sh, uint32_t rows, const MatvecPlan& plan, uint32_t* status)
+        : sh_(sh), rows_(rows), per_row_(plan.per_row), block_rows_(plan.block_rows), status_(status), warp_(threadIdx.x >> 5), lane_(threadIdx.x & 31),
           ring_(reinterpret_cast<__nv_bfloat16*>(smem) + static_cast<size_t>(warp_) * MR_STAGES * MV_CHUNK) {
-        down_ = MR_WARPS / per_row;
-        right_ = MR_WARPS - down_ * per_row;
-        now_.row = next_.row = warp_ / per_row;
-        now_.col = next_.col = warp_ - now_.row * per_row;
+        down_ = MR_WARPS * plan.inv >> 16;
+        right_ = MR_WARPS - down_ * per_row_;
+        now_.row = next_.row = warp_ * plan.inv >> 16;
+        now_.col = next_.col = warp_ - now_.row * per_row_;
     }
 
     // fills the ring; at(row, col) -> MatvecChunk
@@ -75,7 +88,6 @@ private:
     static constexpr int U = MV_CHUNK / 256;                               // 16-byte groups of a chunk per lane
     template <bool PAIRS, bool HELD, class F, class G> __device__ __forceinline__ void run_as(F at, const float* xs, G finish) {
         constexpr uint32_t unit = PAIRS ? 2 : 1;
-        const uint32_t block_rows = max(unit, MR_PART / per_row_ / unit * unit);
         float held[HELD ? U : 1][8];
         uint32_t len = 0;
         if constexpr (HELD) {
@@ -88,8 +100,8 @@ private:
         }
         bool ok = true;
         uint32_t st = 0, ph = 0;                                            // ring slot and parity
-        for (uint32_t r0 = 0, pb = 0; r0 < rows_; r0 += block_rows, pb ^= 1) {
-            const uint32_t nr = min(block_rows, rows_ - r0);
+        for (uint32_t r0 = 0, pb = 0; r0 < rows_; r0 += block_rows_, pb ^= 1) {
+            const uint32_t nr = min(block_rows_, rows_ - r0);
             for (; now_.row < r0 + nr; advance(now_)) {
                 const float* x = xs;
                 if constexpr (!HELD) {
@@ -146,7 +158,7 @@ private:
         advance(next_);
     }
     MatvecShared& sh_;
-    const uint32_t rows_, per_row_;
+    const uint32_t rows_, per_row_, block_rows_;
     uint32_t* const status_;
     const uint32_t warp_, lane_;
     __nv_bfloat16* const ring_;

@@ -284,8 +284,10 @@ __device__ __forceinline__ float hyper_elements(const hf2q_hyper& p, uint32_t t,
     return ss;
 }
 // [S][S] mix, [S] out, [S] in; absent streams have zeros.  The whole block takes part and meets at the end.
-template <int S>
-__device__ __forceinline__ void hyper_coefficients(const hf2q_hyper& p, float* coef) {
+__device__ __forceinline__ void store_coefficient(float* c, float v) { *c = v; }
+__device__ __forceinline__ void store_coefficient(f2* c, float v) { *c = f2_both(v); }
+template <int S, typename C>
+__device__ __forceinline__ void hyper_coefficients(const hf2q_hyper& p, C* coef) {
     for (uint32_t i = threadIdx.x; i < S * S + 2 * S; i += blockDim.x) {
         const uint32_t a = i / S, b = i % S;
         float v = 0.f;
@@ -294,7 +296,7 @@ __device__ __forceinline__ void hyper_coefficients(const hf2q_hyper& p, float* c
             else if (a == S) v = p.y ? p.out[b] : 0.f;
             else v = p.in ? p.in[b] : 1.0f;
         }
-        coef[i] = v;
+        store_coefficient(coef + i, v);
     }
     __syncthreads();
 }
