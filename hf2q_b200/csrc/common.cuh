@@ -249,6 +249,8 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32
 }
 // Programmatic dependent launch.  Every kernel launched with launch_pdl() calls pdl_wait() before it touches
 // memory that an earlier kernel of the stream writes (or still reads); weights and other parameters may be touched before.
+// What an earlier kernel writes comes through pointers without __restrict__ and without __ldg: the compiler may move loads of memory
+// that it takes for read-only in front of the wait (it did, in the launches of a latent-attention step).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... KArgs, typename... Args>

@@ -323,11 +323,11 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_decode_kernel(const float
 //     merge order: bit-reproducible).
 // qkv: one fused QKV row, f32 [(n_q + 2 n_kv) * 128]; the query part is NOT modified.
 template <int G, typename OUT>
-__global__ void __launch_bounds__(ATT_WARPS * 32, 2) attn_decode_fused_kernel(const float* __restrict__ qkv, uint32_t n_q, uint32_t n_kv,
+__global__ void __launch_bounds__(ATT_WARPS * 32, 2) attn_decode_fused_kernel(const float* qkv, uint32_t n_q, uint32_t n_kv,
                                                                            float theta, float q_scale,
                                                                            int8_t* __restrict__ k_codes, float* __restrict__ k_scale,
                                                                            int8_t* __restrict__ v_codes, float* __restrict__ v_scale,
-                                                                           uint32_t max_seq, const uint32_t* __restrict__ pos_dev,
+                                                                           uint32_t max_seq, const uint32_t* pos_dev,
                                                                            float* __restrict__ part, uint32_t* __restrict__ counters,
                                                                            OUT* __restrict__ out, uint32_t* status) {
     __shared__ __align__(16) float qs[G][ATT_HD];

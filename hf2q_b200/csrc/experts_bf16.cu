@@ -7,8 +7,8 @@ namespace {
 using namespace seq;
 
 // sorted row order <- rows of x, 16 bytes per thread and step
-__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ x, uint32_t quads, uint32_t top, const uint32_t* __restrict__ header,
-                                                          const uint32_t* __restrict__ perm, uint4* __restrict__ xg) {
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* x, uint32_t quads, uint32_t top, const uint32_t* header,
+                                                          const uint32_t* perm, uint4* __restrict__ xg) {
     pdl_trigger();
     pdl_wait();
     const uint32_t n = header[1];

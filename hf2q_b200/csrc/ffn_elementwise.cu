@@ -35,9 +35,9 @@ __global__ void __launch_bounds__(256) silu_mul_tail_kernel(const float* gate, c
 __device__ __forceinline__ void add_scaled(float& a, float w, float v) { a += w * v; }
 __device__ __forceinline__ void add_scaled(float4& a, float w, const float4& v) { a.x += w * v.x; a.y += w * v.y; a.z += w * v.z; a.w += w * v.w; }
 template <typename V>
-__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, const float* __restrict__ w,
-                                                          const float* __restrict__ shared, const float* __restrict__ gate_logit,
-                                                          const float* __restrict__ residual, float* __restrict__ out,
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* y, const float* w,
+                                                          const float* shared, const float* gate_logit,
+                                                          const float* residual, float* __restrict__ out,
                                                           uint32_t top_k, uint32_t h) {
     constexpr uint32_t E = sizeof(V) / 4, AHEAD = 8;
     pdl_trigger();
@@ -99,7 +99,7 @@ __device__ __forceinline__ float load1(const void* p, uint32_t bf16, size_t i) {
 
 // VEC: h is a multiple of 4, and x and w allow loads of four elements.
 template <bool VEC>
-__global__ void __launch_bounds__(RV_THREADS) router_vector_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
+__global__ void __launch_bounds__(RV_THREADS) router_vector_kernel(const void* x, uint32_t x_bf16, const float* w,
                                                                    float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
     __shared__ float part[RV_TOKENS][RV_THREADS / 32];
     const uint32_t e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -163,7 +163,7 @@ constexpr int RT = 64, RKT = 32, RT_MAX_PARTS = 8;
 constexpr size_t router_smem(int R) { return 4 * (2 * RKT * RT * R > RT * R * RT * R ? 2 * RKT * RT * R : RT * R * RT * R); }
 
 template <bool VEC, int R>
-__global__ void __launch_bounds__(256, 2) router_tile_kernel(const void* __restrict__ x, uint32_t x_bf16, const float* __restrict__ w,
+__global__ void __launch_bounds__(256, 2) router_tile_kernel(const void* x, uint32_t x_bf16, const float* w,
                                                              float* __restrict__ out, uint32_t n_tokens, uint32_t n_experts, uint32_t h) {
     constexpr int TILE = RT * R;
     extern __shared__ __align__(16) float rsm[];

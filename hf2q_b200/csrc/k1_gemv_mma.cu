@@ -1153,8 +1153,8 @@ cudaError_t launch_mma_tt(MParams p, uint32_t slots, const Plan& pl, const Devic
 }
 
 // Adds the split-k parts: y[i] = sum over parts of scratch[part][i] (+ residual[i]), parts in index order.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ scratch, uint32_t parts, uint64_t count,
-                                                            const float* __restrict__ residual, float* __restrict__ y) {
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* scratch, uint32_t parts, uint64_t count,
+                                                            const float* residual, float* __restrict__ y) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");                    // the parts are the previous kernel's output
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
@@ -1248,7 +1248,7 @@ namespace {
 // (a product whose contraction dimension is sharded): this is the all-reduce of a column-sharded projection,
 // built from the all-gather in the producing product's epilogue and a local sum.
 __global__ void __launch_bounds__(256) gather_sum_kernel(const uint32_t* flag, uint32_t n_ranks, uint32_t rank, long long limit, uint32_t* status,
-                                                         const float* __restrict__ parts, uint32_t stride, uint32_t n_parts, float* __restrict__ x,
+                                                         const float* parts, uint32_t stride, uint32_t n_parts, float* __restrict__ x,
                                                          uint32_t n) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next kernel may start its own prologue
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1264,7 +1264,7 @@ __global__ void __launch_bounds__(256) gather_sum_kernel(const uint32_t* flag, u
 // gathered rows of the most recent product leave the group's buffer in one launch (the sharded host-buffer batch
 // copies them out behind the kernels).
 __global__ void __launch_bounds__(256) gather_take_kernel(const uint32_t* flag, uint32_t n_ranks, uint32_t rank, long long limit, uint32_t* status,
-                                                          const float* __restrict__ src, uint32_t pitch, uint32_t width, uint32_t m,
+                                                          const float* src, uint32_t pitch, uint32_t width, uint32_t m,
                                                           float* __restrict__ dst, uint32_t vec4) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next kernel may start its own prologue
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1299,7 +1299,7 @@ struct GatherCopyParams {
     uint32_t peer_ctas[8];
     uint32_t n_ranks, rank, col0, n;
 };
-__global__ void __launch_bounds__(256) gather_copy_kernel(const float* __restrict__ src, const GatherCopyParams p) {
+__global__ void __launch_bounds__(256) gather_copy_kernel(const float* src, const GatherCopyParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next kernel may start its own prologue
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (uint32_t i = blockIdx.x * GCOPY_PER_CTA + threadIdx.x; i < min((blockIdx.x + 1) * GCOPY_PER_CTA, p.n); i += 256) {

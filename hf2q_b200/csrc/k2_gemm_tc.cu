@@ -445,13 +445,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 // ---------------------------------------------------------------- activations -> f16 panel
 __device__ __forceinline__ void load8_f32(const void* x, uint32_t x_bf16, uint64_t at, float (&v)[8]) {
     if (x_bf16) {
-        const uint4 r = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(x) + at));
+        const uint4 r = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(x) + at);
         const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) { v[2 * j] = __uint_as_float(rr[j] << 16); v[2 * j + 1] = __uint_as_float(rr[j] & 0xffff0000u); }
     } else {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x) + at));
-        const float4 b = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x) + at + 4));
+        const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(x) + at);
+        const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(x) + at + 4);
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
 }
@@ -469,7 +469,7 @@ __device__ __forceinline__ bool store8_f16(__half* out, const float (&v)[8]) {  
 // Bound by memory: 16-byte loads and stores (rows are whole K-blocks, so the count divides by 8), four groups in flight per
 // thread; `wide` is false where x itself starts off a 16-byte boundary.  2048 x (3 x 4096 + 14336) bf16: 46 us in all, one
 // element at a time took 110.
-__global__ void __launch_bounds__(256) x_to_f16_kernel(const void* __restrict__ x, uint32_t x_bf16, __half* __restrict__ out,
+__global__ void __launch_bounds__(256) x_to_f16_kernel(const void* x, uint32_t x_bf16, __half* __restrict__ out,
                                                        uint64_t n_elems, bool wide, uint32_t* status) {
     pdl_trigger();
     pdl_wait();
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(256) x_to_f16_kernel(const void* __restrict__ 
 // The same conversion for activations stored [n_heads][m][head_dim] (the layout flash attention writes; the
 // reference's O projection reads it through quantized_matmul_mm_tensor_perm021, forward_prefill_batched.rs:2218-2258):
 // logical (t, c) is physical (h = c / head_dim, t, f = c % head_dim).  8 elements per thread.
-__global__ void __launch_bounds__(256) x_perm021_to_f16_kernel(const void* __restrict__ x, uint32_t x_bf16, __half* __restrict__ out,
+__global__ void __launch_bounds__(256) x_perm021_to_f16_kernel(const void* x, uint32_t x_bf16, __half* __restrict__ out,
                                                                uint32_t m, uint32_t k, uint32_t head_dim, uint32_t* status) {
     pdl_trigger();
     pdl_wait();

@@ -27,19 +27,19 @@ constexpr unsigned SORT_CTAS = 8;
 // of all counts.  Shared memory: 4 arrays of (E+1) u32 + 66 words of scan scratch.
 // The ids are read 16 per thread and step with all loads in flight (the kernel is one CTA deep in load latency
 // otherwise), the two scans over the experts are block-wide shuffle scans.
-__device__ __forceinline__ void load_ids16(const uint32_t* __restrict__ ids, uint32_t r0, uint32_t rows, bool vec, uint32_t (&e)[16]) {
+__device__ __forceinline__ void load_ids16(const uint32_t* ids, uint32_t r0, uint32_t rows, bool vec, uint32_t (&e)[16]) {
     if (vec && r0 + 16 <= rows) {
         const uint4* p = reinterpret_cast<const uint4*>(ids + r0);
-        const uint4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+        const uint4 a = p[0], b = p[1], c = p[2], d = p[3];
         e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w; e[4] = b.x; e[5] = b.y; e[6] = b.z; e[7] = b.w;
         e[8] = c.x; e[9] = c.y; e[10] = c.z; e[11] = c.w; e[12] = d.x; e[13] = d.y; e[14] = d.z; e[15] = d.w;
     } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) e[j] = r0 + j < rows ? __ldg(ids + r0 + j) : 0xffffffffu;
+        for (int j = 0; j < 16; ++j) e[j] = r0 + j < rows ? ids[r0 + j] : 0xffffffffu;
     }
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* __restrict__ ids, uint32_t rows, uint32_t n_experts,
+__global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* ids, uint32_t rows, uint32_t n_experts,
                                                                 uint32_t nt, uint32_t* __restrict__ header, uint4* __restrict__ tiles,
                                                                 uint32_t* __restrict__ perm, float* __restrict__ y, float* __restrict__ y2,
                                                                 uint32_t n, uint32_t* status) {
@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* 
 // then activations are all on their way at once; one row after the other was bound by two loads' latency a row (16384 rows of
 // 2048: 20.5 -> 15.6 us, 76 MB with the tokens read once).
 constexpr int GATHER_ROWS = 4;
-__global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict__ x, uint32_t x_bf16, uint32_t top_k, uint32_t k,
-                                                         const uint32_t* __restrict__ header, const uint32_t* __restrict__ perm,
+__global__ void __launch_bounds__(256) moe_gather_kernel(const void* x, uint32_t x_bf16, uint32_t top_k, uint32_t k,
+                                                         const uint32_t* header, const uint32_t* perm,
                                                          __half* __restrict__ xg, uint32_t* status) {
     pdl_trigger();
     pdl_wait();
@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict_
             for (int i = 0; i < GATHER_ROWS; ++i) {
                 const size_t at = static_cast<size_t>(tok[i]) * k + e;
                 const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(x) + at * (x_bf16 ? 2 : 4));
-                raw[i][0] = __ldg(src);
-                if (!x_bf16) raw[i][1] = __ldg(src + 1);
+                raw[i][0] = src[0];
+                if (!x_bf16) raw[i][1] = src[1];
             }
 #pragma unroll
             for (int i = 0; i < GATHER_ROWS; ++i) {

@@ -16,7 +16,7 @@ namespace {
 constexpr int WARPS = 4;
 
 template <bool SIGMOID>
-__global__ void __launch_bounds__(WARPS * 32) topk_kernel(const float* __restrict__ logits, uint32_t ld,
+__global__ void __launch_bounds__(WARPS * 32) topk_kernel(const float* logits, uint32_t ld,
                                                                   uint32_t* __restrict__ ids,
                                                                   float* __restrict__ weights,
                                                                   uint32_t n_tokens, uint32_t n_experts,
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(WARPS * 32) topk_kernel(const float* __restric
 // A key is the order of the above: 0 taken or absent, 1 a NaN, from 2 on the bits of a probability (none is negative).  One token
 // in the launch: 5.0 -> 3.0 us, 2048 tokens 7.4 -> 4.6.
 template <bool SIGMOID, int NV>
-__global__ void __launch_bounds__(WARPS * 32) topk_small_kernel(const float* __restrict__ logits, uint32_t ld, uint32_t* __restrict__ ids,
+__global__ void __launch_bounds__(WARPS * 32) topk_small_kernel(const float* logits, uint32_t ld, uint32_t* __restrict__ ids,
                                                                 float* __restrict__ weights, uint32_t n_tokens, uint32_t n_experts, uint32_t top_k) {
     pdl_trigger();
     pdl_wait();

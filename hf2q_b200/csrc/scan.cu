@@ -368,8 +368,8 @@ __device__ __forceinline__ float delta_token(Vec<RQ>& S, const DeltaOperands<RQ>
 }
 
 template <int RQ, int C, int W, uint32_t TB, int PER_SM>
-__global__ void __launch_bounds__((W + 1) * 32, PER_SM) delta_scan_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, const float* __restrict__ qkv,
-                                                                  const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ out) {
+__global__ void __launch_bounds__((W + 1) * 32, PER_SM) delta_scan_kernel(const __grid_constant__ hf2q_delta a, uint32_t m, const float* qkv,
+                                                                  const float* beta, const float* g, float* __restrict__ out) {
     using Place = ScanPlace<RQ, C, W>;
     constexpr uint32_t DP = Place::DP;
     extern __shared__ __align__(16) float dsm[];                    // k, q, g: [2][TB][DP] each
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(const __grid_constant__
     for (uint32_t c = threadIdx.x; c < a.g_rank_ld; c += 256) g1[static_cast<size_t>(t) * a.g_rank_ld + c] = from_f32<LR>(row[a.g1_off + c]);
 }
 
-__global__ void __launch_bounds__(256) delta_decay_kernel(const float* __restrict__ a_log, const float* __restrict__ dt_bias, uint32_t dim, uint32_t per_token,
+__global__ void __launch_bounds__(256) delta_decay_kernel(const float* a_log, const float* dt_bias, uint32_t dim, uint32_t per_token,
                                                           uint64_t n, float* __restrict__ g) {
     pdl_trigger();
     pdl_wait();
@@ -796,8 +796,8 @@ __device__ __forceinline__ uint32_t ssd_channels(const hf2q_ssd& a) { return a.h
 
 // S <- keep S + dt B x^T;  y = S^T C + d x
 template <int RQ, int C, int W, uint32_t TB>
-__global__ void __launch_bounds__((W + 1) * 32, TB == SC_TB ? 1 : RQ <= 4 ? 4 : 2) ssd_scan_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, const float* __restrict__ xbc,
-                                                                const float* __restrict__ dt, const float* __restrict__ la, float* __restrict__ y) {
+__global__ void __launch_bounds__((W + 1) * 32, TB == SC_TB ? 1 : RQ <= 4 ? 4 : 2) ssd_scan_kernel(const __grid_constant__ hf2q_ssd a, uint32_t m, const float* xbc,
+                                                                const float* dt, const float* la, float* __restrict__ y) {
     using Place = ScanPlace<RQ, C, W>;
     constexpr uint32_t DP = Place::DP;
     extern __shared__ __align__(16) float dsm[];                    // B, C: [2][TB][DP] each

@@ -9,7 +9,7 @@ namespace hf2q {
 namespace {
 using namespace seq;
 
-__global__ void __launch_bounds__(256) embed_kernel(const __grid_constant__ hf2q_embed e, const uint32_t* __restrict__ ids, uint32_t m,
+__global__ void __launch_bounds__(256) embed_kernel(const __grid_constant__ hf2q_embed e, const uint32_t* ids, uint32_t m,
                                                     float* __restrict__ x, uint32_t* status) {
     pdl_trigger();
     pdl_wait();
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256) gated_heads_kernel(const __grid_constant_
     else gated_heads_row<OUT>(g, t, row, threadIdx.x >> 5, blockDim.x >> 5);
 }
 
-__global__ void __launch_bounds__(256) state_tail_kernel(const uint32_t* __restrict__ pos_dev, uint32_t m, const float* __restrict__ h_last,
+__global__ void __launch_bounds__(256) state_tail_kernel(const uint32_t* pos_dev, uint32_t m, const float* h_last,
                                                          float* __restrict__ shift_state, uint32_t width, const __grid_constant__ hf2q_delta d,
                                                          uint32_t channels) {
     pdl_trigger();

@@ -506,8 +506,8 @@ __device__ __forceinline__ void f32_query(const hf2q_window_attn& a, uint32_t po
         for (uint32_t i = a.heads * a.vdim + lane; i < ldo; i += 32) out[static_cast<size_t>(t) * ldo + i] = from_f32<OUT>(0.f);
 }
 template <typename T, typename OUT, int NC, bool PLAIN>
-__global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m, const T* __restrict__ q,
-                                                                 const float* __restrict__ gate, uint32_t ldg, OUT* __restrict__ out, uint32_t ldo) {
+__global__ void __launch_bounds__(256) window_prefill_f32_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m, const T* q,
+                                                                 const float* gate, uint32_t ldg, OUT* __restrict__ out, uint32_t ldo) {
     __shared__ __align__(16) float qs[8][QK_MAX];
     __shared__ float ps[8][32];
     pdl_trigger();
@@ -552,7 +552,7 @@ __device__ __noinline__ void wt_again(const hf2q_window_attn& a, uint32_t pos0, 
 
 template <int DK, typename OUT, bool PLAIN>
 __global__ void __launch_bounds__(WT_THREADS, DK <= 128 ? 2 : 1) window_prefill_tc_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m,
-                                                                                          const __nv_bfloat16* __restrict__ q, const float* __restrict__ gate,
+                                                                                          const __nv_bfloat16* q, const float* gate,
                                                                                           uint32_t ldg, OUT* __restrict__ out, uint32_t ldo, uint32_t* status) {
     extern __shared__ __align__(16) uint8_t wt_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -834,7 +834,7 @@ constexpr int WP_WARPS = 4, WP_Q = 16 * WP_WARPS, WP_K = 64;
 // query sees.
 template <int DK, int DV, typename OUT, bool PLAIN>
 __global__ void __launch_bounds__(WP_WARPS * 32) window_prefill_mma_kernel(const __grid_constant__ hf2q_window_attn a, uint32_t m,
-                                                                           const __nv_bfloat16* __restrict__ q, const float* __restrict__ gate, uint32_t ldg,
+                                                                           const __nv_bfloat16* q, const float* gate, uint32_t ldg,
                                                                            OUT* __restrict__ out, uint32_t ldo) {
     constexpr uint32_t KP = DK + 8, VP = DV + 8, K_TILE = WP_K * KP, TILES = K_TILE + WP_K * VP;      // pitches and sizes in elements
     extern __shared__ __align__(16) __nv_bfloat16 kv[];             // [2][K tile, V tile]
