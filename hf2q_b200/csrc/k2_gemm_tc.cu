@@ -104,6 +104,7 @@ struct GParams {
     float* reduce_out;
     uint32_t top_k;
     uint32_t tiles_per_cta; // weight-row tiles (of 128 rows) one CTA walks, re-using its barriers, TMEM and token tile
+    uint32_t sms;              // dense launches: SMs of the device (0: the grid may be of any size)
     uint32_t boxw;          // bytes per weight row in one raw stage
     uint32_t blk_bytes;     // bytes of one 256-element K-block of a row
     uint32_t* status;
@@ -538,17 +539,24 @@ EncodeTiledFn encode_fn() {
 
 uint32_t boxw_of(uint32_t type) { return tc_boxw(type); }
 
+constexpr size_t ALONE_SMEM = 116 * 1024;                 // more than half of an SM's
 template <uint32_t TYPE, int NT, bool GROUPED, bool DUAL, bool SHARED>
 cudaError_t launch_gemm_form(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx, const GParams& p, uint32_t grid_y, cudaStream_t st,
                              uint32_t parts) {
     auto kern = gemm_tc_kernel<TYPE, NT, GROUPED, DUAL, SHARED>;
     const size_t raw_stages = raw_stages_of(TYPE, NT, GROUPED);
-    const size_t smem = 1024 + static_cast<size_t>(x_stages_of(TYPE, NT, GROUPED, SHARED && DUAL)) * NT * 128 + raw_stages * TILE_N * p.boxw + 512;
+    size_t smem = 1024 + static_cast<size_t>(x_stages_of(TYPE, NT, GROUPED, SHARED && DUAL)) * NT * 128 + raw_stages * TILE_N * p.boxw + 512;
     static PerDeviceFlag attr;
     if (const cudaError_t e = ensure_max_dynamic_smem(kern, 227 * 1024, attr); e != cudaSuccess) return e;
     const uint32_t tile_rows = DUAL ? 64 : TILE_N;
     const uint32_t row_tiles = (p.n + tile_rows - 1) / tile_rows;
     const dim3 grid((row_tiles + p.tiles_per_cta - 1) / p.tiles_per_cta, grid_y, parts);
+    // No more CTAs than SMs: one to an SM.  A launch that starts early finds a few SMs free, and two to each of these were slower than
+    // waiting for the others (3072 x 8192 in Q4_K and its pair, us
+    // together: 200 rows 86 launched late, 95 early, 80 early and alone; 300 rows 108, 117 and 101).
+    // (Clusters: three quarters, for one does not span the chip's groups of SMs.)
+    const uint64_t ctas = static_cast<uint64_t>(grid.x) * grid.y * parts;
+    if (ctas <= (parts > 1 ? p.sms / 4 * 3 : p.sms) && smem < ALONE_SMEM) smem = ALONE_SMEM;
     if constexpr (SHARED) return launch_pdl_cluster(kern, grid, dim3(GEMM_THREADS), dim3(1, 1, parts), smem, st, tw, tw2, tx, p);
     else return launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, tw, tw2, tx, p);
 }
@@ -657,6 +665,7 @@ cudaError_t gemm_tc_dense(uint32_t type, const void* w, const void* w_up, const 
     p.residual = residual;
     p.act16 = static_cast<__half*>(act16);
     p.tiles_per_cta = 1;
+    p.sms = static_cast<uint32_t>(sm_count);
     p.boxw = boxw_of(type);
     p.blk_bytes = KB / g.elems * g.bytes;
     p.status = status;
