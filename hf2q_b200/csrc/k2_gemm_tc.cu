@@ -177,9 +177,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // The next launch may start its own prologue.  What earlier launches wrote or still read -- activations, tile table,
-    // outputs -- is touched behind pdl_wait() only; weights do not change.
-    pdl_trigger();
+    // What earlier launches wrote or still read -- activations, tile table, outputs -- is touched behind pdl_wait() only; weights
+    // do not change.
     if constexpr (GROUPED) pdl_wait();
     // this CTA's weight-row tiles: [tile0, tile0 + ntile)
     const uint32_t n_row_tiles = (p.n + TILE_ROWS - 1) / TILE_ROWS;
@@ -207,6 +206,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();                                     // (dependents claim tensor memory too and keep it while they wait: not before this CTA has its own)
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_d = tmem_base;                 // columns [0, NT)
     const uint32_t tmem_a = tmem_base + (A_BUFS == 1 ? 128 : 256);     // A_BUFS buffers of 128 columns
