@@ -29,7 +29,7 @@
 // of them) and add their accumulators through distributed shared memory in rank order.
 //
 // Launched early (launch_pdl): barriers, tensor memory and the first weight stages are ready when the launch in front ends
-// (gate, up and down of 2560 x 9728 in Q8_0 at 37 rows, three launches: 64 -> 57 us).
+// (gate, up and down of 2560 x 9728 in Q8_0 at 37 rows, three launches: 64 -> 56 us).
 //
 // TMEM: 512 columns = D (<= 256) + 2 x 128 (two A buffers of one K-block each).
 // Every mbarrier wait is bounded; a wait that gives up sets the status word and all roles drain to
@@ -214,33 +214,35 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     if (warp == DEQ_WARPS) {
         // ------------------------------ TMA producer: lane 0 streams the weight stages, lane 1 the activation stages
         // (two independent rings: a full activation ring must not hold back the next weight stage)
-        if (lane == 0) {
-            bool ok = true;
-            for (uint32_t tl = 0, gk = 0; tl < ntile && ok; ++tl) {           // gk: K-block count over all tiles
-                const uint32_t row0 = (tile0 + tl) * TILE_ROWS;
-                for (uint32_t kb = 0; kb < nkb && ok; ++kb, ++gk) {
-                    const uint32_t rs = gk % RAW_STAGES;
-                    if (gk == RAW_STAGES) pdl_wait();
-                    if (gk >= RAW_STAGES) ok = mbar_wait_bounded(&raw_empty[rs], ((gk / RAW_STAGES) - 1) & 1, p.status);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(&raw_full[rs], raw_stage);
-                    const uint32_t byte0 = ((kb0 + kb) * p.blk_bytes) & ~15u;       // 16-byte aligned start of the box
-                    if constexpr (GROUPED)
-                        tma_3d(raw + rs * raw_stage, &tmap_w, static_cast<int>(byte0 >> 1), static_cast<int>(row0), static_cast<int>(expert), &raw_full[rs]);
-                    else
-                        tma_2d(raw + rs * raw_stage, &tmap_w, static_cast<int>(byte0 >> 1), static_cast<int>(row0), &raw_full[rs]);
-                    if constexpr (DUAL) {                                   // the up rows: second half of the stage (both boxes hold 64 rows)
-                        uint8_t* dst2 = raw + rs * raw_stage + 64 * p.boxw;
-                        if constexpr (GROUPED)
-                            tma_3d(dst2, &tmap_w2, static_cast<int>(byte0 >> 1), static_cast<int>(row0), static_cast<int>(expert), &raw_full[rs]);
-                        else
-                            tma_2d(dst2, &tmap_w2, static_cast<int>(byte0 >> 1), static_cast<int>(row0), &raw_full[rs]);
-                    }
-                }
+        uint32_t gk = 0, tl = 0, kb = 0;                       // K-blocks asked for over all tiles; the next one's place
+        auto next_raw = [&] {
+            const uint32_t rs = gk % RAW_STAGES, row0 = (tile0 + tl) * TILE_ROWS;
+            mbar_arrive_expect_tx(&raw_full[rs], raw_stage);
+            const uint32_t byte0 = ((kb0 + kb) * p.blk_bytes) & ~15u;       // 16-byte aligned start of the box
+            if constexpr (GROUPED)
+                tma_3d(raw + rs * raw_stage, &tmap_w, static_cast<int>(byte0 >> 1), static_cast<int>(row0), static_cast<int>(expert), &raw_full[rs]);
+            else
+                tma_2d(raw + rs * raw_stage, &tmap_w, static_cast<int>(byte0 >> 1), static_cast<int>(row0), &raw_full[rs]);
+            if constexpr (DUAL) {                                   // the up rows: second half of the stage (both boxes hold 64 rows)
+                uint8_t* dst2 = raw + rs * raw_stage + 64 * p.boxw;
+                if constexpr (GROUPED)
+                    tma_3d(dst2, &tmap_w2, static_cast<int>(byte0 >> 1), static_cast<int>(row0), static_cast<int>(expert), &raw_full[rs]);
+                else
+                    tma_2d(dst2, &tmap_w2, static_cast<int>(byte0 >> 1), static_cast<int>(row0), &raw_full[rs]);
             }
+            ++gk;
+            if (++kb == nkb) { kb = 0; ++tl; }
+        };
+        // A warp stands while one of its lanes is in pdl_wait(): the first stages are asked for before any of them is.
+        if (lane == 0)
+            while (gk < RAW_STAGES && tl < ntile) next_raw();
+        __syncwarp();
+        pdl_wait();
+        if (lane == 0) {
+            for (; tl < ntile; next_raw())
+                if (!mbar_wait_bounded(&raw_empty[gk % RAW_STAGES], ((gk / RAW_STAGES) - 1) & 1, p.status)) break;
         } else if (lane == 1) {
             bool ok = true;
-            pdl_wait();
             const uint32_t nx = ntile * nkb * (KB / XK);
             for (uint32_t xi = 0; xi < nx && ok; ++xi) {
                 const uint32_t st = xi % X_STAGES, kx = kb0 * (KB / XK) + xi % (nkb * (KB / XK));      // K position inside the current tile
@@ -302,8 +304,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             const uint32_t row0 = (tile0 + tl) * TILE_ROWS;
             for (uint32_t kb = 0; kb < nkb; ++kb, ++gk) {
                 const uint32_t rs = gk % RAW_STAGES, ab = gk % A_BUFS;
+                // (from here on the bounded waits measure this kernel only: stages up to here were asked for ahead of the producer's wait)
+                static_assert(A_BUFS <= RAW_STAGES, "");
+                if (gk == A_BUFS) pdl_wait();
                 if (ok) ok = mbar_wait_bounded(&raw_full[rs], (gk / RAW_STAGES) & 1, p.status);
-                if (gk == A_BUFS) pdl_wait();                          // (from here on the bounded waits measure this kernel only)
                 if (ok && gk >= A_BUFS) ok = mbar_wait_bounded(&a_empty[ab * DEQ_GROUPS + grp], ((gk / A_BUFS) - 1) & 1, p.status);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
