@@ -479,7 +479,7 @@ constexpr uint32_t QK_MAX = 320;                        // dim and shared_dim to
 // ---------------------------------------------------------------- prefill, f32: one warp per (query, head)
 // query t of head h by one warp; qs [QK_MAX] and ps [32] of this warp in shared memory
 template <typename T, typename OUT, int NC, bool PLAIN>
-__device__ __forceinline__ void f32_query(const hf2q_window_attn& a, uint32_t pos0, uint32_t t, uint32_t h, const T* __restrict__ q, const float* __restrict__ gate,
+__device__ __forceinline__ void f32_query(const hf2q_window_attn& a, uint32_t pos0, uint32_t t, uint32_t h, const T* q, const float* gate,
                                           uint32_t ldg, OUT* __restrict__ out, uint32_t ldo, float* qs, float* ps) {
     const uint32_t lane = threadIdx.x & 31;
     const KeyRows<T, PLAIN> kv(a, h / (a.heads / a.kv_heads), pos0);

@@ -1,7 +1,9 @@
 """Rules of the kernels that start under the launch in front of them, read off their source:
 
 - one that claims tensor memory lets the next launch start only when it has its own.  That launch may claim tensor memory as well and
-  keeps it until this one has ended, and an allocation waits without a limit."""
+  keeps it until this one has ended, and an allocation waits without a limit;
+- what an earlier launch writes does not come through ``const ... __restrict__`` pointers: the compiler may move such loads in
+  front of the wait."""
 import re
 from pathlib import Path
 
@@ -58,3 +60,17 @@ def test_tensor_memory_is_claimed_before_the_next_launch_may_start(file, name):
     body = next(b for f, _, n, _, b in ALL if (f, n) == (file, name))
     owned = body.index("__syncthreads()", body.index("tmem_alloc("))
     assert all(m.start() > owned for m in TRIGGER.finditer(body))
+
+
+@pytest.mark.parametrize("file,name", EARLY)
+def test_what_earlier_launches_write_is_not_taken_for_read_only(file, name):
+    todo, seen = [name], set()
+    while todo:
+        n = todo.pop()
+        for f, _, fn, params, body in ALL:
+            if fn != n or (f, fn, params) in seen or not (f == file or f.endswith(".cuh")):
+                continue
+            seen.add((f, fn, params))
+            for p in re.findall(r"const[^,*]*\*\s*__restrict__\s*(\w+)", params):
+                assert p in ("w", "b"), f"{fn}: {p}"                        # weights, blocks of them
+            todo += set(re.findall(r"\b([a-z_]\w*)\s*(?:<[^;{}()]*>)?\s*\(", body))
