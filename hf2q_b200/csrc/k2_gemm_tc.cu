@@ -557,10 +557,18 @@ cudaError_t launch_gemm_form(const CUtensorMap& tw, const CUtensorMap& tw2, cons
     const dim3 grid((row_tiles + p.tiles_per_cta - 1) / p.tiles_per_cta, grid_y, parts);
     // No more CTAs than SMs: one to an SM.  A launch that starts early finds a few SMs free, and two to each of these were slower than
     // waiting for the others (3072 x 8192 in Q4_K and its pair, us
-    // together: 200 rows 86 launched late, 95 early, 80 early and alone; 300 rows 108, 117 and 101).
-    // (Clusters: three quarters, for one does not span the chip's groups of SMs.)
+    // together: 200 rows 86 launched late, 95 early, 80 early and alone; 300 rows 108, 117 and 101).  Clusters: no more than run side by
+    // side with one CTA to an SM (pair and down product of 4096 x 14336, 128 CTAs in clusters of four, two to an SM and alone: Q4_K 9 rows
+    // 65.5 and 57.8 us, 64 rows 71.0 and 65.3, 128 rows 124 and 111; Q6_K 9 rows 94.4 and 84.3).
     const uint64_t ctas = static_cast<uint64_t>(grid.x) * grid.y * parts;
-    if (ctas <= (parts > 1 ? p.sms / 4 * 3 : p.sms) && smem < ALONE_SMEM) smem = ALONE_SMEM;
+    if (ctas <= p.sms && smem < ALONE_SMEM) {
+        bool fit = true;
+        if constexpr (SHARED) {
+            static PerDeviceClusters side;
+            fit = ctas <= static_cast<uint64_t>(parts) * clusters_side_by_side(kern, dim3(GEMM_THREADS), parts, ALONE_SMEM, side);
+        }
+        if (fit) smem = ALONE_SMEM;
+    }
     if constexpr (SHARED) return launch_pdl_cluster(kern, grid, dim3(GEMM_THREADS), dim3(1, 1, parts), smem, st, tw, tw2, tx, p);
     else return launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, tw, tw2, tx, p);
 }

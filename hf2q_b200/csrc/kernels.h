@@ -37,6 +37,34 @@ inline cudaError_t ensure_max_dynamic_smem(Kernel kern, int bytes, PerDeviceFlag
     }
     return cudaSuccess;
 }
+// Clusters of `size` CTAs, laid along z, that run side by side: a cluster does not span the device's groups of SMs, which differ in
+// size.  Asked for once per device and size; `counts` belongs to one kernel, block and smem.  0 where the device does not say.
+struct PerDeviceClusters {
+    std::mutex mu;
+    int n[MAX_DEVICES][9] = {};                          // 0: not asked for yet, -1: none
+};
+template <typename Kernel>
+inline uint32_t clusters_side_by_side(Kernel kern, dim3 block, uint32_t size, size_t smem, PerDeviceClusters& counts) {
+    int dev = 0;
+    if (size > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 0;
+    std::lock_guard<std::mutex> lock(counts.mu);
+    int& n = counts.n[dev][size];
+    if (n == 0) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(1, 1, size);
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = size;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
+        if (n <= 0) n = -1;
+    }
+    return n > 0 ? static_cast<uint32_t>(n) : 0u;
+}
 
 // K0 (k0_dequant.cu)
 cudaError_t launch_dequant(uint32_t type, const void* w, void* out, uint32_t out_dtype,
