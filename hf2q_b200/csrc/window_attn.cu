@@ -1004,22 +1004,36 @@ uint32_t decode_gr(const hf2q_window_attn& a) {
     return rep >= 5 ? 8 : rep >= 3 ? 4 : rep;
 }
 uint32_t decode_groups(const hf2q_window_attn& a) { const uint32_t gr = decode_gr(a); return (a.heads / a.kv_heads + gr - 1) / gr; }
+// Splits of a window.  A CTA has an SM to itself and takes WD_PASS keys a pass, so the CTAs of all splits are one wave: eight splits a
+// group of heads, whatever the number of groups, ran in several (bf16 heads of 128, us at 256 / 2048 keys of a window of 2048,
+// eight splits and now: 32 heads of keys and values 15.0 / 23.5 and 5.5 / 13.6, 64 24.7 / 39.4 and 6.1 / 20.4, 128 45.4 / 71.1 and
+// 6.5 / 32.1; 4 shared by 16 heads 8.8 / 12.1 as before).
+// Merged through memory: whole passes, for with twice the CTAs and half a pass each a second wave waits with idle warps (window 16384, us at
+// 256 / 8192 / 16384 keys, before and now: 16 heads of keys and values 16.2 / 35.6 / 55.2 and 7.9 / 22.7 / 35.2, 8 shared by 32
+// 23.2 / 30.2 / 44.8 and 13.3 / 24.2 / 36.6, 4 by 16 26.4 / 29.3 / 34.2 and 16.0 / 19.3 / 26.5; 1 by 8 32.8 / 35.2 / 37.7 as before).
 uint32_t decode_splits(const hf2q_window_attn& a, int sms) {
-    const uint32_t ctas = a.kv_heads * decode_groups(a), by_sm = (2 * sms + ctas - 1) / ctas, by_keys = (a.window + 127) / 128;
+    const uint32_t ctas = a.kv_heads * decode_groups(a), by_sm = static_cast<uint32_t>(sms) / ctas, by_keys = (a.window + WD_PASS - 1) / WD_PASS;
     const uint32_t s = by_sm < by_keys ? by_sm : by_keys;
     return s < 1 ? 1 : s > 64 ? 64 : s;
 }
 size_t counter_bytes(const hf2q_window_attn& a) { return (static_cast<size_t>(a.kv_heads) * decode_groups(a) * 4 + 255) & ~static_cast<size_t>(255); }
 
-// Splits of a window as one cluster, 0 for more of them than a cluster has: up to four passes of a CTA.
-uint32_t cluster_splits(const hf2q_window_attn& a) {
-    const uint32_t s = (a.window + WD_PASS - 1) / WD_PASS;
-    return s <= WD_CLUSTER ? s : s <= 4 * WD_CLUSTER ? WD_CLUSTER : 0;
+// Splits as one cluster, 0 for windows of more than four passes for each of eight: up to there the cluster, which adds through shared
+// memory, is ahead at short fills and at most level at full ones with as many CTAs again that merge through memory (us at 256 / 8192 keys of
+// a window of 8192: 1 head of keys and values shared by 8 13.4 / 50.6, 16 splits through memory 19.0 / 34.3; 4 by 16 8.9 / 30.9 and 11.7 / 22.1;
+// 10 heads 5.4 / 19.0 and 9.0 / 20.4).  One wave: clusters do not span the chip's groups of SMs, and with one CTA an SM those of more
+// than four leave up to a quarter of it unused, smaller ones an eighth (16 heads, window 2048, 256 keys: clusters of 6 5.3 us, of 7 9.7).
+uint32_t cluster_splits(const hf2q_window_attn& a, int sms) {
+    const uint32_t ctas = a.kv_heads * decode_groups(a), n = static_cast<uint32_t>(sms), by_keys = (a.window + WD_PASS - 1) / WD_PASS;
+    if (by_keys > 4 * WD_CLUSTER) return 0;
+    uint32_t s = by_keys < WD_CLUSTER ? by_keys : WD_CLUSTER;
+    while (s > 1 && ctas * s > (s > 4 ? n * 3 / 4 : n * 7 / 8)) --s;
+    return s;
 }
 template <typename T, int GR, int NC>
 cudaError_t launch_decode(const hf2q_window_attn& a, float* out, uint8_t* scratch, int sms, cudaStream_t st) {
     const size_t smem = (static_cast<size_t>(GR) * pad8(a.dim) + WD_WARPS * GR * (2 + WD_KEYS + pad8(a.vdim)) + GR * wd_part(a.vdim)) * sizeof(float);
-    const uint32_t groups = decode_groups(a), cluster = cluster_splits(a);
+    const uint32_t groups = decode_groups(a), cluster = cluster_splits(a, sms);
     uint32_t* counters = reinterpret_cast<uint32_t*>(scratch);
     float* part = reinterpret_cast<float*>(scratch + counter_bytes(a));
     if (cluster) {
