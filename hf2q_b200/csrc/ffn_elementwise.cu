@@ -32,6 +32,9 @@ __global__ void __launch_bounds__(256) silu_mul_tail_kernel(const float* gate, c
 // out[t, :] = sum_s w[t*k+s] * y[t*k+s, :]  (+ sigmoid(gate_logit[t]) * shared[t, :])  (+ residual[t, :])
 // V: float, or float4 where rows are whole 16-byte groups.  Bound by memory: eight rows are asked for before they are added, in
 // slot order, as the reference sums (2048 tokens, 8 rows of 2048 each: 151 MB, 30 -> 28 us).
+// The next launch starts when this one ends: under it a following layer's router got SMs as they fell free, two CTAs to one (layers
+// one behind the other, us with and without: 8 experts of 2048 x 2048, two a token, 200 tokens 69.8 and 62.4; 128 of 768, eight a token,
+// 128 tokens 208 and 201; 256 of 512, 512 tokens 290 and 281).
 __device__ __forceinline__ void add_scaled(float& a, float w, float v) { a += w * v; }
 __device__ __forceinline__ void add_scaled(float4& a, float w, const float4& v) { a.x += w * v.x; a.y += w * v.y; a.z += w * v.z; a.w += w * v.w; }
 template <typename V>
@@ -40,7 +43,6 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* y, const 
                                                           const float* residual, float* __restrict__ out,
                                                           uint32_t top_k, uint32_t h) {
     constexpr uint32_t E = sizeof(V) / 4, AHEAD = 8;
-    pdl_trigger();
     pdl_wait();
     const uint32_t t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x, n = h / E;
     if (c >= n) return;
