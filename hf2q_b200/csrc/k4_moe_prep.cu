@@ -24,7 +24,8 @@ constexpr unsigned SORT_CTAS = 8;
 
 // Histogram, exclusive scans, scatter, by one CTA or by a cluster whose CTAs count and place a share of the rows each: bound by the
 // shared-memory atomics, 16384 of them (16384 rows, 256 experts: 14.2 us by one CTA, 7.0 by eight).  Every CTA scans the sums
-// of all counts.  Shared memory: 4 arrays of (E+1) u32 + 66 words of scan scratch.
+// of all counts.  Shared memory: [E] counts, [E + 1] first rows, [E + 1] first tiles, [E] places, and 68 words of the scans (32 + 32 warp
+// totals, 2 running totals, 2 of the block).
 // The ids are read 16 per thread and step with all loads in flight (the kernel is one CTA deep in load latency
 // otherwise), the two scans over the experts are block-wide shuffle scans.
 __device__ __forceinline__ void load_ids16(const uint32_t* ids, uint32_t r0, uint32_t rows, bool vec, uint32_t (&e)[16]) {
@@ -39,6 +40,7 @@ __device__ __forceinline__ void load_ids16(const uint32_t* ids, uint32_t r0, uin
     }
 }
 
+template <bool CLUSTER>
 __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* ids, uint32_t rows, uint32_t n_experts,
                                                                 uint32_t nt, uint32_t* __restrict__ header, uint4* __restrict__ tiles,
                                                                 uint32_t* __restrict__ perm, float* __restrict__ y, float* __restrict__ y2,
@@ -48,11 +50,14 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* 
     uint32_t* off = cnt + n_experts;          // [E+1] first sorted row of each expert
     uint32_t* toff = off + n_experts + 1;     // [E+1] first tile of each expert
     uint32_t* cur = toff + n_experts + 1;     // [E] place of this CTA's next row of each expert
-    uint32_t* wsum = cur + n_experts;         // [32] + [32] warp totals of the two scans, [2] running totals
+    uint32_t* wsum = cur + n_experts;         // [32] + [32] warp totals of the two scans, [2] running totals, [2] of the block
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool vec = reinterpret_cast<uintptr_t>(ids) % 16 == 0;
-    const cg::cluster_group cl = cg::this_cluster();
-    const uint32_t ctas = gridDim.x, rank = blockIdx.x, share = (rows + 16 * ctas - 1) / (16 * ctas) * 16;       // the cluster is the grid
+    const auto meet = [] {
+        if constexpr (CLUSTER) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    const uint32_t ctas = CLUSTER ? gridDim.x : 1u, rank = CLUSTER ? blockIdx.x : 0u, share = (rows + 16 * ctas - 1) / (16 * ctas) * 16;       // the cluster is the grid
     const uint32_t first = min(rank * share, rows), last = min(first + share, rows);
     pdl_trigger();
     for (uint32_t e = tid; e < n_experts; e += SORT_THREADS) cnt[e] = 0;
@@ -72,17 +77,22 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* 
         }
     }
     if (bad) atomicOr(status, STATUS_BAD_EXPERT_ID);
-    cl.sync();
+    meet();
     // exclusive scans of the row counts and of the tile counts over the experts
     for (uint32_t base = 0; base < n_experts; base += SORT_THREADS) {
         const uint32_t e = base + tid;
         uint32_t c = 0, before = 0;                        // rows of the expert, those of the CTAs in front among them
-        if (e < n_experts)
-            for (uint32_t q = 0; q < ctas; ++q) {
-                const uint32_t v = cl.map_shared_rank(cnt, q)[e];
-                c += v;
-                before += q < rank ? v : 0u;
+        if (e < n_experts) {
+            if constexpr (CLUSTER) {
+                for (uint32_t q = 0; q < ctas; ++q) {
+                    const uint32_t v = cg::this_cluster().map_shared_rank(cnt, q)[e];
+                    c += v;
+                    before += q < rank ? v : 0u;
+                }
+            } else {
+                c = cnt[e];
             }
+        }
         const uint32_t t = (c + nt - 1) / nt;
         uint32_t ic = c, it = t;
 #pragma unroll
@@ -142,7 +152,7 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const uint32_t* 
             }
         }
     }
-    cl.sync();                                                       // the others read this CTA's counts until here
+    if constexpr (CLUSTER) meet();                                   // the others read this CTA's counts until here
 }
 
 // Sorted rows as f16: the routed row's activations (token = routed row / top_k).  A CTA takes four rows at a time, whose places and
@@ -214,8 +224,11 @@ cudaError_t launch_moe_sort(const uint32_t* ids, uint32_t rows, uint32_t n_exper
                             float* y, float* y2, uint32_t n, uint32_t* status, cudaStream_t st) {
     const size_t smem = (4 * static_cast<size_t>(n_experts) + 2 + 68) * 4;
     if (smem > 48 * 1024) return cudaErrorInvalidValue;
-    const dim3 ctas(rows > 2048 ? SORT_CTAS : 1);
-    return launch_pdl_cluster(moe_sort_kernel, ctas, dim3(SORT_THREADS), ctas, smem, st, ids, rows, n_experts, nt, header, static_cast<uint4*>(tiles), perm, y, y2, n, status);
+    // up to here one CTA is ahead, which meets without the cluster (us with the gather behind, one CTA / eight: 256 experts 512 rows 6.3 / 6.6,
+    // 3072 8.2 / 8.6, 4096 9.1 / 8.6; 8 experts 3072 7.7 / 8.0, 4096 8.3 / 8.5; one of 8192 13.5 / 10.4)
+    const dim3 ctas(rows > 4096 ? SORT_CTAS : 1);
+    return launch_pdl_cluster(ctas.x > 1 ? moe_sort_kernel<true> : moe_sort_kernel<false>, ctas, dim3(SORT_THREADS), ctas, smem, st, ids, rows, n_experts, nt, header,
+                              static_cast<uint4*>(tiles), perm, y, y2, n, status);
 }
 
 cudaError_t launch_moe_prep(const uint32_t* ids, uint32_t rows, uint32_t n_experts, uint32_t top_k, uint32_t nt, const void* x,
