@@ -569,8 +569,12 @@ cudaError_t launch_gemm_form(const CUtensorMap& tw, const CUtensorMap& tw2, cons
         }
         if (fit) smem = ALONE_SMEM;
     }
-    if constexpr (SHARED) return launch_pdl_cluster(kern, grid, dim3(GEMM_THREADS), dim3(1, 1, parts), smem, st, tw, tw2, tx, p);
-    else return launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, tw, tw2, tx, p);
+    // Started early a launch gets SMs as they fall free, all over the chip; started behind the end of the one in front it fills one neighbour
+    // after the other (96 CTAs on 48 pairs of SMs, early on 61).  Scattered, the plain product in Q6_K is 7 to 12 % slower, why is not
+    // known; with Q5_K and Q4_K the two are within 1 %, and pairs and clusters of four or eight gain more by the early start
+    // (4096 x 14336 in Q6_K, us early / late: 80 rows 64.9 / 60.6, 160 109 / 101, 300 105 / 94; 9 rows, clusters of four, 31.9 / 34.8).
+    const bool late = TYPE == HF2Q_TYPE_Q6_K && !GROUPED && !DUAL && parts <= 2;
+    return launch_as(!late, dim3(1, 1, parts), kern, grid, dim3(GEMM_THREADS), smem, st, tw, tw2, tx, p);
 }
 
 // parts > 1: the CTAs of a cluster share the K-blocks (dense tiles of up to 128 tokens)
