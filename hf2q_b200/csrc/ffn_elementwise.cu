@@ -281,13 +281,28 @@ __global__ void __launch_bounds__(256, 2) router_tile_kernel(const void* x, uint
     cl.sync();                                                       // peers read this CTA's sums until here
 }
 
+uint64_t router_tiles(uint32_t n_tokens, uint32_t n_experts, uint32_t side) { return static_cast<uint64_t>((n_experts + side - 1) / side) * ((n_tokens + side - 1) / side); }
+// Time of n tiles in so many parts, in eighths of what one tile takes an SM by itself: two CTAs that share an SM take twice as long.
+uint64_t router_time(uint64_t n, uint32_t parts, uint64_t sms) { return (n * parts + sms - 1) / sms * (RT_MAX_PARTS / parts); }
+// Parts of a tile: as many as keep two CTAs on every SM busy.  More tiles than SMs: halves or quarters where whole ones leave a last wave nearly
+// empty (8192 tokens, 384 experts of 2048: 395 us in 192 large tiles, 302 in halves; 5000 tokens, 512 experts: 398 in 160, 249 in
+// quarters; quarters for an eighth of the time were a little slower, 16384 tokens, 8 experts: 131 and 134).
+uint32_t router_parts(uint64_t n, uint32_t h, uint64_t sms) {
+    uint32_t parts = 1;
+    while (parts < RT_MAX_PARTS && parts * n <= sms && h >= 2 * parts * RKT) parts *= 2;
+    if (n > sms) {
+        const uint64_t whole = router_time(n, 1, sms), halves = router_time(n, 2, sms), quarters = router_time(n, 4, sms);
+        if (h >= 2 * RKT && 10 * halves < 9 * whole) parts = 2;
+        if (h >= 4 * RKT && 10 * quarters < 8 * whole && quarters < router_time(n, parts, sms)) parts = 4;
+    }
+    return parts;
+}
+
 template <int R>
 cudaError_t launch_router_tiles(bool vec, const void* x, uint32_t x_bf16, const float* w, float* out, uint32_t n_tokens, uint32_t n_experts, uint32_t h, int sm_count,
                                 cudaStream_t st) {
     const dim3 tiles((n_experts + RT * R - 1) / (RT * R), (n_tokens + RT * R - 1) / (RT * R));
-    // as many parts as keep two CTAs on every SM busy
-    uint32_t parts = 1;
-    while (parts < RT_MAX_PARTS && 2ull * parts * tiles.x * tiles.y <= 2ull * sm_count && h >= 2 * parts * RKT) parts *= 2;
+    const uint32_t parts = router_parts(router_tiles(n_tokens, n_experts, RT * R), h, static_cast<uint64_t>(sm_count));
     const auto kern = vec ? router_tile_kernel<true, R> : router_tile_kernel<false, R>;
     static PerDeviceFlag flag[2];
     if (const cudaError_t e = ensure_max_dynamic_smem(kern, static_cast<int>(router_smem(R)), flag[vec]); e != cudaSuccess) return e;
@@ -302,9 +317,12 @@ cudaError_t launch_router_logits(const void* x, uint32_t x_bf16, const float* w,
     if (n_tokens <= RV_TOKENS)
         return launch_pdl(vec ? router_vector_kernel<true> : router_vector_kernel<false>, dim3(n_experts), dim3(RV_THREADS), 0, st, x, x_bf16, w, out,
                                n_tokens, n_experts, h);
-    // the larger tiles where their parts still fill the chip
-    const uint64_t tiles = static_cast<uint64_t>((n_experts + 2 * RT - 1) / (2 * RT)) * ((n_tokens + 2 * RT - 1) / (2 * RT));
-    if (n_experts > RT && tiles * RT_MAX_PARTS >= static_cast<uint64_t>(sm_count)) return launch_router_tiles<2>(vec, x, x_bf16, w, out, n_tokens, n_experts, h, sm_count, st);
+    // The larger tiles take three times as long as the small ones (2048 columns: 200 and 66 us on an SM) for four times the work: where
+    // their parts fill the chip and their waves, with the ragged edge, come out no longer (us small / large: 2048 tokens, 128 experts
+    // 36.7 / 55.8, 256 experts 69.9 / 57.7; 1500 tokens, 192 experts 52.9 / 57.2; 8192 tokens, 256 experts 264 / 205).
+    const uint64_t sms = static_cast<uint64_t>(sm_count), small = router_tiles(n_tokens, n_experts, RT), large = router_tiles(n_tokens, n_experts, 2 * RT);
+    if (n_experts > RT && large * RT_MAX_PARTS >= sms && 3 * router_time(large, router_parts(large, h, sms), sms) <= router_time(small, router_parts(small, h, sms), sms))
+        return launch_router_tiles<2>(vec, x, x_bf16, w, out, n_tokens, n_experts, h, sm_count, st);
     return launch_router_tiles<1>(vec, x, x_bf16, w, out, n_tokens, n_experts, h, sm_count, st);
 }
 
