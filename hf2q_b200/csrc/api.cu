@@ -1635,7 +1635,7 @@ HF2Q_API int32_t hf2q_cuda_rope_kv_append(hf2q_ctx* ctx, void* stream, float* qk
     if (rc) return rc;
     if (m == 0) return HF2Q_OK;
     DeviceGuard dg(ctx->device);
-    const cudaError_t e = launch_rope_kv_append(qkv, m, n_q_heads, kv->n_kv_heads, kv->head_dim, pos, theta, view_of(kv), ctx->status,
+    const cudaError_t e = launch_rope_kv_append(qkv, m, n_q_heads, kv->n_kv_heads, kv->head_dim, pos, theta, view_of(kv), ctx->status, ctx->dev.sm_count,
                                                 static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "rope_kv_append launch");
     ctx->launches += 1;

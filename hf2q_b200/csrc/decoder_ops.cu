@@ -129,12 +129,14 @@ __global__ void __launch_bounds__(1024) rms_norm_any_kernel(float* __restrict__ 
 
 // ------------------------------------------------------------------ rotary embedding + KV append
 // qkv: [m][(n_q + 2 n_kv) * 128] f32 (fused QKV product).  Token t sits at position *pos + t.
-// One CTA per token, one warp per head at a time, four elements a lane.  The 64 angles of a token are the same for all its
-// heads: pow, sine and cosine are taken once per token, not once per head (2048 tokens, 32 + 16 heads: 43 -> 13 us).  q heads are rotated in place and scaled by `q_scale`
+// One CTA per token, or a share of its heads where the tokens alone would leave SMs idle; one warp per head at a time, four
+// elements a lane.  The 64 angles of a token are the same for all its heads: pow, sine and cosine are taken once per CTA, not
+// once per head (2048 tokens, 32 + 16 heads: 43 -> 13 us).  q heads are rotated in place and scaled by `q_scale`
 // (1/sqrt(hd), so the attention kernels need no multiply); k heads are rotated, then k and v heads are quantized
 // to int8 with one scale per (head, position) and stored in the cache.  Pairs are (2i, 2i+1) with
 // angle pos * theta^(-2i/hd) -- the rotary form of the Llama architecture.
 constexpr uint32_t ROPE_HD = 128;
+template <bool SHARES>
 __global__ void __launch_bounds__(256) rope_kv_append_kernel(float* __restrict__ qkv, uint32_t n_q, uint32_t n_kv, const uint32_t* __restrict__ pos_dev,
                                                              float theta, float q_scale, int8_t* __restrict__ k_codes, float* __restrict__ k_scale,
                                                              int8_t* __restrict__ v_codes, float* __restrict__ v_scale, uint32_t max_seq, bool wide,
@@ -149,7 +151,7 @@ __global__ void __launch_bounds__(256) rope_kv_append_kernel(float* __restrict__
     }
     __syncthreads();
     const float4 cs = *reinterpret_cast<const float4*>(&turn[2 * lane]);
-    for (uint32_t hidx = warp; hidx < heads; hidx += 8) {
+    for (uint32_t hidx = warp + (SHARES ? blockIdx.y * 8 : 0u); hidx < heads; hidx += SHARES ? gridDim.y * 8 : 8u) {
         float* v = qkv + (static_cast<size_t>(t) * heads + hidx) * ROPE_HD + 4 * lane;
         const bool is_q = hidx < n_q, is_k = !is_q && hidx < n_q + n_kv;
         float e[4];
@@ -728,11 +730,15 @@ cudaError_t launch_rms_norm(float* x, const float* delta, const float* weight, f
 }
 
 cudaError_t launch_rope_kv_append(float* qkv, uint32_t m, uint32_t n_q, uint32_t n_kv, uint32_t hd, const uint32_t* pos, float theta,
-                                  const KvCacheView& kv, uint32_t* status, cudaStream_t st) {
+                                  const KvCacheView& kv, uint32_t* status, int sm_count, cudaStream_t st) {
     if (hd != ROPE_HD) return cudaErrorInvalidValue;
+    // shares of a token's heads while two CTAs an SM are not there (us, whole tokens / shares: 32 + 16 heads 1 token 3.4 / 2.0, 64 tokens 3.7 /
+    // 2.7, 128 tokens 3.8 / 3.1; 64 + 16 heads 1 token 4.6 / 2.1)
+    const uint32_t all = (n_q + 2 * n_kv + 7) / 8, room = 2 * static_cast<uint32_t>(sm_count) / m, shares = all < room ? all : room;
     const bool wide = reinterpret_cast<uintptr_t>(qkv) % 16 == 0 && (reinterpret_cast<uintptr_t>(kv.k_codes) | reinterpret_cast<uintptr_t>(kv.v_codes)) % 4 == 0;
-    rope_kv_append_kernel<<<m, 256, 0, st>>>(qkv, n_q, n_kv, pos, theta, 1.0f / sqrtf(static_cast<float>(hd)), kv.k_codes, kv.k_scale, kv.v_codes,
-                                             kv.v_scale, kv.max_seq, wide, status);
+    const auto kern = shares > 1 ? rope_kv_append_kernel<true> : rope_kv_append_kernel<false>;
+    kern<<<dim3(m, shares > 1 ? shares : 1), 256, 0, st>>>(qkv, n_q, n_kv, pos, theta, 1.0f / sqrtf(static_cast<float>(hd)), kv.k_codes, kv.k_scale, kv.v_codes,
+                                                           kv.v_scale, kv.max_seq, wide, status);
     return cudaGetLastError();
 }
 

@@ -211,7 +211,7 @@ cudaError_t launch_get_rows(uint32_t type, const void* w, uint64_t row_bytes, ui
 cudaError_t launch_rms_norm(float* x, const float* delta, const float* weight, float eps, void* out, uint32_t out_dtype, uint32_t m,
                             uint32_t h, uint32_t* status, cudaStream_t st);      // out in f16: an activation panel of the tensor-core products
 cudaError_t launch_rope_kv_append(float* qkv, uint32_t m, uint32_t n_q, uint32_t n_kv, uint32_t hd, const uint32_t* pos, float theta,
-                                  const KvCacheView& kv, uint32_t* status, cudaStream_t st);
+                                  const KvCacheView& kv, uint32_t* status, int sm_count, cudaStream_t st);
 size_t attn_decode_scratch_bytes(uint32_t n_kv, uint32_t group, uint32_t n_splits);
 cudaError_t launch_attn_decode(const float* q, uint32_t n_q, uint32_t n_kv, uint32_t hd, const KvCacheView& kv, const uint32_t* pos,
                                void* out, uint32_t out_dtype, float* scratch, uint32_t n_splits, cudaStream_t st);
