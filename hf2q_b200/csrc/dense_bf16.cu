@@ -85,7 +85,7 @@ struct MatvecSegs {
 // us; 2048 outputs behind a gated row 10.5 -> 7.6.
 constexpr int PRO_GROUPS = 3;
 __device__ __forceinline__ float4 group4(const float* p, uint32_t i, bool in) { return p && in ? *reinterpret_cast<const float4*>(p + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f); }
-__device__ __forceinline__ bool groups_fit(uint32_t width, uintptr_t pointers) { return width % 4 == 0 && width <= 4 * PRO_GROUPS * MR_THREADS && pointers % 16 == 0; }
+__device__ __forceinline__ bool groups_fit(uint32_t width, uintptr_t pointers, int groups = PRO_GROUPS) { return width % 4 == 0 && width <= 4 * groups * MR_THREADS && pointers % 16 == 0; }
 __device__ __forceinline__ uintptr_t bits(const void* p) { return reinterpret_cast<uintptr_t>(p); }
 
 struct NormRow {
@@ -227,18 +227,20 @@ struct HyperRow {
 };
 
 // Gated head outputs of heads of whole 128-element spans, a span to a warp (silu_group_norm_row and gated_heads_row take the others).
+// G: groups a thread.
+template <int G>
 struct GatedRow {
     const hf2q_gated_heads& q;
     const bool silu;
     const uint32_t width, spans, inv;            // of a row; of a head; x / spans = x * inv >> 16
-    float4 norm[PRO_GROUPS];
+    float4 norm[G];
     static __device__ __forceinline__ bool fits(const hf2q_gated_heads& q) {
-        return q.head_dim % 128 == 0 && groups_fit(q.heads * q.head_dim, bits(q.o) | bits(q.gate) | bits(q.norm));
+        return q.head_dim % 128 == 0 && groups_fit(q.heads * q.head_dim, bits(q.o) | bits(q.gate) | bits(q.norm), G);
     }
     __device__ __forceinline__ explicit GatedRow(const hf2q_gated_heads& p)
         : q(p), silu(p.kind == HF2Q_GATE_SILU_FIRST), width(p.heads * p.head_dim), spans(p.head_dim / 128), inv((65535 + spans) / spans) {
 #pragma unroll
-        for (int g = 0; g < PRO_GROUPS; ++g) {
+        for (int g = 0; g < G; ++g) {
             const uint32_t i = threadIdx.x + MR_THREADS * g;
             norm[g] = group4(q.norm, silu || q.norm_all ? i : i - first_span(g) * 32, 4 * i < width);
         }
@@ -248,14 +250,14 @@ struct GatedRow {
     // the row into xs.  sums: a float per span
     __device__ __forceinline__ void run(float* xs, float* sums) const {
         const uint32_t lane = threadIdx.x & 31;
-        float4 v[PRO_GROUPS], x[PRO_GROUPS];
+        float4 v[G], x[G];
 #pragma unroll
-        for (int g = 0; g < PRO_GROUPS; ++g) {
+        for (int g = 0; g < G; ++g) {
             const uint32_t i = threadIdx.x + MR_THREADS * g;
             v[g] = group4(q.o, i, 4 * i < width); x[g] = group4(q.gate, i, 4 * i < width);
         }
 #pragma unroll
-        for (int g = 0; g < PRO_GROUPS; ++g) {
+        for (int g = 0; g < G; ++g) {
             if (4 * MR_THREADS * g >= width) break;
             x[g] = make_float4(gate_of(x[g].x), gate_of(x[g].y), gate_of(x[g].z), gate_of(x[g].w));
             if (silu) v[g] = make_float4(v[g].x * x[g].x, v[g].y * x[g].y, v[g].z * x[g].z, v[g].w * x[g].w);
@@ -264,12 +266,14 @@ struct GatedRow {
         }
         __syncthreads();
 #pragma unroll
-        for (int g = 0; g < PRO_GROUPS; ++g) {
+        for (int g = 0; g < G; ++g) {
             const uint32_t i = threadIdx.x + MR_THREADS * g, first = first_span(g);
             if (4 * i >= width) break;                                      // (whole warps)
             float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
             if (q.norm) {
-                const float s = warp_sum((lane < spans ? sums[first + lane] : 0.f) + (lane + 32 < spans ? sums[first + lane + 32] : 0.f));
+                float part = (lane < spans ? sums[first + lane] : 0.f) + (lane + 32 < spans ? sums[first + lane + 32] : 0.f);
+                if (G * MR_WARPS > 64 && lane + 64 < spans) part += sums[first + lane + 64];
+                const float s = warp_sum(part);
                 const float r = 1.0f / sqrtf(s / static_cast<float>(q.head_dim) + q.eps);
                 w = make_float4(norm[g].x * r, norm[g].y * r, norm[g].z * r, norm[g].w * r);
             }
@@ -281,10 +285,14 @@ struct GatedRow {
 };
 
 // One-row product: the CTA's weight rows run through a MatvecStream; the layer's row prologue fills x in front of it.
-template <int PRO, bool PAIRS>
+// WIDE: rows beyond PRO_GROUPS groups a thread, 16 bytes at a time through shared memory, gated ones with twice the groups (64 outputs behind
+// rows of 8192, us element by element and now: norm 8.9 / 5.1, four streams 13.3 / 9.2, gated 7.6 / 6.6).  A form of its own, for with these
+// paths beside the others a decode step of 200 products took 1.7 % longer.
+template <int PRO, bool PAIRS, bool WIDE>
 __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __grid_constant__ MatvecSegs p, uint32_t* status) {
     extern __shared__ __align__(128) uint8_t mv_smem[];                 // ring, then x [k] f32
-    __shared__ float red[96];
+    __shared__ float red[96];                                           // (a float for every 128 elements of a gated row among them)
+    static_assert(2 * PRO_GROUPS * MR_WARPS <= 96, "");
     __shared__ MatvecShared sh;
     pdl_trigger();
     const bool second = blockIdx.x >= p.blocks0;
@@ -320,7 +328,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __gri
     } else if constexpr (PRO == HF2Q_PRO_NORM) {
         const hf2q_pre_norm& q = s.pre;
         const bool keep = blk == 0;
-        if (NormRow::fits(q)) {
+        if (!WIDE && NormRow::fits(q)) {
             const NormRow row(q);
             pdl_wait();
             add_residual();
@@ -333,7 +341,20 @@ __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __gri
             const uint32_t pos = q.shift ? *q.pos : 0u;
             const float* before = q.shift_state + static_cast<size_t>((pos + 1) & 1) * q.width;
             float* now = q.shift_state + static_cast<size_t>(pos & 1) * q.width;
-            for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) {
+            const uint32_t n4 = WIDE && q.width % 4 == 0 && (bits(q.norm) | bits(q.x_out) | bits(q.shift) | bits(q.shift_state)) % 16 == 0 ? q.width / 4 : 0u;
+#pragma unroll 4
+            for (uint32_t i = threadIdx.x; i < n4; i += MR_THREADS) {
+                const float4 x = *reinterpret_cast<const float4*>(xs + 4 * i), w = group4(q.norm, i, true);
+                if (keep && q.x_out) *reinterpret_cast<float4*>(q.x_out + 4 * i) = x;
+                float4 h = make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w);
+                if (q.shift) {
+                    const float4 was = group4(before, i, true), mu = group4(q.shift, i, true);
+                    if (keep) *reinterpret_cast<float4*>(now + 4 * i) = h;
+                    h = make_float4(h.x + (was.x - h.x) * mu.x, h.y + (was.y - h.y) * mu.y, h.z + (was.z - h.z) * mu.z, h.w + (was.w - h.w) * mu.w);
+                }
+                *reinterpret_cast<float4*>(xs + 4 * i) = h;
+            }
+            for (uint32_t i = 4 * n4 + threadIdx.x; i < s.k; i += MR_THREADS) {
                 float h = 0.f;
                 if (i < q.width) {
                     const float x = xs[i];
@@ -352,7 +373,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __gri
         __shared__ __align__(8) float coef[HYPER_COEF];
         // every CTA makes the whole row and stores its share of the new streams
         const uint32_t lo = min(p.share[second] * blk, q.width), hi = min(lo + p.share[second], q.width);
-        if (HyperRow::fits(q)) {
+        if (!WIDE && HyperRow::fits(q)) {
             f2* pairs = reinterpret_cast<f2*>(coef);
             const HyperRow row(q, pairs);
             pdl_wait();
@@ -363,14 +384,25 @@ __global__ void __launch_bounds__(MR_THREADS, 1) dense_matvec_kernel(const __gri
             pdl_wait();
             add_residual();
             const float inv = hyper_row(q, 0, xs, coef, red, lo, hi);
-            for (uint32_t i = threadIdx.x; i < s.k; i += MR_THREADS) {
+            const uint32_t n4 = WIDE && q.width % 4 == 0 && (bits(q.norm) | bits(q.h_out)) % 16 == 0 ? q.width / 4 : 0u;      // (lo and hi are multiples of four)
+#pragma unroll 4
+            for (uint32_t i = threadIdx.x; i < n4; i += MR_THREADS) {
+                float4 h = *reinterpret_cast<const float4*>(xs + 4 * i);
+                if (q.norm) {
+                    const float4 w = group4(q.norm, i, true);
+                    h = make_float4(h.x * inv * w.x, h.y * inv * w.y, h.z * inv * w.z, h.w * inv * w.w);
+                    *reinterpret_cast<float4*>(xs + 4 * i) = h;
+                }
+                if (q.h_out && 4 * i >= lo && 4 * i < hi) *reinterpret_cast<float4*>(q.h_out + 4 * i) = h;
+            }
+            for (uint32_t i = 4 * n4 + threadIdx.x; i < s.k; i += MR_THREADS) {
                 const float h = i < q.width ? (q.norm ? xs[i] * inv * q.norm[i] : xs[i]) : 0.f;
                 xs[i] = h;
                 if (q.h_out && i >= lo && i < hi) q.h_out[i] = h;
             }
         }
-    } else if (GatedRow::fits(s.gated)) {
-        const GatedRow row(s.gated);
+    } else if (typedef GatedRow<(WIDE ? 2 : 1) * PRO_GROUPS> Row; Row::fits(s.gated)) {
+        const Row row(s.gated);
         pdl_wait();
         add_residual();
         row.run(xs, red);
@@ -802,15 +834,21 @@ cudaError_t dense_any(const DenseArgs& a, int sms, uint32_t* status, cudaStream_
     return launch_pdl(dense_gemm_f32_kernel<X, Y, false>, dim3((a.n + FT - 1) / FT, (a.m + FT - 1) / FT), dim3(256), 0, st, a);
 }
 
-template <int PRO, bool PAIRS>
+template <int PRO, bool PAIRS, bool WIDE>
 cudaError_t launch_fused_as(const MatvecSegs& p, uint32_t blocks, size_t smem, uint32_t* status, cudaStream_t st) {
     static PerDeviceFlag flag;
-    if (const cudaError_t e = ensure_max_dynamic_smem(dense_matvec_kernel<PRO, PAIRS>, MR_RING + MR_MAX_X, flag); e != cudaSuccess) return e;
-    return launch_pdl(dense_matvec_kernel<PRO, PAIRS>, dim3(blocks), dim3(MR_THREADS), smem, st, p, status);
+    const auto kern = dense_matvec_kernel<PRO, PAIRS, WIDE>;
+    if (const cudaError_t e = ensure_max_dynamic_smem(kern, MR_RING + MR_MAX_X, flag); e != cudaSuccess) return e;
+    return launch_pdl(kern, dim3(blocks), dim3(MR_THREADS), smem, st, p, status);
 }
+// width: of the longest row in front of a product
 template <int PRO>
-cudaError_t launch_fused(const MatvecSegs& p, uint32_t blocks, size_t smem, uint32_t* status, cudaStream_t st) {
-    return epi_pairs(p.s[0].epilogue) ? launch_fused_as<PRO, true>(p, blocks, smem, status, st) : launch_fused_as<PRO, false>(p, blocks, smem, status, st);
+cudaError_t launch_fused(const MatvecSegs& p, uint32_t width, uint32_t blocks, size_t smem, uint32_t* status, cudaStream_t st) {
+    const bool pairs = epi_pairs(p.s[0].epilogue);
+    if constexpr (PRO != HF2Q_PRO_NONE)
+        if (width > 4 * PRO_GROUPS * MR_THREADS)
+            return pairs ? launch_fused_as<PRO, true, true>(p, blocks, smem, status, st) : launch_fused_as<PRO, false, true>(p, blocks, smem, status, st);
+    return pairs ? launch_fused_as<PRO, true, false>(p, blocks, smem, status, st) : launch_fused_as<PRO, false, false>(p, blocks, smem, status, st);
 }
 
 }  // namespace
@@ -896,12 +934,18 @@ HF2Q_API int32_t hf2q_cuda_dense_matvec(hf2q_ctx* ctx, void* stream, uint32_t pr
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t smem = MR_RING + static_cast<size_t>(kmax) * 4;
     uint32_t* status = ctx_status_word(ctx);
+    uint32_t width = 0;
+    for (uint32_t i = 0; i < n_segs; ++i) {
+        const hf2q_matvec& s = segs[i];
+        const uint32_t w = prologue == HF2Q_PRO_NORM ? s.pre.width : prologue == HF2Q_PRO_HYPER ? s.hyper.width : s.gated.heads * s.gated.head_dim;
+        width = w > width ? w : width;
+    }
     cudaError_t e;
     switch (prologue) {
-        case HF2Q_PRO_NONE: e = launch_fused<HF2Q_PRO_NONE>(p, blocks, smem, status, st); break;
-        case HF2Q_PRO_NORM: e = launch_fused<HF2Q_PRO_NORM>(p, blocks, smem, status, st); break;
-        case HF2Q_PRO_HYPER: e = launch_fused<HF2Q_PRO_HYPER>(p, blocks, smem, status, st); break;
-        default: e = launch_fused<HF2Q_PRO_GATED>(p, blocks, smem, status, st); break;
+        case HF2Q_PRO_NONE: e = launch_fused<HF2Q_PRO_NONE>(p, width, blocks, smem, status, st); break;
+        case HF2Q_PRO_NORM: e = launch_fused<HF2Q_PRO_NORM>(p, width, blocks, smem, status, st); break;
+        case HF2Q_PRO_HYPER: e = launch_fused<HF2Q_PRO_HYPER>(p, width, blocks, smem, status, st); break;
+        default: e = launch_fused<HF2Q_PRO_GATED>(p, width, blocks, smem, status, st); break;
     }
     return ctx_cuda_result(ctx, e, "dense_matvec", 1);
 }
