@@ -112,30 +112,25 @@ __global__ void __launch_bounds__(256) window_append_kernel(const __grid_constan
     }
 }
 
-// Online softmax of one warp for GR query heads against keys [lo, hi) of KV head g; qs: [GR][dp] f32 in shared
-// memory, ps: [GR][32] of this warp.  Lane = key for the scores, lane = value columns 2 lane + 64 c for the sums.
-template <typename T, int GR, int NC, bool PLAIN>
+// Online softmax of one warp for a query against keys [lo, hi) of its KV head; qs: [dp] f32 in shared memory, ps: [32] of this
+// warp.  Lane = key for the scores, lane = value columns 2 lane + 64 c for the sums.
+template <typename T, int NC, bool PLAIN>
 struct WarpAttn {
-    float mx[GR], l[GR], acc[GR][NC][2];
+    float mx, l, acc[NC][2];
     __device__ __forceinline__ void init() {
+        mx = -CUDART_INF_F;
+        l = 0.f;
 #pragma unroll
-        for (int g = 0; g < GR; ++g) {
-            mx[g] = -CUDART_INF_F;
-            l[g] = 0.f;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) acc[g][c][0] = acc[g][c][1] = 0.f;
-        }
+        for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = 0.f;
     }
-    __device__ __forceinline__ void keys(const hf2q_window_attn& a, const T* kc, const T* vc, const KeyRows<T, PLAIN>* kv, const float* qs, float* ps, const float (&r1)[GR],
-                                         const float (&r2)[GR], uint32_t pos, uint32_t p0, uint32_t hi) {
+    __device__ __forceinline__ void keys(const hf2q_window_attn& a, const T* kc, const T* vc, const KeyRows<T, PLAIN>* kv, const float* qs, float* ps, float r1, float r2,
+                                         uint32_t pos, uint32_t p0, uint32_t hi) {
         const uint32_t lane = threadIdx.x & 31, dp = pad8(a.dim), dvp = pad8(a.vdim);
         uint32_t dq = dp;
         if constexpr (PLAIN) dq += kv->sp;
         const uint32_t p = p0 + lane;
         const bool live = p < hi;
-        float s[GR];
-#pragma unroll
-        for (int g = 0; g < GR; ++g) s[g] = 0.f;
+        float s = 0.f;
         if (live) {
             const T* kr;
             if constexpr (PLAIN) kr = kv->key(p);
@@ -144,11 +139,8 @@ struct WarpAttn {
             for (uint32_t c = 0; c < dp; c += 8) {
                 float k[8];
                 load8(kr + c, k);
-#pragma unroll
-                for (int g = 0; g < GR; ++g) {
-                    const float4 x = *reinterpret_cast<const float4*>(qs + g * dq + c), y = *reinterpret_cast<const float4*>(qs + g * dq + c + 4);
-                    s[g] += k[0] * x.x + k[1] * x.y + k[2] * x.z + k[3] * x.w + k[4] * y.x + k[5] * y.y + k[6] * y.z + k[7] * y.w;
-                }
+                const float4 x = *reinterpret_cast<const float4*>(qs + c), y = *reinterpret_cast<const float4*>(qs + c + 4);
+                s += k[0] * x.x + k[1] * x.y + k[2] * x.z + k[3] * x.w + k[4] * y.x + k[5] * y.y + k[6] * y.z + k[7] * y.w;
             }
             if constexpr (PLAIN) {
                 kr = kv->shared_key(p) - dp;
@@ -156,27 +148,21 @@ struct WarpAttn {
                 for (uint32_t c = dp; c < dq; c += 8) {
                     float k[8];
                     load8(kr + c, k);
-#pragma unroll
-                    for (int g = 0; g < GR; ++g) {
-                        const float4 x = *reinterpret_cast<const float4*>(qs + g * dq + c), y = *reinterpret_cast<const float4*>(qs + g * dq + c + 4);
-                        s[g] += k[0] * x.x + k[1] * x.y + k[2] * x.z + k[3] * x.w + k[4] * y.x + k[5] * y.y + k[6] * y.z + k[7] * y.w;
-                    }
+                    const float4 x = *reinterpret_cast<const float4*>(qs + c), y = *reinterpret_cast<const float4*>(qs + c + 4);
+                    s += k[0] * x.x + k[1] * x.y + k[2] * x.z + k[3] * x.w + k[4] * y.x + k[5] * y.y + k[6] * y.z + k[7] * y.w;
                 }
             }
         }
+        const float sc = live ? score_of(s, a.scale, r1, r2, pos - p, a.r1 != nullptr) : -CUDART_INF_F;
+        float bm = sc;
+        for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+        const float nm = fmaxf(mx, bm);
+        const float corr = expf(mx - nm), pr = live ? expf(sc - nm) : 0.f;
+        l = l * corr + warp_sum(pr);
+        mx = nm;
 #pragma unroll
-        for (int g = 0; g < GR; ++g) {
-            const float sc = live ? score_of(s[g], a.scale, r1[g], r2[g], pos - p, a.r1 != nullptr) : -CUDART_INF_F;
-            float bm = sc;
-            for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
-            const float nm = fmaxf(mx[g], bm);
-            const float corr = expf(mx[g] - nm), pr = live ? expf(sc - nm) : 0.f;
-            l[g] = l[g] * corr + warp_sum(pr);
-            mx[g] = nm;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) { acc[g][c][0] *= corr; acc[g][c][1] *= corr; }
-            ps[g * 32 + lane] = pr;
-        }
+        for (int c = 0; c < NC; ++c) { acc[c][0] *= corr; acc[c][1] *= corr; }
+        ps[lane] = pr;
         __syncwarp();
         const uint32_t cnt = min(32u, hi - p0);
 #pragma unroll 4
@@ -189,12 +175,9 @@ struct WarpAttn {
                 const uint32_t d = 2 * lane + 64 * c;
                 if (d < dvp) {
                     const float v0 = to_f32(vr[d]), v1 = to_f32(vr[d + 1]);
-#pragma unroll
-                    for (int g = 0; g < GR; ++g) {
-                        const float w = ps[g * 32 + i];
-                        acc[g][c][0] = fmaf(w, v0, acc[g][c][0]);
-                        acc[g][c][1] = fmaf(w, v1, acc[g][c][1]);
-                    }
+                    const float w = ps[i];
+                    acc[c][0] = fmaf(w, v0, acc[c][0]);
+                    acc[c][1] = fmaf(w, v1, acc[c][1]);
                 }
             }
         }
@@ -487,8 +470,8 @@ __device__ __forceinline__ void f32_query(const hf2q_window_attn& a, uint32_t po
     for (uint32_t i = lane; i < dq; i += 32) qs[i] = to_f32(q[(static_cast<size_t>(t) * a.heads + h) * dq + i]);
     __syncwarp();
     const uint32_t pos = pos0 + t, n = min(pos + 1, a.window), hi = pos + 1;
-    const float r1[1] = {a.r1 ? a.r1[h] : 0.f}, r2[1] = {a.r1 ? a.r2[h] : 0.f};
-    WarpAttn<T, 1, NC, PLAIN> w;
+    const float r1 = a.r1 ? a.r1[h] : 0.f, r2 = a.r1 ? a.r2[h] : 0.f;
+    WarpAttn<T, NC, PLAIN> w;
     w.init();
     for (uint32_t p0 = hi - n; p0 < hi; p0 += 32) w.keys(a, kv.k, kv.v, &kv, qs, ps, r1, r2, pos, p0, hi);
 #pragma unroll
@@ -497,7 +480,7 @@ __device__ __forceinline__ void f32_query(const hf2q_window_attn& a, uint32_t po
         for (int u = 0; u < 2; ++u) {
             const uint32_t d = 2 * lane + 64 * c + u;
             if (d < a.vdim) {
-                float v = w.acc[0][c][u] / w.l[0];
+                float v = w.acc[c][u] / w.l;
                 if (gate) v *= sigmoidf(gate[static_cast<size_t>(t) * ldg + h * a.vdim + d]);
                 out[static_cast<size_t>(t) * ldo + h * a.vdim + d] = from_f32<OUT>(v);
             }
