@@ -16,6 +16,11 @@
  *     (forward_mlx.rs:9647-9651; weight_loader.rs:1059-1079).
  *   - a context is bound to one device and may be used from one thread at a time; the library
  *     keeps no other mutable global state (decode_pool.rs:51-76, serve/gpu.rs:38-39).
+ *   - launches start under the launch in front of them on their stream: products of any number of
+ *     rows and one-token calls read parameters (weights, biases, norms, coefficients, taps) while it
+ *     still runs; activations, states, positions, expert ids and outputs are touched behind its end.
+ *     So a buffer that a compute call of this library wrote is not a parameter of the call right
+ *     behind it.  Copies, dequantisation, packing and other libraries' launches end first.
  *
  * `stream` arguments are `cudaStream_t` passed as `void*` (NULL = the legacy default stream).
  */
@@ -129,7 +134,8 @@ HF2Q_API int32_t hf2q_cuda_dequantize(hf2q_ctx* ctx, void* stream, const void* w
  * x is row-major [m,k] of x_dtype (F32 or BF16), y is row-major f32 [m,n], w is the raw block
  * bytes of W.  m <= 8 takes the mat-vec kernel (the reference's MM_ROUTING_THRESHOLD,
  * forward_mlx.rs:9800); larger m takes the tensor-core kernel, which needs the workspace reported
- * by hf2q_cuda_qmatmul_workspace_bytes (0 for m <= 8). */
+ * by hf2q_cuda_qmatmul_workspace_bytes (0 for m <= 8).  Both ask for weights while the launch in
+ * front still runs (see the conventions). */
 HF2Q_API int32_t hf2q_cuda_qmatmul(hf2q_ctx* ctx, void* stream, const void* x, uint32_t x_dtype,
                                    const void* w, float* y, uint32_t m, uint32_t n, uint32_t k,
                                    uint32_t ggml_type, void* workspace, uint64_t workspace_bytes);
@@ -640,7 +646,8 @@ HF2Q_API int32_t hf2q_cuda_attn_prefill(hf2q_ctx* ctx, void* stream, const float
 /* ---- panels ----
  * A panel is the f16 [m][k] that a tensor-core product multiplies: the product's own conversion of f32 or bf16 activations gives
  * the same (beyond the f16 range clipped and noted in the status).  The entry in front of a product can write it, which saves the
- * conversion pass and half of the store.  More than 8 rows, 16-byte boundaries. */
+ * conversion pass and half of the store.  More than 8 rows, 16-byte boundaries.  The products ask for weights while the launch in
+ * front, the one that writes the panel, still runs. */
 HF2Q_API int32_t hf2q_cuda_panel_supported(hf2q_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, uint32_t ggml_type);
 /* hf2q_cuda_rms_norm, hf2q_cuda_attn_prefill with a panel as the output */
 HF2Q_API int32_t hf2q_cuda_rms_norm_panel(hf2q_ctx* ctx, void* stream, float* x, const float* delta, const float* weight,
