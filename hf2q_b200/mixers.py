@@ -20,10 +20,11 @@ def _off(t: torch.Tensor, cols: int) -> int:
 
 
 # Portions of this many tokens run a layer's recurrence beside its attention: a scan has fewer CTAs than the chip has SMs and each
-# token waits for the one before, so the attention's tiles take the SMs that it leaves (four layers, two of them such ones, us in turn
-# and beside: 256 tokens 813 and 724, 2048 tokens 2441 and 2293).  Shorter ones gain as well (64: 614 and 557) where the host is ahead of
-# the device, which a portion by itself is not.
-BESIDE_TOKENS = 256
+# token waits for the one before, so the attention's tiles take the SMs that it leaves.  The second stream costs the host some
+# 130 us in four layers, two of them such ones, and a prompt by itself is bound by the host up to about 400 tokens (us in turn and beside, those
+# four layers: 300 tokens 1035 and 1095, 512 tokens 1215 and 1165, 2048 tokens 2640 and 2490).  Where the host is ahead of the device
+# shorter portions gain too (256 tokens: 813 and 724).
+BESIDE_TOKENS = 512
 
 
 class ParallelWindowMLstm:
